@@ -7,8 +7,10 @@
 //   * frac[slot]  : fixed-point fractional coordinates (uint32 per axis for FP32, uint64 for
 //                   FP64) + charge, the input of every k-space phase (exact integer phases);
 //   * meta[slot]  : int2 (type, molecule);
-//   * nbr[p * stride + slot] : neighbour entry (j_slot << 6 | shift code), transposed so that a
-//                   warp of consecutive slots reads one 128-byte line per neighbour index.
+//   * nbr[nbr_at(p, slot, stride)] : neighbour entry p of a slot (j_slot << 6 | shift code), in
+//                   chunks of four entries transposed over the slots, so that a lane takes four
+//                   entries with one 16-byte load and a warp of consecutive slots reads 512
+//                   consecutive bytes.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -18,6 +20,13 @@ namespace rbmd {
 constexpr int kMaxReplicaTypes = 16;   // per-type LJ table lives in shared memory
 constexpr int kMaxCellAtoms = 1024;    // cell rank-sort bound (RBMD_FLAG_CELL_OVERFLOW beyond)
 constexpr int kShiftBits = 6;
+
+constexpr int kNbrChunk = 4;           // list entries per 16-byte chunk; list capacities are multiples of it
+
+// index of entry p of a slot in the neighbour list
+__host__ __device__ __forceinline__ size_t nbr_at(int p, int slot, int stride) {
+  return ((size_t)(p >> 2) * (size_t)stride + (size_t)slot) * kNbrChunk + (size_t)(p & 3);
+}
 
 // status bits (mirrors include/rbmd_force.h)
 constexpr uint32_t kFlagListOverflow = 0x01u;
@@ -102,6 +111,58 @@ template <> struct Acc<double> {
   double hi = 0;
   __device__ __forceinline__ void add(double b) { hi += b; }
   __device__ __forceinline__ double value() const { return hi; }
+};
+
+// Two values of the run precision side by side.  FP32: the packed FP32x2 instructions of sm_100
+// (IEEE rounding per half), which halve the issue slots of paired arithmetic; FP64: two scalar
+// operations.  A packed product that feeds a packed sum may be contracted to one rounding.
+template <class R> struct Pair { R x, y; };
+template <class R> __device__ __forceinline__ Pair<R> both(R a) { return {a, a}; }
+__device__ __forceinline__ Pair<float> mul2(Pair<float> a, Pair<float> b) {
+  const float2 r = __fmul2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ Pair<float> add2(Pair<float> a, Pair<float> b) {
+  const float2 r = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ Pair<float> fma2(Pair<float> a, Pair<float> b, Pair<float> c) {
+  const float2 r = __ffma2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y), make_float2(c.x, c.y));
+  return {r.x, r.y};
+}
+__device__ __forceinline__ Pair<double> mul2(Pair<double> a, Pair<double> b) {
+  return {__dmul_rn(a.x, b.x), __dmul_rn(a.y, b.y)};
+}
+__device__ __forceinline__ Pair<double> add2(Pair<double> a, Pair<double> b) {
+  return {__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y)};
+}
+__device__ __forceinline__ Pair<double> fma2(Pair<double> a, Pair<double> b, Pair<double> c) {
+  return {fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)};
+}
+
+// Acc of a force vector; FP32 runs the x and y sums as one packed TwoSum.
+template <class R> struct Acc3 {
+  Acc<R> ax, ay, az;
+  __device__ __forceinline__ void add(R x, R y, R z) { ax.add(x); ay.add(y); az.add(z); }
+  __device__ __forceinline__ double vx() const { return ax.value(); }
+  __device__ __forceinline__ double vy() const { return ay.value(); }
+  __device__ __forceinline__ double vz() const { return az.value(); }
+};
+template <> struct Acc3<float> {
+  Pair<float> hi{0.f, 0.f}, lo{0.f, 0.f};
+  Acc<float> az;
+  __device__ __forceinline__ void add(float x, float y, float z) {
+    const Pair<float> b{x, y}, m{-1.f, -1.f};
+    const Pair<float> s = add2(hi, b);
+    const Pair<float> bb = fma2(hi, m, s);             // s - hi
+    const Pair<float> t = fma2(bb, m, s);              // s - bb
+    lo = add2(lo, add2(fma2(t, m, hi), fma2(bb, m, b)));
+    hi = s;
+    az.add(z);
+  }
+  __device__ __forceinline__ double vx() const { return (double)hi.x + (double)lo.x; }
+  __device__ __forceinline__ double vy() const { return (double)hi.y + (double)lo.y; }
+  __device__ __forceinline__ double vz() const { return az.value(); }
 };
 
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11), same stream as the oracle's.

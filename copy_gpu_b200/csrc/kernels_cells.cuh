@@ -339,7 +339,7 @@ __device__ __forceinline__ int nlist_range(int s, const int s1, const typename T
     const R r2 = sub_rn(sub_rn(pj.z, off[2]), pix[2]);
     const R d2 = add_rn(add_rn(mul_rn(r0, r0), mul_rn(r1, r1)), mul_rn(r2, r2));
     if (inside_cut(sub_rn(cut2, d2), orig) && gt_small(d2)) {
-      if (idx < cap) __stcs(nbr + (size_t)idx * stride + i, (s << kShiftBits) | code);
+      if (idx < cap) __stcs(nbr + nbr_at(idx, i, stride), (s << kShiftBits) | code);
       ++idx;
     }
   }
@@ -418,9 +418,13 @@ __device__ int nlist_thread(int i, const typename Traits<R>::V4 pi, const RepDev
   return idx;
 }
 
-__device__ __forceinline__ void nlist_finish(int i, int idx, int cap, int* __restrict__ count,
-                                             int* __restrict__ max_count, uint32_t* status) {
+// Count of slot i's row; a last chunk that is not full is filled with the slot itself (distance
+// 0, which no pair predicate accepts), so that a pass may evaluate whole chunks.
+__device__ __forceinline__ void nlist_finish(int i, int idx, int cap, int stride, int* __restrict__ nbr,
+                                             int* __restrict__ count, int* __restrict__ max_count,
+                                             uint32_t* status) {
   count[i] = idx;
+  for (int p = idx; p < cap && (p & (kNbrChunk - 1)) != 0; ++p) nbr[nbr_at(p, i, stride)] = i << kShiftBits;
   if (idx > cap) {
     set_flag(status, kFlagListOverflow);
     atomicMax(max_count, idx);
@@ -442,7 +446,7 @@ __global__ void __launch_bounds__(256) k_nlist(
   const RepDev& rp = reps[r];
   const int idx = nlist_thread<R>(i, pos4[i], rp, pos4, cell_start, num_cycles, rc, cap, stride, nbr,
                                   trim_x != 0, orig);
-  nlist_finish(i, idx, cap, count, max_count, status);
+  nlist_finish(i, idx, cap, stride, nbr, count, max_count, status);
 }
 
 // Warp-per-atom list build for systems with few atoms and many candidates per atom (long
@@ -490,7 +494,7 @@ __global__ void __launch_bounds__(256) k_nlist_warp(
       const unsigned m = __ballot_sync(0xffffffffu, ok);
       if (ok) {
         const int at = idx + __popc(m & below);
-        if (at < cap) __stcs(nbr + (size_t)at * stride + i, (sj << kShiftBits) | code);
+        if (at < cap) __stcs(nbr + nbr_at(at, i, stride), (sj << kShiftBits) | code);
       }
       idx += __popc(m);
     }
@@ -515,148 +519,203 @@ __global__ void __launch_bounds__(256) k_nlist_warp(
         }
       }
     }
-  if (lane == 0) nlist_finish(i, idx, cap, count, max_count, status);
+  if (lane == 0) nlist_finish(i, idx, cap, stride, nbr, count, max_count, status);
 }
 
-// ---- staged list build ------------------------------------------------------------------
-// One block per segment of kSeg consecutive x cells of one (y, z) cell row.  The block copies
-// the positions of its 9 neighbour rows x (segment + 1 cell each side) into shared memory once,
-// already shifted by their periodic offsets and tagged with (slot << 6 | image code), and every
-// atom of the segment walks its 27 cells there.  Cells are visited in the same order, with the
-// same float operations, as k_nlist, so the list is identical entry for entry.  A segment whose
-// staged atoms exceed the shared buffer, or an atom whose own cell index falls outside the
-// segment (binning clamps positions at the upper face), takes k_nlist's global-memory path.
-struct ListSeg { int rep, y, z, x0, x1, pad0, pad1, pad2; };
-constexpr int kStageThreads = 256;
-constexpr int kSegMaxCells = 32;
-constexpr int kStageCells = 9 * (kSegMaxCells + 2);
+// ---- cell-cooperative list build ------------------------------------------------------------
+// One warp per cell (or per 1/nparts of a cell's atoms): the candidates of the cell's 27-cell
+// stencil, flattened in k_nlist's walk order, are held 32 * KC at a time in the registers of the
+// lanes, each shifted by its periodic offset once, and every atom of the cell is tested against
+// them by a broadcast read of its position: one coalesced load serves all atoms of the cell, no
+// lane diverges in the tests, and two candidates share one packed instruction.  A ballot gives
+// the accept bits of (atom, 32 candidates); lane k keeps the bits of atom k, and after a batch of
+// kCellBatch candidates (a whole stencil at the densities of the benchmarks) every lane takes its
+// accepted entries in candidate order, four per 16-byte store, all lanes in step.  Same float operations per pair
+// and same order as k_nlist, so the list is identical entry for entry.  d2_max: the predicate
+// rc^2 - d^2 > 1e-4 (or > 0) as one comparison of d^2 (pair_d2_max).  one = 1, unknown to the
+// compiler: the sums of squares are written as m * one + t, because ptxas contracts a packed
+// multiply and add even with explicit .rn (two pairs at the cutoff changed sides), and m * one
+// + t rounds as the plain sum.  An atom whose own cell index
+// differs from the cell it was binned into (binning clamps positions at the faces) takes
+// k_nlist's path on its lane.  Bound by issue (packed tests, ballots and the walk over the bits).
+// Measured per build: 200,000 electrolyte atoms at rc 2.5 in FP32 99 us (a shared-memory staged
+// build with one thread per atom: 190), 50,021 in FP64 53 us (119); averaged over the steps of a
+// run with list reuse 1,000,000 atoms 103 us (k_nlist: 154), 512 replicas 357 us (staged: 719).
+constexpr int kCellWarps = 4;
+constexpr int kCellBatch = 768;   // candidates whose accept bits are kept before entries are written
 
-__device__ __forceinline__ float pack_tag(float, int v) { return __int_as_float(v); }
-__device__ __forceinline__ double pack_tag(double, int v) { return (double)v; }
-__device__ __forceinline__ int unpack_tag(float v) { return __float_as_int(v); }
-__device__ __forceinline__ int unpack_tag(double v) { return (int)v; }
+template <class R> struct __align__(16) CellWarpMem {
+  struct __align__(16) XY { Pair<R> x, y; } xy[32];   // the atoms' -x and -y, each twice
+  Pair<R> z[32];
+  R off[3][27];        // periodic offset of each stencil cell
+  int start[27];       // its first slot
+  int code[27];        // its image code
+  int pre[28];         // candidates before it
+  int ent[kCellBatch];                      // list entry of each candidate of the batch
+  unsigned word[kCellBatch / 32][32];       // accept bits [32 candidates][atom], first candidate on top
+};
 
-template <class R>
-__global__ void __launch_bounds__(kStageThreads, 2) k_nlist_staged(
-    const ListSeg* __restrict__ segs, int stage_cap, const typename Traits<R>::V4* __restrict__ pos4,
-    const int* __restrict__ cell_start, const RepDev* __restrict__ reps, R rc, int cap, int stride,
+template <class R, int KC>
+__global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
+    int ncell, int nparts, const typename Traits<R>::V4* __restrict__ pos4, const int* __restrict__ cell_start,
+    const RepDev* __restrict__ reps, const int* __restrict__ cell_rep, R rc, R d2_max, R one, int cap, int stride,
     int* __restrict__ nbr, int* __restrict__ count, int* __restrict__ max_count, uint32_t* status,
-    const int* __restrict__ rebuild, unsigned long long* __restrict__ nbuilds, int trim_x, int n_rep,
-    int orig) {
+    const int* __restrict__ rebuild, unsigned long long* __restrict__ nbuilds, int n_rep, int orig) {
+  static_assert(KC == 2 || KC == 4, "candidates per lane");
   using V4 = typename Traits<R>::V4;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && nbuilds) atomicAdd(nbuilds, rebuilt_replicas(rebuild, n_rep));
-  if (rebuild && !rebuild[segs[blockIdx.x].rep]) return;
-  extern __shared__ __align__(16) unsigned char stage_raw[];
-  V4* stage = reinterpret_cast<V4*>(stage_raw);
-  __shared__ int cs[kStageCells + 1];     // staged start of staged cell k = row * W + u
-  __shared__ int cell_k[kStageCells];     // its global cell index
-  __shared__ int cnt_k[kStageCells];      // its atom count
-  const ListSeg sg = segs[blockIdx.x];
-  const RepDev& rp = reps[sg.rep];
-  const int S = sg.x1 - sg.x0, W = S + 2, K = 9 * W;
-  const int d0 = rp.dims[0], d1 = rp.dims[1], d2 = rp.dims[2];
-  for (int k = threadIdx.x; k < K; k += blockDim.x) {
-    const int r = k / W, u = k - r * W;
-    const int wy = wrap_cell(sg.y + r / 3 - 1, d1), wz = wrap_cell(sg.z + r % 3 - 1, d2);
-    const int wx = wrap_cell(sg.x0 - 1 + u, d0);
-    const int cell = rp.cell_base + wx + wy * d0 + wz * d0 * d1;
-    cell_k[k] = cell;
-    cnt_k[k] = cell_start[cell + 1] - cell_start[cell];
+  constexpr unsigned full = 0xffffffffu;
+  __shared__ CellWarpMem<R> mem[kCellWarps];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long item = (long long)blockIdx.x * kCellWarps + w;
+  if (item == 0 && lane == 0 && nbuilds) atomicAdd(nbuilds, rebuilt_replicas(rebuild, n_rep));
+  const int cell = (int)(item / nparts), part = (int)(item % nparts);
+  if (cell >= ncell) return;   // uniform across the warp; the kernel has no block barrier
+  const int r = cell_rep ? cell_rep[cell] : 0;
+  if (rebuild && !rebuild[r]) return;
+  const int s0 = cell_start[cell], ns = cell_start[cell + 1] - s0;
+  const int a0 = s0 + (int)((long long)ns * part / nparts), a1 = s0 + (int)((long long)ns * (part + 1) / nparts);
+  if (a0 == a1) return;
+  CellWarpMem<R>& M = mem[w];
+  const RepDev& rp = reps[r];
+  const int d0 = rp.dims[0], d1 = rp.dims[1], d2n = rp.dims[2];
+  const int cl = cell - rp.cell_base;
+  const int cx = cl % d0, cy = (cl / d0) % d1, cz = cl / (d0 * d1);
+  // stencil cells in walk order: y outermost, then z, then x
+  int cnt = 0;
+  if (lane < 27) {
+    const int nbx = cx + lane % 3 - 1, nbz = cz + (lane / 3) % 3 - 1, nby = cy + lane / 9 - 1;
+    const int wx = wrap_cell(nbx, d0), wy = wrap_cell(nby, d1), wz = wrap_cell(nbz, d2n);
+    const int dx = wx - nbx, dy = wy - nby, dz = wz - nbz;
+    const int c = rp.cell_base + wx + wy * d0 + wz * d0 * d1;
+    const int st = cell_start[c];
+    cnt = cell_start[c + 1] - st;
+    M.off[0][lane] = mul_rn(Traits<R>::dx(rp, 0), (R)dx);
+    M.off[1][lane] = mul_rn(Traits<R>::dx(rp, 1), (R)dy);
+    M.off[2][lane] = mul_rn(Traits<R>::dx(rp, 2), (R)dz);
+    M.start[lane] = st;
+    M.code[lane] = (dx > 0 ? 1 : (dx < 0 ? 2 : 0)) | ((dy > 0 ? 1 : (dy < 0 ? 2 : 0)) << 2) |
+                   ((dz > 0 ? 1 : (dz < 0 ? 2 : 0)) << 4);
   }
-  __syncthreads();
-  if (threadIdx.x < 32) {   // exclusive scan of the K counts: lane chunks, then a warp scan
-    const int lane = threadIdx.x, per = (K + 31) / 32, k0 = min(lane * per, K), k1 = min(k0 + per, K);
-    int sum = 0;
-    for (int k = k0; k < k1; ++k) sum += cnt_k[k];
-    int incl = sum;
+  int incl = cnt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += v;
-    }
-    int run = incl - sum;
-    for (int k = k0; k < k1; ++k) {
-      cs[k] = run;
-      run += cnt_k[k];
-    }
-    if (lane == 31) cs[K] = incl;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(full, incl, o);
+    if (lane >= o) incl += v;
   }
-  __syncthreads();
-  const int total = cs[K];
-  const bool staged = total <= stage_cap;
-  const R cut2 = mul_rn(rc, rc);
-  if (staged) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int k = warp; k < K; k += nw) {
-      const int r = k / W, u = k - r * W;
-      const int nby = sg.y + r / 3 - 1, nbz = sg.z + r % 3 - 1, nbx = sg.x0 - 1 + u;
-      const int dy = wrap_cell(nby, d1) - nby, dz = wrap_cell(nbz, d2) - nbz;
-      const int dx = wrap_cell(nbx, d0) - nbx;
-      const R o0 = mul_rn(Traits<R>::dx(rp, 0), (R)dx), o1 = mul_rn(Traits<R>::dx(rp, 1), (R)dy),
-              o2 = mul_rn(Traits<R>::dx(rp, 2), (R)dz);
-      const int code = (dx > 0 ? 1 : (dx < 0 ? 2 : 0)) | ((dy > 0 ? 1 : (dy < 0 ? 2 : 0)) << 2) |
-                       ((dz > 0 ? 1 : (dz < 0 ? 2 : 0)) << 4);
-      const int c0 = cell_start[cell_k[k]], cnt = cnt_k[k], base = cs[k];
-      for (int t = lane; t < cnt; t += 32) {
-        const V4 pj = pos4[c0 + t];
-        V4 v;
-        v.x = sub_rn(pj.x, o0);
-        v.y = sub_rn(pj.y, o1);
-        v.z = sub_rn(pj.z, o2);
-        v.w = pack_tag(v.x, ((c0 + t) << kShiftBits) | code);
-        stage[base + t] = v;
-      }
-    }
-  }
-  __syncthreads();
-  const int row0 = rp.cell_base + sg.y * d0 + sg.z * d0 * d1;
-  const int s0 = cell_start[row0 + sg.x0], s1 = cell_start[row0 + sg.x1];
-  for (int i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
+  if (lane < 28) M.pre[lane] = incl - cnt;   // lane 27 (count 0) holds the total
+  const int total = __shfl_sync(full, incl, 27);
+  const R d2_lo = (R)1.0e-4;                 // gt_small
+  const Pair<R> unit = both<R>(one);
+  int4* out = reinterpret_cast<int4*>(nbr);
+  for (int g0 = a0; g0 < a1; g0 += 32) {
+    const int m = min(32, a1 - g0);
+    const int i = g0 + min(lane, m - 1);
     const V4 pi = pos4[i];
-    const R pix[3] = {pi.x, pi.y, pi.z};
-    int ci[3];
+    const int ci0 = (int)div_rn(sub_rn(pi.x, Traits<R>::lo(rp, 0)), Traits<R>::dx(rp, 0));
+    const int ci1 = (int)div_rn(sub_rn(pi.y, Traits<R>::lo(rp, 1)), Traits<R>::dx(rp, 1));
+    const int ci2 = (int)div_rn(sub_rn(pi.z, Traits<R>::lo(rp, 2)), Traits<R>::dx(rp, 2));
+    const bool valid = lane < m, mine = valid && ci0 == cx && ci1 == cy && ci2 == cz;
+    __syncwarp();
+    M.xy[lane].x = both<R>(-pi.x);
+    M.xy[lane].y = both<R>(-pi.y);
+    M.z[lane] = both<R>(-pi.z);
+    int idx = 0, have = 0;                     // pairs found; entries of the open chunk in ch
+    int ch[4] = {0, 0, 0, 0};
+    int4* dst = out + i;
+    int row4 = 0;                              // first row of the open chunk
+    for (int b0 = 0; b0 < total; b0 += kCellBatch) {
+      const int b1 = min(total, b0 + kCellBatch);
+      __syncwarp();
+      for (int base = b0; base < b1; base += 32 * KC) {
+        R px[KC], py[KC], pz[KC];
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
-      ci[d] = (int)div_rn(sub_rn(pix[d], Traits<R>::lo(rp, d)), Traits<R>::dx(rp, d));
-    int idx = 0;
-    if (staged && ci[1] == sg.y && ci[2] == sg.z && ci[0] >= sg.x0 && ci[0] < sg.x1) {
-      const int u0 = ci[0] - sg.x0;   // staged cells u0 .. u0 + 2 of every row
-      // staged x already carries the periodic shift, and a row's cells are ordered by x
-      // (rows that wrap in x are walked whole: atoms outside the box, binned into the last or
-      // first cell, break the order across the wrap)
-      const R xm = rc + (fabs(pix[0]) + (R)2 * rc) * (R)1e-5 + (R)1e-6;
-      const bool trim = trim_x && ci[0] - 1 >= 0 && ci[0] + 1 < d0;
-      for (int r = 0; r < 9; ++r) {
-        int t0 = cs[r * W + u0], t1 = cs[r * W + u0 + 3];
-        if (trim) {
-          for (int lo = t0, hi = t1; lo < hi;) {
-            const int mid = (lo + hi) >> 1;
-            if (stage[mid].x < pix[0] - xm) lo = t0 = mid + 1;
-            else hi = mid;
-          }
-          for (int lo = t0, hi = t1; lo < hi;) {
-            const int mid = (lo + hi) >> 1;
-            if (stage[mid].x < pix[0] + xm) lo = mid + 1;
-            else hi = t1 = mid;
+        for (int k = 0; k < KC; ++k) {
+          const int q = base + 32 * k + 31 - lane;
+          px[k] = (R)INFINITY;                 // past the last candidate: never accepted
+          py[k] = pz[k] = (R)0;
+          if (q < b1) {
+            int lo = 0, hi = 27;               // pre[lo] <= q < pre[hi]
+#pragma unroll
+            for (int b = 0; b < 5; ++b) {
+              const int mid = (lo + hi) >> 1;
+              if (M.pre[mid] <= q) lo = mid;
+              else hi = mid;
+            }
+            const int s = M.start[lo] + (q - M.pre[lo]);
+            const V4 pj = pos4[s];
+            px[k] = sub_rn(pj.x, M.off[0][lo]);
+            py[k] = sub_rn(pj.y, M.off[1][lo]);
+            pz[k] = sub_rn(pj.z, M.off[2][lo]);
+            M.ent[q - b0] = (s << kShiftBits) | M.code[lo];
           }
         }
-#pragma unroll 4
-        for (int t = t0; t < t1; ++t) {
-          const V4 q = stage[t];
-          const R r0 = sub_rn(q.x, pix[0]);
-          const R r1 = sub_rn(q.y, pix[1]);
-          const R r2 = sub_rn(q.z, pix[2]);
-          const R dd = add_rn(add_rn(mul_rn(r0, r0), mul_rn(r1, r1)), mul_rn(r2, r2));
-          if (inside_cut(sub_rn(cut2, dd), orig) && gt_small(dd)) {
-            if (idx < cap) __stcs(nbr + (size_t)idx * stride + i, unpack_tag(q.w));
-            ++idx;
+        unsigned word[KC];
+#pragma unroll
+        for (int k = 0; k < KC; ++k) word[k] = 0;
+#pragma unroll 2
+        for (int a = 0; a < m; ++a) {
+          const typename CellWarpMem<R>::XY o = M.xy[a];
+          const Pair<R> oz = M.z[a];
+#pragma unroll
+          for (int h = 0; h < KC; h += 2) {
+            const Pair<R> dx = add2(Pair<R>{px[h], px[h + 1]}, o.x), dy = add2(Pair<R>{py[h], py[h + 1]}, o.y),
+                          dz = add2(Pair<R>{pz[h], pz[h + 1]}, oz);
+            const Pair<R> dd = fma2(mul2(dz, dz), unit, fma2(mul2(dy, dy), unit, mul2(dx, dx)));
+            const unsigned ba = __ballot_sync(full, dd.x > d2_lo && dd.x <= d2_max);
+            const unsigned bb = __ballot_sync(full, dd.y > d2_lo && dd.y <= d2_max);
+            if (a == lane) {
+              word[h] = ba;
+              word[h + 1] = bb;
+            }
           }
         }
+#pragma unroll
+        for (int k = 0; k < KC; ++k) M.word[(base - b0) / 32 + k][lane] = word[k];
       }
-    } else {
-      idx = nlist_thread<R>(i, pi, rp, pos4, cell_start, 1, rc, cap, stride, nbr, false, orig);
+      __syncwarp();
+      if (mine) {
+        const int nw = (b1 - b0 + 31) / 32;
+        int found = 0;
+        for (int k = 0; k < nw; ++k) found += __popc(M.word[k][lane]);
+        idx += found;
+        int wi = 0;
+        unsigned bits = M.word[0][lane];
+        auto next = [&]() -> int {             // entry of the next accepted candidate
+          while (bits == 0) bits = M.word[++wi][lane];
+          const int c = __clz(bits);
+          bits ^= 0x80000000u >> c;
+          return M.ent[32 * wi + c];
+        };
+        const int all = have + found;
+        for (int t = 0; t < all >> 2; ++t) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (k >= have) ch[k] = next();
+          have = 0;
+          if (row4 < cap) __stcs(dst, make_int4(ch[0], ch[1], ch[2], ch[3]));
+          dst += stride;
+          row4 += 4;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (k >= have && k < (all & 3)) ch[k] = next();
+        have = all & 3;
+      }
     }
-    nlist_finish(i, idx, cap, count, max_count, status);
+    if (mine) {   // the last chunk, filled with the slot itself (see nlist_finish)
+      if (have > 0 && row4 < cap) {
+        const int self = i << kShiftBits;
+        __stcs(dst, make_int4(ch[0], have > 1 ? ch[1] : self, have > 2 ? ch[2] : self, self));
+      }
+      count[i] = idx;
+      if (idx > cap) {
+        set_flag(status, kFlagListOverflow);
+        atomicMax(max_count, idx);
+      }
+    } else if (valid) {
+      idx = nlist_thread<R>(i, pi, rp, pos4, cell_start, 1, rc, cap, stride, nbr, false, orig);
+      nlist_finish(i, idx, cap, stride, nbr, count, max_count, status);
+    }
   }
 }
 

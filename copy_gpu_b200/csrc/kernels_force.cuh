@@ -134,7 +134,7 @@ __device__ __forceinline__ float rcp_r(float x) {
 }
 __device__ __forceinline__ double rcp_r(double x) { return 1.0 / x; }
 
-// Near force of one slot per thread over its transposed list row (nbr[p * stride + slot]).
+// Near force of one slot per thread over its list row.
 // Pair physics: ComputeNearForceVerletWorklet / ComputeLJForceVerletWorklet
 // (rbmd/framework/run/worklet/RunWorklet.cpp:170-303) with ComputeLJForce and
 // ComputeNearEnergyForce (rbmd/framework/forceFunction/ExecForceFunction.h:74-140):
@@ -179,15 +179,14 @@ __global__ void __launch_bounds__(256) k_near_force(
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
   const int trow = prm.ntypes > 1 ? mi.x * prm.ntypes : 0;   // one LJ type when all types agree
-  const int* col = nbr + i;
-  const size_t st = (size_t)prm.stride;
+  const int st = prm.stride;
   Acc<R> fx, fy, fz;
   R gx = 0, gy = 0, gz = 0;   // FP32 group sum folded into the accumulators every 4 pairs
   R e_lj = 0, e_coul = 0;
   const int cnt = min(count[i], prm.cap);   // an overflowed row is redone after regrowth
   // pipeline prologue
-  int e_cur = cnt > 0 ? __ldg(col) : 0;
-  int e_nxt = cnt > 1 ? __ldg(col + st) : 0;
+  int e_cur = cnt > 0 ? __ldg(nbr + nbr_at(0, i, st)) : 0;
+  int e_nxt = cnt > 1 ? __ldg(nbr + nbr_at(1, i, st)) : 0;
   V4 pj_cur = pos4[cnt > 0 ? (e_cur >> kShiftBits) : i];
   for (int p = 0; p < cnt; ++p) {
     const int e = e_cur;
@@ -195,7 +194,7 @@ __global__ void __launch_bounds__(256) k_near_force(
     // issue the loads of the next iterations before the arithmetic of this one
     e_cur = e_nxt;
     if (p + 1 < cnt) pj_cur = pos4[e_cur >> kShiftBits];
-    if (p + 2 < cnt) e_nxt = __ldg(col + (size_t)(p + 2) * st);
+    if (p + 2 < cnt) e_nxt = __ldg(nbr + nbr_at(p + 2, i, st));
     R px = pj.x, py = pj.y, pz = pj.z;
     if (e & 63) {   // periodic image: p_j - offset (PeriodicCoordOffset)
       const int c0 = e & 3, c1 = (e >> 2) & 3, c2b = (e >> 4) & 3;
@@ -275,115 +274,125 @@ __global__ void __launch_bounds__(256) k_near_force(
 
 // Near force, one thread per atom, for the common case of one LJ coefficient pair for every type
 // pair and no molecules (the electrolyte benchmarks): the same pair set,
-// predicates and pair arithmetic as k_near_force, with less work per listed pair:
-//   * the LJ coefficients live in registers (no per-pair shared-memory lookups);
-//   * the list is walked four entries at a time, software-pipelined by whole chunks: the entries
-//     of chunk c + 2 and the neighbour positions of chunk c + 1 are in flight while chunk c is
-//     evaluated; the last chunk repeats the row's last entry and masks the repeats (a variant
-//     with rows padded by the atom's own slot instead held more registers and ran 15 % slower);
-//   * the LJ term is evaluated branch-free and selected by the pair predicate (the predicate of
-//     the list at rc under list reuse), so skin pairs cost no divergent branch;
+// predicates and pair physics as k_near_force, with less work per listed pair:
+//   * the list is walked a chunk of four entries at a time: one 16-byte load per chunk, the last
+//     chunk filled with the slot itself by the list build (distance 0, which the predicate
+//     refuses), so no entry is tested against the row's length; the entries of the chunk after
+//     next and the positions of the next are in flight while a chunk is evaluated;
+//   * all lanes of a warp run the chunks of its longest row (lanes past their row hold the slot
+//     itself), so the votes below are on full warps;
 //   * the periodic image offsets are decoded only when some lane of the warp holds an image
-//     entry in the chunk (most warps hold none);
+//     entry in the chunk (most warps hold none), in one branch per chunk;
+//   * the LJ terms of two entries are evaluated side by side in packed FP32x2 instructions,
+//     branch-free, and selected by the predicate d2_lo < d^2 <= d2_max (the list predicate at rc
+//     as one comparison, list_d2_max);
 //   * the four pair forces of a chunk are summed in R and folded into the two-float accumulator.
+// Bound by issue and the latency of the position gathers; 1,000,000 atoms, 72 listed pairs each:
+// 288 -> 219 us, 512 replicas (2.2 M atoms) 685 -> 548 us against one 4-byte list load, one length
+// test and one image branch per entry.
 // Pair physics as k_near_force: ComputeNearForceVerletWorklet / ComputeLJForceVerletWorklet
 // (rbmd/framework/run/worklet/RunWorklet.cpp:170-303), ExecForceFunction::ComputeLJForce and
 // ComputeNearEnergyForce (rbmd/framework/forceFunction/ExecForceFunction.h:74-140).
 template <class R, bool COUL, int MI, bool ENERGY>
 __global__ void __launch_bounds__(256) k_near_lean(
-    NearParams prm, R a24, R s6, const typename Traits<R>::V4* __restrict__ pos4, const int* __restrict__ nbr,
-    const int* __restrict__ count, const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot,
-    const int* __restrict__ slot_atom, double* __restrict__ force, double* __restrict__ energy_slot,
-    uint32_t* status) {
+    NearParams prm, R a24, R s6, R d2_max, const typename Traits<R>::V4* __restrict__ pos4,
+    const int4* __restrict__ nbr4, const int* __restrict__ count, const RepDev* __restrict__ reps,
+    const int* __restrict__ rep_of_slot, const int* __restrict__ slot_atom, double* __restrict__ force,
+    double* __restrict__ energy_slot, uint32_t* status) {
   static_assert((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0, "k_near_lean: no per-pair minimum image, no weights");
   using V4 = typename Traits<R>::V4;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= prm.n) return;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool active = gid < prm.n;   // lanes past the end run along with an empty row
+  const int i = active ? gid : prm.n - 1;
   const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
   const V4 pi = pos4[i];
   const R rc = (R)prm.rc;
-  const R cut2 = rc * rc;
-  const R w0 = Traits<R>::wrap(rp, 0), w1 = Traits<R>::wrap(rp, 1), w2 = Traits<R>::wrap(rp, 2);
   const R sa = (R)prm.sqrt_alpha, aa = (R)prm.alpha, c2 = (R)prm.two_sqrt_alpha_over_sqrt_pi;
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
-  const int cnt = min(count[i], prm.cap);
-  Acc<R> fx, fy, fz;
+  const int cnt = active ? min(count[i], prm.cap) : 0;
+  const int last = __reduce_max_sync(0xffffffffu, cnt);
+  const int self = i << kShiftBits;
+  const int4 idle = make_int4(self, self, self, self);
+  // 24 eps (2 s6 u - 1) s6 u / d^2 with u = d^-6 as (ka u - kb) d^-8
+  const Pair<R> ka = both<R>((R)2 * a24 * s6 * s6), kb = both<R>(-a24 * s6);
+  Acc3<R> F;
   R e_lj = 0, e_coul = 0;
-  // a chunk's entries; indices past the end repeat the last entry (valid memory), masked below
-  const unsigned ust = (unsigned)prm.stride;
-  auto load_chunk = [&](int p0, int (&e)[4]) {
+  const int4* row = nbr4 + i;
+  const size_t st = (size_t)prm.stride;
+  int4 e = cnt > 0 ? __ldg(row) : idle;
+  int4 e_nxt = cnt > 4 ? __ldg(row + st) : idle;
+  row += 2 * st;
+  V4 pj[4] = {pos4[e.x >> kShiftBits], pos4[e.y >> kShiftBits], pos4[e.z >> kShiftBits], pos4[e.w >> kShiftBits]};
+  for (int p = 0; p < last; p += 4, row += st) {
+    if (__any_sync(0xffffffffu, ((e.x | e.y | e.z | e.w) & 63) != 0)) {   // p_j - PeriodicCoordOffset
+      const int ee[4] = {e.x, e.y, e.z, e.w};
+      const R w0 = Traits<R>::wrap(rp, 0), w1 = Traits<R>::wrap(rp, 1), w2 = Traits<R>::wrap(rp, 2);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) e[k] = __ldg(nbr + i + (size_t)min(p0 + k, cnt - 1) * (size_t)ust);
-  };
-  int e_cur[4] = {0, 0, 0, 0}, e_nxt[4] = {0, 0, 0, 0};
-  V4 pj[4];
-  if (cnt > 0) {
-    load_chunk(0, e_cur);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) pj[k] = pos4[e_cur[k] >> kShiftBits];
-    if (cnt > 4) load_chunk(4, e_nxt);
-  }
-  for (int p = 0; p < cnt; p += 4) {
-    const unsigned act = __activemask();
-    const bool img = __any_sync(act, ((e_cur[0] | e_cur[1] | e_cur[2] | e_cur[3]) & 63) != 0);
-    R gx = 0, gy = 0, gz = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      R px = pj[k].x, py = pj[k].y, pz = pj[k].z;
-      if (img) {   // p_j - PeriodicCoordOffset
-        const int e = e_cur[k];
-        const int c0 = e & 3, c1 = (e >> 2) & 3, c2b = (e >> 4) & 3;
-        px = px - (c0 == 1 ? w0 : (c0 == 2 ? -w0 : (R)0));
-        py = py - (c1 == 1 ? w1 : (c1 == 2 ? -w1 : (R)0));
-        pz = pz - (c2b == 1 ? w2 : (c2b == 2 ? -w2 : (R)0));
+      for (int k = 0; k < 4; ++k) {
+        const int k0 = ee[k] & 3, k1 = (ee[k] >> 2) & 3, k2 = (ee[k] >> 4) & 3;
+        pj[k].x -= k0 == 1 ? w0 : (k0 == 2 ? -w0 : (R)0);
+        pj[k].y -= k1 == 1 ? w1 : (k1 == 2 ? -w1 : (R)0);
+        pj[k].z -= k2 == 1 ? w2 : (k2 == 2 ? -w2 : (R)0);
       }
-      const R r0 = px - pi.x, r1 = py - pi.y, r2 = pz - pi.z;
-      const R d2 = r0 * r0 + r1 * r1 + r2 * r2;
-      bool in = (p + k < cnt) && d2 > (R)1.0e-4;
-      if ((MI & 3) == kMiAll) in = in && (prm.orig ? cut2 - d2 > (R)0 : cut2 - d2 > (R)1.0e-4);
-      else in = in && d2 < cut2;
-      const R inv2 = rcp_r(d2);
-      const R sd6 = s6 * inv2 * inv2 * inv2;
-      const R scal = in ? a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2 : (R)0;
-      // 4 eps (s6 - 1) s6 with 4 eps = -lj24/6
-      if (ENERGY && in) e_lj += -a24 / (R)6 * (sd6 - (R)1) * sd6;
-      R f = 0;
+    }
+    Pair<R> gx = both<R>(0), gy = both<R>(0), gz = both<R>(0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const V4 &pa = pj[2 * h], &pb = pj[2 * h + 1];
+      const Pair<R> rx{pa.x - pi.x, pb.x - pi.x}, ry{pa.y - pi.y, pb.y - pi.y}, rz{pa.z - pi.z, pb.z - pi.z};
+      const Pair<R> d2 = fma2(rz, rz, fma2(ry, ry, mul2(rx, rx)));
+      const bool in[2] = {d2.x > (R)1.0e-4 && d2.x <= d2_max, d2.y > (R)1.0e-4 && d2.y <= d2_max};
+      const Pair<R> i2{rcp_r(d2.x), rcp_r(d2.y)};
+      const Pair<R> i4 = mul2(i2, i2), i6 = mul2(i4, i2), i8 = mul2(i4, i4);
+      const Pair<R> lj = mul2(fma2(ka, i6, kb), i8);
+      Pair<R> t{in[0] ? lj.x : (R)0, in[1] ? lj.y : (R)0};
+      if (ENERGY) {
+        // 4 eps (sd6 - 1) sd6 with 4 eps = -a24 / 6
+        const R sx = s6 * i6.x, sy = s6 * i6.y;
+        if (in[0]) e_lj += -a24 / (R)6 * (sx - (R)1) * sx;
+        if (in[1]) e_lj += -a24 / (R)6 * (sy - (R)1) * sy;
+      }
       if (COUL) {
-        const R qq = qi * pj[k].w;
-        if (in && qq != (R)0) {
-          const R inv = rsqrt_r(d2);
-          const R dis = d2 * inv;
-          if (dis < rc && dis > (R)0.01) {
-            const R ex = exp_r(-aa * d2);
-            const R erfcv = erfc_shared(sa * dis, ex);
-            const R g = (erfcv * inv + c2 * ex) * inv;
-            f = -qq * g * inv * cs;
-            if (ENERGY) e_coul += qq * erfcv * inv * cs;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const R qq = qi * (k ? pb.w : pa.w);
+          if (in[k] && qq != (R)0) {
+            const R dd = k ? d2.y : d2.x;
+            const R inv = rsqrt_r(dd);
+            const R dis = dd * inv;
+            if (dis < rc && dis > (R)0.01) {
+              const R ex = exp_r(-aa * dd);
+              const R erfcv = erfc_shared(sa * dis, ex);
+              const R g = (erfcv * inv + c2 * ex) * inv;
+              const R f = -qq * g * inv * cs;
+              if (k) t.y += f;
+              else t.x += f;
+              if (ENERGY) e_coul += qq * erfcv * inv * cs;
+            }
           }
         }
       }
-      const R t = scal + f;
-      gx += t * r0;
-      gy += t * r1;
-      gz += t * r2;
+      gx = fma2(t, rx, gx);
+      gy = fma2(t, ry, gy);
+      gz = fma2(t, rz, gz);
     }
-    fx.add(gx); fy.add(gy); fz.add(gz);
+    F.add(gx.x + gx.y, gy.x + gy.y, gz.x + gz.y);
     // advance the pipeline: positions of the next chunk, entries of the one after
-#pragma unroll
-    for (int k = 0; k < 4; ++k) e_cur[k] = e_nxt[k];
-    if (p + 4 < cnt) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pj[k] = pos4[e_cur[k] >> kShiftBits];
-      if (p + 8 < cnt) load_chunk(p + 8, e_nxt);
-    }
+    e = e_nxt;
+    pj[0] = pos4[e.x >> kShiftBits];
+    pj[1] = pos4[e.y >> kShiftBits];
+    pj[2] = pos4[e.z >> kShiftBits];
+    pj[3] = pos4[e.w >> kShiftBits];
+    e_nxt = p + 8 < cnt ? __ldg(row) : idle;
   }
-  const double F[3] = {fx.value(), fy.value(), fz.value()};
-  if (!isfinite(F[0]) || !isfinite(F[1]) || !isfinite(F[2])) set_flag(status, kFlagNonFinite);
+  if (!active) return;
+  const double Fd[3] = {F.vx(), F.vy(), F.vz()};
+  if (!isfinite(Fd[0]) || !isfinite(Fd[1]) || !isfinite(Fd[2])) set_flag(status, kFlagNonFinite);
   const int id = slot_atom[i];
-  force[3 * id] = F[0];
-  force[3 * id + 1] = F[1];
-  force[3 * id + 2] = F[2];
+  force[3 * id] = Fd[0];
+  force[3 * id + 1] = Fd[1];
+  force[3 * id + 2] = Fd[2];
   if (ENERGY) {
     energy_slot[2 * i] = 0.5 * (double)e_lj;
     energy_slot[2 * i + 1] = 0.5 * (double)e_coul;
@@ -430,14 +439,13 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
   const int trow = prm.ntypes > 1 ? mi.x * prm.ntypes : 0;
-  const size_t st = (size_t)prm.stride;
   Acc<R> fx, fy, fz;
   R gx = 0, gy = 0, gz = 0;
   R e_lj = 0, e_coul = 0;
   const int cnt = active ? min(count[i], prm.cap) : 0;
   int k = 0;
   for (int p = sub; p < cnt; p += G, ++k) {
-    const int e = __ldg(nbr + (size_t)p * st + i);
+    const int e = __ldg(nbr + nbr_at(p, i, prm.stride));
     const V4 pj = pos4[e >> kShiftBits];
     R px = pj.x, py = pj.y, pz = pj.z;
     if (e & 63) {
@@ -947,7 +955,7 @@ __global__ void __launch_bounds__(128) k_eam_fp(int n, int stride, int cap, doub
   Acc<R> rho;
   const int cnt = min(count[i], cap);
   for (int p = 0; p < cnt; ++p) {
-    const int e = __ldg(nbr + (size_t)p * stride + i);
+    const int e = __ldg(nbr + nbr_at(p, i, stride));
     const int j = e >> kShiftBits;
     const typename Traits<R>::V4 pj = pos4[j];
     R r[3];
@@ -1011,7 +1019,7 @@ __global__ void __launch_bounds__(128) k_eam_force(int n, int stride, int cap, d
   R epair = 0;
   const int cnt = min(count[i], cap);
   for (int p = 0; p < cnt; ++p) {
-    const int e = __ldg(nbr + (size_t)p * stride + i);
+    const int e = __ldg(nbr + nbr_at(p, i, stride));
     const int j = e >> kShiftBits;
     const typename Traits<R>::V4 pj = pos4[j];
     R r[3];

@@ -104,13 +104,13 @@ __global__ void __launch_bounds__(128) k_rbl_list(
               const int e = ((s + u) << kShiftBits) | code;
               if (gt_small(sub_rn(rc2, d2)) && gt_small(sub_rn(d2, rs2))) {
                 if (shell_index == next_kept) {   // shell_index % pice == 0
-                  if (n_shell < shell_cap) nbr[(size_t)(core_cap + n_shell) * stride + i] = e;
+                  if (n_shell < shell_cap) nbr[nbr_at(core_cap + n_shell, i, stride)] = e;
                   ++n_shell;
                   next_kept += pice;
                 }
                 ++shell_index;
               } else if (gt_small(sub_rn(rs2, d2)) && gt_small(d2)) {
-                if (n_core < core_cap) nbr[(size_t)n_core * stride + i] = e;
+                if (n_core < core_cap) nbr[nbr_at(n_core, i, stride)] = e;
                 ++n_core;
               }
             }
@@ -236,11 +236,11 @@ __global__ void __launch_bounds__(32 * kRblWarps) k_rbl_list_warp(
     const unsigned bcore = __ballot_sync(full, core);
     if (keep) {
       const int at = n_shell + __popc(bkeep & lt);
-      if (at < shell_cap) nbr[(size_t)(core_cap + at) * stride + i] = entry;
+      if (at < shell_cap) nbr[nbr_at(core_cap + at, i, stride)] = entry;
     }
     if (core) {
       const int at = n_core + __popc(bcore & lt);
-      if (at < core_cap) nbr[(size_t)at * stride + i] = entry;
+      if (at < core_cap) nbr[nbr_at(at, i, stride)] = entry;
     }
     shell_index += __popc(bsh);
     n_shell += __popc(bkeep);
@@ -323,7 +323,6 @@ __global__ void __launch_bounds__(128, 8) k_rbl_force(
   const R sa = (R)prm.sqrt_alpha, aa = (R)prm.alpha, c2 = (R)prm.two_sqrt_alpha_over_sqrt_pi;
   const R qqr2e = (R)prm.qqr2e;
   const R qi = pi.w;
-  const size_t st = (size_t)prm.stride;
   Acc<R> fx, fy, fz;
   double e_lj = 0, e_coul = 0;
   const int nco = min(ncore[i], prm.core_cap), nsh = active ? min(nshell[i], shell_cap) : 0;
@@ -331,7 +330,7 @@ __global__ void __launch_bounds__(128, 8) k_rbl_force(
   for (int p = sub; p < nall; p += G) {
     const bool shell = p >= nco;
     const int row = shell ? prm.core_cap + (p - nco) : p;
-    const int e = __ldg(nbr + (size_t)row * st + i);
+    const int e = __ldg(nbr + nbr_at(row, i, prm.stride));
     const int js = e >> kShiftBits;
     const V4 pj = pos4[js];
     R px = pj.x, py = pj.y, pz = pj.z;
@@ -458,7 +457,7 @@ __global__ void __launch_bounds__(128) k_rbl_eam_fp(int n, int stride, int core_
   const int nco = min(ncore[i], core_cap), nsh = min(nshell[i], shell_cap);
   for (int p = 0; p < nco + nsh; ++p) {
     const bool shell = p >= nco;
-    const int e = __ldg(nbr + (size_t)(shell ? core_cap + (p - nco) : p) * stride + i);
+    const int e = __ldg(nbr + nbr_at(shell ? core_cap + (p - nco) : p, i, stride));
     R r[3];
     rbl_eam_pair<R>(pi, pos4[e >> kShiftBits], e, wrap, box, r);
     const R rsq = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
@@ -514,7 +513,7 @@ __global__ void __launch_bounds__(128) k_rbl_eam_force(int n, int stride, int co
   const int nco = min(ncore[i], core_cap), nsh = min(nshell[i], shell_cap);
   for (int p = 0; p < nco + nsh; ++p) {
     const bool shell = p >= nco;
-    const int e = __ldg(nbr + (size_t)(shell ? core_cap + (p - nco) : p) * stride + i);
+    const int e = __ldg(nbr + nbr_at(shell ? core_cap + (p - nco) : p, i, stride));
     const int j = e >> kShiftBits;
     R r[3];
     rbl_eam_pair<R>(pi, pos4[j], e, wrap, box, r);

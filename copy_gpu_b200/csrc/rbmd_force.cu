@@ -121,13 +121,13 @@ struct rbmd_force {
   double shake_tol = 1e-5;
   int energy_every = 0;   // energies inside step(): every outputs.thermo_out.interval steps
   int cap_override = 0;   // neighbor.capacity: initial list capacity (grown on overflow)
-  int tpa_list = 0, tpa_near = 128;
+  int tpa_list = 0, tpa_near = 128;     // list build: 0 = one warp per cell, 1 = one warp per atom, else
+                                        // threads per block of k_nlist; threads per block of the force pass
   int rbl_list_warp = -1;               // RBL list build: 1 one warp per atom, 0 one thread per atom, -1 by size
   int rbl_lanes = 0;                    // RBL force pass lanes per atom (0: by size)
   int num_sms = 148;                    // SMs of the bound device (cudaDevAttrMultiProcessorCount)
   int near_variant = 1;                 // 1: k_near_lean where it applies (lean_ok), 0: k_near_force
-  int near_lanes = 1;                   // near pass lanes per atom: 1, or 4 / 8 / 16 / 32     // list build: 0 = staged kernel, else threads per block of
-                                        // k_nlist; threads per block of the force pass
+  int near_lanes = 1;                   // near pass lanes per atom: 1, or 4 / 8 / 16 / 32
   bool autotune = false;                // "autotune": true tunes them at the first compute
   bool tuned = false;
   bool list_valid = false;   // a list (and x_ref) exists from an earlier build
@@ -192,8 +192,7 @@ struct rbmd_force {
   int *d_rebuild = nullptr, *d_block_sums = nullptr;   // d_rebuild[nrep + 1]: per replica, then any
   int* d_cell_rep = nullptr;                            // replica of each cell (batches only)
   unsigned long long* d_nbuilds = nullptr;
-  ListSeg* d_segs = nullptr;   // staged list build: one block per segment of a cell row
-  int nsegs = 0, stage_cap = 0;
+  int list_parts = 1;          // warps per cell of k_nlist_cell
   double* d_xref = nullptr;
   uint32_t* d_status = nullptr;
   double* d_eslot = nullptr;   // 2 per slot (lj, coul)
@@ -404,8 +403,6 @@ void free_all(rbmd_force* f) {
   dfree(f->d_prep); dfree(f->d_cdf); dfree(f->d_wbin); dfree(f->d_pw); dfree(f->d_mlp); dfree(f->d_mlp_t); dfree(f->d_h);
   dfree(f->d_spec); dfree(f->d_spec_init);
   dfree(f->d_rebuild); dfree(f->d_block_sums); dfree(f->d_cell_rep); dfree(f->d_xref); dfree(f->d_nbuilds);
-  dfree(f->d_segs);
-  f->nsegs = 0;
   dfree(f->d_eslot); dfree(f->d_esum);
   if (f->d_krec) cudaFree(f->d_krec);
   f->d_krec = nullptr;
@@ -747,15 +744,50 @@ double rbe_S(double alpha, const double* L) {
   return H[0] * H[1] * H[2] - 1.0;
 }
 
+// Largest d^2 that a pair predicate accepts: `reuse` the list predicate rc^2 - d^2 > 1e-4 (with
+// orig: > 0), else d^2 < rc^2.  Rounding rc^2 - d^2 is monotonic in d^2, so the predicate equals
+// d^2 <= this value for every float d^2; found by bisection over the bit patterns (positive
+// floats are ordered as their bits).  Negative when nothing is accepted.
+template <class R>
+R pair_d2_max(R rc, bool reuse, bool orig) {
+  using I = typename std::conditional<sizeof(R) == 4, uint32_t, uint64_t>::type;
+  const volatile R cut2 = rc * rc;
+  auto accepts = [&](R d2) -> bool {
+    if (!reuse) return d2 < cut2;
+    const volatile R margin = cut2 - d2;
+    return orig ? margin > (R)0 : margin > (R)1.0e-4;
+  };
+  if (!accepts((R)0)) return (R)-1;
+  I lo = 0, hi;   // accepts(lo), not accepts(hi)
+  const R c = cut2;
+  std::memcpy(&hi, &c, sizeof hi);
+  while (hi - lo > 1) {
+    const I mid = lo + (hi - lo) / 2;
+    R v;
+    std::memcpy(&v, &mid, sizeof v);
+    (accepts(v) ? lo : hi) = mid;
+  }
+  R v;
+  std::memcpy(&v, &lo, sizeof v);
+  return v;
+}
+
+template <class R>
+R lean_d2_max(const rbmd_force* f) {
+  return pair_d2_max<R>((R)f->rc, f->skin > 0, f->orig_pred);
+}
+
 template <class R>
 void launch_nlist(rbmd_force* f, cudaStream_t s) {
   PhaseScope ps(f, kPhList, s);
-  if (f->tpa_list == 0 && f->nsegs > 0) {
-    const size_t smem = (size_t)f->stage_cap * sizeof(typename Traits<R>::V4);
-    k_nlist_staged<R><<<f->nsegs, kStageThreads, smem, s>>>(
-        f->d_segs, f->stage_cap, (const typename Traits<R>::V4*)f->d_pos4, f->d_cell_start, f->d_reps,
-        (R)f->list_cut(), f->cap, f->stride, f->d_nbr, f->d_count, f->d_maxcount, f->d_status,
-        f->skin > 0 ? f->d_rebuild : nullptr, f->d_nbuilds, f->sort_x() ? 1 : 0, f->nrep, f->orig_pred ? 1 : 0);
+  if (f->tpa_list == 0 && f->num_cycles == 1) {   // warp per cell
+    const long long items = (long long)f->ncell_total * f->list_parts;
+    k_nlist_cell<R, sizeof(R) == 4 ? 4 : 2><<<(unsigned)((items + kCellWarps - 1) / kCellWarps), 32 * kCellWarps, 0, s>>>(
+        f->ncell_total, f->list_parts, (const typename Traits<R>::V4*)f->d_pos4, f->d_cell_start, f->d_reps,
+        f->nrep > 1 ? f->d_cell_rep : nullptr, (R)f->list_cut(),
+        pair_d2_max<R>((R)f->list_cut(), true, f->orig_pred), (R)1, f->cap, f->stride, f->d_nbr, f->d_count,
+        f->d_maxcount, f->d_status, f->skin > 0 ? f->d_rebuild : nullptr, f->d_nbuilds, f->nrep,
+        f->orig_pred ? 1 : 0);
     f->launches++;
     return;
   }
@@ -980,8 +1012,8 @@ void launch_near_t(rbmd_force* f, cudaStream_t s) {
       auto kern = f->want_energy ? k_near_lean<R, COUL, MI, true> : k_near_lean<R, COUL, MI, false>;
       prefer_shared_carveout(f, (const void*)kern);
       kern<<<(f->n + bs - 1) / bs, bs, 0, s>>>(
-          p, lj24<R>(f->ljt_h, 0), sig6<R>(f->ljt_h, 0), (const typename Traits<R>::V4*)f->d_pos4, f->d_nbr,
-          f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
+          p, lj24<R>(f->ljt_h, 0), sig6<R>(f->ljt_h, 0), lean_d2_max<R>(f), (const typename Traits<R>::V4*)f->d_pos4,
+          (const int4*)f->d_nbr, f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
           f->want_energy ? f->d_eslot : nullptr, f->d_status);
       f->launches++;
       return;
@@ -1313,6 +1345,9 @@ void drop_graphs(rbmd_force* f) {
   if (f->graph_multi) cudaGraphExecDestroy(f->graph_multi);
   f->graph_multi = nullptr;
 }
+
+// list capacities hold whole chunks of kNbrChunk entries
+int round_chunk(int cap) { return (cap + kNbrChunk - 1) / kNbrChunk * kNbrChunk; }
 
 rbmd_status grow_list(rbmd_force* f, const int* need) {
   drop_graphs(f);   // buffers move: the captured steps are stale
@@ -1783,10 +1818,9 @@ rbmd_status autotune_impl(rbmd_force* f, cudaStream_t s) {
   };
   float bl = 1e30f, bn = 1e30f;
   int tl = f->tpa_list, tn = f->tpa_near;
-  const int lcand[5] = {0, 1, 64, 128, 256};   // 0: the staged build, 1: warp per atom
+  const int lcand[5] = {0, 1, 64, 128, 256};   // 0: warp per cell, 1: warp per atom
   for (int t : lcand) {
-    if (t == 0 && f->nsegs == 0) continue;
-    if (t == 1 && f->num_cycles != 1) continue;
+    if (t <= 1 && f->num_cycles != 1) continue;
     f->tpa_list = t;
     const float ms = best_of([&] { launch_nlist<R>(f, s); });
     if (ms < bl) { bl = ms; tl = t; }
@@ -2155,7 +2189,7 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     rho_max = std::max(rho_max, (f->rep_off[r + 1] - f->rep_off[r]) / f->reps_h[r].volume);
   const double lc = f->list_cut();
   f->cap = ((int)(1.5 * rho_max * 4.0 / 3.0 * M_PI * lc * lc * lc) + 32 + 7) & ~7;
-  if (f->cap_override > 0) f->cap = f->cap_override;
+  if (f->cap_override > 0) f->cap = round_chunk(f->cap_override);
   if (f->is_rbl()) {
     // pice per replica from the reference's sizing (ExecutionMD.cpp:460-801); capacities from
     // the density with a margin (the reference's rs_num / rc_num rows have no overflow check)
@@ -2174,7 +2208,7 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     const double rs3 = f->rs * f->rs * f->rs, rc3 = f->rc * f->rc * f->rc;
     f->core_cap = ((int)(1.5 * rho_max * 4.0 / 3.0 * M_PI * rs3) + 32 + 7) & ~7;
     f->shell_cap = ((int)(1.5 * rho_max * 4.0 / 3.0 * M_PI * (rc3 - rs3) / pice_min) + 32 + 7) & ~7;
-    if (f->cap_override > 0) f->core_cap = f->cap_override;
+    if (f->cap_override > 0) f->core_cap = round_chunk(f->cap_override);
     f->cap = f->core_cap + f->shell_cap;
   }
   const size_t n = f->n;
@@ -2205,29 +2239,13 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     CK(dalloc(&f->d_erf_tab, tab.size()));
     CK(cudaMemcpy(f->d_erf_tab, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice));
   }
-  if (f->nbr_type != "RBL" && f->num_cycles == 1) {
-    // staged list build: segments of S x cells per (y, z) row, S sized so that a segment holds
-    // about 224 atoms (one 256-thread pass) and its 9 x (S + 2) staged cells fill at most 60 %
-    // of the shared buffer on average
-    f->stage_cap = f->fp64 ? 2048 : 4096;
-    std::vector<ListSeg> sg;
-    for (int r = 0; r < nrep; ++r) {
-      const RepDev& rp = f->reps_h[r];
-      const double apc = std::max(1e-3, (double)(f->rep_off[r + 1] - f->rep_off[r]) / (double)rp.ncell);
-      int S = (int)std::floor(224.0 / apc);
-      S = std::min(S, (int)std::floor(0.6 * f->stage_cap / (9.0 * apc)) - 2);
-      S = std::max(1, std::min(std::min(S, kSegMaxCells), rp.dims[0]));
-      for (int z = 0; z < rp.dims[2]; ++z)
-        for (int y = 0; y < rp.dims[1]; ++y)
-          for (int x0 = 0; x0 < rp.dims[0]; x0 += S)
-            sg.push_back(ListSeg{r, y, z, x0, std::min(x0 + S, rp.dims[0]), 0, 0, 0});
-    }
-    f->nsegs = (int)sg.size();
-    CK(dalloc(&f->d_segs, sg.size()));
-    CK(cudaMemcpy(f->d_segs, sg.data(), sizeof(ListSeg) * sg.size(), cudaMemcpyHostToDevice));
-    const int bytes = f->stage_cap * (f->fp64 ? (int)sizeof(double4) : (int)sizeof(float4));
-    CK(cudaFuncSetAttribute(f->fp64 ? (const void*)k_nlist_staged<double> : (const void*)k_nlist_staged<float>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  {
+    // warps per cell of the list build: at most 32 atoms a warp on average, and for systems with
+    // few cells more warps (down to 4 atoms each), so that every SM gets about 24
+    const double apc = (double)f->n / std::max(1, f->ncell_total);
+    const int few = (24 * f->num_sms + f->ncell_total - 1) / f->ncell_total;
+    f->list_parts = std::max((int)std::ceil(apc / 32.0), std::min(few, (int)std::ceil(apc / 4.0)));
+    f->list_parts = std::max(1, f->list_parts);
   }
   CK(dalloc(&f->d_maxcount, 2));
   CK(dalloc(&f->d_nbuilds, 1));
@@ -2770,7 +2788,7 @@ rbmd_status rbmd_force_get_neighbors(rbmd_force* f, int32_t* counts, int32_t* id
     if (ma + mb > cap) too_small = true;
     for (int p = 0; p < ma + mb && p < cap; ++p) {
       const int row = p < ma ? p : cap_a + (p - ma);
-      ids[(size_t)id * cap + p] = slot_atom[nbr[(size_t)row * f->stride + i] >> kShiftBits];
+      ids[(size_t)id * cap + p] = slot_atom[nbr[nbr_at(row, (int)i, f->stride)] >> kShiftBits];
     }
   }
   return too_small ? RBMD_ERR_ARG : RBMD_OK;

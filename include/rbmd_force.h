@@ -191,7 +191,7 @@ RBMD_API rbmd_status rbmd_force_sample_k(rbmd_force* f, int64_t step, int32_t* m
  * (rbmd/framework/run/ExecutionNVT.cpp:179-222). */
 RBMD_API rbmd_status rbmd_force_compute(rbmd_force* f, void* stream);
 
-/* Time every choice of the neighbour-list build (0: the shared-memory staged kernel, 1: one warp
+/* Time every choice of the neighbour-list build (0: one warp per cell, 1: one warp
  * per atom, or 64, 128, 256 threads per block of the per-atom kernel) and of the force pass (64,
  * 128, 256 threads per block with one thread per atom, or 4 / 8 / 16 / 32 lanes per atom) on the
  * bound system, keep the fastest, and leave the forces of that choice in atoms->force.
