@@ -306,11 +306,11 @@ __global__ void __launch_bounds__(256) k_prop_spectrum(int nrep, const RepDev* _
 // K k-vectors (drawn from p) against the nq charged atoms of one replica in fixed point.
 // Pass 0: partial rho_k; pass 1: partial sum_i q_i^2 (c_i Im rho_k - s_i Re rho_k)^2, the squared
 // norm (up to the factor (4 pi qqr2e |k| / (V k^2))^2) of the force field of this one sample.
-// Grid: (K / 256, atom chunks); thread = one k; atoms staged in shared memory.
-constexpr int kTrainChunk = 4096;
+// Grid: (K / 256, atom chunks); thread = one k; atoms staged in shared memory.  Bound by the two
+// MUFU operations per (atom, k); `chunk` atoms per block are chosen by train_chunk.
 __global__ void __launch_bounds__(256) k_train_pass(int pass, int K, int nq, const Frac32* __restrict__ frac,
-                                                    const int* __restrict__ kv, const double2* __restrict__ rho,
-                                                    float* __restrict__ partial) {
+                                                    int chunk, const int* __restrict__ kv,
+                                                    const double2* __restrict__ rho, float* __restrict__ partial) {
   __shared__ Frac32 stage[256];
   const int k = blockIdx.x * 256 + threadIdx.x;
   const bool ok = k < K;
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(256) k_train_pass(int pass, int K, int nq, con
     rre = (float)rho[k].x;
     rim = (float)rho[k].y;
   }
-  const int a0 = blockIdx.y * kTrainChunk, a1 = min(nq, a0 + kTrainChunk);
+  const int a0 = blockIdx.y * chunk, a1 = min(nq, a0 + chunk);
   float s0 = 0.f, s1 = 0.f;
   for (int base = a0; base < a1; base += 256) {
     const int cnt = min(256, a1 - base);
@@ -373,24 +373,50 @@ __global__ void k_train_finish(int pass, int K, int nchunks, const PropRep* __re
   }
 }
 
-// Per snapshot (one block, thread b = bin): C_b = (1/K) sum of a_k over the samples in bin b (an
-// unbiased estimate of sum_{m in b} a(m) / p(m), since the samples come from p), and the
-// conditioning spectrum of the snapshot (log band means of |rho_k|^2 / N_q).  Deterministic.
-__global__ void k_train_bins(int K, int nq, const int* __restrict__ kbin, const double2* __restrict__ rho,
-                             const double* __restrict__ ak, float* __restrict__ cbin, float* __restrict__ spec) {
-  const int b = threadIdx.x;
-  double cs = 0, bs = 0;
-  int bn = 0;
-  for (int k = 0; k < K; ++k) {
+// Per snapshot: C_b = (1/K) sum of a_k over the samples in bin b (an unbiased estimate of
+// sum_{m in b} a(m) / p(m), since the samples come from p), and the conditioning spectrum of the
+// snapshot (log band means of |rho_k|^2 / N_q).  One block per bin (blocks 0 .. 255) or band
+// (256 .. 263): its threads stride over the sample codes, which stay in L2, and the block sums in
+// a fixed order.  Bound by the K codes read per block; one block walking all of them once per
+// thread took 2.07 ms at K = 16384.
+__global__ void __launch_bounds__(256) k_train_bins(int K, int nq, const int* __restrict__ kbin,
+                                                    const double2* __restrict__ rho, const double* __restrict__ ak,
+                                                    float* __restrict__ cbin, float* __restrict__ spec) {
+  const int b = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const bool band = b >= kPropBins;
+  double s = 0;
+  int cnt = 0;
+#pragma unroll 4
+  for (int k = t; k < K; k += 256) {
     const int code = __ldg(kbin + k);
-    if ((code & 0xFFFF) == b) cs += ak[k];
-    if (b < kPropBands && (code >> 16) == b) {
-      bs += rho[k].x * rho[k].x + rho[k].y * rho[k].y;
-      ++bn;
+    if (band ? (code >> 16) == b - kPropBins : (code & 0xFFFF) == b) {
+      if (band) {
+        s += rho[k].x * rho[k].x + rho[k].y * rho[k].y;
+        ++cnt;
+      } else {
+        s += ak[k];
+      }
     }
   }
-  cbin[b] = (float)(cs / (double)K);
-  if (b < kPropBands) spec[b] = bn > 0 ? (float)log(fmax(bs / ((double)bn * (double)nq), 1e-6)) : 0.f;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, o);
+    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+  }
+  __shared__ double ws[8];
+  __shared__ int wc[8];
+  if (lane == 0) {
+    ws[w] = s;
+    wc[w] = cnt;
+  }
+  __syncthreads();
+  if (t != 0) return;
+  for (int k = 1; k < 8; ++k) {
+    s += ws[k];
+    cnt += wc[k];
+  }
+  if (band) spec[b - kPropBins] = cnt > 0 ? (float)log(fmax(s / ((double)cnt * (double)nq), 1e-6)) : 0.f;
+  else cbin[b] = (float)(s / (double)K);
 }
 
 }  // namespace rbmd

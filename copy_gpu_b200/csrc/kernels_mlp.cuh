@@ -33,6 +33,7 @@ struct __align__(1024) MlpSmem {
   uint16_t w2t[kMlpHid * kMlpHid];      //  8 KB  W2^T [64][64]    (B of dA1 = dZ2 W2)
   uint16_t a1[kMlpRows * kMlpHid];      // 32 KB  A1   [256][64]   (A of layer 2)
   uint16_t dz2[kMlpRows * kMlpHid];     // 32 KB  dZ2  [256][64]   (A of dA1); then dZ1 FP32 over a1+dz2
+  float part[32][kMlpRows / 2];         // 16 KB  partial dW2 of the second half of the rows
   float red[8][kMlpHid];                // per-warp partial sums
   float gsum[8][4];
   float par_b1[kMlpHid], par_b2[kMlpHid], par_w3[kMlpHid];
@@ -49,7 +50,20 @@ __device__ __forceinline__ int core_off(int r, int k, int K) {
 __device__ __forceinline__ uint16_t to_bf16(float v) {
   return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
-__device__ __forceinline__ float from_bf16(uint16_t v) { return __bfloat162float(__ushort_as_bfloat16(v)); }
+
+__device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
+// eight consecutive values of a row, one 16-byte core-matrix row
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  uint32_t u[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) u[k] = (uint32_t)to_bf16(v[2 * k]) | ((uint32_t)to_bf16(v[2 * k + 1]) << 16);
+  return make_uint4(u[0], u[1], u[2], u[3]);
+}
+__device__ __forceinline__ void unpack8(uint4 u, float* v) {
+  v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
+  v[4] = bf16_lo(u.z); v[5] = bf16_hi(u.z); v[6] = bf16_lo(u.w); v[7] = bf16_hi(u.w);
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -126,14 +140,25 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Sum the per-thread values v[64] over the block's 256 rows into out[64] (fixed order).
-__device__ __forceinline__ void block_colsum(MlpSmem& S, const float* v, float* out) {
+// Sum the per-thread values v[64] over the block's 256 rows into out[64] (fixed order): a butterfly
+// that halves the values a lane holds at every exchange (lane l ends with the warp's sums of
+// columns 2l and 2l + 1 after 62 shuffles instead of 64 full butterflies of 5), then the 8 warps
+// in order.  v is used up.
+__device__ __forceinline__ void block_colsum(MlpSmem& S, float* v, float* out) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-  for (int j = 0; j < kMlpHid; ++j) {
-    const float s = warp_sum(v[j]);
-    if (lane == 0) S.red[w][j] = s;
+  for (int o = 16, n = kMlpHid; o > 0; o >>= 1, n >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < kMlpHid / 2; ++k) {
+      if (k < n / 2) {
+        const float keep = up ? v[n / 2 + k] : v[k], give = up ? v[k] : v[n / 2 + k];
+        v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+    }
   }
+  S.red[w][2 * lane] = v[0];
+  S.red[w][2 * lane + 1] = v[1];
   __syncthreads();
   if (threadIdx.x < kMlpHid) {
     float s = 0;
@@ -153,8 +178,13 @@ __global__ void __launch_bounds__(256, 1) k_mlp(MlpArgs args) {
   const float* P = args.params;
 
   // ---- stage operands (generic proxy) ----
+  {
+    float xv[kMlpIn];
 #pragma unroll
-  for (int f = 0; f < kMlpIn; ++f) S.x[core_off(t, f, kMlpIn)] = to_bf16(args.x[row * kMlpIn + f]);
+    for (int f = 0; f < kMlpIn; ++f) xv[f] = args.x[row * kMlpIn + f];
+#pragma unroll
+    for (int f = 0; f < kMlpIn; f += 8) *reinterpret_cast<uint4*>(&S.x[core_off(t, f, kMlpIn)]) = pack8(xv + f);
+  }
   for (int e = t; e < kMlpHid * kMlpIn; e += 256) {
     const int j = e / kMlpIn, f = e % kMlpIn;
     S.w1[core_off(j, f, kMlpIn)] = to_bf16(P[kOW1 + e]);
@@ -207,10 +237,10 @@ __global__ void __launch_bounds__(256, 1) k_mlp(MlpArgs args) {
     for (int c = 0; c < 4; ++c) {
       tmem_ld16(my_lane_addr + 16 * c, z);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const int j = 16 * c + k;
-        S.a1[core_off(t, j, kMlpHid)] = to_bf16(tanhf(z[k] + S.par_b1[j]));
-      }
+      for (int k = 0; k < 16; ++k) z[k] = tanhf(z[k] + S.par_b1[16 * c + k]);
+#pragma unroll
+      for (int k = 0; k < 16; k += 8)
+        *reinterpret_cast<uint4*>(&S.a1[core_off(t, 16 * c + k, kMlpHid)]) = pack8(z + k);
     }
   }
   proxy_fence();
@@ -295,10 +325,9 @@ __global__ void __launch_bounds__(256, 1) k_mlp(MlpArgs args) {
     for (int j = 0; j < kMlpHid; ++j) v[j] = dh * a2[j];
     block_colsum(S, v, G + kOW3);                      // dw3
 #pragma unroll
-    for (int j = 0; j < kMlpHid; ++j) {
-      v[j] = dh * S.par_w3[j] * (1.0f - a2[j] * a2[j]);   // dZ2
-      S.dz2[core_off(t, j, kMlpHid)] = to_bf16(v[j]);
-    }
+    for (int j = 0; j < kMlpHid; ++j) v[j] = dh * S.par_w3[j] * (1.0f - a2[j] * a2[j]);   // dZ2
+#pragma unroll
+    for (int j = 0; j < kMlpHid; j += 8) *reinterpret_cast<uint4*>(&S.dz2[core_off(t, j, kMlpHid)]) = pack8(v + j);
     block_colsum(S, v, G + kOB2);                      // db2 (block_colsum synchronises)
   }
   // ---- dA1 = dZ2 W2 on the tensor cores, dW2 = dZ2^T A1 on the CUDA cores meanwhile ----
@@ -315,17 +344,40 @@ __global__ void __launch_bounds__(256, 1) k_mlp(MlpArgs args) {
   }
   {
     float* G = args.grad_partial + (size_t)g * kMlpNParam;
-    const int j = t >> 2, i0 = (t & 3) * 16;
-    float acc[16];
+    // thread (row half, 4 rows of dW2, 8 columns): per row one 8-byte read of dZ2 and one 16-byte read
+    // of A1 feed 32 FMAs; the halves are added through shared memory
+    const int half = t >> 7, j0 = ((t & 127) >> 3) * 4, i0 = (t & 7) * 8;
+    float acc[4][8];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) acc[k] = 0.f;
-    for (int r = 0; r < kMlpRows; ++r) {
-      const float d = from_bf16(S.dz2[core_off(r, j, kMlpHid)]);
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int k = 0; k < 16; ++k) acc[k] = fmaf(d, from_bf16(S.a1[core_off(r, i0 + k, kMlpHid)]), acc[k]);
+      for (int k = 0; k < 8; ++k) acc[a][k] = 0.f;
+#pragma unroll 4
+    for (int q = half * (kMlpRows / 2); q < (half + 1) * (kMlpRows / 2); ++q) {
+      const int r = (q & ~7) | ((q + t) & 7);   // the 8 column groups of a warp read 8 different rows (no conflicts)
+      const uint2 dv = *reinterpret_cast<const uint2*>(&S.dz2[core_off(r, j0, kMlpHid)]);
+      const float d[4] = {bf16_lo(dv.x), bf16_hi(dv.x), bf16_lo(dv.y), bf16_hi(dv.y)};
+      float x[8];
+      unpack8(*reinterpret_cast<const uint4*>(&S.a1[core_off(r, i0, kMlpHid)]), x);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[a][k] = fmaf(d[a], x[k], acc[a][k]);
     }
+    if (half) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) G[kOW2 + j * kMlpHid + i0 + k] = acc[k];
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) S.part[a * 8 + k][t & 127] = acc[a][k];
+    }
+    __syncthreads();
+    if (!half) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          G[kOW2 + (j0 + a) * kMlpHid + i0 + k] = acc[a][k] + S.part[a * 8 + k][t];
+    }
   }
   ok = mbar_wait(&S.mbar, parity);
   parity ^= 1;
@@ -338,24 +390,29 @@ __global__ void __launch_bounds__(256, 1) k_mlp(MlpArgs args) {
       float z[16];
       tmem_ld16(my_lane_addr + 16 * c, z);
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const int i = 16 * c + k;
-        const float a = from_bf16(S.a1[core_off(t, i, kMlpHid)]);
-        dz1[i] = z[k] * (1.0f - a * a);
+      for (int h = 0; h < 16; h += 8) {
+        float a[8];
+        unpack8(*reinterpret_cast<const uint4*>(&S.a1[core_off(t, 16 * c + h, kMlpHid)]), a);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) dz1[16 * c + h + k] = z[h + k] * (1.0f - a[k] * a[k]);
       }
     }
     float* G = args.grad_partial + (size_t)g * kMlpNParam;
-    block_colsum(S, dz1, G + kOB1);                    // db1 (synchronises: A1 and dZ2 are free now)
+    __syncthreads();                                   // every row of A1 and dZ2 has been read
     float* dz1s = reinterpret_cast<float*>(S.a1);      // [256][64] FP32 over a1 + dz2
 #pragma unroll
     for (int i = 0; i < kMlpHid; ++i) dz1s[t * kMlpHid + ((i + t) & 63)] = dz1[i];
-    __syncthreads();
+    block_colsum(S, dz1, G + kOB1);                    // db1 (synchronises)
     const int i = t >> 2, f0 = (t & 3) * 4;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
     for (int r = 0; r < kMlpRows; ++r) {
       const float d = dz1s[r * kMlpHid + ((i + r) & 63)];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] = fmaf(d, from_bf16(S.x[core_off(r, f0 + k, kMlpIn)]), acc[k]);
+      const uint2 xv = *reinterpret_cast<const uint2*>(&S.x[core_off(r, f0, kMlpIn)]);
+      acc[0] = fmaf(d, bf16_lo(xv.x), acc[0]);
+      acc[1] = fmaf(d, bf16_hi(xv.x), acc[1]);
+      acc[2] = fmaf(d, bf16_lo(xv.y), acc[2]);
+      acc[3] = fmaf(d, bf16_hi(xv.y), acc[3]);
     }
 #pragma unroll
     for (int k = 0; k < 4; ++k) G[kOW1 + i * kMlpIn + f0 + k] = acc[k];
@@ -372,7 +429,6 @@ done:
   }
 }
 
-// Sum of the per-group gradients in group order (deterministic), one thread per parameter.
 // T from the parameter vector P (layout in mlp_forward.cuh), one thread per word
 __global__ void k_mlp_prep(const float* __restrict__ P, float* __restrict__ T) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -400,20 +456,27 @@ __global__ void __launch_bounds__(256) k_mlp_infer(int rows, const float* __rest
   if (row < rows && part == 0) h[row] = v;
 }
 
-__global__ void k_mlp_grad_sum(int groups, const float* __restrict__ partial, float* __restrict__ grad) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= kMlpNParam) return;
+// Sum of the per-group gradients of one parameter in group order (deterministic).
+__device__ __forceinline__ float grad_of_groups(int groups, const float* __restrict__ partial, int p) {
   float s = 0;
+#pragma unroll 8
   for (int g = 0; g < groups; ++g) s += partial[(size_t)g * kMlpNParam + p];
-  grad[p] = s;
+  return s;
 }
 
-// Adam (Kingma & Ba, ICLR 2015) on the FP32 master parameters.
-__global__ void k_adam(float* __restrict__ params, const float* __restrict__ grad, float* __restrict__ m,
-                       float* __restrict__ v, float lr, float b1, float b2, float eps, int step) {
+__global__ void k_mlp_grad_sum(int groups, const float* __restrict__ partial, float* __restrict__ grad) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p < kMlpNParam) grad[p] = grad_of_groups(groups, partial, p);
+}
+
+// Gradient sum and Adam (Kingma & Ba, ICLR 2015) on the FP32 master parameters, one thread per
+// parameter; latency bound, so small blocks spread the 5313 serial sums over the SMs.
+__global__ void k_adam(int groups, const float* __restrict__ partial, float* __restrict__ params,
+                       float* __restrict__ m, float* __restrict__ v, float lr, float b1, float b2, float eps,
+                       int step) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= kMlpNParam) return;
-  const float gr = grad[p];
+  const float gr = grad_of_groups(groups, partial, p);
   const float mm = b1 * m[p] + (1.f - b1) * gr;
   const float vv = b2 * v[p] + (1.f - b2) * gr * gr;
   m[p] = mm;

@@ -52,8 +52,9 @@ cudaError_t mlp_grad_sum(int groups, const float* partial, float* grad, cudaStre
   return cudaGetLastError();
 }
 
-cudaError_t mlp_adam(float* params, const float* grad, float* m, float* v, float lr, int step, cudaStream_t s) {
-  k_adam<<<(kMlpNParam + 255) / 256, 256, 0, s>>>(params, grad, m, v, lr, 0.9f, 0.999f, 1e-8f, step);
+cudaError_t mlp_adam(int groups, const float* partial, float* params, float* m, float* v, float lr, int step,
+                     cudaStream_t s) {
+  k_adam<<<(kMlpNParam + 63) / 64, 64, 0, s>>>(groups, partial, params, m, v, lr, 0.9f, 0.999f, 1e-8f, step);
   return cudaGetLastError();
 }
 

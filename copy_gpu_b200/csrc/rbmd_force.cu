@@ -611,6 +611,16 @@ rbmd_status build_proposal_tables(rbmd_force* f, const std::vector<int64_t>& qof
   return RBMD_OK;
 }
 
+// Charged atoms per block of the training passes: about four resident waves of eight blocks per
+// SM, between 256 atoms (one staged tile) and 4096 (the partial sums are 8 B per chunk and k).
+// At 2,000 charged atoms and K = 16384, 64 blocks of up to 4096 atoms took 62 us a pass.
+int train_chunk(int nq, int K, int sms) {
+  const long long kblocks = (K + 255) / 256;
+  const long long want = std::max(1LL, 32LL * sms / kblocks);
+  const long long c = ((nq + want - 1) / want + 255) / 256 * 256;
+  return (int)std::min(4096LL, std::max(256LL, c));
+}
+
 // Scratch of one training run, freed on every return path.
 struct TrainScratch {
   std::vector<void*> ptrs;
@@ -632,7 +642,7 @@ struct TrainScratch {
 // network's conditioning state starts at the mean training spectrum.
 rbmd_status train_fit(rbmd_force* f, const rbmd_train_opts* o, rbmd_train_report* rep, cudaStream_t s,
                       std::chrono::steady_clock::time_point t0, int S, float* cbin, float* spec, float* wbinf,
-                      float* X, double* loss, float* gpart, float* grad, float* am, float* av) {
+                      float* X, double* loss, float* gpart, float* am, float* av) {
   std::vector<float> wf((size_t)S * kPropBins);
   for (int sn = 0; sn < S; ++sn)
     for (int b = 0; b < kPropBins; ++b) wf[(size_t)sn * kPropBins + b] = (float)f->wbin_h[b];
@@ -676,9 +686,8 @@ rbmd_status train_fit(rbmd_force* f, const rbmd_train_opts* o, rbmd_train_report
   double l_first = 0;
   for (int it = 1; it <= T; ++it) {
     CK(mlp_launch(a, s));
-    CK(mlp_grad_sum(S, gpart, grad, s));
     const float lr = o->learning_rate * (0.1f + 0.45f * (1.0f + std::cos((float)M_PI * (float)(it - 1) / (float)T)));
-    CK(mlp_adam(f->d_mlp, grad, am, av, lr, it, s));
+    CK(mlp_adam(S, gpart, f->d_mlp, am, av, lr, it, s));
     if (it == 1) l_first = mean_loss();
   }
   CK(mlp_launch(a, s));
@@ -2827,13 +2836,13 @@ rbmd_status rbmd_force_train_proposal(rbmd_force* f, const rbmd_train_opts* o, r
   cudaStream_t s = (cudaStream_t)stream;
   const int S = o->n_snapshots, K = o->k_per_snapshot, nq0 = f->prep_h[0].nq;
   if (nq0 < 1) return RBMD_ERR_STATE;
-  const int nch = (nq0 + kTrainChunk - 1) / kTrainChunk;
+  const int chunk = train_chunk(nq0, K, f->num_sms), nch = (nq0 + chunk - 1) / chunk;
   TrainScratch ts;
   int *kv = nullptr, *krec = nullptr, *krep = nullptr, *kbin = nullptr;
   double *kw = nullptr, *ak = nullptr, *loss = nullptr;
   double2* rho = nullptr;
   float *partial = nullptr, *cbin = nullptr, *spec = nullptr, *wbinf = nullptr, *X = nullptr, *gpart = nullptr,
-        *grad = nullptr, *am = nullptr, *av = nullptr;
+        *am = nullptr, *av = nullptr;
   Frac32* frac = nullptr;
   RepDev* rep1 = nullptr;
   CK(ts.get(&kv, 3 * (size_t)K));
@@ -2850,7 +2859,6 @@ rbmd_status rbmd_force_train_proposal(rbmd_force* f, const rbmd_train_opts* o, r
   CK(ts.get(&X, (size_t)S * kPropBins * kMlpIn));
   CK(ts.get(&loss, (size_t)S));
   CK(ts.get(&gpart, (size_t)S * kMlpNParam));
-  CK(ts.get(&grad, (size_t)kMlpNParam));
   CK(ts.get(&am, (size_t)kMlpNParam));
   CK(ts.get(&av, (size_t)kMlpNParam));
   CK(ts.get(&frac, (size_t)nq0));
@@ -2874,14 +2882,14 @@ rbmd_status rbmd_force_train_proposal(rbmd_force* f, const rbmd_train_opts* o, r
                                     (1LL << 40) + sn, nullptr, 4096, kv, krec, 12, krep, kw, f->d_status);
     const dim3 grid((K + 255) / 256, nch);
     for (int pass = 0; pass < 2; ++pass) {
-      k_train_pass<<<grid, 256, 0, s>>>(pass, K, nq0, frac, kv, rho, partial);
+      k_train_pass<<<grid, 256, 0, s>>>(pass, K, nq0, frac, chunk, kv, rho, partial);
       k_train_finish<<<(K + 255) / 256, 256, 0, s>>>(pass, K, nch, f->d_prep, kv, partial, rho, ak, kbin);
     }
-    k_train_bins<<<1, kPropBins, 0, s>>>(K, nq0, kbin, rho, ak, cbin + (size_t)sn * kPropBins,
+    k_train_bins<<<kPropBins + kPropBands, 256, 0, s>>>(K, nq0, kbin, rho, ak, cbin + (size_t)sn * kPropBins,
                                          spec + (size_t)sn * kPropBands);
     CK(cudaGetLastError());
   }
-  return train_fit(f, o, rep, s, t0, S, cbin, spec, wbinf, X, loss, gpart, grad, am, av);
+  return train_fit(f, o, rep, s, t0, S, cbin, spec, wbinf, X, loss, gpart, am, av);
 }
 
 rbmd_status rbmd_force_proposal_params(rbmd_force* f, float* get_host, const float* set_host) {
