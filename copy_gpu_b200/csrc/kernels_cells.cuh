@@ -744,6 +744,10 @@ __global__ void k_frac(int nq, const int* __restrict__ qidx, const double* __res
     for (int d = 0; d < 3; ++d) {
       U[d] = turn32(u[d]);
     }
+template <class R> struct FracT;
+template <> struct FracT<float> { using T = Frac32; };
+template <> struct FracT<double> { using T = Frac64; };
+
     reinterpret_cast<Frac32*>(frac_out)[c] = Frac32{U[0], U[1], U[2], (float)q};
   } else {
     unsigned long long U[3];
