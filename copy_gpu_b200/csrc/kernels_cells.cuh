@@ -724,14 +724,8 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
 // * 2^32) (2^64 for FP64), so integer phases m . U mod 2^32 are exact.  Uncharged atoms add
 // nothing to rho_k or the k-space force and are left out.
 template <class R>
-__global__ void k_frac(int nq, const int* __restrict__ qidx, const double* __restrict__ pos,
-                       const double* __restrict__ charge, const int* __restrict__ rep_of,
-                       const RepDev* __restrict__ reps, void* __restrict__ frac_out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nq) return;
-  const int id = qidx[c];
-  const RepDev& rp = reps[rep_of ? rep_of[id] : 0];
-  const double q = charge[id];
+__device__ __forceinline__ typename FracT<R>::T frac_of(const RepDev& rp, const double* __restrict__ pos,
+                                                        const double* __restrict__ charge, int id) {
   double u[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
