@@ -27,13 +27,11 @@ __device__ __forceinline__ int cell_of_pos(const RepDev& rp, R x, R y, R z) {
 
 // Verlet-skin rebuild flags: rebuild[r] for replica r and rebuild[n_replicas] for "any replica";
 // a replica whose atoms all stayed within skin/2 keeps its cells, slots and list.
-// rebuild (nullable): bin only the atoms of rebuilding replicas.  xref (nullable): the positions of
-// this build, in caller order, so consecutive here (the cell sort would scatter them).
+// rebuild (nullable): bin only the atoms of rebuilding replicas.
 template <class R>
 __global__ void k_bin(int n, const double* __restrict__ pos, const int* __restrict__ rep_of,
                       const RepDev* __restrict__ reps, int* __restrict__ cell_of,
-                      int* __restrict__ cell_count, uint32_t* status, const int* __restrict__ rebuild,
-                      double* __restrict__ xref) {
+                      int* __restrict__ cell_count, uint32_t* status, const int* __restrict__ rebuild) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int r = rep_of ? rep_of[i] : 0;
@@ -41,7 +39,6 @@ __global__ void k_bin(int n, const double* __restrict__ pos, const int* __restri
   const RepDev& rp = reps[r];
   double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
   if (!isfinite(x) || !isfinite(y) || !isfinite(z)) set_flag(status, kFlagNonFinite);
-  if (xref) { xref[3 * i] = x; xref[3 * i + 1] = y; xref[3 * i + 2] = z; }
   int c = cell_of_pos<R>(rp, (R)x, (R)y, (R)z);
   cell_of[i] = c;
   atomicAdd(&cell_count[c], 1);
@@ -172,29 +169,26 @@ __device__ __forceinline__ unsigned long long ord_key(double x) {
 // row of consecutive x cells is ordered by x, which lets the list build skip the candidates
 // beyond the cutoff in x by binary search.  Cells above kMaxCellAtoms keep the scatter order
 // (flagged by the scan).
-// nparts > 1 (cells of many atoms): a cell is shared by nparts warps, each ranking its share of the
-// atoms against all of them (30,000 water atoms fill 216 cells, 54 blocks of one warp per cell).
-constexpr int kSortWarps = 4;   // warps per block of k_cell_sort_gather
+constexpr int kSortWarps = 4;   // cells (one per warp) per block of k_cell_sort_gather
 
 template <class R>
 __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
-    int ncell, int nparts, const int* __restrict__ start, const int* __restrict__ tmp_slot_atom,
+    int ncell, const int* __restrict__ start, const int* __restrict__ tmp_slot_atom,
     const double* __restrict__ pos, const double* __restrict__ charge,
     const int* __restrict__ type, const int* __restrict__ mol, const int* __restrict__ rep_of,
     const RepDev* __restrict__ reps, int* __restrict__ slot_atom, int* __restrict__ atom_slot,
     typename Traits<R>::V4* __restrict__ pos4, void* __restrict__ frac_out,
-    int2* __restrict__ meta, const int* __restrict__ rebuild, int sort_x, const int* __restrict__ cell_rep) {
+    int2* __restrict__ meta, double* __restrict__ xref, const int* __restrict__ rebuild, int sort_x,
+    const int* __restrict__ cell_rep) {
   using Key = decltype(ord_key((R)0));
   __shared__ int ids[kSortWarps][kMaxCellAtoms];
   __shared__ Key keys[kSortWarps][kMaxCellAtoms];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long item = (long long)blockIdx.x * kSortWarps + w;
-  const int cell = (int)(item / nparts), part = (int)(item % nparts);
+  const int cell = blockIdx.x * kSortWarps + w;
   if (cell >= ncell) return;
   if (rebuild && !rebuild[cell_rep ? cell_rep[cell] : 0]) return;
   const int s0 = start[cell], n = start[cell + 1] - s0;
-  const int k0 = (int)((long long)n * part / nparts), k1 = (int)((long long)n * (part + 1) / nparts);
-  if (k0 == k1) return;
+  if (n == 0) return;
   const bool sortable = n <= kMaxCellAtoms;
   if (sortable)
     for (int k = lane; k < n; k += 32) {
@@ -203,7 +197,7 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
       if (sort_x) keys[w][k] = ord_key((R)pos[3 * id]);
     }
   __syncwarp();
-  for (int k = k0 + lane; k < k1; k += 32) {
+  for (int k = lane; k < n; k += 32) {
     int id = sortable ? ids[w][k] : tmp_slot_atom[s0 + k];
     int rank = k;
     if (sortable) {
@@ -223,6 +217,7 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
     atom_slot[id] = slot;
     const double x = pos[3 * id], y = pos[3 * id + 1], z = pos[3 * id + 2];
     const double q = charge ? charge[id] : 0.0;
+    if (xref) { xref[3 * id] = x; xref[3 * id + 1] = y; xref[3 * id + 2] = z; }
     typename Traits<R>::V4 v;
     v.x = (R)x; v.y = (R)y; v.z = (R)z; v.w = (R)q;
     pos4[slot] = v;
@@ -552,10 +547,10 @@ constexpr int kCellBatch = 768;   // candidates whose accept bits are kept befor
 template <class R> struct __align__(16) CellWarpMem {
   struct __align__(16) XY { Pair<R> x, y; } xy[32];   // the atoms' -x and -y, each twice
   Pair<R> z[32];
-  R off[3][27];        // periodic offset of each non-empty stencil cell
+  R off[3][27];        // periodic offset of each stencil cell
   int start[27];       // its first slot
   int code[27];        // its image code
-  int pre[27];         // candidates before it
+  int pre[28];         // candidates before it
   int ent[kCellBatch];                      // list entry of each candidate of the batch
   unsigned word[kCellBatch / 32][32];       // accept bits [32 candidates][atom], first candidate on top
 };
@@ -585,17 +580,21 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
   const int d0 = rp.dims[0], d1 = rp.dims[1], d2n = rp.dims[2];
   const int cl = cell - rp.cell_base;
   const int cx = cl % d0, cy = (cl / d0) % d1, cz = cl / (d0 * d1);
-  // the non-empty stencil cells in walk order: y outermost, then z, then x
-  int cnt = 0, st = 0, dx = 0, dy = 0, dz = 0;
+  // stencil cells in walk order: y outermost, then z, then x
+  int cnt = 0;
   if (lane < 27) {
     const int nbx = cx + lane % 3 - 1, nbz = cz + (lane / 3) % 3 - 1, nby = cy + lane / 9 - 1;
     const int wx = wrap_cell(nbx, d0), wy = wrap_cell(nby, d1), wz = wrap_cell(nbz, d2n);
-    dx = wx - nbx;
-    dy = wy - nby;
-    dz = wz - nbz;
+    const int dx = wx - nbx, dy = wy - nby, dz = wz - nbz;
     const int c = rp.cell_base + wx + wy * d0 + wz * d0 * d1;
-    st = cell_start[c];
+    const int st = cell_start[c];
     cnt = cell_start[c + 1] - st;
+    M.off[0][lane] = mul_rn(Traits<R>::dx(rp, 0), (R)dx);
+    M.off[1][lane] = mul_rn(Traits<R>::dx(rp, 1), (R)dy);
+    M.off[2][lane] = mul_rn(Traits<R>::dx(rp, 2), (R)dz);
+    M.start[lane] = st;
+    M.code[lane] = (dx > 0 ? 1 : (dx < 0 ? 2 : 0)) | ((dy > 0 ? 1 : (dy < 0 ? 2 : 0)) << 2) |
+                   ((dz > 0 ? 1 : (dz < 0 ? 2 : 0)) << 4);
   }
   int incl = cnt;
 #pragma unroll
@@ -603,26 +602,11 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
     const int v = __shfl_up_sync(full, incl, o);
     if (lane >= o) incl += v;
   }
-  const int total = __shfl_sync(full, incl, 31);
-  const unsigned some = __ballot_sync(full, cnt > 0);
-  const int nseg = __popc(some);
-  if (cnt > 0) {
-    const int at = __popc(some & ((1u << lane) - 1u));
-    M.off[0][at] = mul_rn(Traits<R>::dx(rp, 0), (R)dx);
-    M.off[1][at] = mul_rn(Traits<R>::dx(rp, 1), (R)dy);
-    M.off[2][at] = mul_rn(Traits<R>::dx(rp, 2), (R)dz);
-    M.start[at] = st;
-    M.code[at] = (dx > 0 ? 1 : (dx < 0 ? 2 : 0)) | ((dy > 0 ? 1 : (dy < 0 ? 2 : 0)) << 2) |
-                 ((dz > 0 ? 1 : (dz < 0 ? 2 : 0)) << 4);
-    M.pre[at] = incl - cnt;
-  }
-  __syncwarp();
-  // lane l holds the first candidate of segment l + 1, the rest never start
-  const int next_pre = lane + 1 < nseg ? M.pre[lane + 1] : 1 << 30;
+  if (lane < 28) M.pre[lane] = incl - cnt;   // lane 27 (count 0) holds the total
+  const int total = __shfl_sync(full, incl, 27);
   const R d2_lo = (R)1.0e-4;                 // gt_small
   const Pair<R> unit = both<R>(one);
   int4* out = reinterpret_cast<int4*>(nbr);
-  int strays = 0;   // atoms whose own cell is another: after the others
   for (int g0 = a0; g0 < a1; g0 += 32) {
     const int m = min(32, a1 - g0);
     const int i = g0 + min(lane, m - 1);
@@ -649,17 +633,20 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
           const int q = base + 32 * k + 31 - lane;
           px[k] = (R)INFINITY;                 // past the last candidate: never accepted
           py[k] = pz[k] = (R)0;
-          // segments starting at or before q: those before this group of 32, and a mask of the others
-          const int q0 = base + 32 * k, rel = next_pre - q0;
-          const unsigned starts = __reduce_or_sync(full, rel >= 0 && rel < 32 ? 1u << rel : 0u);
-          const int sg = __popc(__ballot_sync(full, rel < 0)) + __popc(starts & (full >> lane));
           if (q < b1) {
-            const int s = M.start[sg] + (q - M.pre[sg]);
+            int lo = 0, hi = 27;               // pre[lo] <= q < pre[hi]
+#pragma unroll
+            for (int b = 0; b < 5; ++b) {
+              const int mid = (lo + hi) >> 1;
+              if (M.pre[mid] <= q) lo = mid;
+              else hi = mid;
+            }
+            const int s = M.start[lo] + (q - M.pre[lo]);
             const V4 pj = pos4[s];
-            px[k] = sub_rn(pj.x, M.off[0][sg]);
-            py[k] = sub_rn(pj.y, M.off[1][sg]);
-            pz[k] = sub_rn(pj.z, M.off[2][sg]);
-            M.ent[q - b0] = (s << kShiftBits) | M.code[sg];
+            px[k] = sub_rn(pj.x, M.off[0][lo]);
+            py[k] = sub_rn(pj.y, M.off[1][lo]);
+            pz[k] = sub_rn(pj.z, M.off[2][lo]);
+            M.ent[q - b0] = (s << kShiftBits) | M.code[lo];
           }
         }
         unsigned word[KC];
@@ -725,18 +712,10 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
         set_flag(status, kFlagListOverflow);
         atomicMax(max_count, idx);
       }
+    } else if (valid) {
+      idx = nlist_thread<R>(i, pi, rp, pos4, cell_start, 1, rc, cap, stride, nbr, false, orig);
+      nlist_finish(i, idx, cap, stride, nbr, count, max_count, status);
     }
-    strays |= __any_sync(full, valid && !mine);
-  }
-  if (!strays) return;
-  for (int i = a0 + lane; i < a1; i += 32) {
-    const V4 pi = pos4[i];
-    if ((int)div_rn(sub_rn(pi.x, Traits<R>::lo(rp, 0)), Traits<R>::dx(rp, 0)) == cx &&
-        (int)div_rn(sub_rn(pi.y, Traits<R>::lo(rp, 1)), Traits<R>::dx(rp, 1)) == cy &&
-        (int)div_rn(sub_rn(pi.z, Traits<R>::lo(rp, 2)), Traits<R>::dx(rp, 2)) == cz)
-      continue;
-    const int idx = nlist_thread<R>(i, pi, rp, pos4, cell_start, 1, rc, cap, stride, nbr, false, orig);
-    nlist_finish(i, idx, cap, stride, nbr, count, max_count, status);
   }
 }
 
@@ -745,8 +724,14 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
 // * 2^32) (2^64 for FP64), so integer phases m . U mod 2^32 are exact.  Uncharged atoms add
 // nothing to rho_k or the k-space force and are left out.
 template <class R>
-__device__ __forceinline__ typename FracT<R>::T frac_of(const RepDev& rp, const double* __restrict__ pos,
-                                                        const double* __restrict__ charge, int id) {
+__global__ void k_frac(int nq, const int* __restrict__ qidx, const double* __restrict__ pos,
+                       const double* __restrict__ charge, const int* __restrict__ rep_of,
+                       const RepDev* __restrict__ reps, void* __restrict__ frac_out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nq) return;
+  const int id = qidx[c];
+  const RepDev& rp = reps[rep_of ? rep_of[id] : 0];
+  const double q = charge[id];
   double u[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -759,10 +744,6 @@ __device__ __forceinline__ typename FracT<R>::T frac_of(const RepDev& rp, const 
     for (int d = 0; d < 3; ++d) {
       U[d] = turn32(u[d]);
     }
-template <class R> struct FracT;
-template <> struct FracT<float> { using T = Frac32; };
-template <> struct FracT<double> { using T = Frac64; };
-
     reinterpret_cast<Frac32*>(frac_out)[c] = Frac32{U[0], U[1], U[2], (float)q};
   } else {
     unsigned long long U[3];

@@ -52,37 +52,22 @@ struct NearParams {
 template <class R> struct KRec;
 template <> struct KRec<float> { using T = KRec32; };
 template <> struct KRec<double> { using T = KRec64; };
-// e^x, 1/sqrt(x) and 1/x by one MUFU operation each.  The flush-to-zero forms leave out the
-// rescaling of denormals, which the arguments here never are: x = -alpha d^2 above -100, d^2 > 1e-4.
-__device__ __forceinline__ float exp_r(float x) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.44269504088896340736f));
-  return r;
-}
+template <class R> struct FracT;
+template <> struct FracT<float> { using T = Frac32; };
+template <> struct FracT<double> { using T = Frac64; };
+
+__device__ __forceinline__ float exp_r(float x) { return __expf(x); }
 __device__ __forceinline__ double exp_r(double x) { return exp(x); }
-__device__ __forceinline__ float rsqrt_r(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
+__device__ __forceinline__ float rsqrt_r(float x) { return rsqrtf(x); }
 __device__ __forceinline__ float sqrt_r(float x) { return sqrtf(x); }
 __device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
 __device__ __forceinline__ double rsqrt_r(double x) { return 1.0 / sqrt(x); }
-
-// approximate reciprocal (one MUFU op, about 1 ulp): the pair terms carry a 1e-5 budget
-__device__ __forceinline__ float rcp_r(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 
 // erfc(x) for x >= 0 given e = exp(-x^2).  FP32: Abramowitz & Stegun, Handbook of Mathematical
 // Functions, eq. 7.1.26 (rational approximation in t = 1/(1 + p x), |error| <= 1.5e-7), which
 // reuses the Gaussian factor the real-space force needs anyway.  FP64: the library erfc.
 __device__ __forceinline__ float erfc_shared(float x, float e) {
-  // 1 / d to within an ulp: the MUFU reciprocal and one Newton step (the correctly rounded one takes
-  // a dozen instructions; both leave the formula's 1.5e-7 as it is)
-  const float d = fmaf(0.3275911f, x, 1.0f), t0 = rcp_r(d), t = fmaf(t0, fmaf(-d, t0, 1.0f), t0);
+  const float t = __frcp_rn(fmaf(0.3275911f, x, 1.0f));
   float poly = fmaf(1.061405429f, t, -1.453152027f);
   poly = fmaf(poly, t, 1.421413741f);
   poly = fmaf(poly, t, -0.284496736f);
@@ -98,12 +83,12 @@ template <class R> __host__ __device__ __forceinline__ R sig6(const LJTable& t, 
 template <> __host__ __device__ __forceinline__ float sig6<float>(const LJTable& t, int k) { return t.sig6_f[k]; }
 template <> __host__ __device__ __forceinline__ double sig6<double>(const LJTable& t, int k) { return t.sig6_d[k]; }
 
-// RBE force terms of one atom over the k records sub, sub + G, .. < P of `kr` (shared or global memory).
-template <class R, int G>
+// RBE force terms of one atom over k records [0, P) of `kr` (shared or global memory).
+template <class R>
 __device__ __forceinline__ void rbe_terms(const typename FracT<R>::T& fr, const typename KRec<R>::T* kr,
-                                          int P, int sub, R& ax, R& ay, R& az) {
+                                          int P, R& ax, R& ay, R& az) {
 #pragma unroll 4
-  for (int l = sub; l < P; l += G) {
+  for (int l = 0; l < P; ++l) {
     const typename KRec<R>::T k = kr[l];
     R s, c;
     if constexpr (sizeof(R) == 4) {
@@ -141,6 +126,12 @@ __device__ __forceinline__ void min_image(R& q0, R& q1, R& q2, const R* box) {
   if (fabs(q2) > box[2] * (R)0.5) q2 -= (q2 > 0 ? box[2] : -box[2]);
 }
 
+// approximate reciprocal (one MUFU op, about 1 ulp): the pair terms carry a 1e-5 budget
+__device__ __forceinline__ float rcp_r(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ double rcp_r(double x) { return 1.0 / x; }
 
 // Near force of one slot per thread over its list row.
@@ -302,18 +293,15 @@ __global__ void __launch_bounds__(256) k_near_force(
 // Pair physics as k_near_force: ComputeNearForceVerletWorklet / ComputeLJForceVerletWorklet
 // (rbmd/framework/run/worklet/RunWorklet.cpp:170-303), ExecForceFunction::ComputeLJForce and
 // ComputeNearEnergyForce (rbmd/framework/forceFunction/ExecForceFunction.h:74-140).
-// G > 1: G lanes per atom for systems with too few atoms to fill the chip; lane s takes the chunks
-// s, s + G, .. and the lanes' sums are combined in FP64 by a fixed butterfly.
-// FP32 is held to 64 registers (32 warps per SM; 74 without): 1,000,000 atoms 191 -> about 183 us.
-template <class R, bool COUL, int MI, bool ENERGY, int G>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_lean(
+template <class R, bool COUL, int MI, bool ENERGY>
+__global__ void __launch_bounds__(256) k_near_lean(
     NearParams prm, R a24, R s6, R d2_max, const typename Traits<R>::V4* __restrict__ pos4,
     const int4* __restrict__ nbr4, const int* __restrict__ count, const RepDev* __restrict__ reps,
     const int* __restrict__ rep_of_slot, const int* __restrict__ slot_atom, double* __restrict__ force,
     double* __restrict__ energy_slot, uint32_t* status) {
   static_assert((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0, "k_near_lean: no per-pair minimum image, no weights");
   using V4 = typename Traits<R>::V4;
-  const int gid = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G), sub = threadIdx.x % G;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = gid < prm.n;   // lanes past the end run along with an empty row
   const int i = active ? gid : prm.n - 1;
   const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
@@ -322,21 +310,21 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_lean(
   const R sa = (R)prm.sqrt_alpha, aa = (R)prm.alpha, c2 = (R)prm.two_sqrt_alpha_over_sqrt_pi;
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
-  const int nch = active ? (min(count[i], prm.cap) + 3) >> 2 : 0;   // chunks of the row
-  const int last = __reduce_max_sync(0xffffffffu, nch);
+  const int cnt = active ? min(count[i], prm.cap) : 0;
+  const int last = __reduce_max_sync(0xffffffffu, cnt);
   const int self = i << kShiftBits;
   const int4 idle = make_int4(self, self, self, self);
   // 24 eps (2 s6 u - 1) s6 u / d^2 with u = d^-6 as (ka u - kb) d^-8
   const Pair<R> ka = both<R>((R)2 * a24 * s6 * s6), kb = both<R>(-a24 * s6);
   Acc3<R> F;
   R e_lj = 0, e_coul = 0;
-  const size_t st = (size_t)prm.stride * G;
-  const int4* row = nbr4 + (size_t)prm.stride * sub + i;
-  int4 e = sub < nch ? __ldg(row) : idle;
-  int4 e_nxt = sub + G < nch ? __ldg(row + st) : idle;
+  const int4* row = nbr4 + i;
+  const size_t st = (size_t)prm.stride;
+  int4 e = cnt > 0 ? __ldg(row) : idle;
+  int4 e_nxt = cnt > 4 ? __ldg(row + st) : idle;
   row += 2 * st;
   V4 pj[4] = {pos4[e.x >> kShiftBits], pos4[e.y >> kShiftBits], pos4[e.z >> kShiftBits], pos4[e.w >> kShiftBits]};
-  for (int c = sub; c - sub < last; c += G, row += st) {
+  for (int p = 0; p < last; p += 4, row += st) {
     if (__any_sync(0xffffffffu, ((e.x | e.y | e.z | e.w) & 63) != 0)) {   // p_j - PeriodicCoordOffset
       const int ee[4] = {e.x, e.y, e.z, e.w};
       const R w0 = Traits<R>::wrap(rp, 0), w1 = Traits<R>::wrap(rp, 1), w2 = Traits<R>::wrap(rp, 2);
@@ -406,20 +394,16 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_lean(
   force[3 * id + 1] = Fd[1];
   force[3 * id + 2] = Fd[2];
   if (ENERGY) {
-    energy_slot[2 * i] = 0.5 * el;
-    energy_slot[2 * i + 1] = 0.5 * ec;
+    energy_slot[2 * i] = 0.5 * (double)e_lj;
+    energy_slot[2 * i + 1] = 0.5 * (double)e_coul;
   }
 }
 
-// Near force with G lanes per atom (G = 4 .. 32) for systems with few atoms or long lists
+// Near force with G lanes per atom (G = 4 .. 32) for systems with few atoms and long lists
 // (water at 10 A: ~550 neighbours, 30,000 atoms), where one thread per atom leaves most of the
-// GPU idle.  Lane s of an atom's group takes the chunks s, s + G, .. of four list entries: one
-// 16-byte load per chunk, the next chunk's entries and the four positions (and, with types or
-// molecules, records) of the current one in flight together, the image offsets decoded in one
-// branch per chunk.  The filler entries of the last chunk hold the slot itself, at distance 0,
-// which no predicate accepts.  The pair terms are those of k_near_force (same predicates and
-// arithmetic); each lane sums the four forces of a chunk and folds them into a two-float
-// accumulator, and the group combines its G partial sums in FP64 with a fixed butterfly, so the
+// GPU idle.  Lane s of an atom's group takes list entries s, s + G, ...; the pair terms are
+// those of k_near_force (same predicates and arithmetic); each lane accumulates in a two-float
+// accumulator and the group combines its G partial sums in FP64 with a fixed butterfly, so the
 // result does not depend on scheduling.
 template <class R, bool COUL, int MI, int G>
 __global__ void __launch_bounds__(256) k_near_force_group(
@@ -439,7 +423,7 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   const bool MOLEC = prm.molecular != 0;
   constexpr bool SPW = (MI & kMiSpecial) != 0;
   const bool ENERGY = energy_slot != nullptr;
-  const int gid = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) / G);
+  const int gid = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G);
   const int sub = threadIdx.x % G;
   const bool active = gid < prm.n;   // inactive groups still join the shuffles below
   const int i = active ? gid : prm.n - 1;
@@ -449,93 +433,85 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   const int2 mi = typed ? meta[i] : make_int2(0, 0);
   const R rc = (R)prm.rc;
   const R cut2 = rc * rc;
+  const R box[3] = {Traits<R>::box(rp, 0), Traits<R>::box(rp, 1), Traits<R>::box(rp, 2)};
+  const R wrap[3] = {Traits<R>::wrap(rp, 0), Traits<R>::wrap(rp, 1), Traits<R>::wrap(rp, 2)};
   const R sa = (R)prm.sqrt_alpha, aa = (R)prm.alpha, c2 = (R)prm.two_sqrt_alpha_over_sqrt_pi;
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
   const int trow = prm.ntypes > 1 ? mi.x * prm.ntypes : 0;
-  const int4* nbr4 = reinterpret_cast<const int4*>(nbr) + i;
-  const int nch = active ? (min(count[i], prm.cap) + 3) >> 2 : 0;
-  const int last = __reduce_max_sync(0xffffffffu, nch);
-  const int self = i << kShiftBits;
-  const int4 idle = make_int4(self, self, self, self);
-  Acc3<R> acc;
+  Acc<R> fx, fy, fz;
+  R gx = 0, gy = 0, gz = 0;
   R e_lj = 0, e_coul = 0;
-  int4 e4 = sub < nch ? __ldg(nbr4 + (size_t)sub * prm.stride) : idle;
-  for (int c = sub; c - sub < last; c += G) {
-    const int ee[4] = {e4.x, e4.y, e4.z, e4.w};
-    V4 pj[4];
-    int2 mj[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) pj[k] = pos4[ee[k] >> kShiftBits];
-    if (typed)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) mj[k] = meta[ee[k] >> kShiftBits];
-    e4 = c + G < nch ? __ldg(nbr4 + (size_t)(c + G) * prm.stride) : idle;
-    if (__any_sync(0xffffffffu, ((ee[0] | ee[1] | ee[2] | ee[3]) & 63) != 0)) {   // p_j - PeriodicCoordOffset
-      const R w0 = Traits<R>::wrap(rp, 0), w1 = Traits<R>::wrap(rp, 1), w2 = Traits<R>::wrap(rp, 2);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int k0 = ee[k] & 3, k1 = (ee[k] >> 2) & 3, k2 = (ee[k] >> 4) & 3;
-        pj[k].x -= k0 == 1 ? w0 : (k0 == 2 ? -w0 : (R)0);
-        pj[k].y -= k1 == 1 ? w1 : (k1 == 2 ? -w1 : (R)0);
-        pj[k].z -= k2 == 1 ? w2 : (k2 == 2 ? -w2 : (R)0);
-      }
+  const int cnt = active ? min(count[i], prm.cap) : 0;
+  int k = 0;
+  for (int p = sub; p < cnt; p += G, ++k) {
+    const int e = __ldg(nbr + nbr_at(p, i, prm.stride));
+    const V4 pj = pos4[e >> kShiftBits];
+    R px = pj.x, py = pj.y, pz = pj.z;
+    if (e & 63) {
+      const int c0 = e & 3, c1 = (e >> 2) & 3, c2b = (e >> 4) & 3;
+      px = px - (c0 == 1 ? wrap[0] : (c0 == 2 ? -wrap[0] : (R)0));
+      py = py - (c1 == 1 ? wrap[1] : (c1 == 2 ? -wrap[1] : (R)0));
+      pz = pz - (c2b == 1 ? wrap[2] : (c2b == 2 ? -wrap[2] : (R)0));
     }
-    R gx = 0, gy = 0, gz = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const R r0 = pj[k].x - pi.x, r1 = pj[k].y - pi.y, r2 = pj[k].z - pi.z;
-      const R d2 = r0 * r0 + r1 * r1 + r2 * r2;
-      if ((MI & 3) == kMiAll && !((prm.orig ? cut2 - d2 > (R)0 : cut2 - d2 > (R)1.0e-4) && d2 > (R)1.0e-4)) continue;
-      R f = 0;
-      if (COUL) {
-        const R qq = qi * pj[k].w;
-        if (qq != (R)0) {
-          const R inv = rsqrt_r(d2);
-          const R dis = d2 * inv;
-          if (dis < rc && dis > (R)0.01) {
-            const R ex = exp_r(-aa * d2);
-            const R erfcv = erfc_shared(sa * dis, ex);
-            const R g = (erfcv * inv + c2 * ex) * inv;
-            f = -qq * g * inv * cs;
-            if (ENERGY) e_coul += qq * erfcv * inv * cs;
-          }
-        }
-      }
-      R fl0 = 0, fl1 = 0, fl2 = 0;
-      bool same = false;
-      int tj = 0;
-      R wsp = (R)1;   // special-bond LJ weight (molecular == 2: meta.y is the bond-graph component)
-      if (typed) {
-        same = MOLEC && (mj[k].y == mi.y);
-        tj = prm.ntypes > 1 ? mj[k].x : 0;
-        if (SPW && same) {
-          wsp = special_weight<R>(prm.sp, slot_atom[i], slot_atom[ee[k] >> kShiftBits]);
-          same = false;
-        }
-      }
-      if (!same) {
-        R q0 = r0, q1 = r1, q2 = r2;
-        R dl2 = d2;
-        if ((MI & 3) == kMiLJ) {
-          const R box[3] = {Traits<R>::box(rp, 0), Traits<R>::box(rp, 1), Traits<R>::box(rp, 2)};
-          min_image(q0, q1, q2, box);
-          dl2 = q0 * q0 + q1 * q1 + q2 * q2;
-        }
-        if (dl2 < cut2 && dl2 > (R)0.0001) {
-          const R inv2 = rcp_r(dl2);
-          const R sd6 = lj_s6[trow + tj] * inv2 * inv2 * inv2;
-          const R a24 = lj_a[trow + tj];
-          R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2;
-          if (SPW) scal *= wsp;
-          fl0 = scal * q0; fl1 = scal * q1; fl2 = scal * q2;
-          if (ENERGY) e_lj += (SPW ? wsp : (R)1) * (-a24 / (R)6 * (sd6 - (R)1) * sd6);
+    const R r0 = px - pi.x, r1 = py - pi.y, r2 = pz - pi.z;
+    const R d2 = r0 * r0 + r1 * r1 + r2 * r2;
+    if ((MI & 3) == kMiAll && !((prm.orig ? cut2 - d2 > (R)0 : cut2 - d2 > (R)1.0e-4) && d2 > (R)1.0e-4)) continue;
+    R f = 0;
+    if (COUL) {
+      const R qq = qi * pj.w;
+      if (qq != (R)0) {
+        const R inv = rsqrt_r(d2);
+        const R dis = d2 * inv;
+        if (dis < rc && dis > (R)0.01) {
+          const R ex = exp_r(-aa * d2);
+          const R erfcv = erfc_shared(sa * dis, ex);
+          const R g = (erfcv * inv + c2 * ex) * inv;
+          f = -qq * g * inv * cs;
+          if (ENERGY) e_coul += qq * erfcv * inv * cs;
         }
       }
     }
-    acc.add(gx, gy, gz);
+    R fl0 = 0, fl1 = 0, fl2 = 0;
+    bool same = false;
+    int tj = 0;
+    R wsp = (R)1;   // special-bond LJ weight (molecular == 2: meta.y is the bond-graph component)
+    if (typed) {
+      const int2 mj = meta[e >> kShiftBits];
+      same = MOLEC && (mj.y == mi.y);
+      tj = prm.ntypes > 1 ? mj.x : 0;
+      if (SPW && same) {
+        wsp = special_weight<R>(prm.sp, slot_atom[i], slot_atom[e >> kShiftBits]);
+        same = false;
+      }
+    }
+    if (!same) {
+      R q0 = r0, q1 = r1, q2 = r2;
+      R dl2 = d2;
+      if ((MI & 3) == kMiLJ) {
+        min_image(q0, q1, q2, box);
+        dl2 = q0 * q0 + q1 * q1 + q2 * q2;
+      }
+      if (dl2 < cut2 && dl2 > (R)0.0001) {
+        const R inv2 = rcp_r(dl2);
+        const R sd6 = lj_s6[trow + tj] * inv2 * inv2 * inv2;
+        const R a24 = lj_a[trow + tj];
+        R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2;
+        if (SPW) scal *= wsp;
+        fl0 = scal * q0; fl1 = scal * q1; fl2 = scal * q2;
+        if (ENERGY) e_lj += (SPW ? wsp : (R)1) * (-a24 / (R)6 * (sd6 - (R)1) * sd6);
+      }
+    }
+    gx += f * r0 + fl0;
+    gy += f * r1 + fl1;
+    gz += f * r2 + fl2;
+    if ((k & 3) == 3) {
+      fx.add(gx); fy.add(gy); fz.add(gz);
+      gx = gy = gz = 0;
+    }
   }
-  double F[3] = {acc.vx(), acc.vy(), acc.vz()};
+  fx.add(gx); fy.add(gy); fz.add(gz);
+  double F[3] = {fx.value(), fy.value(), fz.value()};
   double el = (double)e_lj, ec = (double)e_coul;
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) {
@@ -544,9 +520,6 @@ __global__ void __launch_bounds__(256) k_near_force_group(
     F[2] += __shfl_xor_sync(0xffffffffu, F[2], o);
     el += __shfl_xor_sync(0xffffffffu, el, o);
     ec += __shfl_xor_sync(0xffffffffu, ec, o);
-      gx += f * r0 + fl0;
-      gy += f * r1 + fl1;
-      gz += f * r2 + fl2;
   }
   if (!active || sub != 0) return;
   if (!isfinite(F[0]) || !isfinite(F[1]) || !isfinite(F[2])) set_flag(status, kFlagNonFinite);
@@ -560,18 +533,14 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   }
 }
 
-// RBE k-space force, G lanes per charged atom (compact index c, caller id qidx[c]):
+// RBE k-space force, one thread per charged atom (compact index c, caller id qidx[c]):
 // F_i = q_i sum_l w_l k_l (cos(k_l.r_i) Im rho_l - sin(k_l.r_i) Re rho_l)
 // (ComputeNewRBEForceWorklet, RunWorklet.cpp:1508-1548; S/P and qqr2e are folded into the
 // records).  The block stages the k records of the replicas its atoms belong to in shared
 // memory (two 16-byte broadcast loads per sample) when they fit.  Runs on the k-space stream
 // concurrently with the near pass and writes far_force[c]; k_add_far folds it into the force.
-// Bound by MUFU (two per term) when the chip is full; the lanes of an atom take every G-th sample and
-// are summed in FP64 by a fixed butterfly, so that few charged atoms still fill it (launch_rbe_force).
-constexpr int kRbeThreads = 128;
-
-template <class R, int G>
-__global__ void __launch_bounds__(kRbeThreads) k_rbe_force(int nq, int kstage, const int* __restrict__ qidx,
+template <class R>
+__global__ void __launch_bounds__(128) k_rbe_force(int nq, int kstage, const int* __restrict__ qidx,
                                                    const typename FracT<R>::T* __restrict__ frac,
                                                    const typename KRec<R>::T* __restrict__ krec,
                                                    const RepDev* __restrict__ reps,
@@ -579,11 +548,9 @@ __global__ void __launch_bounds__(kRbeThreads) k_rbe_force(int nq, int kstage, c
                                                    double* __restrict__ far_force) {
   extern __shared__ __align__(16) unsigned char ksm_raw[];
   typename KRec<R>::T* ksm = reinterpret_cast<typename KRec<R>::T*>(ksm_raw);
-  const int c0 = blockIdx.x * (kRbeThreads / G);
-  const int sub = threadIdx.x % G;
-  const int last = min(nq, c0 + kRbeThreads / G) - 1;
-  const int c = min(c0 + (int)threadIdx.x / G, last);   // lanes past the end repeat the last atom
-  const bool active = c0 + (int)threadIdx.x / G < nq;
+  const int c0 = blockIdx.x * blockDim.x;
+  const int c = c0 + threadIdx.x;
+  const int last = min(nq, c0 + (int)blockDim.x) - 1;
   const int ra = rep_of ? rep_of[qidx[c0]] : 0;
   const int rb = rep_of ? rep_of[qidx[last]] : 0;
   const int kfirst = reps[ra].k_begin;
@@ -596,21 +563,16 @@ __global__ void __launch_bounds__(kRbeThreads) k_rbe_force(int nq, int kstage, c
     for (int t = threadIdx.x; t < nwords; t += blockDim.x) dst[t] = src[t];
   }
   __syncthreads();
+  if (c >= nq) return;
   const RepDev& rp = reps[rep_of ? rep_of[qidx[c]] : 0];
   const typename FracT<R>::T fr = frac[c];
   R ax = 0, ay = 0, az = 0;
-  if (staged) rbe_terms<R, G>(fr, ksm + (rp.k_begin - kfirst), rp.P, sub, ax, ay, az);
-  else rbe_terms<R, G>(fr, krec + rp.k_begin, rp.P, sub, ax, ay, az);
-  double F[3] = {(double)ax, (double)ay, (double)az};
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) F[d] += __shfl_xor_sync(0xffffffffu, F[d], o);
-  if (!active || sub != 0) return;
+  if (staged) rbe_terms<R>(fr, ksm + (rp.k_begin - kfirst), rp.P, ax, ay, az);
+  else rbe_terms<R>(fr, krec + rp.k_begin, rp.P, ax, ay, az);
   const double q = (double)fr.q;
-  far_force[3 * c] = q * F[0];
-  far_force[3 * c + 1] = q * F[1];
-  far_force[3 * c + 2] = q * F[2];
+  far_force[3 * c] = q * (double)ax;
+  far_force[3 * c + 1] = q * (double)ay;
+  far_force[3 * c + 2] = q * (double)az;
 }
 
 __global__ void k_add_far(int nq, const int* __restrict__ qidx, const double* __restrict__ far_force,
@@ -637,61 +599,15 @@ struct RhoItem { int atom_begin, atom_end, k_first, k_count; };
 constexpr int kRhoStage = 256;
 
 template <class R, int KL>
-__global__ void __launch_bounds__(256) k_rho_lanes(
-    const RhoItem* __restrict__ items, int P, const int* __restrict__ qidx, const double* __restrict__ pos,
-    const double* __restrict__ charge, const RepDev* __restrict__ reps, const RhoRep* __restrict__ rr,
-    typename FracT<R>::T* __restrict__ frac, R* partial, int ktile, int* __restrict__ rep_done, RhoOut<R> o) {
+__global__ void __launch_bounds__(256) k_rho_lanes(const RhoItem* __restrict__ items,
+                                                   const typename FracT<R>::T* __restrict__ frac,
+                                                   const typename KRec<R>::T* __restrict__ krec,
+                                                   R* __restrict__ partial, int ktile) {
   using FT = typename FracT<R>::T;
   __shared__ FT stage[kRhoStage];
-// Per-replica reduction layout: items are ordered (replica, chunk, tile); replica r's partials
-// for tile t and chunk c sit at item_base_r + c * ntiles_r + t.
-struct RhoRep { int item_base, ntiles, nchunks, pad; };
-
-// What a finished structure factor fills in.
-template <class R> struct RhoOut {
-  const double* weights;           // importance weights (nullable)
-  double qqr2e;
-  typename KRec<R>::T* krec;
-  double2* rho;
-  double* ek;
-};
-
-// Sample l of a replica from its summed partials: undo the half-turn phase convention (rho = -sum)
-// and fill the force coefficients of the k record, rho, and the k-space energy estimate
-// (S/P) qqr2e w_l (2 pi / V) |rho_l|^2 / k_l^2.
-template <class R>
-__device__ __forceinline__ void rho_record(const RepDev& rp, int l, double re, double im, const RhoOut<R>& o) {
-  const int g = rp.k_begin + l;
-  typename KRec<R>::T k = o.krec[g];
-  re = -re;
-  im = -im;
-  const double twopi = 6.283185307179586476925;
-  const double kx = twopi * k.mx / rp.box_d[0], ky = twopi * k.my / rp.box_d[1],
-               kz = twopi * k.mz / rp.box_d[2];
-  const double k2 = kx * kx + ky * ky + kz * kz;
-  const double wgt = o.weights ? o.weights[g] : 1.0;
-  // F_i = q_i (S/P) qqr2e sum_l wgt (-4 pi /(V k^2)) k (cos Im - sin Re); the kernel evaluates
-  // the angle shifted by half a turn, which flips cos and sin: store -w.
-  const double w0 = -(rp.S / rp.P) * o.qqr2e * wgt * (-4.0 * 3.14159265358979323846 / (rp.volume * k2));
-  k.wx = (decltype(k.wx))(w0 * kx);
-  k.wy = (decltype(k.wy))(w0 * ky);
-  k.wz = (decltype(k.wz))(w0 * kz);
-  k.re = (decltype(k.re))re;
-  k.im = (decltype(k.im))im;
-  o.krec[g] = k;
-  o.rho[g] = make_double2(re, im);
-  o.ek[g] = (rp.S / rp.P) * o.qqr2e * wgt * (2.0 * 3.14159265358979323846 / rp.volume) *
-                (re * re + im * im) / k2;
-}
-
   const RhoItem it = items[blockIdx.x];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   using MT = typename std::conditional<sizeof(R) == 4, uint32_t, unsigned long long>::type;
-// The fixed-point coordinates are formed while staging (k tile 0 also writes them for k_rbe_force).
-// rep_done: with few chunks per replica the block that finishes a replica's last item sums its
-// partials in chunk order and fills the records (kFusedChunks); otherwise k_rho_finish does.
-constexpr int kFusedChunks = 32;
-
   MT mx[KL], my[KL], mz[KL];
   R re[KL], im[KL];
   int kk[KL];
@@ -699,12 +615,7 @@ constexpr int kFusedChunks = 32;
 #pragma unroll
   for (int j = 0; j < KL; ++j) {
     kk[j] = w * 32 * KL + j * 32 + lane;
-  __shared__ int last;
     const bool ok = kk[j] < it.k_count;
-  const int r = it.k_first / P;   // replicas hold P samples each
-  const RepDev& rp = reps[r];
-  const bool first_tile = it.k_first == rp.k_begin;
-  const typename KRec<R>::T* krec = o.krec;
     any |= ok;
     const typename KRec<R>::T k = ok ? krec[it.k_first + kk[j]] : typename KRec<R>::T{};
     mx[j] = (MT)(long long)k.mx;
@@ -717,11 +628,7 @@ constexpr int kFusedChunks = 32;
   for (int base = it.atom_begin; base < it.atom_end; base += kRhoStage) {
     const int cnt = min(kRhoStage, it.atom_end - base);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-      const FT f = frac_of<R>(rp, pos, charge, qidx[base + t]);
-      stage[t] = f;
-      if (first_tile) frac[base + t] = f;
-    }
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x) stage[t] = frac[base + t];
     __syncthreads();
     if (!warp_any) continue;
 #pragma unroll 4
@@ -745,62 +652,61 @@ constexpr int kFusedChunks = 32;
     }
 }
 
-// Sum of the chunk partials of 32 consecutive k samples of one tile per block: lane = sample, so a
-// warp reads 32 consecutive partials, warp w takes the chunks w, w + warps, .. (FP64) and the warps
-// are added in order through shared memory (deterministic).
-// (One warp per sample read one 8-byte partial per 32-byte sector: 12.4 us at 390 chunks, 35 us for
-// 512 replicas of 100 samples.)
-constexpr int kFinishWarps = 16;   // at most; the launch uses as many as the longest chunk list needs
+// Per-replica reduction layout: items are ordered (replica, chunk, tile); replica r's partials
+// for tile t and chunk c sit at item_base_r + c * ntiles_r + t.
+struct RhoRep { int item_base, ntiles, nchunks, pad; };
 
-  if (!rep_done) return;
-  __threadfence();   // the partials before the count
-  __syncthreads();
-  const RhoRep q = rr[r];
-  if (threadIdx.x == 0) last = atomicAdd(rep_done + r, 1) == q.nchunks * q.ntiles - 1;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();   // the count before the other blocks' partials
-  for (int l = threadIdx.x; l < P; l += blockDim.x) {
-    const int tile = l / ktile, k = l % ktile;
-    double sr = 0, si = 0;
-#pragma unroll 4
-    for (int c = 0; c < q.nchunks; ++c) {
-      const size_t at = (((size_t)q.item_base + (size_t)c * q.ntiles + tile) * ktile + k) * 2;
-      sr += (double)__ldcg(partial + at);
-      si += (double)__ldcg(partial + at + 1);
-    }
-    rho_record<R>(rp, l, sr, si, o);
-  }
-  if (threadIdx.x == 0) rep_done[r] = 0;
+// One warp per k sample: lanes sum the chunk partials in a fixed strided order (FP64) and a
+// butterfly combines them (deterministic); then undo the half-turn phase convention
+// (rho = -sum) and fill the force coefficients of the k record.
+// k-space energy estimate per replica: (S/P) qqr2e sum_l w_l (2 pi / V) |rho_l|^2 / k_l^2.
 template <class R>
-__global__ void __launch_bounds__(32 * kFinishWarps) k_rho_finish(
-    int nrep, int groups, int P, int ktile, const RhoRep* __restrict__ rr, const RepDev* __restrict__ reps,
-    const R* __restrict__ partial, RhoOut<R> o) {
-  __shared__ double sre[kFinishWarps][32], sim[kFinishWarps][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int r = blockIdx.x / groups;               // groups = ceil(P / 32) blocks per replica
-  const int l = (blockIdx.x % groups) * 32 + lane;
+__global__ void k_rho_finish(int nk_total, int ktile, const int* __restrict__ krep,
+                             const RhoRep* __restrict__ rr, const RepDev* __restrict__ reps,
+                             const R* __restrict__ partial, const double* __restrict__ weights,
+                             double qqr2e, typename KRec<R>::T* __restrict__ krec,
+                             double2* __restrict__ rho_out, double* __restrict__ ek_out) {
+  const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (g >= nk_total) return;
+  const int r = krep[g];
   const RepDev& rp = reps[r];
   const RhoRep q = rr[r];
-  const int tile = l / ktile, kk = l % ktile;      // ktile is a multiple of 32: one tile per block
+  const int l = g - rp.k_begin;
+  const int tile = l / ktile, kk = l % ktile;
   double re = 0, im = 0;
-  if (l < P) {
-#pragma unroll 4
-    for (int c = w; c < q.nchunks; c += nw) {
-      const size_t at = (((size_t)q.item_base + (size_t)c * q.ntiles + tile) * ktile + kk) * 2;
-      re += (double)partial[at];
-      im += (double)partial[at + 1];
-    }
+  for (int c = lane; c < q.nchunks; c += 32) {
+    const size_t item = (size_t)q.item_base + (size_t)c * q.ntiles + tile;
+    re += (double)partial[(item * ktile + kk) * 2];
+    im += (double)partial[(item * ktile + kk) * 2 + 1];
   }
-  sre[w][lane] = re;
-  sim[w][lane] = im;
-  __syncthreads();
-  if (w != 0 || l >= P) return;
-  for (int k = 1; k < nw; ++k) {
-    re += sre[k][lane];
-    im += sim[k][lane];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    re += __shfl_xor_sync(0xffffffffu, re, o);
+    im += __shfl_xor_sync(0xffffffffu, im, o);
   }
-  rho_record<R>(rp, l, re, im, o);
+  if (lane != 0) return;
+  typename KRec<R>::T k = krec[g];
+  re = -re;
+  im = -im;
+  const double twopi = 6.283185307179586476925;
+  const double kx = twopi * k.mx / rp.box_d[0], ky = twopi * k.my / rp.box_d[1],
+               kz = twopi * k.mz / rp.box_d[2];
+  const double k2 = kx * kx + ky * ky + kz * kz;
+  const double wgt = weights ? weights[g] : 1.0;
+  // F_i = q_i (S/P) qqr2e sum_l wgt (-4 pi /(V k^2)) k (cos Im - sin Re); the kernel evaluates
+  // the angle shifted by half a turn, which flips cos and sin: store -w.
+  const double w = -(rp.S / rp.P) * qqr2e * wgt * (-4.0 * 3.14159265358979323846 / (rp.volume * k2));
+  k.wx = (decltype(k.wx))(w * kx);
+  k.wy = (decltype(k.wy))(w * ky);
+  k.wz = (decltype(k.wz))(w * kz);
+  k.re = (decltype(k.re))re;
+  k.im = (decltype(k.im))im;
+  krec[g] = k;
+  if (rho_out) rho_out[g] = make_double2(re, im);
+  if (ek_out)
+    ek_out[g] = (rp.S / rp.P) * qqr2e * wgt * (2.0 * 3.14159265358979323846 / rp.volume) *
+                (re * re + im * im) / k2;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1125,7 +1031,6 @@ __global__ void __launch_bounds__(128) k_eam_force(int n, int stride, int cap, d
       // pair vector p_i - p_j' (the sign for which F = -grad E, as LAMMPS' pair_eam and the
       // reference's RBL pass, RunWorklet.cpp:1180); ref_sign: the reference's Verlet pass uses
       // MinDistanceVec(p_j, p_i) (RunWorklet.cpp:402), which reverses the force
-  const float4* rows;   // value rows (c3, c4, c5, c6) of rho(r) [nr + 1], then of z2(r) [nr + 1]
       R v = ref_sign ? (pjv[d] - off) - piv[d] : piv[d] - (pjv[d] - off);
       if (MI) v -= box[d] * rint(v * ibox[d]);
       r[d] = v;
@@ -1165,175 +1070,3 @@ __global__ void __launch_bounds__(128) k_eam_force(int n, int stride, int cap, d
 }
 
 }  // namespace rbmd
-// EAM passes in FP32 with the spline tables in shared memory, for tables whose value rows fit
-// (launch_eam).  The per-pair work is a gather of 16-byte spline rows at random indexes: from L1 it
-// takes a tag lookup per lane, from shared memory about 11 cycles a warp, so one block per SM copies
-// the rows once and walks the atoms.  Rows hold the value polynomial alone, (c3, c4, c5, c6) of
-// rho(r) and of z2(r): the derivative is (3 c3 p^2 + 2 c4 p + c5) / dr, which the seven-coefficient
-// rows store rounded (their c0..c2).  G lanes per atom share a row of the list, lane s taking the
-// chunks s, s + G, .. of four entries (the last chunk is filled with the slot itself, which the
-// predicate 0.01 < r^2 < rc^2 refuses); each term goes into a two-float accumulator, the lanes'
-// sums are combined in FP64 by a fixed butterfly.  Pass 1 also writes (x, y, z, F'(rho)) per slot, so
-// that pass 2 needs one gather per neighbour.  Pair physics as k_eam_fp and k_eam_force.
-constexpr int kEamThreads = 1024;
-
-template <bool MI>
-__device__ __forceinline__ void eam_vec(const float4& pi, const float4& pj, int e, const float* wrap, const float* box,
-                                        const float* ibox, float* r) {
-  r[0] = pj.x;
-  r[1] = pj.y;
-  r[2] = pj.z;
-  if ((e & 63) != 0) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const int cd = (e >> (2 * d)) & 3;
-      r[d] -= cd == 1 ? wrap[d] : (cd == 2 ? -wrap[d] : 0.f);
-    }
-  }
-  r[0] = pi.x - r[0];
-  r[1] = pi.y - r[1];
-  r[2] = pi.z - r[2];
-  if (MI) {   // MinDistanceVec
-#pragma unroll
-    for (int d = 0; d < 3; ++d) r[d] -= box[d] * rint(r[d] * ibox[d]);
-  }
-}
-
-// spline row and offset of distance r; row 0 (for a NaN of the filler entries) exists
-__device__ __forceinline__ int eam_row(float r, float rdr, int nr, float& p) {
-  const float pp = r * rdr + 1.0f;
-  const int m = max(0, min((int)pp, nr - 1));
-  p = fminf(pp - (float)m, 1.0f);
-  return m;
-}
-
-template <bool MI, int G>
-__global__ void __launch_bounds__(kEamThreads, 1) k_eam_fp_smem(
-    int n, int stride, int cap, float rc, EamDev eam, const float4* __restrict__ pos4, const int4* __restrict__ nbr4,
-    const int* __restrict__ count, const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot,
-    float4* __restrict__ posf, double* __restrict__ embed_slot) {
-  extern __shared__ float4 eam_tab[];
-  for (int t = threadIdx.x; t <= eam.nr; t += blockDim.x) eam_tab[t] = eam.rows[t];
-  __syncthreads();
-  const int sub = threadIdx.x % G;
-  const float cut2 = rc * rc;
-  for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; (at & ~31LL) < (long long)n * G;
-       at += (long long)gridDim.x * blockDim.x) {
-    const bool active = at / G < n;
-    const int i = active ? (int)(at / G) : n - 1;
-    const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
-    const float4 pi = pos4[i];
-    const float box[3] = {rp.box_f[0], rp.box_f[1], rp.box_f[2]};
-    const float ibox[3] = {1.f / box[0], 1.f / box[1], 1.f / box[2]};
-    const int nch = active ? (min(count[i], cap) + 3) >> 2 : 0;
-    const int last = __reduce_max_sync(0xffffffffu, nch);
-    const int self = i << kShiftBits;
-    const int4 idle = make_int4(self, self, self, self);
-    Acc<float> rho;
-    int4 e = sub < nch ? __ldg(nbr4 + (size_t)sub * stride + i) : idle;
-    for (int c = sub; c - sub < last; c += G) {
-      const int ee[4] = {e.x, e.y, e.z, e.w};
-      float4 pj[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pj[k] = pos4[ee[k] >> kShiftBits];
-      e = c + G < nch ? __ldg(nbr4 + (size_t)(c + G) * stride + i) : idle;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        float r[3], p;
-        eam_vec<MI>(pi, pj[k], ee[k], rp.wrap_f, box, ibox, r);
-        const float rsq = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-        const bool in = rsq < cut2 && rsq > 0.01f;
-        const float4 a = eam_tab[eam_row(rsq * rsqrt_r(rsq), eam.rdr, eam.nr, p)];
-        rho.add(in ? ((a.x * p + a.y) * p + a.z) * p + a.w : 0.f);
-      }
-    }
-    double sum = rho.value();
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (!active || sub != 0) continue;
-    const float rr = (float)sum;
-    float pp = rr * eam.rdrho + 1.0f;
-    const int m = max(1, min((int)pp, eam.nrho - 1));
-    pp = fminf(pp - (float)m, 1.0f);
-    const float4 a = __ldg(eam.frho + 2 * m + 0), b = __ldg(eam.frho + 2 * m + 1);
-    const float fp = (a.x * pp + a.y) * pp + a.z;
-    posf[i] = make_float4(pi.x, pi.y, pi.z, fp);
-    double phi = (((double)a.w * pp + (double)b.x) * pp + (double)b.y) * pp + (double)b.z;
-    if ((double)rr > eam.rhomax) phi += (double)fp * ((double)rr - eam.rhomax);
-    embed_slot[i] = phi;
-  }
-}
-
-template <bool MI, int G>
-__global__ void __launch_bounds__(kEamThreads, 1) k_eam_force_smem(
-    int n, int stride, int cap, float rc, EamDev eam, const float4* __restrict__ posf, const int4* __restrict__ nbr4,
-    const int* __restrict__ count, const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot,
-    const int* __restrict__ slot_atom, double* __restrict__ force, double* __restrict__ pair_slot, uint32_t* status,
-    int ref_sign) {
-  extern __shared__ float4 eam_tab[];   // rows of rho, then of z2
-  for (int t = threadIdx.x; t < 2 * (eam.nr + 1); t += blockDim.x) eam_tab[t] = eam.rows[t];
-  __syncthreads();
-  const float4* ztab = eam_tab + eam.nr + 1;
-  const int sub = threadIdx.x % G;
-  const float cut2 = rc * rc;
-  // ref_sign: the reference's Verlet pass uses MinDistanceVec(p_j, p_i) (RunWorklet.cpp:402)
-  const float sgn = ref_sign ? 1.f : -1.f;
-  for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; (at & ~31LL) < (long long)n * G;
-       at += (long long)gridDim.x * blockDim.x) {
-    const bool active = at / G < n;
-    const int i = active ? (int)(at / G) : n - 1;
-    const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
-    const float4 pi = posf[i];
-    const float box[3] = {rp.box_f[0], rp.box_f[1], rp.box_f[2]};
-    const float ibox[3] = {1.f / box[0], 1.f / box[1], 1.f / box[2]};
-    const int nch = active ? (min(count[i], cap) + 3) >> 2 : 0;
-    const int last = __reduce_max_sync(0xffffffffu, nch);
-    const int self = i << kShiftBits;
-    const int4 idle = make_int4(self, self, self, self);
-    Acc3<float> F;
-    float epair = 0.f;
-    int4 e = sub < nch ? __ldg(nbr4 + (size_t)sub * stride + i) : idle;
-    for (int c = sub; c - sub < last; c += G) {
-      const int ee[4] = {e.x, e.y, e.z, e.w};
-      float4 pj[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pj[k] = posf[ee[k] >> kShiftBits];
-      e = c + G < nch ? __ldg(nbr4 + (size_t)(c + G) * stride + i) : idle;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        float r[3], p;
-        eam_vec<MI>(pi, pj[k], ee[k], rp.wrap_f, box, ibox, r);
-        const float rsq = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-        const bool in = rsq < cut2 && rsq > 0.01f;
-        const float recip = rsqrt_r(rsq);
-        const int m = eam_row(rsq * recip, eam.rdr, eam.nr, p);
-        const float4 a = eam_tab[m], z = ztab[m];
-        const float rhop = (((a.x * 3.f) * p + (a.y + a.y)) * p + a.z) * eam.rdr;
-        const float z2p = (((z.x * 3.f) * p + (z.y + z.y)) * p + z.z) * eam.rdr;
-        const float z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
-        const float phi = z2 * recip;
-        const float phip = z2p * recip - phi * recip;
-        const float psip = pi.w * rhop + pj[k].w * rhop + phip;
-        const float fpair = in ? sgn * psip * recip : 0.f;
-        F.add(r[0] * fpair, r[1] * fpair, r[2] * fpair);
-        epair += in ? phi : 0.f;
-      }
-    }
-    double Fd[3] = {F.vx(), F.vy(), F.vz()}, ep = (double)epair;
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-      Fd[0] += __shfl_xor_sync(0xffffffffu, Fd[0], o);
-      Fd[1] += __shfl_xor_sync(0xffffffffu, Fd[1], o);
-      Fd[2] += __shfl_xor_sync(0xffffffffu, Fd[2], o);
-      ep += __shfl_xor_sync(0xffffffffu, ep, o);
-    }
-    if (!active || sub != 0) continue;
-    if (!isfinite(Fd[0]) || !isfinite(Fd[1]) || !isfinite(Fd[2])) set_flag(status, kFlagNonFinite);
-    const int id = slot_atom[i];
-    force[3 * id] = Fd[0];
-    force[3 * id + 1] = Fd[1];
-    force[3 * id + 2] = Fd[2];
-    pair_slot[i] = 0.5 * ep;
-  }
-}
-

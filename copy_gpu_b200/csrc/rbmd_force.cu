@@ -43,7 +43,7 @@ namespace {
 constexpr int kKL = 2;           // k samples per lane in the structure-factor kernel
 constexpr int kStageBytes = 48 * 1024;   // shared memory for k staging in the force pass
 constexpr int kSamplerD = 640;   // pre-drawn proposals per axis in the sampler kernel (38 KB smem)
-constexpr int kMdChunkMax = 1024;   // atoms per kinetic-energy chunk: at most
+constexpr int kMdChunk = 2048;   // atoms per kinetic-energy chunk
 
 }  // namespace
 
@@ -123,17 +123,14 @@ struct rbmd_force {
   int cap_override = 0;   // neighbor.capacity: initial list capacity (grown on overflow)
   int tpa_list = 0, tpa_near = 128;     // list build: 0 = one warp per cell, 1 = one warp per atom, else
                                         // threads per block of k_nlist; threads per block of the force pass
-  double mean_listed = 0;               // listed neighbours per atom expected from the density
-  int rbl_list_warp = -1;               // RBL list build: -1 one warp per cell, 1 one warp per atom, 0 one thread per atom
+  int rbl_list_warp = -1;               // RBL list build: 1 one warp per atom, 0 one thread per atom, -1 by size
   int rbl_lanes = 0;                    // RBL force pass lanes per atom (0: by size)
   int num_sms = 148;                    // SMs of the bound device (cudaDevAttrMultiProcessorCount)
   int near_variant = 1;                 // 1: k_near_lean where it applies (lean_ok), 0: k_near_force
   int near_lanes = 1;                   // near pass lanes per atom: 1, or 4 / 8 / 16 / 32
-  bool lanes_set = false;               // given by the configuration or tuned (else near_lanes())
   bool autotune = false;                // "autotune": true tunes them at the first compute
   bool tuned = false;
   bool list_valid = false;   // a list (and x_ref) exists from an earlier build
-  bool rebuild_clear = false;   // d_rebuild is zero: the last thing that ran was a whole step
   int shake_max_iter = 5000;
   std::string potential_file, potential_format;   // format: "", "funcfl" or "setfl"
 
@@ -201,7 +198,7 @@ struct rbmd_force {
   double* d_eslot = nullptr;   // 2 per slot (lj, coul)
   double* d_esum = nullptr;    // scratch sums
   // RBE
-  int Ptot = 0, nitems = 0, finish_warps = 1, rho_threads = 64, ktile = 128, kstage = 0;
+  int Ptot = 0, nitems = 0, rho_threads = 64, ktile = 128, kstage = 0;
   bool minimg = true, want_energy = true;
   bool kspace_priority = true;
   bool orig_pred = false;        // neighbor.type "ORIGINAL": pair predicate d^2 < rc^2   // execution.kspace_priority: side stream at the highest priority
@@ -214,8 +211,6 @@ struct rbmd_force {
   RhoRep* d_rhorep = nullptr;
   void* d_partial = nullptr;
   double2* d_rho = nullptr;
-  int* d_rho_done = nullptr;   // finished structure-factor items per replica (few chunks: kFusedChunks)
-  int* d_cidx = nullptr;       // charged atom of each atom, or -1
   double* d_ek = nullptr;
   double* d_far = nullptr;
   double* d_weights = nullptr;
@@ -225,7 +220,7 @@ struct rbmd_force {
   // MD
   MdChunk* d_chunks = nullptr;
   int nchunks = 0;
-  int *d_chunk_rep_begin = nullptr, *d_chunk_done = nullptr;
+  int* d_chunk_rep_begin = nullptr;
   double *d_ke_partial = nullptr, *d_ke = nullptr, *d_T = nullptr, *d_lambda = nullptr,
          *d_xi = nullptr, *d_xold = nullptr, *d_vold = nullptr;
   bool pending_scale = false;
@@ -236,8 +231,6 @@ struct rbmd_force {
   float* d_host32 = nullptr;   // [3 n] staging of rbmd_force_compute_host_f32 (positions in, forces out)
   // topology device
   int *d_term_atom = nullptr, *d_tmult = nullptr, *d_sc_off = nullptr, *d_sc_id = nullptr, *d_row_off = nullptr,
-  float4 *d_eam_rows = nullptr, *d_posf = nullptr;   // value rows of rho and z2; (x, y, z, F'(rho)) per slot
-  bool eam_smem = false;        // FP32 tables small enough for the passes with rows in shared memory
       *d_row_idx = nullptr, *d_sp_off = nullptr, *d_sp_id = nullptr, *d_comp = nullptr;
   double *d_tk = nullptr, *d_ta = nullptr, *d_sc_fac = nullptr, *d_rows = nullptr, *d_eterm = nullptr,
          *d_esc = nullptr, *d_sp_wd = nullptr;
@@ -364,28 +357,11 @@ int molecular_mode(const rbmd_force* f) {
   return f->at.molecule != nullptr ? 1 : 0;
 }
 
-// k_near_lean applies: one LJ coefficient pair for all types, no molecules, no per-pair minimum
-// image (a Verlet skin, or boxes of >= 3 cells per axis).
+// k_near_lean applies: one LJ coefficient pair for all types, no molecules, one thread per atom,
+// no per-pair minimum image (a Verlet skin, or boxes of >= 3 cells per axis).
 bool lean_ok(const rbmd_force* f) {
   return f->near_variant >= 1 && !f->is_rbl() && !f->is_eam() && f->nt_eff == 1 && molecular_mode(f) == 0 &&
-         (f->skin > 0 || !f->minimg);
-}
-
-// Lanes per atom of the near pass when neither the configuration nor the autotuner gave them
-// (B200, microseconds a pass).  Lean pass, electrolyte lists of 78 entries, FP32: 4,000 atoms 1 lane
-// 29 / 16 lanes 10.1; 8,000 8 lanes 14.2 / 16 lanes 15.5; 16,000 1 lane 28 / 8 lanes 15.6; 32,000
-// 4 lanes 21.6 / 8 lanes 22.5; 128,000 1 lane 49 / 4 lanes 44; 256,000 82 / 80, beyond which the
-// FP64 sums of the lanes cost more than they spread (FP64 crosses at 128,000: 109 / 110).  General
-// pass with long lists: water (556 listed) 30,000 atoms 1 lane 409 / 4 lanes 165 / 16 lanes 120 / 32
-// lanes 132, 4,800 359 / 78 / 32 / 37; chains (505 listed) 22,824 427 / 179 / 125 / 142.
-int near_lanes(const rbmd_force* f) {
-  if (f->lanes_set) return f->near_lanes;
-  const int per_sm = f->n / f->num_sms;
-  const bool lean = lean_ok(f);
-  if (!lean && f->mean_listed >= 128.0) return 16;
-  if (per_sm < 40) return 16;
-  if (per_sm < 160) return 8;
-  return !lean || per_sm < (f->fp64 ? 700 : 1400) ? 4 : 1;
+         f->near_lanes == 1 && (f->skin > 0 || !f->minimg);
 }
 
 // The lean near pass and the per-atom list build run beside the k-space stream and use no shared
@@ -434,10 +410,9 @@ void free_all(rbmd_force* f) {
   if (f->d_partial) cudaFree(f->d_partial);
   f->d_partial = nullptr;
   dfree(f->d_rho); dfree(f->d_ek); dfree(f->d_far); dfree(f->d_weights); dfree(f->d_srep); dfree(f->d_qtab);
-  dfree(f->d_rho_done); dfree(f->d_cidx);
   dfree(f->d_chunks); dfree(f->d_chunk_rep_begin); dfree(f->d_ke_partial); dfree(f->d_ke);
   dfree(f->d_T); dfree(f->d_lambda); dfree(f->d_xi); dfree(f->d_xold); dfree(f->d_vold);
-  dfree(f->d_frho); dfree(f->d_rhor); dfree(f->d_z2r); dfree(f->d_eam_rows); dfree(f->d_posf);
+  dfree(f->d_frho); dfree(f->d_rhor); dfree(f->d_z2r);
   if (f->d_fp) cudaFree(f->d_fp);
   f->d_fp = nullptr;
   dfree(f->d_emb); dfree(f->d_epair); dfree(f->d_hoh); dfree(f->d_ebond); dfree(f->d_eangle); dfree(f->d_ewcoul);
@@ -806,30 +781,6 @@ R pair_d2_max(R rc, bool reuse, bool orig) {
   return v;
 }
 
-// Smallest d^2 with d^2 - rs^2 > 1e-4, found the same way.
-template <class R>
-R pair_d2_min(R rs) {
-  using I = typename std::conditional<sizeof(R) == 4, uint32_t, uint64_t>::type;
-  const volatile R cut2 = rs * rs;
-  auto accepts = [&](R d2) -> bool {
-    const volatile R margin = d2 - cut2;
-    return margin > (R)1.0e-4;
-  };
-  I lo, hi;   // not accepts(lo), accepts(hi)
-  const R c = cut2, top = (R)2 * c + (R)1;
-  std::memcpy(&lo, &c, sizeof lo);
-  std::memcpy(&hi, &top, sizeof hi);
-  while (hi - lo > 1) {
-    const I mid = lo + (hi - lo) / 2;
-    R v;
-    std::memcpy(&v, &mid, sizeof v);
-    (accepts(v) ? hi : lo) = mid;
-  }
-  R v;
-  std::memcpy(&v, &hi, sizeof v);
-  return v;
-}
-
 template <class R>
 R lean_d2_max(const rbmd_force* f) {
   return pair_d2_max<R>((R)f->rc, f->skin > 0, f->orig_pred);
@@ -872,17 +823,11 @@ template <class R>
 void launch_rbl_list(rbmd_force* f, cudaStream_t s) {
   PhaseScope ps(f, kPhList, s);
   const int* rp = f->nrep > 1 ? f->d_rep_of : nullptr;
-  const int side = 2 * f->num_cycles + 1, ncs = side * side * side;
-  if (f->rbl_list_warp < 0 && ncs <= kRblStencilMax) {   // warp per cell
-    const long long items = (long long)f->ncell_total * f->list_parts;
-    const size_t smem = (size_t)kRblWarps * rbl_cell_bytes<R>(ncs);
-    k_rbl_list_cell<R, sizeof(R) == 4 ? 4 : 2>
-        <<<(unsigned)((items + kRblWarps - 1) / kRblWarps), 32 * kRblWarps, smem, s>>>(
-            f->ncell_total, f->list_parts, (const typename Traits<R>::V4*)f->d_pos4, f->d_cell_start, f->d_reps,
-            f->nrep > 1 ? f->d_cell_rep : nullptr, f->num_cycles, (R)f->rc, (R)f->rs,
-            pair_d2_max<R>((R)f->rs, true, false), pair_d2_min<R>((R)f->rs), pair_d2_max<R>((R)f->rc, true, false),
-            (R)1, f->core_cap, f->shell_cap, f->stride, f->d_nbr, f->d_count, f->d_count2, f->d_maxcount, f->d_status);
-  } else if (f->rbl_list_warp > 0 && ncs <= kRblStencilMax) {
+  const int side = 2 * f->num_cycles + 1;
+  // one warp per atom below 10 warps' worth of atoms per SM (measured crossover between 21k and
+  // 98k atoms on B200), where one thread per atom leaves most SMs idle
+  const bool warp = f->rbl_list_warp > 0 || (f->rbl_list_warp < 0 && f->n < 10 * 32 * f->num_sms);
+  if (warp && side * side * side <= kRblStencilMax) {
     k_rbl_list_warp<R><<<(f->n + kRblWarps - 1) / kRblWarps, 32 * kRblWarps, 0, s>>>(
         f->n, (const typename Traits<R>::V4*)f->d_pos4, f->d_cell_start, f->d_reps, rp, f->num_cycles, (R)f->rc,
         (R)f->rs, f->core_cap, f->shell_cap, f->stride, f->d_nbr, f->d_count, f->d_count2, f->d_maxcount,
@@ -926,7 +871,7 @@ void launch_sort(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
       cudaMemsetAsync(f->d_cell_count, 0, sizeof(int) * f->ncell_total, s);
     }
     k_bin<R><<<(n + 255) / 256, 256, 0, s>>>(n, f->at.pos, rep_of, f->d_reps, f->d_cell_of, f->d_cell_count,
-                                             f->d_status, rb, f->skin > 0 ? f->d_xref : nullptr);
+                                             f->d_status, rb);
     f->launches++;
   }
   const int nblk = (f->ncell_total + kScanBlock - 1) / kScanBlock;
@@ -936,14 +881,11 @@ void launch_sort(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
                                     f->d_cursor, rb_any);
   k_scatter<<<(n + 255) / 256, 256, 0, s>>>(n, f->d_cell_of, f->d_cell_start, f->d_cursor, f->d_tmp, rep_of,
                                             rb);
-  // one warp per 32 atoms of a cell on average
-  const int parts = std::max(1, (int)((f->n + 32LL * f->ncell_total - 1) / (32LL * f->ncell_total)));
-  const long long sort_items = (long long)f->ncell_total * parts;
-  k_cell_sort_gather<R><<<(unsigned)((sort_items + kSortWarps - 1) / kSortWarps), 32 * kSortWarps, 0, s>>>(
-      f->ncell_total, parts, f->d_cell_start, f->d_tmp, f->at.pos, f->at.charge, f->at.type,
+  k_cell_sort_gather<R><<<(f->ncell_total + kSortWarps - 1) / kSortWarps, 32 * kSortWarps, 0, s>>>(
+      f->ncell_total, f->d_cell_start, f->d_tmp, f->at.pos, f->at.charge, f->at.type,
       molecular_mode(f) == 2 ? f->d_comp : f->at.molecule,
       rep_of, f->d_reps, f->d_slot_atom, f->d_atom_slot, (typename Traits<R>::V4*)f->d_pos4, nullptr,
-      f->d_meta, rb, f->sort_x() ? 1 : 0, f->d_cell_rep);
+      f->d_meta, f->d_xref, rb, f->sort_x() ? 1 : 0, f->d_cell_rep);
   f->launches += 4;
   if (rb && regather) launch_regather<R>(f, s);
 }
@@ -999,45 +941,26 @@ void launch_kspace(rbmd_force* f, cudaStream_t s, cudaEvent_t ready) {
     cudaEventRecord(f->ev_tail, s);
     return;
   }
-// RBE force: lanes per charged atom so that the launch holds about eight warps per scheduler (one
-// thread per atom at 100,000 charged atoms and more, 8 lanes below 19,000); beyond that, lanes only
-// add copies of the staged records.
-template <class R>
-void launch_rbe_force(rbmd_force* f, cudaStream_t s) {
-  const size_t smem = (size_t)f->kstage * sizeof(typename KRec<R>::T);
-  const long long want = 1024LL * f->num_sms;
-  const int g = 8LL * f->nq <= want ? 8 : (4LL * f->nq <= want ? 4 : (2LL * f->nq <= want ? 2 : 1));
-  auto kern = g == 8 ? k_rbe_force<R, 8> : g == 4 ? k_rbe_force<R, 4> : g == 2 ? k_rbe_force<R, 2> : k_rbe_force<R, 1>;
-  const int per = kRbeThreads / g;
-  kern<<<(f->nq + per - 1) / per, kRbeThreads, smem, s>>>(
-      f->nq, f->kstage, f->d_qidx, (const typename FracT<R>::T*)f->d_frac, (const typename KRec<R>::T*)f->d_krec,
-      f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_far);
-}
-
+  const int* rep_of = f->nrep > 1 ? f->d_rep_of : nullptr;
   {
     PhaseScope ps(f, kPhK, s);
-    RhoOut<R> o;
-    o.weights = own_prop ? f->d_pw : f->d_weights;
-    o.qqr2e = f->u.qqr2e;
-    o.krec = (typename KRec<R>::T*)f->d_krec;
-    o.rho = f->d_rho;
-    o.ek = f->d_ek;
+    k_frac<R><<<(f->nq + 255) / 256, 256, 0, s>>>(f->nq, f->d_qidx, f->at.pos, f->at.charge, rep_of,
+                                                   f->d_reps, f->d_frac);
     k_rho_lanes<R, kKL><<<f->nitems, f->rho_threads, 0, s>>>(
-        f->d_items, f->P, f->d_qidx, f->at.pos, f->at.charge, f->d_reps, f->d_rhorep,
-        (typename FracT<R>::T*)f->d_frac, (R*)f->d_partial, f->ktile, f->d_rho_done, o);
-    f->launches++;
-    if (!f->d_rho_done) {
-      const int groups = (f->P + 31) / 32;
-      k_rho_finish<R><<<f->nrep * groups, 32 * f->finish_warps, 0, s>>>(
-          f->nrep, groups, f->P, f->ktile, f->d_rhorep, f->d_reps, (const R*)f->d_partial, o);
-      f->launches++;
-    }
+        f->d_items, (const typename FracT<R>::T*)f->d_frac, (const typename KRec<R>::T*)f->d_krec,
+        (R*)f->d_partial, f->ktile);
+    k_rho_finish<R><<<(f->Ptot + 3) / 4, 128, 0, s>>>(
+        f->Ptot, f->ktile, f->d_krep, f->d_rhorep, f->d_reps, (const R*)f->d_partial,
+        own_prop ? f->d_pw : f->d_weights, f->u.qqr2e, (typename KRec<R>::T*)f->d_krec, f->d_rho, f->d_ek);
   }
   {
     PhaseScope ps(f, kPhRbeF, s);
-    launch_rbe_force<R>(f, s);
+    const size_t smem = (size_t)f->kstage * sizeof(typename KRec<R>::T);
+    k_rbe_force<R><<<(f->nq + 127) / 128, 128, smem, s>>>(
+        f->nq, f->kstage, f->d_qidx, (const typename FracT<R>::T*)f->d_frac,
+        (const typename KRec<R>::T*)f->d_krec, f->d_reps, rep_of, f->d_far);
   }
-  f->launches++;
+  f->launches += 4;
   // conditioning of the next step's proposal, after the force kernels of this one
   if (own_prop && f->proposal == "learned" && f->prop_trained) {
     k_prop_spectrum<<<f->nrep, 256, 0, s>>>(f->nrep, f->d_reps, f->d_prep, f->d_kvec, f->d_rho, f->d_pw, 0.1f,
@@ -1078,24 +1001,13 @@ void launch_near_t(rbmd_force* f, cudaStream_t s) {
   p.two_sqrt_alpha_over_sqrt_pi = 2.0 * std::sqrt(f->alpha) / std::sqrt(M_PI);
   p.kstage = 0;
   p.orig = f->orig_pred ? 1 : 0;
-  const int g = near_lanes(f);
-  if constexpr ((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0) {
-    // one LJ coefficient pair for all types, no molecules: the lean pass
-    if (lean_ok(f)) {
-      if (g >= 16) launch_near_lean<R, COUL, MI, 16>(f, s, p);
-      else if (g == 8) launch_near_lean<R, COUL, MI, 8>(f, s, p);
-      else if (g == 4) launch_near_lean<R, COUL, MI, 4>(f, s, p);
-      else launch_near_lean<R, COUL, MI, 1>(f, s, p);
-      return;
-    }
-  }
-  if (g > 1) {
-    const long long threads = (long long)f->n * g;
+  if (f->near_lanes > 1) {
+    const long long threads = (long long)f->n * f->near_lanes;
     const int grid = (int)((threads + 255) / 256);
-    auto kern = g == 4    ? k_near_force_group<R, COUL, MI, 4>
-                : g == 8  ? k_near_force_group<R, COUL, MI, 8>
-                : g == 16 ? k_near_force_group<R, COUL, MI, 16>
-                          : k_near_force_group<R, COUL, MI, 32>;
+    auto kern = f->near_lanes == 4    ? k_near_force_group<R, COUL, MI, 4>
+                : f->near_lanes == 8  ? k_near_force_group<R, COUL, MI, 8>
+                : f->near_lanes == 16 ? k_near_force_group<R, COUL, MI, 16>
+                                      : k_near_force_group<R, COUL, MI, 32>;
     kern<<<grid, 256, 0, s>>>(p, f->d_ljt, (const typename Traits<R>::V4*)f->d_pos4, f->d_meta, f->d_nbr,
                               f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom,
                               f->at.force, f->want_energy ? f->d_eslot : nullptr, f->d_status);
@@ -1103,6 +1015,19 @@ void launch_near_t(rbmd_force* f, cudaStream_t s) {
     return;
   }
   const int bs = f->tpa_near;
+  if constexpr ((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0) {
+    // one LJ coefficient pair for all types, no molecules: the lean pass
+    if (lean_ok(f)) {
+      auto kern = f->want_energy ? k_near_lean<R, COUL, MI, true> : k_near_lean<R, COUL, MI, false>;
+      prefer_shared_carveout(f, (const void*)kern);
+      kern<<<(f->n + bs - 1) / bs, bs, 0, s>>>(
+          p, lj24<R>(f->ljt_h, 0), sig6<R>(f->ljt_h, 0), lean_d2_max<R>(f), (const typename Traits<R>::V4*)f->d_pos4,
+          (const int4*)f->d_nbr, f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
+          f->want_energy ? f->d_eslot : nullptr, f->d_status);
+      f->launches++;
+      return;
+    }
+  }
   k_near_force<R, COUL, MI><<<(f->n + bs - 1) / bs, bs, 0, s>>>(
       p, f->d_ljt, (const typename Traits<R>::V4*)f->d_pos4, f->d_meta, f->d_nbr, f->d_count,
       f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
@@ -1114,19 +1039,6 @@ template <class R, bool COUL>
 void launch_near_m(rbmd_force* f, cudaStream_t s) {
   const int mi = f->skin > 0 ? kMiAll : (f->minimg ? kMiLJ : kMiNone);
   if (molecular_mode(f) == 2) {   // special-bond LJ weights: their own instantiations
-template <class R, bool COUL, int MI, int G>
-void launch_near_lean(rbmd_force* f, cudaStream_t s, const NearParams& p) {
-  const int bs = G == 1 ? f->tpa_near : 128;
-  const long long threads = (long long)f->n * G;
-  auto kern = f->want_energy ? k_near_lean<R, COUL, MI, true, G> : k_near_lean<R, COUL, MI, false, G>;
-  if (G == 1) prefer_shared_carveout(f, (const void*)kern);
-  kern<<<(unsigned)((threads + bs - 1) / bs), bs, 0, s>>>(
-      p, lj24<R>(f->ljt_h, 0), sig6<R>(f->ljt_h, 0), lean_d2_max<R>(f), (const typename Traits<R>::V4*)f->d_pos4,
-      (const int4*)f->d_nbr, f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
-      f->want_energy ? f->d_eslot : nullptr, f->d_status);
-  f->launches++;
-}
-
     if (mi == kMiAll) launch_near_t<R, COUL, kMiAll | kMiSpecial>(f, s);
     else if (mi == kMiLJ) launch_near_t<R, COUL, kMiLJ | kMiSpecial>(f, s);
     else launch_near_t<R, COUL, kMiNone | kMiSpecial>(f, s);
@@ -1143,7 +1055,8 @@ void launch_near(rbmd_force* f, cudaStream_t s) {
   else launch_near_m<R, false>(f, s);
 }
 
-EamDev eam_dev(const rbmd_force* f) {
+template <class R>
+void launch_eam(rbmd_force* f, cudaStream_t s) {
   EamDev e;
   e.frho = f->d_frho;
   e.rhor = f->d_rhor;
@@ -1199,7 +1112,17 @@ void launch_rbl_force(rbmd_force* f, cudaStream_t s) {
   const int* rp = f->nrep > 1 ? f->d_rep_of : nullptr;
   const int nb = (f->n + 127) / 128;
   if (f->is_eam()) {
-    const EamDev e = eam_dev(f);
+    EamDev e;
+    e.frho = f->d_frho;
+    e.rhor = f->d_rhor;
+    e.z2r = f->d_z2r;
+    e.nrho = f->eam_h.nrho;
+    e.nr = f->eam_h.nr;
+    e.rdr = 1.0f / f->eam_h.dr;
+    e.rdrho = 1.0f / f->eam_h.drho;
+    e.rdr_d = 1.0 / (double)f->eam_h.dr;
+    e.rdrho_d = 1.0 / (double)f->eam_h.drho;
+    e.rhomax = f->eam_h.rhomax;
     k_rbl_eam_fp<R><<<nb, 128, 0, s>>>(f->n, f->stride, f->core_cap, f->shell_cap, f->rc, f->rs, e,
                                         (const typename Traits<R>::V4*)f->d_pos4, f->d_nbr, f->d_count,
                                         f->d_count2, f->d_reps, rp, (R*)f->d_fp, f->d_emb);
@@ -1221,7 +1144,6 @@ void launch_rbl_force(rbmd_force* f, cudaStream_t s) {
     p.erf_tab = f->d_erf_tab;
     p.rc = f->rc;
     p.rs = f->rs;
-  e.rows = f->d_eam_rows;
     p.alpha = f->alpha;
     p.qqr2e = f->u.qqr2e;
     p.sqrt_alpha = std::sqrt(f->alpha);
@@ -1232,37 +1154,7 @@ void launch_rbl_force(rbmd_force* f, cudaStream_t s) {
     auto kern = pick_rbl_force<R>(f->with_coul_near(), spw, g);
     const int grid = (int)(((long long)f->n * g + 127) / 128);
     kern<<<grid, 128, 0, s>>>(p, f->d_ljt, (const typename Traits<R>::V4*)f->d_pos4, f->d_meta, f->d_nbr,
-  return e;
-}
-
-// FP32 passes with the spline rows in shared memory (k_eam_fp_smem, k_eam_force_smem): one block of
-// 1024 threads per SM at most.  Four lanes per atom balance the blocks' shares and keep the rows of
-// about 53 listed neighbours four iterations long; systems that would leave SMs idle with four
-// lanes take 16.
-template <bool MI, int G>
-void launch_eam_smem(rbmd_force* f, cudaStream_t s, const EamDev& e, const int* rp) {
-  const long long blocks = ((long long)f->n * G + kEamThreads - 1) / kEamThreads;
-  const int grid = (int)std::min<long long>(blocks, f->num_sms);
-  const size_t row_bytes = (size_t)(e.nr + 1) * sizeof(float4);
-  k_eam_fp_smem<MI, G><<<grid, kEamThreads, row_bytes, s>>>(
-      f->n, f->stride, f->cap, (float)f->rc, e, (const float4*)f->d_pos4, (const int4*)f->d_nbr, f->d_count, f->d_reps,
-      rp, f->d_posf, f->d_emb);
-  k_eam_force_smem<MI, G><<<grid, kEamThreads, 2 * row_bytes, s>>>(
-      f->n, f->stride, f->cap, (float)f->rc, e, f->d_posf, (const int4*)f->d_nbr, f->d_count, f->d_reps, rp,
-      f->d_slot_atom, f->at.force, f->d_epair, f->d_status, f->eam_ref_sign ? 1 : 0);
-  f->launches += 2;
-}
-
-template <class R>
-void launch_eam(rbmd_force* f, cudaStream_t s) {
-  const EamDev e = eam_dev(f);
                               f->d_count, f->d_count2, f->d_reps, rp, f->d_slot_atom, f->shell_cap, f->at.force, es,
-  if (sizeof(R) == 4 && f->eam_smem) {
-    const bool few = 4LL * f->n < (long long)kEamThreads * f->num_sms;
-    if (f->minimg) few ? launch_eam_smem<true, 16>(f, s, e, rp) : launch_eam_smem<true, 4>(f, s, e, rp);
-    else few ? launch_eam_smem<false, 16>(f, s, e, rp) : launch_eam_smem<false, 4>(f, s, e, rp);
-    return;
-  }
                               f->d_status);
     f->launches++;
   }
@@ -1374,7 +1266,7 @@ bool launch_rebuild_conditional(rbmd_force* f, cudaStream_t s, bool bin) {
 // stream, the cell sort / neighbour list / near pass / intramolecular terms run on the caller's
 // stream, and the far force is folded in after the join.
 template <class R>
-void launch_force_tail(rbmd_force* f, cudaStream_t s, bool bin, bool regather, bool fold_far) {
+void launch_force_tail(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
   const bool kspace = f->is_rbe();
   if (kspace) {
     cudaEventRecord(f->ev_fork, s);
@@ -1405,8 +1297,7 @@ void launch_force_tail(rbmd_force* f, cudaStream_t s, bool bin, bool regather, b
   }
   if (kspace) {
     cudaStreamWaitEvent(s, f->ev_join, 0);
-    if (f->nq > 0 && fold_far) {
-// fold_far: add the k-space force here (a step without a Langevin force leaves it to its kick).
+    if (f->nq > 0) {
       k_add_far<<<(3 * f->nq + 255) / 256, 256, 0, s>>>(f->nq, f->d_qidx, f->d_far, f->at.force, f->d_status);
       f->launches++;
     }
@@ -1443,7 +1334,7 @@ void launch_compute(rbmd_force* f, cudaStream_t s) {
   } else if (f->d_rebuild) {
     cudaMemsetAsync(f->d_rebuild, 1, sizeof(int) * (f->nrep + 1), s);   // nonzero: rebuild
   }
-  launch_force_tail<R>(f, s, true, true, true);
+  launch_force_tail<R>(f, s, true, true);
   f->list_valid = true;
 }
 
@@ -1465,7 +1356,6 @@ void drop_graphs(rbmd_force* f) {
 }
 
 // list capacities hold whole chunks of kNbrChunk entries
-  f->rebuild_clear = false;
 int round_chunk(int cap) { return (cap + kNbrChunk - 1) / kNbrChunk * kNbrChunk; }
 
 rbmd_status grow_list(rbmd_force* f, const int* need) {
@@ -1516,14 +1406,13 @@ void launch_step(rbmd_force* f, cudaStream_t s) {
   mp.apply_scale = f->pending_scale ? 1 : 0;
   mp.nh = f->tstat == 3;
   f->want_energy = f->energy_every > 0 && ((f->step_count + 1) % f->energy_every == 0);
+  cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s);
   const bool skin = f->skin > 0;
   // without a skin the drift bins every step; with one it writes the slot caches (unless SHAKE
   // moves the atoms afterwards) and k_bin bins on rebuild steps only
   if (!skin) cudaMemsetAsync(f->d_cell_count, 0, sizeof(int) * f->ncell_total, s);
-  // with a skin the drift kernel decides, on flags that the end of the last step cleared; a missing
-  // or overflowed list forces a rebuild
-  if (skin && !(f->list_valid && f->rebuild_clear))
-    cudaMemsetAsync(f->d_rebuild, f->list_valid ? 0 : 1, sizeof(int) * (f->nrep + 1), s);
+  // with a skin the drift kernel decides; a missing or overflowed list forces a rebuild
+  if (skin) cudaMemsetAsync(f->d_rebuild, f->list_valid ? 0 : 1, sizeof(int) * (f->nrep + 1), s);
   // (the slot map exists once a cell sort has run: list_valid)
   const bool drift_cache = skin && !shake && f->list_valid;
   // stages 1-2: kick, drift + wrap, bin (binning sees the unconstrained positions, as the
@@ -1556,13 +1445,29 @@ void launch_step(rbmd_force* f, cudaStream_t s) {
     f->launches++;
   }
   // stage 3: force (cell sort of the pre-constraint binning, then list and forces)
-  const bool kick_folds = f->is_rbe() && f->nq > 0 && f->tstat != 4;
-  launch_force_tail<R>(f, s, skin, skin && !drift_cache, !kick_folds);
+  launch_force_tail<R>(f, s, skin, skin && !drift_cache);
   f->list_valid = true;
-  // stage 3: kick (+ RATTLE), temperature, thermostat.  The temperature and thermostat run at the
-  // end of the last kernel that sums the kinetic energy; Nose-Hoover's extra kick uses the xi of
-  // before the update, so there they follow in their own launch.
+  // stage 3: kick (+ RATTLE), temperature, thermostat
   PhaseScope ps_int(f, kPhInt, s);
+  if (shake) {
+    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 1,
+                                        nullptr, nullptr);
+    k_rattle<<<((int)f->n_mol + 127) / 128, 128, 0, s>>>((int)f->n_mol, f->d_hoh, f->at.pos, f->at.vel,
+                                                         f->at.mass, f->nrep > 1 ? f->d_rep_of : nullptr,
+                                                         f->d_reps, f->d_status);
+    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 0,
+                                        nullptr, f->d_ke_partial);
+    f->launches += 3;
+  } else {
+    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 1,
+                                        nullptr, f->d_ke_partial);
+    f->launches++;
+  }
+  if (f->tstat == 3) {
+    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 2,
+                                        f->d_xi, nullptr);
+    f->launches++;
+  }
   ThermoParams tp;
   tp.nrep = f->nrep;
   tp.tstat = f->tstat;
@@ -1572,38 +1477,9 @@ void launch_step(rbmd_force* f, cudaStream_t s) {
   tp.Tdamp = f->Tdamp;
   tp.T0 = f->T0;
   tp.dof_mode = f->dof_mode;
-  ThermoDev td;
-  td.chunk_begin_of_rep = f->d_chunk_rep_begin;
-  td.ke_partial = f->d_ke_partial;
-  td.ke = f->d_ke;
-  td.T = f->d_T;
-  td.lambda = f->d_lambda;
-  td.xi = f->d_xi;
-  td.rebuild = skin ? f->d_rebuild : nullptr;
-  td.done = f->d_chunk_done;
-  const int fused = f->tstat != 3;
-  auto kick = [&](int do_kick, const double* xi, double* ke, int thermo) {
-    const FarFold far{kick_folds && do_kick == 1 ? f->d_cidx : nullptr, f->d_far, f->d_status};
-    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, do_kick, xi, ke, far,
-                                         thermo, tp, td, f->d_reps);
-    f->launches++;
-  };
-  if (shake) {
-    kick(1, nullptr, nullptr, 0);
-    k_rattle<<<((int)f->n_mol + 127) / 128, 128, 0, s>>>((int)f->n_mol, f->d_hoh, f->at.pos, f->at.vel,
-                                                         f->at.mass, f->nrep > 1 ? f->d_rep_of : nullptr,
-                                                         f->d_reps, f->d_status);
-    f->launches++;
-    kick(0, nullptr, f->d_ke_partial, fused);
-  } else {
-    kick(1, nullptr, f->d_ke_partial, fused);
-  }
-  if (f->tstat == 3) {
-    kick(2, f->d_xi, nullptr, 0);
-    k_thermo<<<f->nrep, 128, 0, s>>>(tp, td, f->d_reps);
-    f->launches++;
-  }
-  f->rebuild_clear = skin;
+  k_thermo<<<(f->nrep + 3) / 4, 128, 0, s>>>(tp, f->d_chunk_rep_begin, f->d_ke_partial, f->d_ke,
+                                                f->d_T, f->d_lambda, f->d_xi, f->d_reps);
+  f->launches++;
   f->pending_scale = (f->tstat == 1 || f->tstat == 2);
   f->step_count++;
 }
@@ -1732,11 +1608,11 @@ rbmd_status parse_config(rbmd_force* f, const char* text) {
     auto ok = [](int t) { return t == 64 || t == 128 || t == 256; };
     const Value* tlv = root.path("tuning.list_block");
     if (ok(tl) || (tlv && (tl == 0 || tl == 1))) { f->tpa_list = tl; f->autotune = false; }
-    if (ok(tn)) { f->tpa_near = tn; f->autotune = false; f->lanes_set = true; }
+    if (ok(tn)) { f->tpa_near = tn; f->autotune = false; }
     const Value* nv = root.path("tuning.near_variant");
     if (nv) f->near_variant = (int)num(root, "tuning.near_variant", 1.0) == 0 ? 0 : 1;
     const int ln = (int)num(root, "tuning.force_lanes", 0.0);
-    if (ln == 1 || ln == 4 || ln == 8 || ln == 16 || ln == 32) { f->near_lanes = ln; f->autotune = false; f->lanes_set = true; }
+    if (ln == 1 || ln == 4 || ln == 8 || ln == 16 || ln == 32) { f->near_lanes = ln; f->autotune = false; }
     const std::string rl = rbmdjson::text(root, "tuning.rbl_list", "auto");
     if (rl != "warp" && rl != "thread" && rl != "auto") {
       std::snprintf(g_last_error, sizeof g_last_error,
@@ -1999,7 +1875,6 @@ rbmd_status rbmd_force_create(const char* json_text, int32_t n_replicas, const r
                               rbmd_force** out) {
   if (!out || !boxes || n_replicas < 1) return RBMD_ERR_ARG;
   *out = nullptr;
-  f->lanes_set = true;   // the trials set near_lanes
   rbmd_force* f = new rbmd_force();
   rbmd_status st = parse_config(f, json_text);
   if (st) { delete f; return st; }
@@ -2382,14 +2257,6 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     f->list_parts = std::max(1, f->list_parts);
   }
   CK(dalloc(&f->d_maxcount, 2));
-  if (f->is_rbl()) {   // the cell-cooperative list build of the largest stencils asks for more than 48 KB
-    const int side = 2 * f->num_cycles + 1, ncs = side * side * side;
-    if (ncs <= kRblStencilMax) {
-      const int bytes = kRblWarps * (fp64 ? rbl_cell_bytes<double>(kRblStencilMax) : rbl_cell_bytes<float>(kRblStencilMax));
-      CK(cudaFuncSetAttribute(fp64 ? (const void*)k_rbl_list_cell<double, 2> : (const void*)k_rbl_list_cell<float, 4>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    }
-  }
   CK(dalloc(&f->d_nbuilds, 1));
   CK(cudaMemset(f->d_nbuilds, 0, sizeof(unsigned long long)));
   CK(dalloc(&f->d_rebuild, (size_t)nrep + 1));
@@ -2402,7 +2269,6 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     CK(cudaMemcpy(f->d_cell_rep, cr.data(), sizeof(int) * cr.size(), cudaMemcpyHostToDevice));
   }
   CK(dalloc(&f->d_block_sums, (size_t)(f->ncell_total + kScanBlock - 1) / kScanBlock + 1));
-  f->mean_listed = rho_max * 4.0 / 3.0 * M_PI * lc * lc * lc;
   if (f->skin > 0) CK(dalloc(&f->d_xref, 3 * n));
   CK(dalloc(&f->d_status, 1));
   CK(cudaMemset(f->d_status, 0, sizeof(uint32_t)));
@@ -2496,12 +2362,8 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     std::vector<RhoItem> items;
     std::vector<RhoRep> rr(nrep);
     const int ntiles = (f->P + f->ktile - 1) / f->ktile;
-    // chunks: three blocks per SM, between 64 charged atoms (16,000-atom systems otherwise filled 6
-    // of the SMs) and 256 (one staged tile), longer only to bound the number of partial sums
-    const double target_blocks = (double)f->num_sms * (2048 / f->rho_threads) * 2.0;
-    const double per_item = (double)std::max(1, f->nq) * ntiles;
-    const double chunk_atoms = std::max(std::min(256.0, std::max(64.0, per_item / (3.0 * f->num_sms))),
-                                        per_item / target_blocks);
+    const double target_blocks = 148.0 * (2048 / f->rho_threads) * 2.0;
+    const double chunk_atoms = std::max(256.0, (double)std::max(1, f->nq) * ntiles / target_blocks);
     for (int r = 0; r < nrep; ++r) {
       const int Nr = (int)(qoff[r + 1] - qoff[r]);   // charged atoms of replica r
       const int nch = std::max(1, (int)std::lround(Nr / chunk_atoms));
@@ -2525,10 +2387,6 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     CK(dalloc(&f->d_items, items.size()));
     CK(cudaMemcpy(f->d_items, items.data(), sizeof(RhoItem) * items.size(), cudaMemcpyHostToDevice));
     CK(dalloc(&f->d_rhorep, (size_t)nrep));
-    std::vector<int> cidx(n, -1);
-    for (int c = 0; c < f->nq; ++c) cidx[qidx[c]] = c;
-    CK(dalloc(&f->d_cidx, n));
-    CK(cudaMemcpy(f->d_cidx, cidx.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(f->d_rhorep, rr.data(), sizeof(RhoRep) * nrep, cudaMemcpyHostToDevice));
     CK(cudaMalloc(&f->d_partial, (size_t)f->nitems * f->ktile * 2 * (fp64 ? sizeof(double) : sizeof(float))));
     // shared-memory staging of k records in the force pass: the largest k range a 128-slot block
@@ -2584,14 +2442,6 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
       for (int r = 0; r < nrep; ++r) {
         const double* L = f->reps_h[r].box_d;
         const int K = f->kmax;
-    int most = 1;
-    for (const RhoRep& q : rr) most = std::max(most, q.nchunks);
-    f->finish_warps = 1;
-    if (most <= kFusedChunks) {
-      CK(dalloc(&f->d_rho_done, (size_t)nrep));
-      CK(cudaMemset(f->d_rho_done, 0, sizeof(int) * nrep));
-    }
-    while (f->finish_warps < kFinishWarps && 2 * f->finish_warps <= most) f->finish_warps *= 2;
         for (int i = -K; i <= K; ++i)
           for (int j = -K; j <= K; ++j)
             for (int k = -K; k <= K; ++k) {
@@ -2613,10 +2463,10 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     std::vector<int> crb(nrep + 1);
     for (int r = 0; r < nrep; ++r) {
       crb[r] = (int)ch.size();
-      for (int64_t b = f->rep_off[r]; b < f->rep_off[r + 1]; b += chunk) {
+      for (int64_t b = f->rep_off[r]; b < f->rep_off[r + 1]; b += kMdChunk) {
         MdChunk c;
         c.begin = (int)b;
-        c.end = (int)std::min<int64_t>(b + chunk, f->rep_off[r + 1]);
+        c.end = (int)std::min<int64_t>(b + kMdChunk, f->rep_off[r + 1]);
         c.rep = r;
         c.pad = 0;
         ch.push_back(c);
@@ -2650,10 +2500,6 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
       const size_t rows = s.size() / 7;
       std::vector<float4> v(2 * rows);
       for (size_t m = 0; m < rows; ++m) {
-    // about eight blocks of 256 threads per SM, one to four atoms a thread: a block of 2048 atoms
-    // walks eight atoms a thread in FP64 (10 us), 4,000 atoms filled two such blocks, and the
-    // ragged last chunks of 512 replicas left a long tail (75 us)
-    const int chunk = std::min(kMdChunkMax, std::max(256, (f->n / (8 * f->num_sms) + 255) / 256 * 256));
         v[2 * m] = make_float4(s[7 * m], s[7 * m + 1], s[7 * m + 2], s[7 * m + 3]);
         v[2 * m + 1] = make_float4(s[7 * m + 4], s[7 * m + 5], s[7 * m + 6], 0.f);
       }
@@ -2674,8 +2520,6 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
   // water
   if (f->n_mol > 0) {
     CK(dalloc(&f->d_hoh, (size_t)3 * f->n_mol));
-    CK(dalloc(&f->d_chunk_done, (size_t)nrep));
-    CK(cudaMemset(f->d_chunk_done, 0, sizeof(int) * nrep));
     CK(cudaMemcpy(f->d_hoh, f->hoh_h.data(), sizeof(int) * 3 * f->n_mol, cudaMemcpyHostToDevice));
     CK(dalloc(&f->d_ebond, (size_t)f->n_mol));
     CK(dalloc(&f->d_eangle, (size_t)f->n_mol));
@@ -2757,7 +2601,6 @@ rbmd_status rbmd_force_autotune(rbmd_force* f, void* stream, int32_t* list_lanes
   if (st) return st;
   if (list_lanes) *list_lanes = f->tpa_list;
   if (force_lanes) *force_lanes = f->near_lanes > 1 ? -f->near_lanes : f->tpa_near;
-  f->rebuild_clear = false;
   return RBMD_OK;
 }
 
@@ -2805,34 +2648,6 @@ rbmd_status rbmd_force_compute_host_f32(rbmd_force* f, const float* pos_host, fl
   const int grid = (int)std::min<long long>((m + 255) / 256, 8LL * f->num_sms);
   CK(cudaMemcpyAsync(f->d_host32, pos_host, sizeof(float) * m, cudaMemcpyHostToDevice, s));
   k_f32_to_f64<<<grid, 256, 0, s>>>(m, f->d_host32, f->at.pos);
-    {
-      // the value rows, and whether two tables of them fit the shared memory of a block
-      const size_t rows = (size_t)f->eam_h.nr + 1;
-      int dev = 0, limit = 0;
-      CK(cudaGetDevice(&dev));
-      CK(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-      const size_t bytes = 2 * rows * sizeof(float4);
-      f->eam_smem = !fp64 && !f->is_rbl() && bytes <= (size_t)limit && f->eam_h.rhor.size() >= 7 * rows &&
-                    f->eam_h.z2r.size() >= 7 * rows;
-      if (f->eam_smem) {
-        std::vector<float4> v(2 * rows);
-        for (size_t m = 0; m < rows; ++m) {
-          const float *r = &f->eam_h.rhor[7 * m], *z = &f->eam_h.z2r[7 * m];
-          v[m] = make_float4(r[3], r[4], r[5], r[6]);
-          v[rows + m] = make_float4(z[3], z[4], z[5], z[6]);
-        }
-        CK(dalloc(&f->d_eam_rows, v.size()));
-        CK(cudaMemcpy(f->d_eam_rows, v.data(), bytes, cudaMemcpyHostToDevice));
-        CK(dalloc(&f->d_posf, n));
-        const void* kerns[8] = {
-            (const void*)k_eam_fp_smem<false, 4>,    (const void*)k_eam_fp_smem<false, 16>,
-            (const void*)k_eam_fp_smem<true, 4>,     (const void*)k_eam_fp_smem<true, 16>,
-            (const void*)k_eam_force_smem<false, 4>, (const void*)k_eam_force_smem<false, 16>,
-            (const void*)k_eam_force_smem<true, 4>,  (const void*)k_eam_force_smem<true, 16>};
-        for (const void* k : kerns)
-          CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
-      }
-    }
   for (int attempt = 0; attempt < 4; ++attempt) {
     f->launches = 1;
     launch_compute_any(f, s);
@@ -2906,7 +2721,6 @@ rbmd_status rbmd_force_sync_velocities(rbmd_force* f, void* stream) {
 rbmd_status rbmd_force_energy(rbmd_force* f, rbmd_energy* out, void* stream) {
   if (!f || !out) return RBMD_ERR_ARG;
   if (!f->bound) return RBMD_ERR_STATE;
-    CK(cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s));   // longest overflowed row of this call
   cudaStream_t s = (cudaStream_t)stream;
   std::memset(out, 0, sizeof *out);
   CK(cudaMemsetAsync(f->d_esum, 0, sizeof(double) * 32, s));
