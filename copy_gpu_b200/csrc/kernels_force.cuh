@@ -927,6 +927,7 @@ __global__ void __launch_bounds__(256) k_sample(int nrep, const SamplerRep* __re
 // unwrapped since the build).  FP32 uses r = rsq * rsqrt(rsq) and 1/r = rsqrt(rsq).
 // ------------------------------------------------------------------------------------------
 struct EamDev {
+  const float4* rows;   // value rows (c3, c4, c5, c6) of rho(r) [nr + 1], then of z2(r) [nr + 1]
   const float4* frho;   // 2 float4 per row
   const float4* rhor;
   const float4* z2r;
@@ -1067,6 +1068,178 @@ __global__ void __launch_bounds__(128) k_eam_force(int n, int stride, int cap, d
   force[3 * id + 1] = F[1];
   force[3 * id + 2] = F[2];
   if (pair_slot) pair_slot[i] = 0.5 * (double)epair;
+}
+
+// EAM passes in FP32 with the spline tables in shared memory, for tables whose value rows fit
+// (launch_eam).  The per-pair work is a gather of 16-byte spline rows at random indexes: from L1 it
+// takes a tag lookup per lane, from shared memory about 11 cycles a warp, so one block per SM copies
+// the rows once and walks the atoms.  Rows hold the value polynomial alone, (c3, c4, c5, c6) of
+// rho(r) and of z2(r): the derivative is (3 c3 p^2 + 2 c4 p + c5) / dr, which the seven-coefficient
+// rows store rounded (their c0..c2).  G lanes per atom share a row of the list, lane s taking the
+// chunks s, s + G, .. of four entries (the last chunk is filled with the slot itself, which the
+// predicate 0.01 < r^2 < rc^2 refuses); each term goes into a two-float accumulator, the lanes'
+// sums are combined in FP64 by a fixed butterfly.  Pass 1 also writes (x, y, z, F'(rho)) per slot, so
+// that pass 2 needs one gather per neighbour.  Pair physics as k_eam_fp and k_eam_force.
+constexpr int kEamThreads = 1024;
+
+template <bool MI>
+__device__ __forceinline__ void eam_vec(const float4& pi, const float4& pj, int e, const float* wrap, const float* box,
+                                        const float* ibox, float* r) {
+  r[0] = pj.x;
+  r[1] = pj.y;
+  r[2] = pj.z;
+  if ((e & 63) != 0) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int cd = (e >> (2 * d)) & 3;
+      r[d] -= cd == 1 ? wrap[d] : (cd == 2 ? -wrap[d] : 0.f);
+    }
+  }
+  r[0] = pi.x - r[0];
+  r[1] = pi.y - r[1];
+  r[2] = pi.z - r[2];
+  if (MI) {   // MinDistanceVec
+#pragma unroll
+    for (int d = 0; d < 3; ++d) r[d] -= box[d] * rint(r[d] * ibox[d]);
+  }
+}
+
+// spline row and offset of distance r; row 0 (for a NaN of the filler entries) exists
+__device__ __forceinline__ int eam_row(float r, float rdr, int nr, float& p) {
+  const float pp = r * rdr + 1.0f;
+  const int m = max(0, min((int)pp, nr - 1));
+  p = fminf(pp - (float)m, 1.0f);
+  return m;
+}
+
+template <bool MI, int G>
+__global__ void __launch_bounds__(kEamThreads, 1) k_eam_fp_smem(
+    int n, int stride, int cap, float rc, EamDev eam, const float4* __restrict__ pos4, const int4* __restrict__ nbr4,
+    const int* __restrict__ count, const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot,
+    float4* __restrict__ posf, double* __restrict__ embed_slot) {
+  extern __shared__ float4 eam_tab[];
+  for (int t = threadIdx.x; t <= eam.nr; t += blockDim.x) eam_tab[t] = eam.rows[t];
+  __syncthreads();
+  const int sub = threadIdx.x % G;
+  const float cut2 = rc * rc;
+  for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; (at & ~31LL) < (long long)n * G;
+       at += (long long)gridDim.x * blockDim.x) {
+    const bool active = at / G < n;
+    const int i = active ? (int)(at / G) : n - 1;
+    const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
+    const float4 pi = pos4[i];
+    const float box[3] = {rp.box_f[0], rp.box_f[1], rp.box_f[2]};
+    const float ibox[3] = {1.f / box[0], 1.f / box[1], 1.f / box[2]};
+    const int nch = active ? (min(count[i], cap) + 3) >> 2 : 0;
+    const int last = __reduce_max_sync(0xffffffffu, nch);
+    const int self = i << kShiftBits;
+    const int4 idle = make_int4(self, self, self, self);
+    Acc<float> rho;
+    int4 e = sub < nch ? __ldg(nbr4 + (size_t)sub * stride + i) : idle;
+    for (int c = sub; c - sub < last; c += G) {
+      const int ee[4] = {e.x, e.y, e.z, e.w};
+      float4 pj[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) pj[k] = pos4[ee[k] >> kShiftBits];
+      e = c + G < nch ? __ldg(nbr4 + (size_t)(c + G) * stride + i) : idle;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float r[3], p;
+        eam_vec<MI>(pi, pj[k], ee[k], rp.wrap_f, box, ibox, r);
+        const float rsq = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+        const bool in = rsq < cut2 && rsq > 0.01f;
+        const float4 a = eam_tab[eam_row(rsq * rsqrt_r(rsq), eam.rdr, eam.nr, p)];
+        rho.add(in ? ((a.x * p + a.y) * p + a.z) * p + a.w : 0.f);
+      }
+    }
+    double sum = rho.value();
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (!active || sub != 0) continue;
+    const float rr = (float)sum;
+    float pp = rr * eam.rdrho + 1.0f;
+    const int m = max(1, min((int)pp, eam.nrho - 1));
+    pp = fminf(pp - (float)m, 1.0f);
+    const float4 a = __ldg(eam.frho + 2 * m + 0), b = __ldg(eam.frho + 2 * m + 1);
+    const float fp = (a.x * pp + a.y) * pp + a.z;
+    posf[i] = make_float4(pi.x, pi.y, pi.z, fp);
+    double phi = (((double)a.w * pp + (double)b.x) * pp + (double)b.y) * pp + (double)b.z;
+    if ((double)rr > eam.rhomax) phi += (double)fp * ((double)rr - eam.rhomax);
+    embed_slot[i] = phi;
+  }
+}
+
+template <bool MI, int G>
+__global__ void __launch_bounds__(kEamThreads, 1) k_eam_force_smem(
+    int n, int stride, int cap, float rc, EamDev eam, const float4* __restrict__ posf, const int4* __restrict__ nbr4,
+    const int* __restrict__ count, const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot,
+    const int* __restrict__ slot_atom, double* __restrict__ force, double* __restrict__ pair_slot, uint32_t* status,
+    int ref_sign) {
+  extern __shared__ float4 eam_tab[];   // rows of rho, then of z2
+  for (int t = threadIdx.x; t < 2 * (eam.nr + 1); t += blockDim.x) eam_tab[t] = eam.rows[t];
+  __syncthreads();
+  const float4* ztab = eam_tab + eam.nr + 1;
+  const int sub = threadIdx.x % G;
+  const float cut2 = rc * rc;
+  // ref_sign: the reference's Verlet pass uses MinDistanceVec(p_j, p_i) (RunWorklet.cpp:402)
+  const float sgn = ref_sign ? 1.f : -1.f;
+  for (long long at = (long long)blockIdx.x * blockDim.x + threadIdx.x; (at & ~31LL) < (long long)n * G;
+       at += (long long)gridDim.x * blockDim.x) {
+    const bool active = at / G < n;
+    const int i = active ? (int)(at / G) : n - 1;
+    const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
+    const float4 pi = posf[i];
+    const float box[3] = {rp.box_f[0], rp.box_f[1], rp.box_f[2]};
+    const float ibox[3] = {1.f / box[0], 1.f / box[1], 1.f / box[2]};
+    const int nch = active ? (min(count[i], cap) + 3) >> 2 : 0;
+    const int last = __reduce_max_sync(0xffffffffu, nch);
+    const int self = i << kShiftBits;
+    const int4 idle = make_int4(self, self, self, self);
+    Acc3<float> F;
+    float epair = 0.f;
+    int4 e = sub < nch ? __ldg(nbr4 + (size_t)sub * stride + i) : idle;
+    for (int c = sub; c - sub < last; c += G) {
+      const int ee[4] = {e.x, e.y, e.z, e.w};
+      float4 pj[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) pj[k] = posf[ee[k] >> kShiftBits];
+      e = c + G < nch ? __ldg(nbr4 + (size_t)(c + G) * stride + i) : idle;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float r[3], p;
+        eam_vec<MI>(pi, pj[k], ee[k], rp.wrap_f, box, ibox, r);
+        const float rsq = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+        const bool in = rsq < cut2 && rsq > 0.01f;
+        const float recip = rsqrt_r(rsq);
+        const int m = eam_row(rsq * recip, eam.rdr, eam.nr, p);
+        const float4 a = eam_tab[m], z = ztab[m];
+        const float rhop = (((a.x * 3.f) * p + (a.y + a.y)) * p + a.z) * eam.rdr;
+        const float z2p = (((z.x * 3.f) * p + (z.y + z.y)) * p + z.z) * eam.rdr;
+        const float z2 = ((z.x * p + z.y) * p + z.z) * p + z.w;
+        const float phi = z2 * recip;
+        const float phip = z2p * recip - phi * recip;
+        const float psip = pi.w * rhop + pj[k].w * rhop + phip;
+        const float fpair = in ? sgn * psip * recip : 0.f;
+        F.add(r[0] * fpair, r[1] * fpair, r[2] * fpair);
+        epair += in ? phi : 0.f;
+      }
+    }
+    double Fd[3] = {F.vx(), F.vy(), F.vz()}, ep = (double)epair;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      Fd[0] += __shfl_xor_sync(0xffffffffu, Fd[0], o);
+      Fd[1] += __shfl_xor_sync(0xffffffffu, Fd[1], o);
+      Fd[2] += __shfl_xor_sync(0xffffffffu, Fd[2], o);
+      ep += __shfl_xor_sync(0xffffffffu, ep, o);
+    }
+    if (!active || sub != 0) continue;
+    if (!isfinite(Fd[0]) || !isfinite(Fd[1]) || !isfinite(Fd[2])) set_flag(status, kFlagNonFinite);
+    const int id = slot_atom[i];
+    force[3 * id] = Fd[0];
+    force[3 * id + 1] = Fd[1];
+    force[3 * id + 2] = Fd[2];
+    pair_slot[i] = 0.5 * ep;
+  }
 }
 
 }  // namespace rbmd

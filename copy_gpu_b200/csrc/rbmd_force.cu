@@ -226,6 +226,8 @@ struct rbmd_force {
   bool pending_scale = false;
   // EAM device
   float4 *d_frho = nullptr, *d_rhor = nullptr, *d_z2r = nullptr;
+  float4 *d_eam_rows = nullptr, *d_posf = nullptr;   // value rows of rho and z2; (x, y, z, F'(rho)) per slot
+  bool eam_smem = false;        // FP32 tables small enough for the passes with rows in shared memory
   void* d_fp = nullptr;
   double *d_emb = nullptr, *d_epair = nullptr;
   float* d_host32 = nullptr;   // [3 n] staging of rbmd_force_compute_host_f32 (positions in, forces out)
@@ -412,7 +414,7 @@ void free_all(rbmd_force* f) {
   dfree(f->d_rho); dfree(f->d_ek); dfree(f->d_far); dfree(f->d_weights); dfree(f->d_srep); dfree(f->d_qtab);
   dfree(f->d_chunks); dfree(f->d_chunk_rep_begin); dfree(f->d_ke_partial); dfree(f->d_ke);
   dfree(f->d_T); dfree(f->d_lambda); dfree(f->d_xi); dfree(f->d_xold); dfree(f->d_vold);
-  dfree(f->d_frho); dfree(f->d_rhor); dfree(f->d_z2r);
+  dfree(f->d_frho); dfree(f->d_rhor); dfree(f->d_z2r); dfree(f->d_eam_rows); dfree(f->d_posf);
   if (f->d_fp) cudaFree(f->d_fp);
   f->d_fp = nullptr;
   dfree(f->d_emb); dfree(f->d_epair); dfree(f->d_hoh); dfree(f->d_ebond); dfree(f->d_eangle); dfree(f->d_ewcoul);
@@ -1055,9 +1057,9 @@ void launch_near(rbmd_force* f, cudaStream_t s) {
   else launch_near_m<R, false>(f, s);
 }
 
-template <class R>
-void launch_eam(rbmd_force* f, cudaStream_t s) {
+EamDev eam_dev(const rbmd_force* f) {
   EamDev e;
+  e.rows = f->d_eam_rows;
   e.frho = f->d_frho;
   e.rhor = f->d_rhor;
   e.z2r = f->d_z2r;
@@ -1068,7 +1070,37 @@ void launch_eam(rbmd_force* f, cudaStream_t s) {
   e.rdr_d = 1.0 / (double)f->eam_h.dr;
   e.rdrho_d = 1.0 / (double)f->eam_h.drho;
   e.rhomax = f->eam_h.rhomax;
+  return e;
+}
+
+// FP32 passes with the spline rows in shared memory (k_eam_fp_smem, k_eam_force_smem): one block of
+// 1024 threads per SM at most.  Four lanes per atom balance the blocks' shares and keep the rows of
+// about 53 listed neighbours four iterations long; systems that would leave SMs idle with four
+// lanes take 16.
+template <bool MI, int G>
+void launch_eam_smem(rbmd_force* f, cudaStream_t s, const EamDev& e, const int* rp) {
+  const long long blocks = ((long long)f->n * G + kEamThreads - 1) / kEamThreads;
+  const int grid = (int)std::min<long long>(blocks, f->num_sms);
+  const size_t row_bytes = (size_t)(e.nr + 1) * sizeof(float4);
+  k_eam_fp_smem<MI, G><<<grid, kEamThreads, row_bytes, s>>>(
+      f->n, f->stride, f->cap, (float)f->rc, e, (const float4*)f->d_pos4, (const int4*)f->d_nbr, f->d_count, f->d_reps,
+      rp, f->d_posf, f->d_emb);
+  k_eam_force_smem<MI, G><<<grid, kEamThreads, 2 * row_bytes, s>>>(
+      f->n, f->stride, f->cap, (float)f->rc, e, f->d_posf, (const int4*)f->d_nbr, f->d_count, f->d_reps, rp,
+      f->d_slot_atom, f->at.force, f->d_epair, f->d_status, f->eam_ref_sign ? 1 : 0);
+  f->launches += 2;
+}
+
+template <class R>
+void launch_eam(rbmd_force* f, cudaStream_t s) {
+  const EamDev e = eam_dev(f);
   const int* rp = f->nrep > 1 ? f->d_rep_of : nullptr;
+  if (sizeof(R) == 4 && f->eam_smem) {
+    const bool few = 4LL * f->n < (long long)kEamThreads * f->num_sms;
+    if (f->minimg) few ? launch_eam_smem<true, 16>(f, s, e, rp) : launch_eam_smem<true, 4>(f, s, e, rp);
+    else few ? launch_eam_smem<false, 16>(f, s, e, rp) : launch_eam_smem<false, 4>(f, s, e, rp);
+    return;
+  }
   const int bs = 128;
   const int nb = (f->n + bs - 1) / bs;
   auto fp_kern = f->minimg ? k_eam_fp<R, true> : k_eam_fp<R, false>;
@@ -1112,17 +1144,7 @@ void launch_rbl_force(rbmd_force* f, cudaStream_t s) {
   const int* rp = f->nrep > 1 ? f->d_rep_of : nullptr;
   const int nb = (f->n + 127) / 128;
   if (f->is_eam()) {
-    EamDev e;
-    e.frho = f->d_frho;
-    e.rhor = f->d_rhor;
-    e.z2r = f->d_z2r;
-    e.nrho = f->eam_h.nrho;
-    e.nr = f->eam_h.nr;
-    e.rdr = 1.0f / f->eam_h.dr;
-    e.rdrho = 1.0f / f->eam_h.drho;
-    e.rdr_d = 1.0 / (double)f->eam_h.dr;
-    e.rdrho_d = 1.0 / (double)f->eam_h.drho;
-    e.rhomax = f->eam_h.rhomax;
+    const EamDev e = eam_dev(f);
     k_rbl_eam_fp<R><<<nb, 128, 0, s>>>(f->n, f->stride, f->core_cap, f->shell_cap, f->rc, f->rs, e,
                                         (const typename Traits<R>::V4*)f->d_pos4, f->d_nbr, f->d_count,
                                         f->d_count2, f->d_reps, rp, (R*)f->d_fp, f->d_emb);
@@ -2514,6 +2536,34 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     s1 = up(f->eam_h.z2r, &f->d_z2r);
     if (s1) return s1;
     CK(cudaMalloc(&f->d_fp, n * (fp64 ? sizeof(double) : sizeof(float))));
+    {
+      // the value rows, and whether two tables of them fit the shared memory of a block
+      const size_t rows = (size_t)f->eam_h.nr + 1;
+      int dev = 0, limit = 0;
+      CK(cudaGetDevice(&dev));
+      CK(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+      const size_t bytes = 2 * rows * sizeof(float4);
+      f->eam_smem = !fp64 && !f->is_rbl() && bytes <= (size_t)limit && f->eam_h.rhor.size() >= 7 * rows &&
+                    f->eam_h.z2r.size() >= 7 * rows;
+      if (f->eam_smem) {
+        std::vector<float4> v(2 * rows);
+        for (size_t m = 0; m < rows; ++m) {
+          const float *r = &f->eam_h.rhor[7 * m], *z = &f->eam_h.z2r[7 * m];
+          v[m] = make_float4(r[3], r[4], r[5], r[6]);
+          v[rows + m] = make_float4(z[3], z[4], z[5], z[6]);
+        }
+        CK(dalloc(&f->d_eam_rows, v.size()));
+        CK(cudaMemcpy(f->d_eam_rows, v.data(), bytes, cudaMemcpyHostToDevice));
+        CK(dalloc(&f->d_posf, n));
+        const void* kerns[8] = {
+            (const void*)k_eam_fp_smem<false, 4>,    (const void*)k_eam_fp_smem<false, 16>,
+            (const void*)k_eam_fp_smem<true, 4>,     (const void*)k_eam_fp_smem<true, 16>,
+            (const void*)k_eam_force_smem<false, 4>, (const void*)k_eam_force_smem<false, 16>,
+            (const void*)k_eam_force_smem<true, 4>,  (const void*)k_eam_force_smem<true, 16>};
+        for (const void* k : kerns)
+          CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+      }
+    }
     CK(dalloc(&f->d_emb, n));
     CK(dalloc(&f->d_epair, n));
   }

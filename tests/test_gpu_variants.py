@@ -1,0 +1,96 @@
+"""Kernel variants chosen by size, at the edges of their rules.
+
+* EAM in FP32 with the spline rows in shared memory (tables up to the shared-memory limit, one row
+  longer falls back to the global tables) against the FP64 passes on the same file: 1e-5 of the force
+  rms, the FP32 parity bar; boxes of 2 cells per axis (per-pair minimum image) and of 3.
+* RBL lists built by one warp per cell (the default) equal those of one thread per atom entry for
+  entry, from a few atoms to cells of more than 32 atoms and several batches of candidates.
+* Lanes per charged atom of the RBE force and short structure-factor chunks: one to a few thousand
+  charged atoms against the FP64 oracle, no worse than 1e-5 of the largest force (FP32 bar).
+"""
+import numpy as np
+import pytest
+
+from copy_gpu_b200 import systems
+from tests.helpers import jitter, make_ff, rel_err, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _eam_force(s, path, prec, cuda):
+    import torch
+    cfg = systems.eam_config(path, precision=prec)
+    cfg["hyper_parameters"]["force_field"]["potential_format"] = "setfl"
+    dev = to_dev(s, cuda)
+    ff = make_ff(cfg, s, dev)
+    ff.Execute()
+    torch.cuda.synchronize()
+    assert ff.status() == 0
+    e = ff.energy()
+    return dev["force"].cpu().numpy(), e["eam_embed"] + e["eam_pair"]
+
+
+@pytest.mark.parametrize("ncell,npts", [(4, 5000), (5, 5000), (5, 64), (9, 5000), (6, 7262), (6, 9000)])
+def test_eam_rows_in_shared_memory(cuda, tmp_path, ncell, npts):
+    p = dict(systems.JOHNSON_CU, npts=npts)
+    path = systems.write_johnson_setfl(str(tmp_path / "j.setfl"), p)
+    s = systems.eam_fcc(ncell=ncell, seed=3)
+    f32, e32 = _eam_force(s, path, "fp32", cuda)
+    f64, e64 = _eam_force(s, path, "fp64", cuda)
+    # the FP32 pass differentiates the value rows, the FP64 pass reads the rounded derivative rows:
+    # with npts rows over 5 A the float row values carry 6e-8 npts / 12 of a row's slope
+    bar = 1e-5 + 6e-8 * npts / 12
+    assert rel_err(f32, f64) <= bar, rel_err(f32, f64)
+    assert abs(e32 - e64) <= 1e-6 * abs(e64)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("case", ["tiny", "chains", "dense", "wide", "outside"])
+def test_rbl_cell_list_identical(cuda, prec, case):
+    import torch
+    if case == "chains":
+        s = systems.molecular(n_chain=27, chain_len=12, n_ion_pairs=4, step=1.5, cell=8.0, seed=5)
+        rc, rcore = 10.0, 5.0
+    else:
+        s = systems.lj_fcc(ncell={"tiny": 2, "dense": 8, "wide": 6, "outside": 7}[case], seed=4)
+        s["pos"] = jitter(s["pos"], s["lo"], s["hi"], 0.08, seed=5)
+        # tiny: fewer cells than the stencil; dense: about 75 atoms a cell; wide: num_cycles 3;
+        # outside: atoms up to 1.2 beyond the faces, binned into the boundary cells
+        rc, rcore = {"tiny": (1.6, 0.8), "dense": (8.0, 4.5), "wide": (3.4, 1.2), "outside": (3.0, 1.6)}[case]
+        if case == "outside":
+            rng = np.random.default_rng(8)
+            s["pos"][:200] += rng.uniform(-1.2, 1.2, size=(200, 3))
+    out = []
+    for mode in ("auto", "thread"):
+        cfg = systems.lj_config(cutoff=rc, precision=prec)
+        cfg["hyper_parameters"]["neighbor"].update(type="RBL", r_core=rcore, neighbor_sample_num=20)
+        cfg["tuning"] = {"rbl_list": mode}
+        dev = to_dev(s, cuda)
+        ff = make_ff(cfg, s, dev)
+        ff.Execute()
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        c, ids = ff.neighbors(1024)
+        ncore, nshell, _ = ff.rbl_lists()
+        out.append((c, ids, ncore, nshell, dev["force"].cpu().numpy()))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("nq,P", [(2, 1), (2, 33), (66, 100), (258, 305), (3000, 64), (5000, 520)])
+def test_kspace_small_counts(cuda, oracle_lib, nq, P):
+    import torch
+    s = systems.electrolyte(max(600, nq), ion_frac=min(1.0, nq / max(600, nq)), seed=5)
+    cfg = systems.electrolyte_config(P=P, precision="fp32", seed=2)
+    alpha = cfg["hyper_parameters"]["coulomb"]["alpha"]
+    L = s["hi"] - s["lo"]
+    m = oracle_lib.rbe_sample(alpha, L, seed=5, step=0, rep=0, P=P)
+    dev = to_dev(s, cuda)
+    ff = make_ff(cfg, s, dev)
+    ff.set_ksamples(m)
+    ff.Execute()
+    torch.cuda.synchronize()
+    rho = oracle_lib.rhok(s["pos"], s["charge"], L, m)
+    far = oracle_lib.rbe_force(s["pos"], s["charge"], L, alpha, 1.0, m, rho)
+    got = ff.far_force()
+    assert np.abs(got - far).max() <= 1e-5 * np.abs(far).max()
