@@ -293,15 +293,18 @@ __global__ void __launch_bounds__(256) k_near_force(
 // Pair physics as k_near_force: ComputeNearForceVerletWorklet / ComputeLJForceVerletWorklet
 // (rbmd/framework/run/worklet/RunWorklet.cpp:170-303), ExecForceFunction::ComputeLJForce and
 // ComputeNearEnergyForce (rbmd/framework/forceFunction/ExecForceFunction.h:74-140).
-template <class R, bool COUL, int MI, bool ENERGY>
-__global__ void __launch_bounds__(256) k_near_lean(
+// G > 1: G lanes per atom for systems with too few atoms to fill the chip; lane s takes the chunks
+// s, s + G, .. and the lanes' sums are combined in FP64 by a fixed butterfly.
+// FP32 is held to 64 registers (32 warps per SM; 74 without): 1,000,000 atoms 191 -> about 183 us.
+template <class R, bool COUL, int MI, bool ENERGY, int G>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_lean(
     NearParams prm, R a24, R s6, R d2_max, const typename Traits<R>::V4* __restrict__ pos4,
     const int4* __restrict__ nbr4, const int* __restrict__ count, const RepDev* __restrict__ reps,
     const int* __restrict__ rep_of_slot, const int* __restrict__ slot_atom, double* __restrict__ force,
     double* __restrict__ energy_slot, uint32_t* status) {
   static_assert((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0, "k_near_lean: no per-pair minimum image, no weights");
   using V4 = typename Traits<R>::V4;
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gid = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G), sub = threadIdx.x % G;
   const bool active = gid < prm.n;   // lanes past the end run along with an empty row
   const int i = active ? gid : prm.n - 1;
   const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
@@ -310,21 +313,21 @@ __global__ void __launch_bounds__(256) k_near_lean(
   const R sa = (R)prm.sqrt_alpha, aa = (R)prm.alpha, c2 = (R)prm.two_sqrt_alpha_over_sqrt_pi;
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
-  const int cnt = active ? min(count[i], prm.cap) : 0;
-  const int last = __reduce_max_sync(0xffffffffu, cnt);
+  const int nch = active ? (min(count[i], prm.cap) + 3) >> 2 : 0;   // chunks of the row
+  const int last = __reduce_max_sync(0xffffffffu, nch);
   const int self = i << kShiftBits;
   const int4 idle = make_int4(self, self, self, self);
   // 24 eps (2 s6 u - 1) s6 u / d^2 with u = d^-6 as (ka u - kb) d^-8
   const Pair<R> ka = both<R>((R)2 * a24 * s6 * s6), kb = both<R>(-a24 * s6);
   Acc3<R> F;
   R e_lj = 0, e_coul = 0;
-  const int4* row = nbr4 + i;
-  const size_t st = (size_t)prm.stride;
-  int4 e = cnt > 0 ? __ldg(row) : idle;
-  int4 e_nxt = cnt > 4 ? __ldg(row + st) : idle;
+  const size_t st = (size_t)prm.stride * G;
+  const int4* row = nbr4 + (size_t)prm.stride * sub + i;
+  int4 e = sub < nch ? __ldg(row) : idle;
+  int4 e_nxt = sub + G < nch ? __ldg(row + st) : idle;
   row += 2 * st;
   V4 pj[4] = {pos4[e.x >> kShiftBits], pos4[e.y >> kShiftBits], pos4[e.z >> kShiftBits], pos4[e.w >> kShiftBits]};
-  for (int p = 0; p < last; p += 4, row += st) {
+  for (int c = sub; c - sub < last; c += G, row += st) {
     if (__any_sync(0xffffffffu, ((e.x | e.y | e.z | e.w) & 63) != 0)) {   // p_j - PeriodicCoordOffset
       const int ee[4] = {e.x, e.y, e.z, e.w};
       const R w0 = Traits<R>::wrap(rp, 0), w1 = Traits<R>::wrap(rp, 1), w2 = Traits<R>::wrap(rp, 2);
@@ -384,26 +387,40 @@ __global__ void __launch_bounds__(256) k_near_lean(
     pj[1] = pos4[e.y >> kShiftBits];
     pj[2] = pos4[e.z >> kShiftBits];
     pj[3] = pos4[e.w >> kShiftBits];
-    e_nxt = p + 8 < cnt ? __ldg(row) : idle;
+    e_nxt = c + 2 * G < nch ? __ldg(row) : idle;
   }
-  if (!active) return;
-  const double Fd[3] = {F.vx(), F.vy(), F.vz()};
+  double Fd[3] = {F.vx(), F.vy(), F.vz()}, el = (double)e_lj, ec = (double)e_coul;
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    Fd[0] += __shfl_xor_sync(0xffffffffu, Fd[0], o);
+    Fd[1] += __shfl_xor_sync(0xffffffffu, Fd[1], o);
+    Fd[2] += __shfl_xor_sync(0xffffffffu, Fd[2], o);
+    if (ENERGY) {
+      el += __shfl_xor_sync(0xffffffffu, el, o);
+      ec += __shfl_xor_sync(0xffffffffu, ec, o);
+    }
+  }
+  if (!active || sub != 0) return;
   if (!isfinite(Fd[0]) || !isfinite(Fd[1]) || !isfinite(Fd[2])) set_flag(status, kFlagNonFinite);
   const int id = slot_atom[i];
   force[3 * id] = Fd[0];
   force[3 * id + 1] = Fd[1];
   force[3 * id + 2] = Fd[2];
   if (ENERGY) {
-    energy_slot[2 * i] = 0.5 * (double)e_lj;
-    energy_slot[2 * i + 1] = 0.5 * (double)e_coul;
+    energy_slot[2 * i] = 0.5 * el;
+    energy_slot[2 * i + 1] = 0.5 * ec;
   }
 }
 
-// Near force with G lanes per atom (G = 4 .. 32) for systems with few atoms and long lists
+// Near force with G lanes per atom (G = 4 .. 32) for systems with few atoms or long lists
 // (water at 10 A: ~550 neighbours, 30,000 atoms), where one thread per atom leaves most of the
-// GPU idle.  Lane s of an atom's group takes list entries s, s + G, ...; the pair terms are
-// those of k_near_force (same predicates and arithmetic); each lane accumulates in a two-float
-// accumulator and the group combines its G partial sums in FP64 with a fixed butterfly, so the
+// GPU idle.  Lane s of an atom's group takes the chunks s, s + G, .. of four list entries: one
+// 16-byte load per chunk, the next chunk's entries and the four positions (and, with types or
+// molecules, records) of the current one in flight together, the image offsets decoded in one
+// branch per chunk.  The filler entries of the last chunk hold the slot itself, at distance 0,
+// which no predicate accepts.  The pair terms are those of k_near_force (same predicates and
+// arithmetic); each lane sums the four forces of a chunk and folds them into a two-float
+// accumulator, and the group combines its G partial sums in FP64 with a fixed butterfly, so the
 // result does not depend on scheduling.
 template <class R, bool COUL, int MI, int G>
 __global__ void __launch_bounds__(256) k_near_force_group(
@@ -423,7 +440,7 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   const bool MOLEC = prm.molecular != 0;
   constexpr bool SPW = (MI & kMiSpecial) != 0;
   const bool ENERGY = energy_slot != nullptr;
-  const int gid = (int)((blockIdx.x * blockDim.x + threadIdx.x) / G);
+  const int gid = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) / G);
   const int sub = threadIdx.x % G;
   const bool active = gid < prm.n;   // inactive groups still join the shuffles below
   const int i = active ? gid : prm.n - 1;
@@ -433,85 +450,96 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   const int2 mi = typed ? meta[i] : make_int2(0, 0);
   const R rc = (R)prm.rc;
   const R cut2 = rc * rc;
-  const R box[3] = {Traits<R>::box(rp, 0), Traits<R>::box(rp, 1), Traits<R>::box(rp, 2)};
-  const R wrap[3] = {Traits<R>::wrap(rp, 0), Traits<R>::wrap(rp, 1), Traits<R>::wrap(rp, 2)};
   const R sa = (R)prm.sqrt_alpha, aa = (R)prm.alpha, c2 = (R)prm.two_sqrt_alpha_over_sqrt_pi;
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
   const int trow = prm.ntypes > 1 ? mi.x * prm.ntypes : 0;
-  Acc<R> fx, fy, fz;
-  R gx = 0, gy = 0, gz = 0;
+  const int4* nbr4 = reinterpret_cast<const int4*>(nbr) + i;
+  const int nch = active ? (min(count[i], prm.cap) + 3) >> 2 : 0;
+  const int last = __reduce_max_sync(0xffffffffu, nch);
+  const int self = i << kShiftBits;
+  const int4 idle = make_int4(self, self, self, self);
+  Acc3<R> acc;
   R e_lj = 0, e_coul = 0;
-  const int cnt = active ? min(count[i], prm.cap) : 0;
-  int k = 0;
-  for (int p = sub; p < cnt; p += G, ++k) {
-    const int e = __ldg(nbr + nbr_at(p, i, prm.stride));
-    const V4 pj = pos4[e >> kShiftBits];
-    R px = pj.x, py = pj.y, pz = pj.z;
-    if (e & 63) {
-      const int c0 = e & 3, c1 = (e >> 2) & 3, c2b = (e >> 4) & 3;
-      px = px - (c0 == 1 ? wrap[0] : (c0 == 2 ? -wrap[0] : (R)0));
-      py = py - (c1 == 1 ? wrap[1] : (c1 == 2 ? -wrap[1] : (R)0));
-      pz = pz - (c2b == 1 ? wrap[2] : (c2b == 2 ? -wrap[2] : (R)0));
+  int4 e4 = sub < nch ? __ldg(nbr4 + (size_t)sub * prm.stride) : idle;
+  for (int c = sub; c - sub < last; c += G) {
+    const int ee[4] = {e4.x, e4.y, e4.z, e4.w};
+    V4 pj[4];
+    int2 mj[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) pj[k] = pos4[ee[k] >> kShiftBits];
+    if (typed)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) mj[k] = meta[ee[k] >> kShiftBits];
+    e4 = c + G < nch ? __ldg(nbr4 + (size_t)(c + G) * prm.stride) : idle;
+    if (__any_sync(0xffffffffu, ((ee[0] | ee[1] | ee[2] | ee[3]) & 63) != 0)) {   // p_j - PeriodicCoordOffset
+      const R w0 = Traits<R>::wrap(rp, 0), w1 = Traits<R>::wrap(rp, 1), w2 = Traits<R>::wrap(rp, 2);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int k0 = ee[k] & 3, k1 = (ee[k] >> 2) & 3, k2 = (ee[k] >> 4) & 3;
+        pj[k].x -= k0 == 1 ? w0 : (k0 == 2 ? -w0 : (R)0);
+        pj[k].y -= k1 == 1 ? w1 : (k1 == 2 ? -w1 : (R)0);
+        pj[k].z -= k2 == 1 ? w2 : (k2 == 2 ? -w2 : (R)0);
+      }
     }
-    const R r0 = px - pi.x, r1 = py - pi.y, r2 = pz - pi.z;
-    const R d2 = r0 * r0 + r1 * r1 + r2 * r2;
-    if ((MI & 3) == kMiAll && !((prm.orig ? cut2 - d2 > (R)0 : cut2 - d2 > (R)1.0e-4) && d2 > (R)1.0e-4)) continue;
-    R f = 0;
-    if (COUL) {
-      const R qq = qi * pj.w;
-      if (qq != (R)0) {
-        const R inv = rsqrt_r(d2);
-        const R dis = d2 * inv;
-        if (dis < rc && dis > (R)0.01) {
-          const R ex = exp_r(-aa * d2);
-          const R erfcv = erfc_shared(sa * dis, ex);
-          const R g = (erfcv * inv + c2 * ex) * inv;
-          f = -qq * g * inv * cs;
-          if (ENERGY) e_coul += qq * erfcv * inv * cs;
+    R gx = 0, gy = 0, gz = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const R r0 = pj[k].x - pi.x, r1 = pj[k].y - pi.y, r2 = pj[k].z - pi.z;
+      const R d2 = r0 * r0 + r1 * r1 + r2 * r2;
+      if ((MI & 3) == kMiAll && !((prm.orig ? cut2 - d2 > (R)0 : cut2 - d2 > (R)1.0e-4) && d2 > (R)1.0e-4)) continue;
+      R f = 0;
+      if (COUL) {
+        const R qq = qi * pj[k].w;
+        if (qq != (R)0) {
+          const R inv = rsqrt_r(d2);
+          const R dis = d2 * inv;
+          if (dis < rc && dis > (R)0.01) {
+            const R ex = exp_r(-aa * d2);
+            const R erfcv = erfc_shared(sa * dis, ex);
+            const R g = (erfcv * inv + c2 * ex) * inv;
+            f = -qq * g * inv * cs;
+            if (ENERGY) e_coul += qq * erfcv * inv * cs;
+          }
         }
       }
-    }
-    R fl0 = 0, fl1 = 0, fl2 = 0;
-    bool same = false;
-    int tj = 0;
-    R wsp = (R)1;   // special-bond LJ weight (molecular == 2: meta.y is the bond-graph component)
-    if (typed) {
-      const int2 mj = meta[e >> kShiftBits];
-      same = MOLEC && (mj.y == mi.y);
-      tj = prm.ntypes > 1 ? mj.x : 0;
-      if (SPW && same) {
-        wsp = special_weight<R>(prm.sp, slot_atom[i], slot_atom[e >> kShiftBits]);
-        same = false;
+      R fl0 = 0, fl1 = 0, fl2 = 0;
+      bool same = false;
+      int tj = 0;
+      R wsp = (R)1;   // special-bond LJ weight (molecular == 2: meta.y is the bond-graph component)
+      if (typed) {
+        same = MOLEC && (mj[k].y == mi.y);
+        tj = prm.ntypes > 1 ? mj[k].x : 0;
+        if (SPW && same) {
+          wsp = special_weight<R>(prm.sp, slot_atom[i], slot_atom[ee[k] >> kShiftBits]);
+          same = false;
+        }
       }
-    }
-    if (!same) {
-      R q0 = r0, q1 = r1, q2 = r2;
-      R dl2 = d2;
-      if ((MI & 3) == kMiLJ) {
-        min_image(q0, q1, q2, box);
-        dl2 = q0 * q0 + q1 * q1 + q2 * q2;
+      if (!same) {
+        R q0 = r0, q1 = r1, q2 = r2;
+        R dl2 = d2;
+        if ((MI & 3) == kMiLJ) {
+          const R box[3] = {Traits<R>::box(rp, 0), Traits<R>::box(rp, 1), Traits<R>::box(rp, 2)};
+          min_image(q0, q1, q2, box);
+          dl2 = q0 * q0 + q1 * q1 + q2 * q2;
+        }
+        if (dl2 < cut2 && dl2 > (R)0.0001) {
+          const R inv2 = rcp_r(dl2);
+          const R sd6 = lj_s6[trow + tj] * inv2 * inv2 * inv2;
+          const R a24 = lj_a[trow + tj];
+          R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2;
+          if (SPW) scal *= wsp;
+          fl0 = scal * q0; fl1 = scal * q1; fl2 = scal * q2;
+          if (ENERGY) e_lj += (SPW ? wsp : (R)1) * (-a24 / (R)6 * (sd6 - (R)1) * sd6);
+        }
       }
-      if (dl2 < cut2 && dl2 > (R)0.0001) {
-        const R inv2 = rcp_r(dl2);
-        const R sd6 = lj_s6[trow + tj] * inv2 * inv2 * inv2;
-        const R a24 = lj_a[trow + tj];
-        R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2;
-        if (SPW) scal *= wsp;
-        fl0 = scal * q0; fl1 = scal * q1; fl2 = scal * q2;
-        if (ENERGY) e_lj += (SPW ? wsp : (R)1) * (-a24 / (R)6 * (sd6 - (R)1) * sd6);
-      }
+      gx += f * r0 + fl0;
+      gy += f * r1 + fl1;
+      gz += f * r2 + fl2;
     }
-    gx += f * r0 + fl0;
-    gy += f * r1 + fl1;
-    gz += f * r2 + fl2;
-    if ((k & 3) == 3) {
-      fx.add(gx); fy.add(gy); fz.add(gz);
-      gx = gy = gz = 0;
-    }
+    acc.add(gx, gy, gz);
   }
-  fx.add(gx); fy.add(gy); fz.add(gz);
-  double F[3] = {fx.value(), fy.value(), fz.value()};
+  double F[3] = {acc.vx(), acc.vy(), acc.vz()};
   double el = (double)e_lj, ec = (double)e_coul;
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) {

@@ -123,11 +123,13 @@ struct rbmd_force {
   int cap_override = 0;   // neighbor.capacity: initial list capacity (grown on overflow)
   int tpa_list = 0, tpa_near = 128;     // list build: 0 = one warp per cell, 1 = one warp per atom, else
                                         // threads per block of k_nlist; threads per block of the force pass
-  int rbl_list_warp = -1;               // RBL list build: 1 one warp per atom, 0 one thread per atom, -1 by size
+  double mean_listed = 0;               // listed neighbours per atom expected from the density
+  int rbl_list_warp = -1;               // RBL list build: -1 one warp per cell, 1 one warp per atom, 0 one thread per atom
   int rbl_lanes = 0;                    // RBL force pass lanes per atom (0: by size)
   int num_sms = 148;                    // SMs of the bound device (cudaDevAttrMultiProcessorCount)
   int near_variant = 1;                 // 1: k_near_lean where it applies (lean_ok), 0: k_near_force
   int near_lanes = 1;                   // near pass lanes per atom: 1, or 4 / 8 / 16 / 32
+  bool lanes_set = false;               // given by the configuration or tuned (else near_lanes())
   bool autotune = false;                // "autotune": true tunes them at the first compute
   bool tuned = false;
   bool list_valid = false;   // a list (and x_ref) exists from an earlier build
@@ -359,11 +361,28 @@ int molecular_mode(const rbmd_force* f) {
   return f->at.molecule != nullptr ? 1 : 0;
 }
 
-// k_near_lean applies: one LJ coefficient pair for all types, no molecules, one thread per atom,
-// no per-pair minimum image (a Verlet skin, or boxes of >= 3 cells per axis).
+// k_near_lean applies: one LJ coefficient pair for all types, no molecules, no per-pair minimum
+// image (a Verlet skin, or boxes of >= 3 cells per axis).
 bool lean_ok(const rbmd_force* f) {
   return f->near_variant >= 1 && !f->is_rbl() && !f->is_eam() && f->nt_eff == 1 && molecular_mode(f) == 0 &&
-         f->near_lanes == 1 && (f->skin > 0 || !f->minimg);
+         (f->skin > 0 || !f->minimg);
+}
+
+// Lanes per atom of the near pass when neither the configuration nor the autotuner gave them
+// (B200, microseconds a pass).  Lean pass, electrolyte lists of 78 entries, FP32: 4,000 atoms 1 lane
+// 29 / 16 lanes 10.1; 8,000 8 lanes 14.2 / 16 lanes 15.5; 16,000 1 lane 28 / 8 lanes 15.6; 32,000
+// 4 lanes 21.6 / 8 lanes 22.5; 128,000 1 lane 49 / 4 lanes 44; 256,000 82 / 80, beyond which the
+// FP64 sums of the lanes cost more than they spread (FP64 crosses at 128,000: 109 / 110).  General
+// pass with long lists: water (556 listed) 30,000 atoms 1 lane 409 / 4 lanes 165 / 16 lanes 120 / 32
+// lanes 132, 4,800 359 / 78 / 32 / 37; chains (505 listed) 22,824 427 / 179 / 125 / 142.
+int near_lanes(const rbmd_force* f) {
+  if (f->lanes_set) return f->near_lanes;
+  const int per_sm = f->n / f->num_sms;
+  const bool lean = lean_ok(f);
+  if (!lean && f->mean_listed >= 128.0) return 16;
+  if (per_sm < 40) return 16;
+  if (per_sm < 160) return 8;
+  return !lean || per_sm < (f->fp64 ? 700 : 1400) ? 4 : 1;
 }
 
 // The lean near pass and the per-atom list build run beside the k-space stream and use no shared
@@ -985,6 +1004,19 @@ void launch_kspace(rbmd_force* f, cudaStream_t s, cudaEvent_t ready) {
   cudaEventRecord(f->ev_tail, s);
 }
 
+template <class R, bool COUL, int MI, int G>
+void launch_near_lean(rbmd_force* f, cudaStream_t s, const NearParams& p) {
+  const int bs = G == 1 ? f->tpa_near : 128;
+  const long long threads = (long long)f->n * G;
+  auto kern = f->want_energy ? k_near_lean<R, COUL, MI, true, G> : k_near_lean<R, COUL, MI, false, G>;
+  if (G == 1) prefer_shared_carveout(f, (const void*)kern);
+  kern<<<(unsigned)((threads + bs - 1) / bs), bs, 0, s>>>(
+      p, lj24<R>(f->ljt_h, 0), sig6<R>(f->ljt_h, 0), lean_d2_max<R>(f), (const typename Traits<R>::V4*)f->d_pos4,
+      (const int4*)f->d_nbr, f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
+      f->want_energy ? f->d_eslot : nullptr, f->d_status);
+  f->launches++;
+}
+
 template <class R, bool COUL, int MI>
 void launch_near_t(rbmd_force* f, cudaStream_t s) {
   NearParams p;
@@ -1003,13 +1035,24 @@ void launch_near_t(rbmd_force* f, cudaStream_t s) {
   p.two_sqrt_alpha_over_sqrt_pi = 2.0 * std::sqrt(f->alpha) / std::sqrt(M_PI);
   p.kstage = 0;
   p.orig = f->orig_pred ? 1 : 0;
-  if (f->near_lanes > 1) {
-    const long long threads = (long long)f->n * f->near_lanes;
+  const int g = near_lanes(f);
+  if constexpr ((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0) {
+    // one LJ coefficient pair for all types, no molecules: the lean pass
+    if (lean_ok(f)) {
+      if (g >= 16) launch_near_lean<R, COUL, MI, 16>(f, s, p);
+      else if (g == 8) launch_near_lean<R, COUL, MI, 8>(f, s, p);
+      else if (g == 4) launch_near_lean<R, COUL, MI, 4>(f, s, p);
+      else launch_near_lean<R, COUL, MI, 1>(f, s, p);
+      return;
+    }
+  }
+  if (g > 1) {
+    const long long threads = (long long)f->n * g;
     const int grid = (int)((threads + 255) / 256);
-    auto kern = f->near_lanes == 4    ? k_near_force_group<R, COUL, MI, 4>
-                : f->near_lanes == 8  ? k_near_force_group<R, COUL, MI, 8>
-                : f->near_lanes == 16 ? k_near_force_group<R, COUL, MI, 16>
-                                      : k_near_force_group<R, COUL, MI, 32>;
+    auto kern = g == 4    ? k_near_force_group<R, COUL, MI, 4>
+                : g == 8  ? k_near_force_group<R, COUL, MI, 8>
+                : g == 16 ? k_near_force_group<R, COUL, MI, 16>
+                          : k_near_force_group<R, COUL, MI, 32>;
     kern<<<grid, 256, 0, s>>>(p, f->d_ljt, (const typename Traits<R>::V4*)f->d_pos4, f->d_meta, f->d_nbr,
                               f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom,
                               f->at.force, f->want_energy ? f->d_eslot : nullptr, f->d_status);
@@ -1017,19 +1060,6 @@ void launch_near_t(rbmd_force* f, cudaStream_t s) {
     return;
   }
   const int bs = f->tpa_near;
-  if constexpr ((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0) {
-    // one LJ coefficient pair for all types, no molecules: the lean pass
-    if (lean_ok(f)) {
-      auto kern = f->want_energy ? k_near_lean<R, COUL, MI, true> : k_near_lean<R, COUL, MI, false>;
-      prefer_shared_carveout(f, (const void*)kern);
-      kern<<<(f->n + bs - 1) / bs, bs, 0, s>>>(
-          p, lj24<R>(f->ljt_h, 0), sig6<R>(f->ljt_h, 0), lean_d2_max<R>(f), (const typename Traits<R>::V4*)f->d_pos4,
-          (const int4*)f->d_nbr, f->d_count, f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
-          f->want_energy ? f->d_eslot : nullptr, f->d_status);
-      f->launches++;
-      return;
-    }
-  }
   k_near_force<R, COUL, MI><<<(f->n + bs - 1) / bs, bs, 0, s>>>(
       p, f->d_ljt, (const typename Traits<R>::V4*)f->d_pos4, f->d_meta, f->d_nbr, f->d_count,
       f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_slot_atom, f->at.force,
@@ -1630,11 +1660,11 @@ rbmd_status parse_config(rbmd_force* f, const char* text) {
     auto ok = [](int t) { return t == 64 || t == 128 || t == 256; };
     const Value* tlv = root.path("tuning.list_block");
     if (ok(tl) || (tlv && (tl == 0 || tl == 1))) { f->tpa_list = tl; f->autotune = false; }
-    if (ok(tn)) { f->tpa_near = tn; f->autotune = false; }
+    if (ok(tn)) { f->tpa_near = tn; f->autotune = false; f->lanes_set = true; }
     const Value* nv = root.path("tuning.near_variant");
     if (nv) f->near_variant = (int)num(root, "tuning.near_variant", 1.0) == 0 ? 0 : 1;
     const int ln = (int)num(root, "tuning.force_lanes", 0.0);
-    if (ln == 1 || ln == 4 || ln == 8 || ln == 16 || ln == 32) { f->near_lanes = ln; f->autotune = false; }
+    if (ln == 1 || ln == 4 || ln == 8 || ln == 16 || ln == 32) { f->near_lanes = ln; f->autotune = false; f->lanes_set = true; }
     const std::string rl = rbmdjson::text(root, "tuning.rbl_list", "auto");
     if (rl != "warp" && rl != "thread" && rl != "auto") {
       std::snprintf(g_last_error, sizeof g_last_error,
@@ -1825,6 +1855,7 @@ rbmd_status autotune_impl(rbmd_force* f, cudaStream_t s) {
   const bool prof = f->prof_on;
   f->prof_on = false;
   const int cand[3] = {64, 128, 256};
+  f->lanes_set = true;   // the trials set near_lanes
   // rebuild pattern of the timed list builds: every replica of a single system; in a batch with
   // a Verlet skin about one replica in five rebuilds per step (each decides alone), and the list
   // variants rank differently on such partial rebuilds than on full ones, so one in five is
@@ -2219,6 +2250,7 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
   for (int r = 0; r < nrep; ++r)
     rho_max = std::max(rho_max, (f->rep_off[r + 1] - f->rep_off[r]) / f->reps_h[r].volume);
   const double lc = f->list_cut();
+  f->mean_listed = rho_max * 4.0 / 3.0 * M_PI * lc * lc * lc;
   f->cap = ((int)(1.5 * rho_max * 4.0 / 3.0 * M_PI * lc * lc * lc) + 32 + 7) & ~7;
   if (f->cap_override > 0) f->cap = round_chunk(f->cap_override);
   if (f->is_rbl()) {

@@ -197,7 +197,8 @@ RBMD_API rbmd_status rbmd_force_compute(rbmd_force* f, void* stream);
  * bound system, keep the fastest, and leave the forces of that choice in atoms->force.
  * force_block returns the threads per block, or -G for G lanes per atom.  Config "autotune":
  * true runs it at the first compute; "tuning.list_block" / "tuning.force_block" /
- * "tuning.force_lanes" fix the choices instead (default 0 / 128 / 1).  Lists are identical entry
+ * "tuning.force_lanes" fix the choices instead (default 0 / 128 / by
+ * size: 1 to 16 lanes; 1 when only force_block is given).  Lists are identical entry
  * for entry whatever the choice; forces agree to rounding (lanes per atom change the summation
  * order).  No reference counterpart. */
 RBMD_API rbmd_status rbmd_force_autotune(rbmd_force* f, void* stream, int32_t* list_block,
