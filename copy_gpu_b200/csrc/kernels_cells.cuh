@@ -723,6 +723,10 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
 // grouped per replica), the input of every k-space phase: U_d = floor(frac((x_d - lo_d)/L_d)
 // * 2^32) (2^64 for FP64), so integer phases m . U mod 2^32 are exact.  Uncharged atoms add
 // nothing to rho_k or the k-space force and are left out.
+template <class R> struct FracT;
+template <> struct FracT<float> { using T = Frac32; };
+template <> struct FracT<double> { using T = Frac64; };
+
 template <class R>
 __global__ void k_frac(int nq, const int* __restrict__ qidx, const double* __restrict__ pos,
                        const double* __restrict__ charge, const int* __restrict__ rep_of,

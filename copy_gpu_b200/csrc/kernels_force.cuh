@@ -52,22 +52,37 @@ struct NearParams {
 template <class R> struct KRec;
 template <> struct KRec<float> { using T = KRec32; };
 template <> struct KRec<double> { using T = KRec64; };
-template <class R> struct FracT;
-template <> struct FracT<float> { using T = Frac32; };
-template <> struct FracT<double> { using T = Frac64; };
-
-__device__ __forceinline__ float exp_r(float x) { return __expf(x); }
+// e^x, 1/sqrt(x) and 1/x by one MUFU operation each.  The flush-to-zero forms leave out the
+// rescaling of denormals, which the arguments here never are: x = -alpha d^2 above -100, d^2 > 1e-4.
+__device__ __forceinline__ float exp_r(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.44269504088896340736f));
+  return r;
+}
 __device__ __forceinline__ double exp_r(double x) { return exp(x); }
-__device__ __forceinline__ float rsqrt_r(float x) { return rsqrtf(x); }
+__device__ __forceinline__ float rsqrt_r(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 __device__ __forceinline__ float sqrt_r(float x) { return sqrtf(x); }
 __device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
 __device__ __forceinline__ double rsqrt_r(double x) { return 1.0 / sqrt(x); }
+
+// approximate reciprocal (one MUFU op, about 1 ulp): the pair terms carry a 1e-5 budget
+__device__ __forceinline__ float rcp_r(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 
 // erfc(x) for x >= 0 given e = exp(-x^2).  FP32: Abramowitz & Stegun, Handbook of Mathematical
 // Functions, eq. 7.1.26 (rational approximation in t = 1/(1 + p x), |error| <= 1.5e-7), which
 // reuses the Gaussian factor the real-space force needs anyway.  FP64: the library erfc.
 __device__ __forceinline__ float erfc_shared(float x, float e) {
-  const float t = __frcp_rn(fmaf(0.3275911f, x, 1.0f));
+  // 1 / d to within an ulp: the MUFU reciprocal and one Newton step (the correctly rounded one takes
+  // a dozen instructions; both leave the formula's 1.5e-7 as it is)
+  const float d = fmaf(0.3275911f, x, 1.0f), t0 = rcp_r(d), t = fmaf(t0, fmaf(-d, t0, 1.0f), t0);
   float poly = fmaf(1.061405429f, t, -1.453152027f);
   poly = fmaf(poly, t, 1.421413741f);
   poly = fmaf(poly, t, -0.284496736f);
@@ -126,12 +141,6 @@ __device__ __forceinline__ void min_image(R& q0, R& q1, R& q2, const R* box) {
   if (fabs(q2) > box[2] * (R)0.5) q2 -= (q2 > 0 ? box[2] : -box[2]);
 }
 
-// approximate reciprocal (one MUFU op, about 1 ulp): the pair terms carry a 1e-5 budget
-__device__ __forceinline__ float rcp_r(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 __device__ __forceinline__ double rcp_r(double x) { return 1.0 / x; }
 
 // Near force of one slot per thread over its list row.
