@@ -728,35 +728,27 @@ template <> struct FracT<float> { using T = Frac32; };
 template <> struct FracT<double> { using T = Frac64; };
 
 template <class R>
-__global__ void k_frac(int nq, const int* __restrict__ qidx, const double* __restrict__ pos,
-                       const double* __restrict__ charge, const int* __restrict__ rep_of,
-                       const RepDev* __restrict__ reps, void* __restrict__ frac_out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nq) return;
-  const int id = qidx[c];
-  const RepDev& rp = reps[rep_of ? rep_of[id] : 0];
-  const double q = charge[id];
+__device__ __forceinline__ typename FracT<R>::T frac_of(const RepDev& rp, const double* __restrict__ pos,
+                                                        const double* __restrict__ charge, int id) {
   double u[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     u[d] = (pos[3 * id + d] - rp.lo_d[d]) / rp.box_d[d];
     u[d] -= floor(u[d]);
   }
-  if (sizeof(R) == 4) {
-    uint32_t U[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      U[d] = turn32(u[d]);
-    }
-    reinterpret_cast<Frac32*>(frac_out)[c] = Frac32{U[0], U[1], U[2], (float)q};
-  } else {
-    unsigned long long U[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      U[d] = turn64(u[d]);
-    }
-    reinterpret_cast<Frac64*>(frac_out)[c] = Frac64{U[0], U[1], U[2], q};
-  }
+  const double q = charge[id];
+  if constexpr (sizeof(R) == 4) return Frac32{turn32(u[0]), turn32(u[1]), turn32(u[2]), (float)q};
+  else return Frac64{turn64(u[0]), turn64(u[1]), turn64(u[2]), q};
+}
+
+template <class R>
+__global__ void k_frac(int nq, const int* __restrict__ qidx, const double* __restrict__ pos,
+                       const double* __restrict__ charge, const int* __restrict__ rep_of,
+                       const RepDev* __restrict__ reps, void* __restrict__ frac_out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= nq) return;
+  const int id = qidx[c];
+  reinterpret_cast<typename FracT<R>::T*>(frac_out)[c] = frac_of<R>(reps[rep_of ? rep_of[id] : 0], pos, charge, id);
 }
 
 }  // namespace rbmd

@@ -98,12 +98,12 @@ template <class R> __host__ __device__ __forceinline__ R sig6(const LJTable& t, 
 template <> __host__ __device__ __forceinline__ float sig6<float>(const LJTable& t, int k) { return t.sig6_f[k]; }
 template <> __host__ __device__ __forceinline__ double sig6<double>(const LJTable& t, int k) { return t.sig6_d[k]; }
 
-// RBE force terms of one atom over k records [0, P) of `kr` (shared or global memory).
-template <class R>
+// RBE force terms of one atom over the k records sub, sub + G, .. < P of `kr` (shared or global memory).
+template <class R, int G>
 __device__ __forceinline__ void rbe_terms(const typename FracT<R>::T& fr, const typename KRec<R>::T* kr,
-                                          int P, R& ax, R& ay, R& az) {
+                                          int P, int sub, R& ax, R& ay, R& az) {
 #pragma unroll 4
-  for (int l = 0; l < P; ++l) {
+  for (int l = sub; l < P; l += G) {
     const typename KRec<R>::T k = kr[l];
     R s, c;
     if constexpr (sizeof(R) == 4) {
@@ -570,14 +570,18 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   }
 }
 
-// RBE k-space force, one thread per charged atom (compact index c, caller id qidx[c]):
+// RBE k-space force, G lanes per charged atom (compact index c, caller id qidx[c]):
 // F_i = q_i sum_l w_l k_l (cos(k_l.r_i) Im rho_l - sin(k_l.r_i) Re rho_l)
 // (ComputeNewRBEForceWorklet, RunWorklet.cpp:1508-1548; S/P and qqr2e are folded into the
 // records).  The block stages the k records of the replicas its atoms belong to in shared
 // memory (two 16-byte broadcast loads per sample) when they fit.  Runs on the k-space stream
 // concurrently with the near pass and writes far_force[c]; k_add_far folds it into the force.
-template <class R>
-__global__ void __launch_bounds__(128) k_rbe_force(int nq, int kstage, const int* __restrict__ qidx,
+// Bound by MUFU (two per term) when the chip is full; the lanes of an atom take every G-th sample and
+// are summed in FP64 by a fixed butterfly, so that few charged atoms still fill it (launch_rbe_force).
+constexpr int kRbeThreads = 128;
+
+template <class R, int G>
+__global__ void __launch_bounds__(kRbeThreads) k_rbe_force(int nq, int kstage, const int* __restrict__ qidx,
                                                    const typename FracT<R>::T* __restrict__ frac,
                                                    const typename KRec<R>::T* __restrict__ krec,
                                                    const RepDev* __restrict__ reps,
@@ -585,9 +589,11 @@ __global__ void __launch_bounds__(128) k_rbe_force(int nq, int kstage, const int
                                                    double* __restrict__ far_force) {
   extern __shared__ __align__(16) unsigned char ksm_raw[];
   typename KRec<R>::T* ksm = reinterpret_cast<typename KRec<R>::T*>(ksm_raw);
-  const int c0 = blockIdx.x * blockDim.x;
-  const int c = c0 + threadIdx.x;
-  const int last = min(nq, c0 + (int)blockDim.x) - 1;
+  const int c0 = blockIdx.x * (kRbeThreads / G);
+  const int sub = threadIdx.x % G;
+  const int last = min(nq, c0 + kRbeThreads / G) - 1;
+  const int c = min(c0 + (int)threadIdx.x / G, last);   // lanes past the end repeat the last atom
+  const bool active = c0 + (int)threadIdx.x / G < nq;
   const int ra = rep_of ? rep_of[qidx[c0]] : 0;
   const int rb = rep_of ? rep_of[qidx[last]] : 0;
   const int kfirst = reps[ra].k_begin;
@@ -600,16 +606,21 @@ __global__ void __launch_bounds__(128) k_rbe_force(int nq, int kstage, const int
     for (int t = threadIdx.x; t < nwords; t += blockDim.x) dst[t] = src[t];
   }
   __syncthreads();
-  if (c >= nq) return;
   const RepDev& rp = reps[rep_of ? rep_of[qidx[c]] : 0];
   const typename FracT<R>::T fr = frac[c];
   R ax = 0, ay = 0, az = 0;
-  if (staged) rbe_terms<R>(fr, ksm + (rp.k_begin - kfirst), rp.P, ax, ay, az);
-  else rbe_terms<R>(fr, krec + rp.k_begin, rp.P, ax, ay, az);
+  if (staged) rbe_terms<R, G>(fr, ksm + (rp.k_begin - kfirst), rp.P, sub, ax, ay, az);
+  else rbe_terms<R, G>(fr, krec + rp.k_begin, rp.P, sub, ax, ay, az);
+  double F[3] = {(double)ax, (double)ay, (double)az};
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) F[d] += __shfl_xor_sync(0xffffffffu, F[d], o);
+  if (!active || sub != 0) return;
   const double q = (double)fr.q;
-  far_force[3 * c] = q * (double)ax;
-  far_force[3 * c + 1] = q * (double)ay;
-  far_force[3 * c + 2] = q * (double)az;
+  far_force[3 * c] = q * F[0];
+  far_force[3 * c + 1] = q * F[1];
+  far_force[3 * c + 2] = q * F[2];
 }
 
 __global__ void k_add_far(int nq, const int* __restrict__ qidx, const double* __restrict__ far_force,
@@ -632,17 +643,68 @@ __global__ void k_add_far(int nq, const int* __restrict__ qidx, const double* __
 // Each (item, k) partial is owned by one lane: no cross-lane reduction.  There is no N x P
 // buffer (the reference materialises rho_Re/Im[P*N] and reduces by key, ExecutionMD.cpp:412-448).
 // ------------------------------------------------------------------------------------------
+// Per-replica reduction layout: items are ordered (replica, chunk, tile); replica r's partials
+// for tile t and chunk c sit at item_base_r + c * ntiles_r + t.
+struct RhoRep { int item_base, ntiles, nchunks, pad; };
+
+// What a finished structure factor fills in.
+template <class R> struct RhoOut {
+  const double* weights;           // importance weights (nullable)
+  double qqr2e;
+  typename KRec<R>::T* krec;
+  double2* rho;
+  double* ek;
+};
+
+// Sample l of a replica from its summed partials: undo the half-turn phase convention (rho = -sum)
+// and fill the force coefficients of the k record, rho, and the k-space energy estimate
+// (S/P) qqr2e w_l (2 pi / V) |rho_l|^2 / k_l^2.
+template <class R>
+__device__ __forceinline__ void rho_record(const RepDev& rp, int l, double re, double im, const RhoOut<R>& o) {
+  const int g = rp.k_begin + l;
+  typename KRec<R>::T k = o.krec[g];
+  re = -re;
+  im = -im;
+  const double twopi = 6.283185307179586476925;
+  const double kx = twopi * k.mx / rp.box_d[0], ky = twopi * k.my / rp.box_d[1],
+               kz = twopi * k.mz / rp.box_d[2];
+  const double k2 = kx * kx + ky * ky + kz * kz;
+  const double wgt = o.weights ? o.weights[g] : 1.0;
+  // F_i = q_i (S/P) qqr2e sum_l wgt (-4 pi /(V k^2)) k (cos Im - sin Re); the kernel evaluates
+  // the angle shifted by half a turn, which flips cos and sin: store -w.
+  const double w0 = -(rp.S / rp.P) * o.qqr2e * wgt * (-4.0 * 3.14159265358979323846 / (rp.volume * k2));
+  k.wx = (decltype(k.wx))(w0 * kx);
+  k.wy = (decltype(k.wy))(w0 * ky);
+  k.wz = (decltype(k.wz))(w0 * kz);
+  k.re = (decltype(k.re))re;
+  k.im = (decltype(k.im))im;
+  o.krec[g] = k;
+  o.rho[g] = make_double2(re, im);
+  o.ek[g] = (rp.S / rp.P) * o.qqr2e * wgt * (2.0 * 3.14159265358979323846 / rp.volume) *
+                (re * re + im * im) / k2;
+}
+
 struct RhoItem { int atom_begin, atom_end, k_first, k_count; };
 constexpr int kRhoStage = 256;
 
+// The fixed-point coordinates are formed while staging (k tile 0 also writes them for k_rbe_force).
+// rep_done: with few chunks per replica the block that finishes a replica's last item sums its
+// partials in chunk order and fills the records (kFusedChunks); otherwise k_rho_finish does.
+constexpr int kFusedChunks = 32;
+
 template <class R, int KL>
-__global__ void __launch_bounds__(256) k_rho_lanes(const RhoItem* __restrict__ items,
-                                                   const typename FracT<R>::T* __restrict__ frac,
-                                                   const typename KRec<R>::T* __restrict__ krec,
-                                                   R* __restrict__ partial, int ktile) {
+__global__ void __launch_bounds__(256) k_rho_lanes(
+    const RhoItem* __restrict__ items, int P, const int* __restrict__ qidx, const double* __restrict__ pos,
+    const double* __restrict__ charge, const RepDev* __restrict__ reps, const RhoRep* __restrict__ rr,
+    typename FracT<R>::T* __restrict__ frac, R* partial, int ktile, int* __restrict__ rep_done, RhoOut<R> o) {
   using FT = typename FracT<R>::T;
   __shared__ FT stage[kRhoStage];
+  __shared__ int last;
   const RhoItem it = items[blockIdx.x];
+  const int r = it.k_first / P;   // replicas hold P samples each
+  const RepDev& rp = reps[r];
+  const bool first_tile = it.k_first == rp.k_begin;
+  const typename KRec<R>::T* krec = o.krec;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   using MT = typename std::conditional<sizeof(R) == 4, uint32_t, unsigned long long>::type;
   MT mx[KL], my[KL], mz[KL];
@@ -665,7 +727,11 @@ __global__ void __launch_bounds__(256) k_rho_lanes(const RhoItem* __restrict__ i
   for (int base = it.atom_begin; base < it.atom_end; base += kRhoStage) {
     const int cnt = min(kRhoStage, it.atom_end - base);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) stage[t] = frac[base + t];
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
+      const FT f = frac_of<R>(rp, pos, charge, qidx[base + t]);
+      stage[t] = f;
+      if (first_tile) frac[base + t] = f;
+    }
     __syncthreads();
     if (!warp_any) continue;
 #pragma unroll 4
@@ -687,63 +753,64 @@ __global__ void __launch_bounds__(256) k_rho_lanes(const RhoItem* __restrict__ i
       partial[((size_t)blockIdx.x * ktile + kk[j]) * 2] = re[j];
       partial[((size_t)blockIdx.x * ktile + kk[j]) * 2 + 1] = im[j];
     }
+  if (!rep_done) return;
+  __threadfence();   // the partials before the count
+  __syncthreads();
+  const RhoRep q = rr[r];
+  if (threadIdx.x == 0) last = atomicAdd(rep_done + r, 1) == q.nchunks * q.ntiles - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();   // the count before the other blocks' partials
+  for (int l = threadIdx.x; l < P; l += blockDim.x) {
+    const int tile = l / ktile, k = l % ktile;
+    double sr = 0, si = 0;
+#pragma unroll 4
+    for (int c = 0; c < q.nchunks; ++c) {
+      const size_t at = (((size_t)q.item_base + (size_t)c * q.ntiles + tile) * ktile + k) * 2;
+      sr += (double)__ldcg(partial + at);
+      si += (double)__ldcg(partial + at + 1);
+    }
+    rho_record<R>(rp, l, sr, si, o);
+  }
+  if (threadIdx.x == 0) rep_done[r] = 0;
 }
 
-// Per-replica reduction layout: items are ordered (replica, chunk, tile); replica r's partials
-// for tile t and chunk c sit at item_base_r + c * ntiles_r + t.
-struct RhoRep { int item_base, ntiles, nchunks, pad; };
+// Sum of the chunk partials of 32 consecutive k samples of one tile per block: lane = sample, so a
+// warp reads 32 consecutive partials, warp w takes the chunks w, w + warps, .. (FP64) and the warps
+// are added in order through shared memory (deterministic).
+// (One warp per sample read one 8-byte partial per 32-byte sector: 12.4 us at 390 chunks, 35 us for
+// 512 replicas of 100 samples.)
+constexpr int kFinishWarps = 16;   // at most; the launch uses as many as the longest chunk list needs
 
-// One warp per k sample: lanes sum the chunk partials in a fixed strided order (FP64) and a
-// butterfly combines them (deterministic); then undo the half-turn phase convention
-// (rho = -sum) and fill the force coefficients of the k record.
-// k-space energy estimate per replica: (S/P) qqr2e sum_l w_l (2 pi / V) |rho_l|^2 / k_l^2.
 template <class R>
-__global__ void k_rho_finish(int nk_total, int ktile, const int* __restrict__ krep,
-                             const RhoRep* __restrict__ rr, const RepDev* __restrict__ reps,
-                             const R* __restrict__ partial, const double* __restrict__ weights,
-                             double qqr2e, typename KRec<R>::T* __restrict__ krec,
-                             double2* __restrict__ rho_out, double* __restrict__ ek_out) {
-  const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (g >= nk_total) return;
-  const int r = krep[g];
+__global__ void __launch_bounds__(32 * kFinishWarps) k_rho_finish(
+    int nrep, int groups, int P, int ktile, const RhoRep* __restrict__ rr, const RepDev* __restrict__ reps,
+    const R* __restrict__ partial, RhoOut<R> o) {
+  __shared__ double sre[kFinishWarps][32], sim[kFinishWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int r = blockIdx.x / groups;               // groups = ceil(P / 32) blocks per replica
+  const int l = (blockIdx.x % groups) * 32 + lane;
   const RepDev& rp = reps[r];
   const RhoRep q = rr[r];
-  const int l = g - rp.k_begin;
-  const int tile = l / ktile, kk = l % ktile;
+  const int tile = l / ktile, kk = l % ktile;      // ktile is a multiple of 32: one tile per block
   double re = 0, im = 0;
-  for (int c = lane; c < q.nchunks; c += 32) {
-    const size_t item = (size_t)q.item_base + (size_t)c * q.ntiles + tile;
-    re += (double)partial[(item * ktile + kk) * 2];
-    im += (double)partial[(item * ktile + kk) * 2 + 1];
+  if (l < P) {
+#pragma unroll 4
+    for (int c = w; c < q.nchunks; c += nw) {
+      const size_t at = (((size_t)q.item_base + (size_t)c * q.ntiles + tile) * ktile + kk) * 2;
+      re += (double)partial[at];
+      im += (double)partial[at + 1];
+    }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    re += __shfl_xor_sync(0xffffffffu, re, o);
-    im += __shfl_xor_sync(0xffffffffu, im, o);
+  sre[w][lane] = re;
+  sim[w][lane] = im;
+  __syncthreads();
+  if (w != 0 || l >= P) return;
+  for (int k = 1; k < nw; ++k) {
+    re += sre[k][lane];
+    im += sim[k][lane];
   }
-  if (lane != 0) return;
-  typename KRec<R>::T k = krec[g];
-  re = -re;
-  im = -im;
-  const double twopi = 6.283185307179586476925;
-  const double kx = twopi * k.mx / rp.box_d[0], ky = twopi * k.my / rp.box_d[1],
-               kz = twopi * k.mz / rp.box_d[2];
-  const double k2 = kx * kx + ky * ky + kz * kz;
-  const double wgt = weights ? weights[g] : 1.0;
-  // F_i = q_i (S/P) qqr2e sum_l wgt (-4 pi /(V k^2)) k (cos Im - sin Re); the kernel evaluates
-  // the angle shifted by half a turn, which flips cos and sin: store -w.
-  const double w = -(rp.S / rp.P) * qqr2e * wgt * (-4.0 * 3.14159265358979323846 / (rp.volume * k2));
-  k.wx = (decltype(k.wx))(w * kx);
-  k.wy = (decltype(k.wy))(w * ky);
-  k.wz = (decltype(k.wz))(w * kz);
-  k.re = (decltype(k.re))re;
-  k.im = (decltype(k.im))im;
-  krec[g] = k;
-  if (rho_out) rho_out[g] = make_double2(re, im);
-  if (ek_out)
-    ek_out[g] = (rp.S / rp.P) * qqr2e * wgt * (2.0 * 3.14159265358979323846 / rp.volume) *
-                (re * re + im * im) / k2;
+  rho_record<R>(rp, l, re, im, o);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -200,7 +200,7 @@ struct rbmd_force {
   double* d_eslot = nullptr;   // 2 per slot (lj, coul)
   double* d_esum = nullptr;    // scratch sums
   // RBE
-  int Ptot = 0, nitems = 0, rho_threads = 64, ktile = 128, kstage = 0;
+  int Ptot = 0, nitems = 0, finish_warps = 1, rho_threads = 64, ktile = 128, kstage = 0;
   bool minimg = true, want_energy = true;
   bool kspace_priority = true;
   bool orig_pred = false;        // neighbor.type "ORIGINAL": pair predicate d^2 < rc^2   // execution.kspace_priority: side stream at the highest priority
@@ -212,6 +212,8 @@ struct rbmd_force {
   RhoItem* d_items = nullptr;
   RhoRep* d_rhorep = nullptr;
   void* d_partial = nullptr;
+  int* d_rho_done = nullptr;   // finished structure-factor items per replica (few chunks: kFusedChunks)
+  int* d_cidx = nullptr;       // charged atom of each atom, or -1
   double2* d_rho = nullptr;
   double* d_ek = nullptr;
   double* d_far = nullptr;
@@ -430,6 +432,7 @@ void free_all(rbmd_force* f) {
   dfree(f->d_kvec); dfree(f->d_krep); dfree(f->d_qidx); dfree(f->d_items); dfree(f->d_rhorep);
   if (f->d_partial) cudaFree(f->d_partial);
   f->d_partial = nullptr;
+  dfree(f->d_rho_done); dfree(f->d_cidx);
   dfree(f->d_rho); dfree(f->d_ek); dfree(f->d_far); dfree(f->d_weights); dfree(f->d_srep); dfree(f->d_qtab);
   dfree(f->d_chunks); dfree(f->d_chunk_rep_begin); dfree(f->d_ke_partial); dfree(f->d_ke);
   dfree(f->d_T); dfree(f->d_lambda); dfree(f->d_xi); dfree(f->d_xold); dfree(f->d_vold);
@@ -928,6 +931,21 @@ void launch_prop_sample(rbmd_force* f, cudaStream_t s, long long step, int rec_b
   f->launches++;
 }
 
+// RBE force: lanes per charged atom so that the launch holds about eight warps per scheduler (one
+// thread per atom at 100,000 charged atoms and more, 8 lanes below 19,000); beyond that, lanes only
+// add copies of the staged records.
+template <class R>
+void launch_rbe_force(rbmd_force* f, cudaStream_t s) {
+  const size_t smem = (size_t)f->kstage * sizeof(typename KRec<R>::T);
+  const long long want = 1024LL * f->num_sms;
+  const int g = 8LL * f->nq <= want ? 8 : (4LL * f->nq <= want ? 4 : (2LL * f->nq <= want ? 2 : 1));
+  auto kern = g == 8 ? k_rbe_force<R, 8> : g == 4 ? k_rbe_force<R, 4> : g == 2 ? k_rbe_force<R, 2> : k_rbe_force<R, 1>;
+  const int per = kRbeThreads / g;
+  kern<<<(f->nq + per - 1) / per, kRbeThreads, smem, s>>>(
+      f->nq, f->kstage, f->d_qidx, (const typename FracT<R>::T*)f->d_frac, (const typename KRec<R>::T*)f->d_krec,
+      f->d_reps, f->nrep > 1 ? f->d_rep_of : nullptr, f->d_far);
+}
+
 // k-space chain on the side stream: sampler (depends only on the step counter, so it runs
 // before the fork wait), fixed-point fractional coordinates, structure factors, coefficients,
 // RBE force into d_far.
@@ -962,26 +980,30 @@ void launch_kspace(rbmd_force* f, cudaStream_t s, cudaEvent_t ready) {
     cudaEventRecord(f->ev_tail, s);
     return;
   }
-  const int* rep_of = f->nrep > 1 ? f->d_rep_of : nullptr;
   {
     PhaseScope ps(f, kPhK, s);
-    k_frac<R><<<(f->nq + 255) / 256, 256, 0, s>>>(f->nq, f->d_qidx, f->at.pos, f->at.charge, rep_of,
-                                                   f->d_reps, f->d_frac);
+    RhoOut<R> o;
+    o.weights = own_prop ? f->d_pw : f->d_weights;
+    o.qqr2e = f->u.qqr2e;
+    o.krec = (typename KRec<R>::T*)f->d_krec;
+    o.rho = f->d_rho;
+    o.ek = f->d_ek;
     k_rho_lanes<R, kKL><<<f->nitems, f->rho_threads, 0, s>>>(
-        f->d_items, (const typename FracT<R>::T*)f->d_frac, (const typename KRec<R>::T*)f->d_krec,
-        (R*)f->d_partial, f->ktile);
-    k_rho_finish<R><<<(f->Ptot + 3) / 4, 128, 0, s>>>(
-        f->Ptot, f->ktile, f->d_krep, f->d_rhorep, f->d_reps, (const R*)f->d_partial,
-        own_prop ? f->d_pw : f->d_weights, f->u.qqr2e, (typename KRec<R>::T*)f->d_krec, f->d_rho, f->d_ek);
+        f->d_items, f->P, f->d_qidx, f->at.pos, f->at.charge, f->d_reps, f->d_rhorep,
+        (typename FracT<R>::T*)f->d_frac, (R*)f->d_partial, f->ktile, f->d_rho_done, o);
+    f->launches++;
+    if (!f->d_rho_done) {
+      const int groups = (f->P + 31) / 32;
+      k_rho_finish<R><<<f->nrep * groups, 32 * f->finish_warps, 0, s>>>(
+          f->nrep, groups, f->P, f->ktile, f->d_rhorep, f->d_reps, (const R*)f->d_partial, o);
+      f->launches++;
+    }
   }
   {
     PhaseScope ps(f, kPhRbeF, s);
-    const size_t smem = (size_t)f->kstage * sizeof(typename KRec<R>::T);
-    k_rbe_force<R><<<(f->nq + 127) / 128, 128, smem, s>>>(
-        f->nq, f->kstage, f->d_qidx, (const typename FracT<R>::T*)f->d_frac,
-        (const typename KRec<R>::T*)f->d_krec, f->d_reps, rep_of, f->d_far);
+    launch_rbe_force<R>(f, s);
   }
-  f->launches += 4;
+  f->launches++;
   // conditioning of the next step's proposal, after the force kernels of this one
   if (own_prop && f->proposal == "learned" && f->prop_trained) {
     k_prop_spectrum<<<f->nrep, 256, 0, s>>>(f->nrep, f->d_reps, f->d_prep, f->d_kvec, f->d_rho, f->d_pw, 0.1f,
@@ -2383,6 +2405,10 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     CK(dalloc(&f->d_qidx, (size_t)std::max(1, f->nq)));
     if (f->nq > 0)
       CK(cudaMemcpy(f->d_qidx, qidx.data(), sizeof(int) * f->nq, cudaMemcpyHostToDevice));
+    std::vector<int> cidx(n, -1);
+    for (int c = 0; c < f->nq; ++c) cidx[qidx[c]] = c;
+    CK(dalloc(&f->d_cidx, n));
+    CK(cudaMemcpy(f->d_cidx, cidx.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
     const int recb = fp64 ? sizeof(KRec64) : sizeof(KRec32);
     if (f->coul_type == "EWALD") {
       // EWALD: the cube m in [-kmax, kmax]^3 \ {0} (ExecPointLocator::ExecuteOnKNeighbor,
@@ -2416,8 +2442,12 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     std::vector<RhoItem> items;
     std::vector<RhoRep> rr(nrep);
     const int ntiles = (f->P + f->ktile - 1) / f->ktile;
-    const double target_blocks = 148.0 * (2048 / f->rho_threads) * 2.0;
-    const double chunk_atoms = std::max(256.0, (double)std::max(1, f->nq) * ntiles / target_blocks);
+    // chunks: three blocks per SM, between 64 charged atoms (16,000-atom systems otherwise filled 6
+    // of the SMs) and 256 (one staged tile), longer only to bound the number of partial sums
+    const double target_blocks = (double)f->num_sms * (2048 / f->rho_threads) * 2.0;
+    const double per_item = (double)std::max(1, f->nq) * ntiles;
+    const double chunk_atoms = std::max(std::min(256.0, std::max(64.0, per_item / (3.0 * f->num_sms))),
+                                        per_item / target_blocks);
     for (int r = 0; r < nrep; ++r) {
       const int Nr = (int)(qoff[r + 1] - qoff[r]);   // charged atoms of replica r
       const int nch = std::max(1, (int)std::lround(Nr / chunk_atoms));
@@ -2438,6 +2468,14 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
       }
     }
     f->nitems = (int)items.size();
+    int most = 1;
+    for (const RhoRep& q : rr) most = std::max(most, q.nchunks);
+    f->finish_warps = 1;
+    if (most <= kFusedChunks) {
+      CK(dalloc(&f->d_rho_done, (size_t)nrep));
+      CK(cudaMemset(f->d_rho_done, 0, sizeof(int) * nrep));
+    }
+    while (f->finish_warps < kFinishWarps && 2 * f->finish_warps <= most) f->finish_warps *= 2;
     CK(dalloc(&f->d_items, items.size()));
     CK(cudaMemcpy(f->d_items, items.data(), sizeof(RhoItem) * items.size(), cudaMemcpyHostToDevice));
     CK(dalloc(&f->d_rhorep, (size_t)nrep));
