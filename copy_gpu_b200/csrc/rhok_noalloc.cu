@@ -6,8 +6,8 @@
 // fragment that pool), or a time-step loop that keeps several streams busy and cannot take
 // the device-wide synchronisation that cudaFree implies.  For them this file provides one
 // entry point, rbmd_rhok_noalloc, that computes rho_k = sum_j q_j exp(i k.r_j) with the same
-// fixed-point phase arithmetic as the force path but keeps all of its scratch (fixed-point
-// coordinates and per-block partial sums) in a file-scope static device array of fixed size.
+// fixed-point phase arithmetic as the force path but keeps all of its scratch (per-block partial
+// sums) in a file-scope static device array of fixed size.
 // The caller still passes the inputs and the output.
 //
 // Limits and sharing rules:
@@ -28,6 +28,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdarg>
@@ -43,10 +44,9 @@ extern char g_last_error[512];   // shared with rbmd_force.cu (rbmd_last_error)
 
 namespace {
 
-constexpr int kNoAllocMaxAtoms = 262144;                 // fixed-point coordinates: 4 MiB
+constexpr int kNoAllocMaxAtoms = 262144;
 constexpr int kNoAllocMaxK = 1024;
-constexpr int kNoAllocChunk = 2048;                      // atoms per structure-factor block
-constexpr size_t kNoAllocFracBytes = (size_t)kNoAllocMaxAtoms * sizeof(rbmd::Frac32);
+constexpr int kNoAllocChunkMin = 32, kNoAllocChunkMax = 2048;   // atoms per structure-factor block (na_chunk)
 constexpr size_t kNoAllocScratchBytes = 8u << 20;        // 8 MiB in total
 constexpr int kMaxDevices = 64;
 
@@ -93,38 +93,39 @@ unsigned long long current_context_id() {
   return id;
 }
 
-__global__ void k_na_frac(int n, const double* __restrict__ pos, const double* __restrict__ charge,
-                          double lo0, double lo1, double lo2, double L0, double L1, double L2,
-                          rbmd::Frac32* __restrict__ frac) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double lo[3] = {lo0, lo1, lo2}, L[3] = {L0, L1, L2};
+// Fixed-point coordinates and charge of one atom.
+struct NaBox { double lo[3], L[3]; };
+__device__ __forceinline__ rbmd::Frac32 na_frac(const NaBox& b, const double* __restrict__ pos,
+                                               const double* __restrict__ charge, int i) {
   uint32_t U[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const double u = (pos[3 * i + d] - lo[d]) / L[d];
+    const double u = (pos[3 * i + d] - b.lo[d]) / b.L[d];
     U[d] = rbmd::turn32(u - floor(u));   // a whole turn wraps to 0
   }
-  frac[i] = rbmd::Frac32{U[0], U[1], U[2], (float)charge[i]};
+  return rbmd::Frac32{U[0], U[1], U[2], (float)charge[i]};
 }
 
-// One sample per lane (up to 32 per warp, P <= 32 * warps), the block's chunk of atoms staged
-// in shared memory and read by broadcast; partial[(chunk * P + k) * 2 + {0,1}] in FP32.
-__global__ void __launch_bounds__(1024) k_na_rho(int n, int P, const rbmd::Frac32* __restrict__ frac,
-                                                 const int* __restrict__ m, float* __restrict__ partial) {
+// One sample per lane (up to 32 per warp, P <= 32 * warps), the block's chunk of atoms converted
+// to fixed point into shared memory (one block holds every sample, so each atom is converted once)
+// and read by broadcast; partial[(chunk * P + k) * 2 + {0,1}] in FP32.
+__global__ void __launch_bounds__(1024) k_na_rho(int n, int P, int chunk, NaBox box, const double* __restrict__ pos,
+                                                 const double* __restrict__ charge, const int* __restrict__ m,
+                                                 float* __restrict__ partial) {
   __shared__ rbmd::Frac32 stage[256];
   const int k = threadIdx.x;
   const bool ok = k < P;
   const uint32_t mx = ok ? (uint32_t)m[3 * k] : 0u, my = ok ? (uint32_t)m[3 * k + 1] : 0u,
                  mz = ok ? (uint32_t)m[3 * k + 2] : 0u;
-  const int a0 = blockIdx.x * kNoAllocChunk, a1 = min(n, a0 + kNoAllocChunk);
+  const int a0 = blockIdx.x * chunk, a1 = min(n, a0 + chunk);
   float re = 0.f, im = 0.f;
   for (int base = a0; base < a1; base += 256) {
     const int cnt = min(256, a1 - base);
     __syncthreads();
-    for (int t = threadIdx.x; t < cnt; t += blockDim.x) stage[t] = frac[base + t];
+    for (int t = threadIdx.x; t < cnt; t += blockDim.x) stage[t] = na_frac(box, pos, charge, base + t);
     __syncthreads();
     if (!ok) continue;
+#pragma unroll 4
     for (int a = 0; a < cnt; ++a) {
       const rbmd::Frac32 f = stage[a];
       const uint32_t ph = mx * f.x + my * f.y + mz * f.z;
@@ -142,26 +143,46 @@ __global__ void __launch_bounds__(1024) k_na_rho(int n, int P, const rbmd::Frac3
   }
 }
 
-// One warp per sample: fixed-order FP64 sum of the chunk partials; the angle was shifted by half
-// a turn, which negates both components.
-__global__ void k_na_finish(int P, int nchunks, const float* __restrict__ partial, double* __restrict__ rho) {
-  const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (k >= P) return;
+// Atoms per structure-factor block: about two waves of the blocks that an SM holds (2048 threads),
+// and no more partial sums than the scratch has room for.  The kernel is bound by MUFU (two per
+// term) once the chip is full; 20,011 atoms x 500 samples in 10 blocks of 2048 atoms took 82 us.
+int na_chunk(int n, int P, int threads, int sms) {
+  const long long blocks = 2LL * sms * (2048 / threads);
+  long long c = (n + blocks - 1) / blocks;
+  const long long most = (long long)(kNoAllocScratchBytes / (2 * sizeof(float) * (size_t)P));
+  c = std::max(c, (n + most - 1) / most);
+  return (int)std::min<long long>(kNoAllocChunkMax, std::max<long long>(kNoAllocChunkMin, c));
+}
+
+// Sum of the chunk partials of 32 samples per block: lane = sample (consecutive partials), warp w
+// takes the chunks w, w + 16, .. in FP64, the warps are added in order; the angle was shifted by
+// half a turn, which negates both components.
+constexpr int kNaFinishWarps = 16;
+
+__global__ void __launch_bounds__(32 * kNaFinishWarps) k_na_finish(int P, int nchunks,
+                                                                   const float* __restrict__ partial,
+                                                                   double* __restrict__ rho) {
+  __shared__ double sre[kNaFinishWarps][32], sim[kNaFinishWarps][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
   double re = 0, im = 0;
-  for (int c = lane; c < nchunks; c += 32) {
-    re += (double)partial[((size_t)c * P + k) * 2];
-    im += (double)partial[((size_t)c * P + k) * 2 + 1];
+  if (k < P) {
+#pragma unroll 4
+    for (int c = w; c < nchunks; c += kNaFinishWarps) {
+      re += (double)partial[((size_t)c * P + k) * 2];
+      im += (double)partial[((size_t)c * P + k) * 2 + 1];
+    }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    re += __shfl_xor_sync(0xffffffffu, re, o);
-    im += __shfl_xor_sync(0xffffffffu, im, o);
+  sre[w][lane] = re;
+  sim[w][lane] = im;
+  __syncthreads();
+  if (w != 0 || k >= P) return;
+  for (int v = 1; v < kNaFinishWarps; ++v) {
+    re += sre[v][lane];
+    im += sim[v][lane];
   }
-  if (lane == 0) {
-    rho[2 * k] = -re;
-    rho[2 * k + 1] = -im;
-  }
+  rho[2 * k] = -re;
+  rho[2 * k + 1] = -im;
 }
 
 }  // namespace
@@ -175,9 +196,8 @@ RBMD_API rbmd_status rbmd_rhok_noalloc(const double* pos_dev, const double* char
     set_error("rbmd_rhok_noalloc: null pointer or non-positive size (n=%d, P=%d)", n, P);
     return RBMD_ERR_ARG;
   }
-  const int nchunks = (n + kNoAllocChunk - 1) / kNoAllocChunk;
-  const size_t partial_bytes = (size_t)nchunks * P * 2 * sizeof(float);
-  if (n > kNoAllocMaxAtoms || P > kNoAllocMaxK || kNoAllocFracBytes + partial_bytes > kNoAllocScratchBytes) {
+  // every n and P within the limits fits: at the longest chunks 128 x 1024 partial sums, 1 MiB of 8
+  if (n > kNoAllocMaxAtoms || P > kNoAllocMaxK) {
     set_error("rbmd_rhok_noalloc: n=%d, P=%d exceed the fixed scratch (n <= %d, P <= %d)", n, P,
               kNoAllocMaxAtoms, kNoAllocMaxK);
     return RBMD_ERR_ARG;
@@ -207,6 +227,11 @@ RBMD_API rbmd_status rbmd_rhok_noalloc(const double* pos_dev, const double* char
     set_error("rbmd_rhok_noalloc: device %d is beyond the %d devices this entry point serves", dev, kMaxDevices);
     return RBMD_ERR_CUDA;
   }
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    cudaGetLastError();
+    sms = 148;
+  }
   cudaStream_t s = (cudaStream_t)stream;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
@@ -234,13 +259,16 @@ RBMD_API rbmd_status rbmd_rhok_noalloc(const double* pos_dev, const double* char
     }
     base = g_scratch_ptr[dev];
   }
-  rbmd::Frac32* frac = reinterpret_cast<rbmd::Frac32*>(base);
-  float* partial = reinterpret_cast<float*>(static_cast<unsigned char*>(base) + kNoAllocFracBytes);
-  k_na_frac<<<(n + 255) / 256, 256, 0, s>>>(n, pos_dev, charge_dev, box->lo[0], box->lo[1], box->lo[2], L[0],
-                                           L[1], L[2], frac);
+  float* partial = static_cast<float*>(base);
+  NaBox nb;
+  for (int d = 0; d < 3; ++d) {
+    nb.lo[d] = box->lo[d];
+    nb.L[d] = L[d];
+  }
   const int threads = ((P + 31) / 32) * 32;
-  k_na_rho<<<nchunks, threads, 0, s>>>(n, P, frac, m_dev, partial);
-  k_na_finish<<<(P + 3) / 4, 128, 0, s>>>(P, nchunks, partial, rho_dev);
+  const int chunk = na_chunk(n, P, threads, sms), nchunks = (n + chunk - 1) / chunk;
+  k_na_rho<<<nchunks, threads, 0, s>>>(n, P, chunk, nb, pos_dev, charge_dev, m_dev, partial);
+  k_na_finish<<<(P + 31) / 32, 32 * kNaFinishWarps, 0, s>>>(P, nchunks, partial, rho_dev);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error("rbmd_rhok_noalloc: launch failed: %s", cudaGetErrorString(e));
