@@ -41,6 +41,7 @@ __global__ void k_kick_drift(MdParams mp, double* __restrict__ pos, double* __re
   const RepDev& rp = reps[r];
   const double m = mass[i];
   const double lam = (mp.apply_scale && lambda) ? lambda[r] : 1.0;
+  const double hk = 0.5 * mp.dt * mp.fmt2v / m;   // one FP64 division per atom instead of one per axis
   double x[3];
   bool bad = false;
 #pragma unroll
@@ -48,7 +49,7 @@ __global__ void k_kick_drift(MdParams mp, double* __restrict__ pos, double* __re
     double v = vel[3 * i + d] * lam;
     const double xo = pos[3 * i + d];
     if (mp.save_old) { x_old[3 * i + d] = xo; v_old[3 * i + d] = v; }
-    v += 0.5 * force[3 * i + d] / m * mp.dt * mp.fmt2v;
+    v += force[3 * i + d] * hk;
     double xn = xo + v * mp.dt;
     if (xn < rp.lo_d[d]) {
       xn += rp.hi_d[d] - rp.lo_d[d];
@@ -169,33 +170,133 @@ __global__ void k_open_rebuild(cudaGraphConditionalHandle h, const int* __restri
 // Chunk of atoms inside one replica (kinetic-energy partials, ordered per replica).
 struct MdChunk { int begin, end, rep, pad; };
 
+struct ThermoParams {
+  int nrep;
+  int tstat;          // 0 none, 1 BERENDSEN, 2 TEMP_RESCALE, 3 NOSE_HOOVER
+  double mvv2e, kB, dt, Tdamp, T0;
+  int dof_mode;       // 0: 3n-3, 1: 3n-n-3 (shake), 2: 3n, 3: 3n/2 (inbuild)
+};
+
+// Device state of the end of a step.
+struct ThermoDev {
+  const int* chunk_begin_of_rep;   // chunks of replica r: [r], [r + 1)
+  const double* ke_partial;
+  double *ke, *T, *lambda, *xi;
+  int* rebuild;                    // Verlet-skin flags, cleared for the next step (nullable)
+  int* done;                       // finished chunks of each replica (0 between launches)
+};
+
+// ExecutionNVT::ComputeTempe + UpdateVelocityByTempConType
+// (rbmd/framework/run/ExecutionNVT.cpp:256-290,749-786) of replica r by one block: T from the
+// chunk partials (threads stride over them, butterflies, then the warps in order: fixed order),
+// lambda for the deferred rescale, NH xi update; and the replica's rebuild flags cleared.
+__device__ __forceinline__ void thermo_replica(const ThermoParams& tp, const ThermoDev& td, int r,
+                                               const RepDev* __restrict__ reps) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  __shared__ double red[32];
+  double s = 0;
+  for (int c = td.chunk_begin_of_rep[r] + threadIdx.x; c < td.chunk_begin_of_rep[r + 1]; c += blockDim.x)
+    s += __ldcg(td.ke_partial + c);   // written by other blocks of the same launch
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  s = red[0];
+  for (int w = 1; w < nw; ++w) s += red[w];
+  s *= tp.mvv2e;
+  const double n = (double)(reps[r].atom_end - reps[r].atom_begin);
+  double T;
+  switch (tp.dof_mode) {
+    case 1: T = 0.5 * s / ((3 * n - n - 3) * tp.kB / 2.0); break;
+    case 2: T = 0.5 * s / ((3 * n) * tp.kB / 2.0); break;
+    case 3: T = 0.5 * s / (3 * n / 2.0); break;
+    default: T = 0.5 * s / ((3 * n - 3) * tp.kB / 2.0); break;
+  }
+  td.ke[r] = 0.5 * s;
+  td.T[r] = T;
+  double lam = 1.0;
+  if (tp.tstat == 1) lam = sqrt(1.0 + (tp.dt / tp.Tdamp) * (tp.T0 / T - 1.0));
+  else if (tp.tstat == 2) lam = sqrt(tp.T0 / T);
+  else if (tp.tstat == 3 && td.xi) {
+    const double tauT = 0.1 * tp.dt;
+    td.xi[r] += 0.5 * tp.dt * (T / tp.T0 - 1.0) / tauT;
+  }
+  td.lambda[r] = lam;
+  if (td.rebuild) {
+    td.rebuild[r] = 0;
+    td.rebuild[tp.nrep] = 0;
+  }
+}
+
+__global__ void k_thermo(ThermoParams tp, ThermoDev td, const RepDev* __restrict__ reps) {
+  thermo_replica(tp, td, blockIdx.x, reps);   // one block per replica
+}
+
+// k-space force folded into the force by the first kick of a step (index == nullptr: nothing to
+// fold): index[i] = charged atom of atom i or -1, force[3 c] its k-space force.
+struct FarFold {
+  const int* index;
+  const double* force;
+  uint32_t* status;
+};
+
 // Stage 3 kick (+ NH variant) and per-chunk sum m v^2 (ComputerKineticEnergyWorklet,
-// RunWorklet.cpp:1806-1816).  One block per chunk; deterministic block reduction.
+// RunWorklet.cpp:1806-1816).  One block per chunk; deterministic block reduction.  With `thermo` the
+// block that finishes a replica's last chunk also does the replica's temperature and thermostat
+// (thermo_replica), which would otherwise be a launch of its own at the end of the step.
 __global__ void __launch_bounds__(256) k_kick_ke(MdParams mp, const MdChunk* __restrict__ chunks,
-                                                 double* __restrict__ vel, const double* __restrict__ force,
+                                                 double* __restrict__ vel, double* __restrict__ force,
                                                  const double* __restrict__ mass, int do_kick,
                                                  const double* __restrict__ xi_rep,
-                                                 double* __restrict__ ke_partial) {
+                                                 double* __restrict__ ke_partial, FarFold far, int thermo, ThermoParams tp,
+                                                 ThermoDev td, const RepDev* __restrict__ reps) {
   const MdChunk ch = chunks[blockIdx.x];
   const double xi = (do_kick == 2 && xi_rep) ? xi_rep[ch.rep] : 0.0;
   double ke = 0;
-  for (int i = ch.begin + threadIdx.x; i < ch.end; i += blockDim.x) {
-    const double m = mass[i];
-    double v2 = 0;
+  bool bad = false;
+  const double c1 = 0.5 * mp.dt * mp.fmt2v;
+  // one coordinate per thread and four in flight: the loads of a group are all issued before its
+  // first store (a thread per atom read three strided words in turn, and the k-space force behind
+  // the stores of the atom before: 90 us for 2.2 M atoms without it, 158 us with it)
+  constexpr int U = 4;
+  for (int t0 = 3 * ch.begin + threadIdx.x; t0 < 3 * ch.end; t0 += 256 * U) {
+    double v[U], f[U], m[U];
+    int fc[U];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      double v = vel[3 * i + d];
-      if (do_kick == 1) {
-        v += 0.5 * force[3 * i + d] / m * mp.dt * mp.fmt2v;
-        vel[3 * i + d] = v;
-      } else if (do_kick == 2) {   // UpdateVelocityNoseHooverWorklet (RunWorklet.cpp:1784-1804)
-        v += 0.5 * mp.dt * (force[3 * i + d] / m - xi * v) * mp.fmt2v;
-        vel[3 * i + d] = v;
-      }
-      v2 += v * v;
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + 256 * u;
+      const bool in = t < 3 * ch.end;
+      const int i = t / 3;
+      fc[u] = in && far.index ? __ldg(far.index + i) : -1;
+      v[u] = in ? vel[t] : 0.0;
+      f[u] = in && do_kick ? force[t] : 0.0;
+      m[u] = in ? __ldg(mass + i) : 1.0;
     }
-    ke += m * v2;
+    double g[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) g[u] = fc[u] >= 0 ? __ldg(far.force + 3 * fc[u] + (t0 + 256 * u) % 3) : 0.0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + 256 * u;
+      if (t >= 3 * ch.end) break;
+      double x = v[u];
+      if (do_kick == 1) {
+        double fx = f[u];
+        if (fc[u] >= 0) {
+          fx += g[u];
+          force[t] = fx;
+          bad |= !isfinite(fx);
+        }
+        x += fx * (c1 / m[u]);
+        vel[t] = x;
+      } else if (do_kick == 2) {   // UpdateVelocityNoseHooverWorklet (RunWorklet.cpp:1784-1804)
+        x += 0.5 * mp.dt * (f[u] / m[u] - xi * x) * mp.fmt2v;
+        vel[t] = x;
+      }
+      ke += m[u] * x * x;
+    }
   }
+  if (bad) set_flag(far.status, kFlagNonFinite);
   if (!ke_partial) return;
   __shared__ double red[8];
   for (int o = 16; o > 0; o >>= 1) ke += __shfl_xor_sync(0xffffffffu, ke, o);
@@ -206,49 +307,18 @@ __global__ void __launch_bounds__(256) k_kick_ke(MdParams mp, const MdChunk* __r
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
     ke_partial[blockIdx.x] = s;
   }
-}
-
-struct ThermoParams {
-  int nrep;
-  int tstat;          // 0 none, 1 BERENDSEN, 2 TEMP_RESCALE, 3 NOSE_HOOVER
-  double mvv2e, kB, dt, Tdamp, T0;
-  int dof_mode;       // 0: 3n-3, 1: 3n-n-3 (shake), 2: 3n, 3: 3n/2 (inbuild)
-};
-
-// ExecutionNVT::ComputeTempe + UpdateVelocityByTempConType
-// (rbmd/framework/run/ExecutionNVT.cpp:256-290,749-786) per replica: T from the chunk
-// partials (fixed order), lambda for the deferred rescale, NH xi update.
-__global__ void k_thermo(ThermoParams tp, const int* __restrict__ chunk_begin_of_rep,
-                         const double* __restrict__ ke_partial, double* __restrict__ ke_out,
-                         double* __restrict__ T_out, double* __restrict__ lambda,
-                         double* __restrict__ xi, const RepDev* __restrict__ reps) {
-  // one warp per replica, fixed-order lane sums then a butterfly: deterministic
-  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= tp.nrep) return;
-  double s = 0;
-  for (int c = chunk_begin_of_rep[r] + lane; c < chunk_begin_of_rep[r + 1]; c += 32) s += ke_partial[c];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane != 0) return;
-  s *= tp.mvv2e;
-  const double n = (double)(reps[r].atom_end - reps[r].atom_begin);
-  double T;
-  switch (tp.dof_mode) {
-    case 1: T = 0.5 * s / ((3 * n - n - 3) * tp.kB / 2.0); break;
-    case 2: T = 0.5 * s / ((3 * n) * tp.kB / 2.0); break;
-    case 3: T = 0.5 * s / (3 * n / 2.0); break;
-    default: T = 0.5 * s / ((3 * n - 3) * tp.kB / 2.0); break;
+  if (!thermo) return;
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    __threadfence();   // the partial before the count
+    const int nch = td.chunk_begin_of_rep[ch.rep + 1] - td.chunk_begin_of_rep[ch.rep];
+    last = atomicAdd(td.done + ch.rep, 1) == nch - 1;
   }
-  ke_out[r] = 0.5 * s;
-  T_out[r] = T;
-  double lam = 1.0;
-  if (tp.tstat == 1) lam = sqrt(1.0 + (tp.dt / tp.Tdamp) * (tp.T0 / T - 1.0));
-  else if (tp.tstat == 2) lam = sqrt(tp.T0 / T);
-  else if (tp.tstat == 3 && xi) {
-    const double tauT = 0.1 * tp.dt;
-    xi[r] += 0.5 * tp.dt * (T / tp.T0 - 1.0) / tauT;
-  }
-  lambda[r] = lam;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();     // the count before the other blocks' partials
+  thermo_replica(tp, td, ch.rep, reps);
+  if (threadIdx.x == 0) td.done[ch.rep] = 0;
 }
 
 __global__ void k_scale_vel(int n, const int* __restrict__ rep_of, const double* __restrict__ lambda,

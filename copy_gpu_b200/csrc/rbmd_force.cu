@@ -43,7 +43,7 @@ namespace {
 constexpr int kKL = 2;           // k samples per lane in the structure-factor kernel
 constexpr int kStageBytes = 48 * 1024;   // shared memory for k staging in the force pass
 constexpr int kSamplerD = 640;   // pre-drawn proposals per axis in the sampler kernel (38 KB smem)
-constexpr int kMdChunk = 2048;   // atoms per kinetic-energy chunk
+constexpr int kMdChunkMax = 1024;   // atoms per kinetic-energy chunk: at most
 
 }  // namespace
 
@@ -133,6 +133,7 @@ struct rbmd_force {
   bool autotune = false;                // "autotune": true tunes them at the first compute
   bool tuned = false;
   bool list_valid = false;   // a list (and x_ref) exists from an earlier build
+  bool rebuild_clear = false;   // d_rebuild is zero: the last thing that ran was a whole step
   int shake_max_iter = 5000;
   std::string potential_file, potential_format;   // format: "", "funcfl" or "setfl"
 
@@ -224,7 +225,7 @@ struct rbmd_force {
   // MD
   MdChunk* d_chunks = nullptr;
   int nchunks = 0;
-  int* d_chunk_rep_begin = nullptr;
+  int *d_chunk_rep_begin = nullptr, *d_chunk_done = nullptr;
   double *d_ke_partial = nullptr, *d_ke = nullptr, *d_T = nullptr, *d_lambda = nullptr,
          *d_xi = nullptr, *d_xold = nullptr, *d_vold = nullptr;
   bool pending_scale = false;
@@ -434,7 +435,7 @@ void free_all(rbmd_force* f) {
   f->d_partial = nullptr;
   dfree(f->d_rho_done); dfree(f->d_cidx);
   dfree(f->d_rho); dfree(f->d_ek); dfree(f->d_far); dfree(f->d_weights); dfree(f->d_srep); dfree(f->d_qtab);
-  dfree(f->d_chunks); dfree(f->d_chunk_rep_begin); dfree(f->d_ke_partial); dfree(f->d_ke);
+  dfree(f->d_chunks); dfree(f->d_chunk_rep_begin); dfree(f->d_chunk_done); dfree(f->d_ke_partial); dfree(f->d_ke);
   dfree(f->d_T); dfree(f->d_lambda); dfree(f->d_xi); dfree(f->d_xold); dfree(f->d_vold);
   dfree(f->d_frho); dfree(f->d_rhor); dfree(f->d_z2r); dfree(f->d_eam_rows); dfree(f->d_posf);
   if (f->d_fp) cudaFree(f->d_fp);
@@ -1339,8 +1340,9 @@ bool launch_rebuild_conditional(rbmd_force* f, cudaStream_t s, bool bin) {
 // Force evaluation from the current master positions: the k-space chain forks onto the side
 // stream, the cell sort / neighbour list / near pass / intramolecular terms run on the caller's
 // stream, and the far force is folded in after the join.
+// fold_far: add the k-space force here (a step without a Langevin force leaves it to its kick).
 template <class R>
-void launch_force_tail(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
+void launch_force_tail(rbmd_force* f, cudaStream_t s, bool bin, bool regather, bool fold_far) {
   const bool kspace = f->is_rbe();
   if (kspace) {
     cudaEventRecord(f->ev_fork, s);
@@ -1371,7 +1373,7 @@ void launch_force_tail(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
   }
   if (kspace) {
     cudaStreamWaitEvent(s, f->ev_join, 0);
-    if (f->nq > 0) {
+    if (f->nq > 0 && fold_far) {
       k_add_far<<<(3 * f->nq + 255) / 256, 256, 0, s>>>(f->nq, f->d_qidx, f->d_far, f->at.force, f->d_status);
       f->launches++;
     }
@@ -1397,6 +1399,7 @@ template <class R>
 void launch_compute(rbmd_force* f, cudaStream_t s) {
   f->want_energy = true;
   f->presampled = false;   // a force call draws the k-set of the current step counter itself
+  f->rebuild_clear = false;
   cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s);
   if (f->skin > 0 && f->list_valid) {
     // reuse the list when no atom moved more than skin/2 since it was built
@@ -1408,7 +1411,7 @@ void launch_compute(rbmd_force* f, cudaStream_t s) {
   } else if (f->d_rebuild) {
     cudaMemsetAsync(f->d_rebuild, 1, sizeof(int) * (f->nrep + 1), s);   // nonzero: rebuild
   }
-  launch_force_tail<R>(f, s, true, true);
+  launch_force_tail<R>(f, s, true, true, true);
   f->list_valid = true;
 }
 
@@ -1480,13 +1483,14 @@ void launch_step(rbmd_force* f, cudaStream_t s) {
   mp.apply_scale = f->pending_scale ? 1 : 0;
   mp.nh = f->tstat == 3;
   f->want_energy = f->energy_every > 0 && ((f->step_count + 1) % f->energy_every == 0);
-  cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s);
   const bool skin = f->skin > 0;
   // without a skin the drift bins every step; with one it writes the slot caches (unless SHAKE
   // moves the atoms afterwards) and k_bin bins on rebuild steps only
   if (!skin) cudaMemsetAsync(f->d_cell_count, 0, sizeof(int) * f->ncell_total, s);
-  // with a skin the drift kernel decides; a missing or overflowed list forces a rebuild
-  if (skin) cudaMemsetAsync(f->d_rebuild, f->list_valid ? 0 : 1, sizeof(int) * (f->nrep + 1), s);
+  // with a skin the drift kernel decides, on flags that the end of the last step cleared; a missing
+  // or overflowed list forces a rebuild
+  if (skin && !(f->list_valid && f->rebuild_clear))
+    cudaMemsetAsync(f->d_rebuild, f->list_valid ? 0 : 1, sizeof(int) * (f->nrep + 1), s);
   // (the slot map exists once a cell sort has run: list_valid)
   const bool drift_cache = skin && !shake && f->list_valid;
   // stages 1-2: kick, drift + wrap, bin (binning sees the unconstrained positions, as the
@@ -1519,29 +1523,13 @@ void launch_step(rbmd_force* f, cudaStream_t s) {
     f->launches++;
   }
   // stage 3: force (cell sort of the pre-constraint binning, then list and forces)
-  launch_force_tail<R>(f, s, skin, skin && !drift_cache);
+  const bool kick_folds = f->is_rbe() && f->nq > 0 && f->tstat != 4;
+  launch_force_tail<R>(f, s, skin, skin && !drift_cache, !kick_folds);
   f->list_valid = true;
-  // stage 3: kick (+ RATTLE), temperature, thermostat
+  // stage 3: kick (+ RATTLE), temperature, thermostat.  The temperature and thermostat run at the
+  // end of the last kernel that sums the kinetic energy; Nose-Hoover's extra kick uses the xi of
+  // before the update, so there they follow in their own launch.
   PhaseScope ps_int(f, kPhInt, s);
-  if (shake) {
-    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 1,
-                                        nullptr, nullptr);
-    k_rattle<<<((int)f->n_mol + 127) / 128, 128, 0, s>>>((int)f->n_mol, f->d_hoh, f->at.pos, f->at.vel,
-                                                         f->at.mass, f->nrep > 1 ? f->d_rep_of : nullptr,
-                                                         f->d_reps, f->d_status);
-    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 0,
-                                        nullptr, f->d_ke_partial);
-    f->launches += 3;
-  } else {
-    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 1,
-                                        nullptr, f->d_ke_partial);
-    f->launches++;
-  }
-  if (f->tstat == 3) {
-    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, 2,
-                                        f->d_xi, nullptr);
-    f->launches++;
-  }
   ThermoParams tp;
   tp.nrep = f->nrep;
   tp.tstat = f->tstat;
@@ -1551,9 +1539,38 @@ void launch_step(rbmd_force* f, cudaStream_t s) {
   tp.Tdamp = f->Tdamp;
   tp.T0 = f->T0;
   tp.dof_mode = f->dof_mode;
-  k_thermo<<<(f->nrep + 3) / 4, 128, 0, s>>>(tp, f->d_chunk_rep_begin, f->d_ke_partial, f->d_ke,
-                                                f->d_T, f->d_lambda, f->d_xi, f->d_reps);
-  f->launches++;
+  ThermoDev td;
+  td.chunk_begin_of_rep = f->d_chunk_rep_begin;
+  td.ke_partial = f->d_ke_partial;
+  td.ke = f->d_ke;
+  td.T = f->d_T;
+  td.lambda = f->d_lambda;
+  td.xi = f->d_xi;
+  td.rebuild = skin ? f->d_rebuild : nullptr;
+  td.done = f->d_chunk_done;
+  const int fused = f->tstat != 3;
+  auto kick = [&](int do_kick, const double* xi, double* ke, int thermo) {
+    const FarFold far{kick_folds && do_kick == 1 ? f->d_cidx : nullptr, f->d_far, f->d_status};
+    k_kick_ke<<<f->nchunks, 256, 0, s>>>(mp, f->d_chunks, f->at.vel, f->at.force, f->at.mass, do_kick, xi, ke, far,
+                                         thermo, tp, td, f->d_reps);
+    f->launches++;
+  };
+  if (shake) {
+    kick(1, nullptr, nullptr, 0);
+    k_rattle<<<((int)f->n_mol + 127) / 128, 128, 0, s>>>((int)f->n_mol, f->d_hoh, f->at.pos, f->at.vel,
+                                                         f->at.mass, f->nrep > 1 ? f->d_rep_of : nullptr,
+                                                         f->d_reps, f->d_status);
+    f->launches++;
+    kick(0, nullptr, f->d_ke_partial, fused);
+  } else {
+    kick(1, nullptr, f->d_ke_partial, fused);
+  }
+  if (f->tstat == 3) {
+    kick(2, f->d_xi, nullptr, 0);
+    k_thermo<<<f->nrep, 128, 0, s>>>(tp, td, f->d_reps);
+    f->launches++;
+  }
+  f->rebuild_clear = skin;
   f->pending_scale = (f->tstat == 1 || f->tstat == 2);
   f->step_count++;
 }
@@ -2551,14 +2568,18 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
   }
   // MD chunks
   {
+    // about eight blocks of 256 threads per SM, one to four atoms a thread: a block of 2048 atoms
+    // walks eight atoms a thread in FP64 (10 us), 4,000 atoms filled two such blocks, and the
+    // ragged last chunks of 512 replicas left a long tail (75 us)
+    const int chunk = std::min(kMdChunkMax, std::max(256, (f->n / (8 * f->num_sms) + 255) / 256 * 256));
     std::vector<MdChunk> ch;
     std::vector<int> crb(nrep + 1);
     for (int r = 0; r < nrep; ++r) {
       crb[r] = (int)ch.size();
-      for (int64_t b = f->rep_off[r]; b < f->rep_off[r + 1]; b += kMdChunk) {
+      for (int64_t b = f->rep_off[r]; b < f->rep_off[r + 1]; b += chunk) {
         MdChunk c;
         c.begin = (int)b;
-        c.end = (int)std::min<int64_t>(b + kMdChunk, f->rep_off[r + 1]);
+        c.end = (int)std::min<int64_t>(b + chunk, f->rep_off[r + 1]);
         c.rep = r;
         c.pad = 0;
         ch.push_back(c);
@@ -2571,6 +2592,8 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     CK(dalloc(&f->d_chunk_rep_begin, (size_t)nrep + 1));
     CK(cudaMemcpy(f->d_chunk_rep_begin, crb.data(), sizeof(int) * (nrep + 1), cudaMemcpyHostToDevice));
     CK(dalloc(&f->d_ke_partial, ch.size()));
+    CK(dalloc(&f->d_chunk_done, (size_t)nrep));
+    CK(cudaMemset(f->d_chunk_done, 0, sizeof(int) * nrep));
     if (f->is_rbl()) CK(dalloc(&f->d_mean_partial, 3 * ch.size()));
     CK(dalloc(&f->d_ke, (size_t)nrep));
     CK(dalloc(&f->d_T, (size_t)nrep));
@@ -2652,6 +2675,7 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
   CK(dalloc(&f->d_host32, (size_t)3 * f->n));
   f->bound = true;
   f->list_valid = false;
+  f->rebuild_clear = false;
   f->step_count = 0;
   f->pending_scale = false;
   return RBMD_OK;
@@ -2800,6 +2824,7 @@ rbmd_status rbmd_force_step(rbmd_force* f, int32_t n_steps, void* stream) {
     if (f->at.image)
       CK(cudaMemcpyAsync(f->d_snap_img, f->at.image, sizeof(int) * 3 * n, cudaMemcpyDeviceToDevice, s));
     f->launches = 0;
+    CK(cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s));   // longest overflowed row of this call
     CK(cudaMemcpyAsync(f->d_step, &f->step_count, sizeof(long long), cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));
     f->in_step = true;
