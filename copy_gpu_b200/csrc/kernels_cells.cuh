@@ -27,11 +27,13 @@ __device__ __forceinline__ int cell_of_pos(const RepDev& rp, R x, R y, R z) {
 
 // Verlet-skin rebuild flags: rebuild[r] for replica r and rebuild[n_replicas] for "any replica";
 // a replica whose atoms all stayed within skin/2 keeps its cells, slots and list.
-// rebuild (nullable): bin only the atoms of rebuilding replicas.
+// rebuild (nullable): bin only the atoms of rebuilding replicas.  xref (nullable): the positions of
+// this build, in caller order, so consecutive here (the cell sort would scatter them).
 template <class R>
 __global__ void k_bin(int n, const double* __restrict__ pos, const int* __restrict__ rep_of,
                       const RepDev* __restrict__ reps, int* __restrict__ cell_of,
-                      int* __restrict__ cell_count, uint32_t* status, const int* __restrict__ rebuild) {
+                      int* __restrict__ cell_count, uint32_t* status, const int* __restrict__ rebuild,
+                      double* __restrict__ xref) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int r = rep_of ? rep_of[i] : 0;
@@ -39,6 +41,7 @@ __global__ void k_bin(int n, const double* __restrict__ pos, const int* __restri
   const RepDev& rp = reps[r];
   double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
   if (!isfinite(x) || !isfinite(y) || !isfinite(z)) set_flag(status, kFlagNonFinite);
+  if (xref) { xref[3 * i] = x; xref[3 * i + 1] = y; xref[3 * i + 2] = z; }
   int c = cell_of_pos<R>(rp, (R)x, (R)y, (R)z);
   cell_of[i] = c;
   atomicAdd(&cell_count[c], 1);
@@ -169,26 +172,29 @@ __device__ __forceinline__ unsigned long long ord_key(double x) {
 // row of consecutive x cells is ordered by x, which lets the list build skip the candidates
 // beyond the cutoff in x by binary search.  Cells above kMaxCellAtoms keep the scatter order
 // (flagged by the scan).
-constexpr int kSortWarps = 4;   // cells (one per warp) per block of k_cell_sort_gather
+// nparts > 1 (cells of many atoms): a cell is shared by nparts warps, each ranking its share of the
+// atoms against all of them (30,000 water atoms fill 216 cells, 54 blocks of one warp per cell).
+constexpr int kSortWarps = 4;   // warps per block of k_cell_sort_gather
 
 template <class R>
 __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
-    int ncell, const int* __restrict__ start, const int* __restrict__ tmp_slot_atom,
+    int ncell, int nparts, const int* __restrict__ start, const int* __restrict__ tmp_slot_atom,
     const double* __restrict__ pos, const double* __restrict__ charge,
     const int* __restrict__ type, const int* __restrict__ mol, const int* __restrict__ rep_of,
     const RepDev* __restrict__ reps, int* __restrict__ slot_atom, int* __restrict__ atom_slot,
     typename Traits<R>::V4* __restrict__ pos4, void* __restrict__ frac_out,
-    int2* __restrict__ meta, double* __restrict__ xref, const int* __restrict__ rebuild, int sort_x,
-    const int* __restrict__ cell_rep) {
+    int2* __restrict__ meta, const int* __restrict__ rebuild, int sort_x, const int* __restrict__ cell_rep) {
   using Key = decltype(ord_key((R)0));
   __shared__ int ids[kSortWarps][kMaxCellAtoms];
   __shared__ Key keys[kSortWarps][kMaxCellAtoms];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int cell = blockIdx.x * kSortWarps + w;
+  const long long item = (long long)blockIdx.x * kSortWarps + w;
+  const int cell = (int)(item / nparts), part = (int)(item % nparts);
   if (cell >= ncell) return;
   if (rebuild && !rebuild[cell_rep ? cell_rep[cell] : 0]) return;
   const int s0 = start[cell], n = start[cell + 1] - s0;
-  if (n == 0) return;
+  const int k0 = (int)((long long)n * part / nparts), k1 = (int)((long long)n * (part + 1) / nparts);
+  if (k0 == k1) return;
   const bool sortable = n <= kMaxCellAtoms;
   if (sortable)
     for (int k = lane; k < n; k += 32) {
@@ -197,7 +203,7 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
       if (sort_x) keys[w][k] = ord_key((R)pos[3 * id]);
     }
   __syncwarp();
-  for (int k = lane; k < n; k += 32) {
+  for (int k = k0 + lane; k < k1; k += 32) {
     int id = sortable ? ids[w][k] : tmp_slot_atom[s0 + k];
     int rank = k;
     if (sortable) {
@@ -217,7 +223,6 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
     atom_slot[id] = slot;
     const double x = pos[3 * id], y = pos[3 * id + 1], z = pos[3 * id + 2];
     const double q = charge ? charge[id] : 0.0;
-    if (xref) { xref[3 * id] = x; xref[3 * id + 1] = y; xref[3 * id + 2] = z; }
     typename Traits<R>::V4 v;
     v.x = (R)x; v.y = (R)y; v.z = (R)z; v.w = (R)q;
     pos4[slot] = v;

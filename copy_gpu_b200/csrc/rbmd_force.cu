@@ -896,7 +896,7 @@ void launch_sort(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
       cudaMemsetAsync(f->d_cell_count, 0, sizeof(int) * f->ncell_total, s);
     }
     k_bin<R><<<(n + 255) / 256, 256, 0, s>>>(n, f->at.pos, rep_of, f->d_reps, f->d_cell_of, f->d_cell_count,
-                                             f->d_status, rb);
+                                             f->d_status, rb, f->skin > 0 ? f->d_xref : nullptr);
     f->launches++;
   }
   const int nblk = (f->ncell_total + kScanBlock - 1) / kScanBlock;
@@ -906,11 +906,14 @@ void launch_sort(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
                                     f->d_cursor, rb_any);
   k_scatter<<<(n + 255) / 256, 256, 0, s>>>(n, f->d_cell_of, f->d_cell_start, f->d_cursor, f->d_tmp, rep_of,
                                             rb);
-  k_cell_sort_gather<R><<<(f->ncell_total + kSortWarps - 1) / kSortWarps, 32 * kSortWarps, 0, s>>>(
-      f->ncell_total, f->d_cell_start, f->d_tmp, f->at.pos, f->at.charge, f->at.type,
+  // one warp per 32 atoms of a cell on average
+  const int parts = std::max(1, (int)((f->n + 32LL * f->ncell_total - 1) / (32LL * f->ncell_total)));
+  const long long sort_items = (long long)f->ncell_total * parts;
+  k_cell_sort_gather<R><<<(unsigned)((sort_items + kSortWarps - 1) / kSortWarps), 32 * kSortWarps, 0, s>>>(
+      f->ncell_total, parts, f->d_cell_start, f->d_tmp, f->at.pos, f->at.charge, f->at.type,
       molecular_mode(f) == 2 ? f->d_comp : f->at.molecule,
       rep_of, f->d_reps, f->d_slot_atom, f->d_atom_slot, (typename Traits<R>::V4*)f->d_pos4, nullptr,
-      f->d_meta, f->d_xref, rb, f->sort_x() ? 1 : 0, f->d_cell_rep);
+      f->d_meta, rb, f->sort_x() ? 1 : 0, f->d_cell_rep);
   f->launches += 4;
   if (rb && regather) launch_regather<R>(f, s);
 }
