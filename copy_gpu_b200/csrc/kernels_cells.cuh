@@ -552,10 +552,10 @@ constexpr int kCellBatch = 768;   // candidates whose accept bits are kept befor
 template <class R> struct __align__(16) CellWarpMem {
   struct __align__(16) XY { Pair<R> x, y; } xy[32];   // the atoms' -x and -y, each twice
   Pair<R> z[32];
-  R off[3][27];        // periodic offset of each stencil cell
+  R off[3][27];        // periodic offset of each non-empty stencil cell
   int start[27];       // its first slot
   int code[27];        // its image code
-  int pre[28];         // candidates before it
+  int pre[27];         // candidates before it
   int ent[kCellBatch];                      // list entry of each candidate of the batch
   unsigned word[kCellBatch / 32][32];       // accept bits [32 candidates][atom], first candidate on top
 };
@@ -585,21 +585,17 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
   const int d0 = rp.dims[0], d1 = rp.dims[1], d2n = rp.dims[2];
   const int cl = cell - rp.cell_base;
   const int cx = cl % d0, cy = (cl / d0) % d1, cz = cl / (d0 * d1);
-  // stencil cells in walk order: y outermost, then z, then x
-  int cnt = 0;
+  // the non-empty stencil cells in walk order: y outermost, then z, then x
+  int cnt = 0, st = 0, dx = 0, dy = 0, dz = 0;
   if (lane < 27) {
     const int nbx = cx + lane % 3 - 1, nbz = cz + (lane / 3) % 3 - 1, nby = cy + lane / 9 - 1;
     const int wx = wrap_cell(nbx, d0), wy = wrap_cell(nby, d1), wz = wrap_cell(nbz, d2n);
-    const int dx = wx - nbx, dy = wy - nby, dz = wz - nbz;
+    dx = wx - nbx;
+    dy = wy - nby;
+    dz = wz - nbz;
     const int c = rp.cell_base + wx + wy * d0 + wz * d0 * d1;
-    const int st = cell_start[c];
+    st = cell_start[c];
     cnt = cell_start[c + 1] - st;
-    M.off[0][lane] = mul_rn(Traits<R>::dx(rp, 0), (R)dx);
-    M.off[1][lane] = mul_rn(Traits<R>::dx(rp, 1), (R)dy);
-    M.off[2][lane] = mul_rn(Traits<R>::dx(rp, 2), (R)dz);
-    M.start[lane] = st;
-    M.code[lane] = (dx > 0 ? 1 : (dx < 0 ? 2 : 0)) | ((dy > 0 ? 1 : (dy < 0 ? 2 : 0)) << 2) |
-                   ((dz > 0 ? 1 : (dz < 0 ? 2 : 0)) << 4);
   }
   int incl = cnt;
 #pragma unroll
@@ -607,11 +603,26 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
     const int v = __shfl_up_sync(full, incl, o);
     if (lane >= o) incl += v;
   }
-  if (lane < 28) M.pre[lane] = incl - cnt;   // lane 27 (count 0) holds the total
-  const int total = __shfl_sync(full, incl, 27);
+  const int total = __shfl_sync(full, incl, 31);
+  const unsigned some = __ballot_sync(full, cnt > 0);
+  const int nseg = __popc(some);
+  if (cnt > 0) {
+    const int at = __popc(some & ((1u << lane) - 1u));
+    M.off[0][at] = mul_rn(Traits<R>::dx(rp, 0), (R)dx);
+    M.off[1][at] = mul_rn(Traits<R>::dx(rp, 1), (R)dy);
+    M.off[2][at] = mul_rn(Traits<R>::dx(rp, 2), (R)dz);
+    M.start[at] = st;
+    M.code[at] = (dx > 0 ? 1 : (dx < 0 ? 2 : 0)) | ((dy > 0 ? 1 : (dy < 0 ? 2 : 0)) << 2) |
+                 ((dz > 0 ? 1 : (dz < 0 ? 2 : 0)) << 4);
+    M.pre[at] = incl - cnt;
+  }
+  __syncwarp();
+  // lane l holds the first candidate of segment l + 1, the rest never start
+  const int next_pre = lane + 1 < nseg ? M.pre[lane + 1] : 1 << 30;
   const R d2_lo = (R)1.0e-4;                 // gt_small
   const Pair<R> unit = both<R>(one);
   int4* out = reinterpret_cast<int4*>(nbr);
+  int strays = 0;   // atoms whose own cell is another: after the others
   for (int g0 = a0; g0 < a1; g0 += 32) {
     const int m = min(32, a1 - g0);
     const int i = g0 + min(lane, m - 1);
@@ -638,20 +649,17 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
           const int q = base + 32 * k + 31 - lane;
           px[k] = (R)INFINITY;                 // past the last candidate: never accepted
           py[k] = pz[k] = (R)0;
+          // segments starting at or before q: those before this group of 32, and a mask of the others
+          const int q0 = base + 32 * k, rel = next_pre - q0;
+          const unsigned starts = __reduce_or_sync(full, rel >= 0 && rel < 32 ? 1u << rel : 0u);
+          const int sg = __popc(__ballot_sync(full, rel < 0)) + __popc(starts & (full >> lane));
           if (q < b1) {
-            int lo = 0, hi = 27;               // pre[lo] <= q < pre[hi]
-#pragma unroll
-            for (int b = 0; b < 5; ++b) {
-              const int mid = (lo + hi) >> 1;
-              if (M.pre[mid] <= q) lo = mid;
-              else hi = mid;
-            }
-            const int s = M.start[lo] + (q - M.pre[lo]);
+            const int s = M.start[sg] + (q - M.pre[sg]);
             const V4 pj = pos4[s];
-            px[k] = sub_rn(pj.x, M.off[0][lo]);
-            py[k] = sub_rn(pj.y, M.off[1][lo]);
-            pz[k] = sub_rn(pj.z, M.off[2][lo]);
-            M.ent[q - b0] = (s << kShiftBits) | M.code[lo];
+            px[k] = sub_rn(pj.x, M.off[0][sg]);
+            py[k] = sub_rn(pj.y, M.off[1][sg]);
+            pz[k] = sub_rn(pj.z, M.off[2][sg]);
+            M.ent[q - b0] = (s << kShiftBits) | M.code[sg];
           }
         }
         unsigned word[KC];
@@ -717,10 +725,18 @@ __global__ void __launch_bounds__(32 * kCellWarps) k_nlist_cell(
         set_flag(status, kFlagListOverflow);
         atomicMax(max_count, idx);
       }
-    } else if (valid) {
-      idx = nlist_thread<R>(i, pi, rp, pos4, cell_start, 1, rc, cap, stride, nbr, false, orig);
-      nlist_finish(i, idx, cap, stride, nbr, count, max_count, status);
     }
+    strays |= __any_sync(full, valid && !mine);
+  }
+  if (!strays) return;
+  for (int i = a0 + lane; i < a1; i += 32) {
+    const V4 pi = pos4[i];
+    if ((int)div_rn(sub_rn(pi.x, Traits<R>::lo(rp, 0)), Traits<R>::dx(rp, 0)) == cx &&
+        (int)div_rn(sub_rn(pi.y, Traits<R>::lo(rp, 1)), Traits<R>::dx(rp, 1)) == cy &&
+        (int)div_rn(sub_rn(pi.z, Traits<R>::lo(rp, 2)), Traits<R>::dx(rp, 2)) == cz)
+      continue;
+    const int idx = nlist_thread<R>(i, pi, rp, pos4, cell_start, 1, rc, cap, stride, nbr, false, orig);
+    nlist_finish(i, idx, cap, stride, nbr, count, max_count, status);
   }
 }
 
