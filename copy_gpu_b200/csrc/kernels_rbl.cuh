@@ -43,14 +43,10 @@ __device__ __forceinline__ R rbl_slack(const RepDev& rp, int d, R x, R rc) {
 constexpr int kRblBatch = 4;   // candidate positions loaded ahead of their classification (8: slower)
 
 template <class R>
-__global__ void __launch_bounds__(128) k_rbl_list(
-    int n, const typename Traits<R>::V4* __restrict__ pos4, const int* __restrict__ cell_start,
-    const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot, int num_cycles, R rc, R rs,
-    int core_cap, int shell_cap, int stride, int* __restrict__ nbr, int* __restrict__ ncore,
-    int* __restrict__ nshell, int* __restrict__ max_count, uint32_t* status) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const RepDev& rp = reps[rep_of_slot ? rep_of_slot[i] : 0];
+__device__ __forceinline__ void rbl_list_slot(
+    int i, const RepDev& rp, const typename Traits<R>::V4* __restrict__ pos4, const int* __restrict__ cell_start,
+    int num_cycles, R rc, R rs, int core_cap, int shell_cap, int stride, int* __restrict__ nbr,
+    int* __restrict__ ncore, int* __restrict__ nshell, int* __restrict__ max_count, uint32_t* status) {
   const int pice = rp.rbl_pice;
   const typename Traits<R>::V4 pi = pos4[i];
   const R pix[3] = {pi.x, pi.y, pi.z};
@@ -126,6 +122,18 @@ __global__ void __launch_bounds__(128) k_rbl_list(
     atomicMax(max_count, n_core);
     atomicMax(max_count + 1, n_shell);
   }
+}
+
+template <class R>
+__global__ void __launch_bounds__(128) k_rbl_list(
+    int n, const typename Traits<R>::V4* __restrict__ pos4, const int* __restrict__ cell_start,
+    const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot, int num_cycles, R rc, R rs,
+    int core_cap, int shell_cap, int stride, int* __restrict__ nbr, int* __restrict__ ncore,
+    int* __restrict__ nshell, int* __restrict__ max_count, uint32_t* status) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  rbl_list_slot<R>(i, reps[rep_of_slot ? rep_of_slot[i] : 0], pos4, cell_start, num_cycles, rc, rs, core_cap,
+                   shell_cap, stride, nbr, ncore, nshell, max_count, status);
 }
 
 // The same list with one warp per atom (systems of 10^4 - 10^5 atoms leave the thread-per-atom
@@ -254,6 +262,302 @@ __global__ void __launch_bounds__(32 * kRblWarps) k_rbl_list_warp(
       atomicMax(max_count, n_core);
       atomicMax(max_count + 1, n_shell);
     }
+  }
+}
+
+// The same list with one warp per cell (or 1/nparts of its atoms), as k_nlist_cell builds the Verlet
+// list: the candidates of the (2 num_cycles + 1)^3 stencil, flattened over its non-empty cells in the
+// reference's walk order, sit 32 * KC at a time in the lanes' registers, every atom of the cell is
+// tested against them by a broadcast read, and two ballots give its core and shell bits.  After
+// kRblBatch candidates lane k walks the bits of atom k in candidate order: core entries four per
+// store, shell entries every pice-th of the running index.  d^2 <= core_hi (core) and shell_lo <=
+// d^2 <= shell_hi (shell) are the reference's predicates as single comparisons (pair_d2_max,
+// pair_d2_min).  Stencil cells farther than rc from the box of the warp's atoms hold no pair and
+// are left out (rbl_gap2).  Lists identical entry for entry to k_rbl_list's, which also serves the
+// atoms whose own cell index differs from the cell they were binned into.
+constexpr int kRblBatch32 = 12;              // words of 32 candidates per batch
+constexpr int kRblBatchN = 32 * kRblBatch32;
+
+template <class R> struct __align__(16) RblCellMem {
+  typename CellWarpMem<R>::XY xy[32];
+  Pair<R> z[32];
+  int ent[kRblBatchN];
+  unsigned core[kRblBatch32][32], shell[kRblBatch32][32];
+  // followed by R off[3][S], int start[S], code[S], pre[S + 1] for S stencil cells
+};
+template <class R>
+__host__ __device__ __forceinline__ int rbl_cell_bytes(int S) {
+  return ((int)sizeof(RblCellMem<R>) + S * (3 * (int)sizeof(R) + 8) + 4 * (S + 1) + 15) & ~15;
+}
+
+template <class R, int KC>
+__global__ void __launch_bounds__(32 * kRblWarps) k_rbl_list_cell(
+    int ncell, int nparts, const typename Traits<R>::V4* __restrict__ pos4, const int* __restrict__ cell_start,
+    const RepDev* __restrict__ reps, const int* __restrict__ cell_rep, int num_cycles, R rc, R rs, R core_hi,
+    R shell_lo, R shell_hi, R one, int core_cap, int shell_cap, int stride, int* __restrict__ nbr,
+    int* __restrict__ ncore, int* __restrict__ nshell, int* __restrict__ max_count, uint32_t* status) {
+  using V4 = typename Traits<R>::V4;
+  constexpr unsigned full = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char rbl_raw[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long item = (long long)blockIdx.x * kRblWarps + w;
+  const int cell = (int)(item / nparts), part = (int)(item % nparts);
+  if (cell >= ncell) return;   // uniform across the warp; the kernel has no block barrier
+  const int s0 = cell_start[cell], ns = cell_start[cell + 1] - s0;
+  const int a0 = s0 + (int)((long long)ns * part / nparts), a1 = s0 + (int)((long long)ns * (part + 1) / nparts);
+  if (a0 == a1) return;
+  const RepDev& rp = reps[cell_rep ? cell_rep[cell] : 0];
+  const int nc = num_cycles, side = 2 * nc + 1, S = side * side * side;
+  unsigned char* base_mem = rbl_raw + (size_t)w * rbl_cell_bytes<R>(S);
+  RblCellMem<R>& M = *reinterpret_cast<RblCellMem<R>*>(base_mem);
+  R* off = reinterpret_cast<R*>(base_mem + sizeof(RblCellMem<R>));
+  int* seg_start = reinterpret_cast<int*>(off + 3 * S);
+  int* seg_code = seg_start + S;
+  int* seg_pre = seg_code + S;
+  const int dims[3] = {rp.dims[0], rp.dims[1], rp.dims[2]};
+  const int cl = cell - rp.cell_base;
+  const int cc[3] = {cl % dims[0], (cl / dims[0]) % dims[1], cl / (dims[0] * dims[1])};
+  const unsigned below = (1u << lane) - 1u;
+  // box of the warp's atoms
+  R lo3[3], hi3[3];
+  {
+    V4 p = pos4[a0];
+    lo3[0] = hi3[0] = p.x; lo3[1] = hi3[1] = p.y; lo3[2] = hi3[2] = p.z;
+    for (int i = a0 + lane; i < a1; i += 32) {
+      p = pos4[i];
+      lo3[0] = fmin(lo3[0], p.x); hi3[0] = fmax(hi3[0], p.x);
+      lo3[1] = fmin(lo3[1], p.y); hi3[1] = fmax(hi3[1], p.y);
+      lo3[2] = fmin(lo3[2], p.z); hi3[2] = fmax(hi3[2], p.z);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        lo3[d] = fmin(lo3[d], __shfl_xor_sync(full, lo3[d], o));
+        hi3[d] = fmax(hi3[d], __shfl_xor_sync(full, hi3[d], o));
+      }
+  }
+  const R rc2 = mul_rn(rc, rc);
+  // stencil table of the non-empty cells in walk order: x outermost, z innermost
+  int nseg = 0, total = 0;
+  for (int k0 = 0; k0 < S; k0 += 32) {
+    const int k = k0 + lane;
+    int cnt = 0, st = 0, dd[3] = {0, 0, 0};
+    if (k < S) {
+      const int o[3] = {k / (side * side) - nc, (k / side) % side - nc, k % side - nc};
+      int wr[3];
+      R g2 = (R)0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const int nb = cc[d] + o[d];
+        wr[d] = wrap_cell(nb, dims[d]);
+        dd[d] = wr[d] - nb;
+        // the point of the atoms' box nearest to the stencil cell stands for every atom
+        const R sl = Traits<R>::lo(rp, d) + (R)nb * Traits<R>::dx(rp, d);
+        const R x = hi3[d] < sl ? hi3[d] : fmax(lo3[d], sl);
+        g2 += rbl_gap2(rp, d, nb, wr[d], x, rbl_slack(rp, d, fmax(fabs(lo3[d]), fabs(hi3[d])), rc));
+      }
+      const int c = rp.cell_base + wr[0] + wr[1] * dims[0] + wr[2] * dims[0] * dims[1];
+      st = cell_start[c];
+      cnt = g2 > rc2 ? 0 : cell_start[c + 1] - st;
+    }
+    const unsigned some = __ballot_sync(full, cnt > 0);
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(full, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (cnt > 0) {
+      const int at = nseg + __popc(some & below);
+      off[at] = mul_rn(Traits<R>::dx(rp, 0), (R)dd[0]);
+      off[S + at] = mul_rn(Traits<R>::dx(rp, 1), (R)dd[1]);
+      off[2 * S + at] = mul_rn(Traits<R>::dx(rp, 2), (R)dd[2]);
+      seg_start[at] = st;
+      seg_code[at] = (dd[0] > 0 ? 1 : (dd[0] < 0 ? 2 : 0)) | ((dd[1] > 0 ? 1 : (dd[1] < 0 ? 2 : 0)) << 2) |
+                     ((dd[2] > 0 ? 1 : (dd[2] < 0 ? 2 : 0)) << 4);
+      seg_pre[at] = total + incl - cnt;
+    }
+    nseg += __popc(some);
+    total += __shfl_sync(full, incl, 31);
+  }
+  const R d2_lo = (R)1.0e-4;
+  const Pair<R> unit = both<R>(one);
+  const int pice = rp.rbl_pice;
+  int4* out = reinterpret_cast<int4*>(nbr);
+  int strays = 0;   // atoms whose own cell is another: after the others
+  for (int g0 = a0; g0 < a1; g0 += 32) {
+    const int m = min(32, a1 - g0);
+    const int i = g0 + min(lane, m - 1);
+    const V4 pi = pos4[i];
+    const int ci0 = (int)div_rn(sub_rn(pi.x, Traits<R>::lo(rp, 0)), Traits<R>::dx(rp, 0));
+    const int ci1 = (int)div_rn(sub_rn(pi.y, Traits<R>::lo(rp, 1)), Traits<R>::dx(rp, 1));
+    const int ci2 = (int)div_rn(sub_rn(pi.z, Traits<R>::lo(rp, 2)), Traits<R>::dx(rp, 2));
+    const bool valid = lane < m, mine = valid && ci0 == cc[0] && ci1 == cc[1] && ci2 == cc[2];
+    __syncwarp();
+    M.xy[lane].x = both<R>(-pi.x);
+    M.xy[lane].y = both<R>(-pi.y);
+    M.z[lane] = both<R>(-pi.z);
+    int n_core = 0, n_shell = 0;
+    int skip = 0;                              // shell pairs before the next kept one
+    int cch[4] = {0, 0, 0, 0}, sch[4] = {0, 0, 0, 0}, chave = 0, shave = 0;   // open chunks
+    int4 *cdst = out + i, *sdst = out + (size_t)(core_cap >> 2) * stride + i;
+    int crow = 0, srow = 0;
+    int seg0 = 0;                              // segment of the next candidate
+    for (int b0 = 0; b0 < total; b0 += kRblBatchN) {
+      const int b1 = min(total, b0 + kRblBatchN);
+      __syncwarp();
+      for (int base = b0; base < b1; base += 32 * KC) {
+        R px[KC], py[KC], pz[KC];
+#pragma unroll
+        for (int k = 0; k < KC; ++k) {
+          const int q0 = base + 32 * k, q = q0 + 31 - lane;
+          px[k] = (R)INFINITY;                 // past the last candidate: never accepted
+          py[k] = pz[k] = (R)0;
+          if (q0 < b1) {                       // uniform
+            // segments that start inside (q0, q0 + 32]: at most 32, their positions as a bit mask
+            const int nx = seg0 + 1 + lane;
+            const int at = nx < nseg ? seg_pre[nx] - q0 : 64;
+            const unsigned starts = __reduce_or_sync(full, at < 32 ? 1u << at : 0u);
+            const int edge = __any_sync(full, at == 32);
+            const int sg = seg0 + __popc(starts & (full >> lane));   // starts at or before q (31 - lane)
+            if (q < b1) {
+              const int s = seg_start[sg] + (q - seg_pre[sg]);
+              const V4 pj = pos4[s];
+              px[k] = sub_rn(pj.x, off[sg]);
+              py[k] = sub_rn(pj.y, off[S + sg]);
+              pz[k] = sub_rn(pj.z, off[2 * S + sg]);
+              M.ent[q - b0] = (s << kShiftBits) | seg_code[sg];
+            }
+            seg0 += __popc(starts) + edge;
+          }
+        }
+        unsigned wc[KC], ws[KC];
+#pragma unroll
+        for (int k = 0; k < KC; ++k) wc[k] = ws[k] = 0;
+        for (int a = 0; a < m; ++a) {
+          const typename CellWarpMem<R>::XY o = M.xy[a];
+          const Pair<R> oz = M.z[a];
+#pragma unroll
+          for (int h = 0; h < KC; h += 2) {
+            const Pair<R> dx = add2(Pair<R>{px[h], px[h + 1]}, o.x), dy = add2(Pair<R>{py[h], py[h + 1]}, o.y),
+                          dz = add2(Pair<R>{pz[h], pz[h + 1]}, oz);
+            const Pair<R> dd = fma2(mul2(dz, dz), unit, fma2(mul2(dy, dy), unit, mul2(dx, dx)));
+            const unsigned ca = __ballot_sync(full, dd.x > d2_lo && dd.x <= core_hi);
+            const unsigned cb = __ballot_sync(full, dd.y > d2_lo && dd.y <= core_hi);
+            const unsigned sa = __ballot_sync(full, dd.x >= shell_lo && dd.x <= shell_hi);
+            const unsigned sb = __ballot_sync(full, dd.y >= shell_lo && dd.y <= shell_hi);
+            if (a == lane) {
+              wc[h] = ca;
+              wc[h + 1] = cb;
+              ws[h] = sa;
+              ws[h + 1] = sb;
+            }
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < KC; ++k) {
+          M.core[(base - b0) / 32 + k][lane] = wc[k];
+          M.shell[(base - b0) / 32 + k][lane] = ws[k];
+        }
+      }
+      __syncwarp();
+      if (mine) {
+        const int nw = (b1 - b0 + 31) / 32;
+        int found = 0, shells = 0;
+        for (int k = 0; k < nw; ++k) {
+          found += __popc(M.core[k][lane]);
+          shells += __popc(M.shell[k][lane]);
+        }
+        // core entries of the batch
+        {
+          int wi = 0;
+          unsigned bits = M.core[0][lane];
+          auto next = [&]() -> int {
+            while (bits == 0) bits = M.core[++wi][lane];
+            const int c = __clz(bits);
+            bits ^= 0x80000000u >> c;
+            return M.ent[32 * wi + c];
+          };
+          const int all = chave + found;
+          n_core += found;
+          for (int t = 0; t < all >> 2; ++t) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (k >= chave) cch[k] = next();
+            chave = 0;
+            if (crow < core_cap) *cdst = make_int4(cch[0], cch[1], cch[2], cch[3]);
+            cdst += stride;
+            crow += 4;
+          }
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            if (k >= chave && k < (all & 3)) cch[k] = next();
+          chave = all & 3;
+        }
+        // kept shell entries: after `skip` dropped pairs, then every pice-th
+        if (shells > skip) {
+          const int kept = (shells - skip - 1) / pice + 1;
+          int wi = 0, drop = skip;
+          unsigned bits = M.shell[0][lane];
+          auto next = [&]() -> int {
+            int c;
+            for (;;) {
+              while (bits == 0) bits = M.shell[++wi][lane];
+              c = __clz(bits);
+              bits ^= 0x80000000u >> c;
+              if (drop == 0) break;
+              --drop;
+            }
+            drop = pice - 1;
+            return M.ent[32 * wi + c];
+          };
+          const int all = shave + kept;
+          n_shell += kept;
+          for (int t = 0; t < all >> 2; ++t) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (k >= shave) sch[k] = next();
+            shave = 0;
+            if (srow < shell_cap) *sdst = make_int4(sch[0], sch[1], sch[2], sch[3]);
+            sdst += stride;
+            srow += 4;
+          }
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+            if (k >= shave && k < (all & 3)) sch[k] = next();
+          shave = all & 3;
+          skip = pice - 1 - (shells - 1 - (skip + (kept - 1) * pice));
+        } else {
+          skip -= shells;
+        }
+      }
+    }
+    if (mine) {
+      const int self = i << kShiftBits;
+      if (chave > 0 && crow < core_cap)
+        *cdst = make_int4(cch[0], chave > 1 ? cch[1] : self, chave > 2 ? cch[2] : self, self);
+      if (shave > 0 && srow < shell_cap)
+        *sdst = make_int4(sch[0], shave > 1 ? sch[1] : self, shave > 2 ? sch[2] : self, self);
+      ncore[i] = n_core;
+      nshell[i] = n_shell;
+      if (n_core > core_cap || n_shell > shell_cap) {
+        set_flag(status, kFlagListOverflow);
+        atomicMax(max_count, n_core);
+        atomicMax(max_count + 1, n_shell);
+      }
+    }
+    strays |= __any_sync(full, valid && !mine);
+  }
+  if (!strays) return;
+  for (int i = a0 + lane; i < a1; i += 32) {
+    const V4 pi = pos4[i];
+    if ((int)div_rn(sub_rn(pi.x, Traits<R>::lo(rp, 0)), Traits<R>::dx(rp, 0)) == cc[0] &&
+        (int)div_rn(sub_rn(pi.y, Traits<R>::lo(rp, 1)), Traits<R>::dx(rp, 1)) == cc[1] &&
+        (int)div_rn(sub_rn(pi.z, Traits<R>::lo(rp, 2)), Traits<R>::dx(rp, 2)) == cc[2])
+      continue;
+    rbl_list_slot<R>(i, rp, pos4, cell_start, num_cycles, rc, rs, core_cap, shell_cap, stride, nbr, ncore, nshell,
+                     max_count, status);
   }
 }
 
@@ -553,7 +857,7 @@ __global__ void __launch_bounds__(128) k_rbl_eam_force(int n, int stride, int co
 
 // Mean removal F_i -= (sum_j F_j) / N_replica (SumRBLCorrForceWorklet, RunWorklet.cpp:1304-1321,
 // after the Reduce of ExecutionMD.cpp:568-569): per-chunk FP64 sums in a fixed order, then every
-// block re-sums its replica's chunk partials in chunk order (deterministic) and subtracts.
+// block re-sums its replica's chunk partials in a fixed order (deterministic) and subtracts.
 __global__ void __launch_bounds__(256) k_force_chunk_sum(const MdChunk* __restrict__ chunks,
                                                          const double* __restrict__ force,
                                                          double* __restrict__ partial) {
@@ -585,12 +889,24 @@ __global__ void __launch_bounds__(256) k_force_sub_mean(const MdChunk* __restric
                                                         const double* __restrict__ partial,
                                                         double* __restrict__ force) {
   const MdChunk c = chunks[blockIdx.x];
-  __shared__ double mean[3];
+  __shared__ double mean[3], red[3][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[3] = {0, 0, 0};
+  for (int k = chunk_rep_begin[c.rep] + threadIdx.x; k < chunk_rep_begin[c.rep + 1]; k += blockDim.x)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[d] += partial[3 * k + d];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[d] += __shfl_xor_sync(0xffffffffu, v[d], o);
+    if (lane == 0) red[d][warp] = v[d];
+  }
+  __syncthreads();
   if (threadIdx.x < 3) {
-    double v = 0;
-    for (int k = chunk_rep_begin[c.rep]; k < chunk_rep_begin[c.rep + 1]; ++k) v += partial[3 * k + threadIdx.x];
+    double t = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[threadIdx.x][w];
     const RepDev& rp = reps[c.rep];
-    mean[threadIdx.x] = v / (double)(rp.atom_end - rp.atom_begin);
+    mean[threadIdx.x] = t / (double)(rp.atom_end - rp.atom_begin);
   }
   __syncthreads();
   for (int a = c.begin + threadIdx.x; a < c.end; a += blockDim.x)

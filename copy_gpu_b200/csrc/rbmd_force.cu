@@ -806,6 +806,30 @@ R pair_d2_max(R rc, bool reuse, bool orig) {
   return v;
 }
 
+// Smallest d^2 with d^2 - rs^2 > 1e-4, found the same way.
+template <class R>
+R pair_d2_min(R rs) {
+  using I = typename std::conditional<sizeof(R) == 4, uint32_t, uint64_t>::type;
+  const volatile R cut2 = rs * rs;
+  auto accepts = [&](R d2) -> bool {
+    const volatile R margin = d2 - cut2;
+    return margin > (R)1.0e-4;
+  };
+  I lo, hi;   // not accepts(lo), accepts(hi)
+  const R c = cut2, top = (R)2 * c + (R)1;
+  std::memcpy(&lo, &c, sizeof lo);
+  std::memcpy(&hi, &top, sizeof hi);
+  while (hi - lo > 1) {
+    const I mid = lo + (hi - lo) / 2;
+    R v;
+    std::memcpy(&v, &mid, sizeof v);
+    (accepts(v) ? hi : lo) = mid;
+  }
+  R v;
+  std::memcpy(&v, &hi, sizeof v);
+  return v;
+}
+
 template <class R>
 R lean_d2_max(const rbmd_force* f) {
   return pair_d2_max<R>((R)f->rc, f->skin > 0, f->orig_pred);
@@ -848,11 +872,17 @@ template <class R>
 void launch_rbl_list(rbmd_force* f, cudaStream_t s) {
   PhaseScope ps(f, kPhList, s);
   const int* rp = f->nrep > 1 ? f->d_rep_of : nullptr;
-  const int side = 2 * f->num_cycles + 1;
-  // one warp per atom below 10 warps' worth of atoms per SM (measured crossover between 21k and
-  // 98k atoms on B200), where one thread per atom leaves most SMs idle
-  const bool warp = f->rbl_list_warp > 0 || (f->rbl_list_warp < 0 && f->n < 10 * 32 * f->num_sms);
-  if (warp && side * side * side <= kRblStencilMax) {
+  const int side = 2 * f->num_cycles + 1, ncs = side * side * side;
+  if (f->rbl_list_warp < 0 && ncs <= kRblStencilMax) {   // warp per cell
+    const long long items = (long long)f->ncell_total * f->list_parts;
+    const size_t smem = (size_t)kRblWarps * rbl_cell_bytes<R>(ncs);
+    k_rbl_list_cell<R, sizeof(R) == 4 ? 4 : 2>
+        <<<(unsigned)((items + kRblWarps - 1) / kRblWarps), 32 * kRblWarps, smem, s>>>(
+            f->ncell_total, f->list_parts, (const typename Traits<R>::V4*)f->d_pos4, f->d_cell_start, f->d_reps,
+            f->nrep > 1 ? f->d_cell_rep : nullptr, f->num_cycles, (R)f->rc, (R)f->rs,
+            pair_d2_max<R>((R)f->rs, true, false), pair_d2_min<R>((R)f->rs), pair_d2_max<R>((R)f->rc, true, false),
+            (R)1, f->core_cap, f->shell_cap, f->stride, f->d_nbr, f->d_count, f->d_count2, f->d_maxcount, f->d_status);
+  } else if (f->rbl_list_warp > 0 && ncs <= kRblStencilMax) {
     k_rbl_list_warp<R><<<(f->n + kRblWarps - 1) / kRblWarps, 32 * kRblWarps, 0, s>>>(
         f->n, (const typename Traits<R>::V4*)f->d_pos4, f->d_cell_start, f->d_reps, rp, f->num_cycles, (R)f->rc,
         (R)f->rs, f->core_cap, f->shell_cap, f->stride, f->d_nbr, f->d_count, f->d_count2, f->d_maxcount,
@@ -2351,6 +2381,14 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     const int few = (24 * f->num_sms + f->ncell_total - 1) / f->ncell_total;
     f->list_parts = std::max((int)std::ceil(apc / 32.0), std::min(few, (int)std::ceil(apc / 4.0)));
     f->list_parts = std::max(1, f->list_parts);
+  }
+  if (f->is_rbl()) {   // the cell-cooperative list build of the largest stencils asks for more than 48 KB
+    const int side = 2 * f->num_cycles + 1, ncs = side * side * side;
+    if (ncs <= kRblStencilMax) {
+      const int bytes = kRblWarps * (fp64 ? rbl_cell_bytes<double>(kRblStencilMax) : rbl_cell_bytes<float>(kRblStencilMax));
+      CK(cudaFuncSetAttribute(fp64 ? (const void*)k_rbl_list_cell<double, 2> : (const void*)k_rbl_list_cell<float, 4>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    }
   }
   CK(dalloc(&f->d_maxcount, 2));
   CK(dalloc(&f->d_nbuilds, 1));
