@@ -33,7 +33,6 @@ struct __align__(1024) MlpSmem {
   uint16_t w2t[kMlpHid * kMlpHid];      //  8 KB  W2^T [64][64]    (B of dA1 = dZ2 W2)
   uint16_t a1[kMlpRows * kMlpHid];      // 32 KB  A1   [256][64]   (A of layer 2)
   uint16_t dz2[kMlpRows * kMlpHid];     // 32 KB  dZ2  [256][64]   (A of dA1); then dZ1 FP32 over a1+dz2
-  float part[32][kMlpRows / 2];         // 16 KB  partial dW2 of the second half of the rows
   float red[8][kMlpHid];                // per-warp partial sums
   float gsum[8][4];
   float par_b1[kMlpHid], par_b2[kMlpHid], par_w3[kMlpHid];
@@ -344,40 +343,30 @@ __global__ void __launch_bounds__(256, 1) k_mlp(MlpArgs args) {
   }
   {
     float* G = args.grad_partial + (size_t)g * kMlpNParam;
-    // thread (row half, 4 rows of dW2, 8 columns): per row one 8-byte read of dZ2 and one 16-byte read
-    // of A1 feed 32 FMAs; the halves are added through shared memory
-    const int half = t >> 7, j0 = ((t & 127) >> 3) * 4, i0 = (t & 7) * 8;
-    float acc[4][8];
+    // 4 x 4 values of dW2 per thread: per row one 8-byte read each of dZ2 and A1 feed 16 FMAs (the rows
+    // in order, one FP32 chain per value).  A warp covers 32 outputs x 16 inputs, which keeps the
+    // core-matrix columns it reads, 128 bytes apart, to four and two.
+    const int j0 = (w >> 2) * 32 + (lane >> 2) * 4, i0 = (w & 3) * 16 + (lane & 3) * 4;
+    float acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[a][k] = 0.f;
-#pragma unroll 4
-    for (int q = half * (kMlpRows / 2); q < (half + 1) * (kMlpRows / 2); ++q) {
-      const int r = (q & ~7) | ((q + t) & 7);   // the 8 column groups of a warp read 8 different rows (no conflicts)
+      for (int k = 0; k < 4; ++k) acc[a][k] = 0.f;
+#pragma unroll 8
+    for (int r = 0; r < kMlpRows; ++r) {
       const uint2 dv = *reinterpret_cast<const uint2*>(&S.dz2[core_off(r, j0, kMlpHid)]);
+      const uint2 av = *reinterpret_cast<const uint2*>(&S.a1[core_off(r, i0, kMlpHid)]);
       const float d[4] = {bf16_lo(dv.x), bf16_hi(dv.x), bf16_lo(dv.y), bf16_hi(dv.y)};
-      float x[8];
-      unpack8(*reinterpret_cast<const uint4*>(&S.a1[core_off(r, i0, kMlpHid)]), x);
+      const float x[4] = {bf16_lo(av.x), bf16_hi(av.x), bf16_lo(av.y), bf16_hi(av.y)};
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[a][k] = fmaf(d[a], x[k], acc[a][k]);
+        for (int k = 0; k < 4; ++k) acc[a][k] = fmaf(d[a], x[k], acc[a][k]);
     }
-    if (half) {
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) S.part[a * 8 + k][t & 127] = acc[a][k];
-    }
-    __syncthreads();
-    if (!half) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          G[kOW2 + (j0 + a) * kMlpHid + i0 + k] = acc[a][k] + S.part[a * 8 + k][t];
-    }
+      for (int k = 0; k < 4; ++k) G[kOW2 + (j0 + a) * kMlpHid + i0 + k] = acc[a][k];
   }
   ok = mbar_wait(&S.mbar, parity);
   parity ^= 1;
