@@ -76,13 +76,17 @@ __device__ __forceinline__ float rcp_r(float x) {
   return r;
 }
 
+// The same with one Newton step, to within about an ulp (the IEEE form takes a dozen instructions).
+__device__ __forceinline__ float rcp_nr(float x) {
+  const float t = rcp_r(x);
+  return fmaf(t, fmaf(-x, t, 1.0f), t);
+}
+
 // erfc(x) for x >= 0 given e = exp(-x^2).  FP32: Abramowitz & Stegun, Handbook of Mathematical
 // Functions, eq. 7.1.26 (rational approximation in t = 1/(1 + p x), |error| <= 1.5e-7), which
 // reuses the Gaussian factor the real-space force needs anyway.  FP64: the library erfc.
 __device__ __forceinline__ float erfc_shared(float x, float e) {
-  // 1 / d to within an ulp: the MUFU reciprocal and one Newton step (the correctly rounded one takes
-  // a dozen instructions; both leave the formula's 1.5e-7 as it is)
-  const float d = fmaf(0.3275911f, x, 1.0f), t0 = rcp_r(d), t = fmaf(t0, fmaf(-d, t0, 1.0f), t0);
+  const float t = rcp_nr(fmaf(0.3275911f, x, 1.0f));   // an ulp of t leaves the formula's 1.5e-7 as it is
   float poly = fmaf(1.061405429f, t, -1.453152027f);
   poly = fmaf(poly, t, 1.421413741f);
   poly = fmaf(poly, t, -0.284496736f);
@@ -492,6 +496,7 @@ __global__ void __launch_bounds__(256) k_near_force_group(
       }
     }
     R gx = 0, gy = 0, gz = 0;
+    unsigned bonded = 0;   // entries of the atom's own bond-graph component (SPW)
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const R r0 = pj[k].x - pi.x, r1 = pj[k].y - pi.y, r2 = pj[k].z - pi.z;
@@ -515,14 +520,10 @@ __global__ void __launch_bounds__(256) k_near_force_group(
       R fl0 = 0, fl1 = 0, fl2 = 0;
       bool same = false;
       int tj = 0;
-      R wsp = (R)1;   // special-bond LJ weight (molecular == 2: meta.y is the bond-graph component)
       if (typed) {
         same = MOLEC && (mj[k].y == mi.y);
         tj = prm.ntypes > 1 ? mj[k].x : 0;
-        if (SPW && same) {
-          wsp = special_weight<R>(prm.sp, slot_atom[i], slot_atom[ee[k] >> kShiftBits]);
-          same = false;
-        }
+        if (SPW && same) bonded |= 1u << k;
       }
       if (!same) {
         R q0 = r0, q1 = r1, q2 = r2;
@@ -536,15 +537,45 @@ __global__ void __launch_bounds__(256) k_near_force_group(
           const R inv2 = rcp_r(dl2);
           const R sd6 = lj_s6[trow + tj] * inv2 * inv2 * inv2;
           const R a24 = lj_a[trow + tj];
-          R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2;
-          if (SPW) scal *= wsp;
+          const R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2;
           fl0 = scal * q0; fl1 = scal * q1; fl2 = scal * q2;
-          if (ENERGY) e_lj += (SPW ? wsp : (R)1) * (-a24 / (R)6 * (sd6 - (R)1) * sd6);
+          if (ENERGY) e_lj += -a24 / (R)6 * (sd6 - (R)1) * sd6;
         }
       }
       gx += f * r0 + fl0;
       gy += f * r1 + fl1;
       gz += f * r2 + fl2;
+    }
+    if (SPW) {
+      // LJ of pairs inside the component, a dozen per atom, with the special-bond weight of the
+      // pair: one copy of the partner search, outside the unrolled entries
+      while (bonded) {
+        const int b = __ffs(bonded) - 1;
+        bonded &= bonded - 1;
+        const int e = b & 2 ? (b & 1 ? ee[3] : ee[2]) : (b & 1 ? ee[1] : ee[0]);
+        const int k0 = e & 3, k1 = (e >> 2) & 3, k2 = (e >> 4) & 3;
+        const V4 q = pos4[e >> kShiftBits];
+        R q0 = (k0 == 0 ? q.x : q.x - (k0 == 1 ? Traits<R>::wrap(rp, 0) : -Traits<R>::wrap(rp, 0))) - pi.x;
+        R q1 = (k1 == 0 ? q.y : q.y - (k1 == 1 ? Traits<R>::wrap(rp, 1) : -Traits<R>::wrap(rp, 1))) - pi.y;
+        R q2 = (k2 == 0 ? q.z : q.z - (k2 == 1 ? Traits<R>::wrap(rp, 2) : -Traits<R>::wrap(rp, 2))) - pi.z;
+        if ((MI & 3) == kMiLJ) {
+          const R box[3] = {Traits<R>::box(rp, 0), Traits<R>::box(rp, 1), Traits<R>::box(rp, 2)};
+          min_image(q0, q1, q2, box);
+        }
+        const R dl2 = q0 * q0 + q1 * q1 + q2 * q2;
+        if (dl2 < cut2 && dl2 > (R)0.0001) {
+          const int tj = prm.ntypes > 1 ? meta[e >> kShiftBits].x : 0;
+          const R wsp = special_weight<R>(prm.sp, slot_atom[i], slot_atom[e >> kShiftBits]);
+          const R inv2 = rcp_r(dl2);
+          const R sd6 = lj_s6[trow + tj] * inv2 * inv2 * inv2;
+          const R a24 = lj_a[trow + tj];
+          const R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2 * wsp;
+          gx += scal * q0;
+          gy += scal * q1;
+          gz += scal * q2;
+          if (ENERGY) e_lj += wsp * (-a24 / (R)6 * (sd6 - (R)1) * sd6);
+        }
+      }
     }
     acc.add(gx, gy, gz);
   }
