@@ -273,6 +273,7 @@ struct rbmd_force {
   bool graph_multi_pending = false;
   int graph_launches = 0;
   bool graph_pending = false;    // pending_scale the graph was captured with
+  bool graph_presampled = false; // presampled the graph was captured with
   bool capturing = false;
   cudaStream_t gstream = nullptr;
   cudaEvent_t ev_begin = nullptr;
@@ -1283,6 +1284,24 @@ __global__ void k_f64_to_f32(long long m, const double* __restrict__ a, float* _
     b[k] = (float)a[k];
 }
 
+// State at the start of a step call, for its replay when a list overflows: one launch for the four
+// arrays.
+__global__ void k_snapshot(long long m, const double* __restrict__ pos, const double* __restrict__ vel,
+                           const double* __restrict__ force, const int* __restrict__ image,
+                           double* __restrict__ snap, int* __restrict__ snap_img) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x) {
+    const double x = pos[k], v = vel[k], f = force[k];
+    const int g = image ? image[k] : 0;
+    snap[k] = x;
+    snap[m + k] = v;
+    snap[2 * m + k] = f;
+    if (image) snap_img[k] = g;
+  }
+}
+
+// The samplers' step index (by value: the host counter moves on while the call's work is queued).
+__global__ void k_set_step(long long* step, long long value) { *step = value; }
+
 // General topology: per-term forces, then the per-atom gather with the Coulomb correction.
 void launch_bonded(rbmd_force* f, cudaStream_t s) {
   BondedParams bp;
@@ -1610,7 +1629,8 @@ void launch_step(rbmd_force* f, cudaStream_t s) {
 
 // n_steps MD steps on stream s.  With execution.cuda_graph (default on) and no per-step host
 // decisions (no energy output, no profiling), the first step runs directly (it brings the lazy
-// thermostat state and the list flag to their steady values), the next step is captured once on
+// thermostat state and the list flag to their steady values; a later call that finds them so starts
+// with the graph), the next step is captured once on
 // an internal stream (the k-space stream joins the capture) and then replayed with one
 // cudaGraphLaunch per step on s.  The samplers read the step index from a device counter that
 // the k-space chain advances, so every replay draws new k-samples.  The captured step is
@@ -1623,8 +1643,13 @@ rbmd_status run_steps(rbmd_force* f, int n_steps, cudaStream_t s) {
     if (f->is_rbe()) cudaStreamWaitEvent(s, f->ev_tail, 0);   // the k-space stream's tail joins s
     return RBMD_OK;
   }
-  launch_step<R>(f, s);
-  if (f->is_rbe()) cudaStreamWaitEvent(s, f->ev_tail, 0);   // graph launches on s follow the whole step
+  // the first step runs directly, unless the state is the one that the captured steps start from
+  const bool steady = f->graph_exec && f->graph_pending == f->pending_scale && f->list_valid &&
+                      (f->skin == 0 || f->rebuild_clear) && f->graph_presampled == f->presampled;
+  if (!steady) {
+    launch_step<R>(f, s);
+    if (f->is_rbe()) cudaStreamWaitEvent(s, f->ev_tail, 0);   // graph launches on s follow the whole step
+  }
   const int per_step = f->launches;
   if (!f->gstream) CK(cudaStreamCreateWithFlags(&f->gstream, cudaStreamNonBlocking));
   if (!f->ev_begin) CK(cudaEventCreateWithFlags(&f->ev_begin, cudaEventDisableTiming));
@@ -1670,8 +1695,9 @@ rbmd_status run_steps(rbmd_force* f, int n_steps, cudaStream_t s) {
     rbmd_status st = capture(1, &f->graph_exec, &f->graph_launches);
     if (st) return st;
     f->graph_pending = f->pending_scale;
+    f->graph_presampled = f->presampled;
   }
-  int remaining = n_steps - 1;
+  int remaining = steady ? n_steps : n_steps - 1;
   const int m = f->graph_steps;
   if (m > 1 && remaining >= m) {
     // several steps per graph launch: small systems pay the graph launch once per m steps
@@ -2859,15 +2885,13 @@ rbmd_status rbmd_force_step(rbmd_force* f, int32_t n_steps, void* stream) {
   const long long step0 = f->step_count;
   const bool pend0 = f->pending_scale;
   for (int attempt = 0; attempt < 4; ++attempt) {
-    CK(cudaMemcpyAsync(f->d_snap, f->at.pos, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(f->d_snap + 3 * n, f->at.vel, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(f->d_snap + 6 * n, f->at.force, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s));
-    if (f->at.image)
-      CK(cudaMemcpyAsync(f->d_snap_img, f->at.image, sizeof(int) * 3 * n, cudaMemcpyDeviceToDevice, s));
+    k_snapshot<<<(unsigned)std::min<size_t>((3 * n + 255) / 256, 32ull * f->num_sms), 256, 0, s>>>(
+        3 * (long long)n, f->at.pos, f->at.vel, f->at.force, f->at.image, f->d_snap, f->d_snap_img);
+    CK(cudaGetLastError());
     f->launches = 0;
     CK(cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s));   // longest overflowed row of this call
-    CK(cudaMemcpyAsync(f->d_step, &f->step_count, sizeof(long long), cudaMemcpyHostToDevice, s));
-    CK(cudaStreamSynchronize(s));
+    k_set_step<<<1, 1, 0, s>>>(f->d_step, f->step_count);
+    CK(cudaGetLastError());
     f->in_step = true;
     rbmd_status gs = f->fp64 ? run_steps<double>(f, n_steps, s) : run_steps<float>(f, n_steps, s);
     f->in_step = false;
