@@ -169,15 +169,14 @@ def algorithmic(n, nq, n_nbr_mean, P, pair="near"):
 # case named beside each entry; a full-size launch has the same per-atom work (same density and
 # neighbour count), so the figures scale by atoms.  Summaries under profiles/.
 PAIR_PROFILE = {
-    # profiles/k_near_lean_electrolyte_200k.md, profiles/pair_kernels_all_workloads.md
-    "electrolyte": {"kernel": "k_near_lean", "atoms": 200_000, "dram_bytes": 68.64e6, "warp_inst": 45.68e6},
-    "batched": {"kernel": "k_near_lean", "atoms": 2_164_302, "dram_bytes": 775.98e6, "warp_inst": 556.30e6},
-    "eam": {"kernel": "k_eam_fp + k_eam_force", "atoms": 256_000, "dram_bytes": 124.95e6, "warp_inst": 91.38e6},
-    "water": {"kernel": "k_near_force_group (16 lanes)", "atoms": 30_000, "dram_bytes": 70.59e6,
-              "warp_inst": 89.23e6},
-    "lj": {"kernel": "k_near_force_group (32 lanes, FP64)", "atoms": 4_000, "dram_bytes": 1.42e6,
-           "warp_inst": 2.09e6},
-    "molecular": {"kernel": "k_rbl_force (8 lanes)", "atoms": 97_600, "dram_bytes": 44.68e6, "warp_inst": 81.31e6},
+    # profiles/pair_kernels_all_workloads.md
+    "electrolyte": {"kernel": "k_near_lean", "atoms": 1_000_000, "dram_bytes": 390.7e6, "warp_inst": 111.9e6},
+    "batched": {"kernel": "k_near_lean", "atoms": 2_266_365, "dram_bytes": 813.0e6, "warp_inst": 339.2e6},
+    "eam": {"kernel": "k_eam_fp_smem + k_eam_force_smem", "atoms": 256_000, "dram_bytes": 126.3e6, "warp_inst": 77.44e6},
+    "water": {"kernel": "k_near_force_group (16 lanes)", "atoms": 30_000, "dram_bytes": 69.85e6,
+              "warp_inst": 75.92e6},
+    "lj": {"kernel": "k_near_lean (16 lanes, FP64)", "atoms": 4_000, "dram_bytes": 1.45e6, "warp_inst": 1.55e6},
+    "molecular": {"kernel": "k_rbl_force (8 lanes)", "atoms": 101_440, "dram_bytes": 47.9e6, "warp_inst": 89.4e6},
     "molecular_verlet": {"kernel": "k_near_force_group (16 lanes)", "atoms": 97_600, "dram_bytes": 175.68e6,
                          "warp_inst": 233.34e6},
 }

@@ -173,7 +173,8 @@ __device__ __forceinline__ unsigned long long ord_key(double x) {
 // beyond the cutoff in x by binary search.  Cells above kMaxCellAtoms keep the scatter order
 // (flagged by the scan).
 // nparts > 1 (cells of many atoms): a cell is shared by nparts warps, each ranking its share of the
-// atoms against all of them (30,000 water atoms fill 216 cells, 54 blocks of one warp per cell).
+// atoms against all of them (30,000 water atoms fill 216 cells, 54 blocks of one warp per cell:
+// 37 -> 16 us with parts).
 constexpr int kSortWarps = 4;   // warps per block of k_cell_sort_gather
 
 template <class R>
@@ -543,9 +544,11 @@ __global__ void __launch_bounds__(256) k_nlist_warp(
 // + t rounds as the plain sum.  An atom whose own cell index
 // differs from the cell it was binned into (binning clamps positions at the faces) takes
 // k_nlist's path on its lane.  Bound by issue (packed tests, ballots and the walk over the bits).
-// Measured per build: 200,000 electrolyte atoms at rc 2.5 in FP32 99 us (a shared-memory staged
+// Measured per build: 200,000 electrolyte atoms at rc 2.5 in FP32 98 us (a shared-memory staged
 // build with one thread per atom: 190), 50,021 in FP64 53 us (119); averaged over the steps of a
-// run with list reuse 1,000,000 atoms 103 us (k_nlist: 154), 512 replicas 357 us (staged: 719).
+// run with list reuse 1,000,000 atoms 96 us (k_nlist: 154), 512 replicas 331 us (staged: 719).
+// Two cells in turn per warp for such batches, whose steps rebuild about one replica in five, made
+// the step 3 % slower.
 constexpr int kCellWarps = 4;
 constexpr int kCellBatch = 768;   // candidates whose accept bits are kept before entries are written
 

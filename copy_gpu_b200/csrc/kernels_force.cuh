@@ -308,7 +308,9 @@ __global__ void __launch_bounds__(256) k_near_force(
 // ComputeNearEnergyForce (rbmd/framework/forceFunction/ExecForceFunction.h:74-140).
 // G > 1: G lanes per atom for systems with too few atoms to fill the chip; lane s takes the chunks
 // s, s + G, .. and the lanes' sums are combined in FP64 by a fixed butterfly.
-// FP32 is held to 64 registers (32 warps per SM; 74 without): 1,000,000 atoms 191 -> about 183 us.
+// FP32 is held to 64 registers (32 warps per SM; 74 without).  With that and the .ftz forms of exp_r
+// and rsqrt_r: 1,000,000 atoms 219 -> 191 -> 181 us, 512 replicas 548 -> 478 -> 448 us (69 % of the
+// issue slots, 28.9 of 32 lanes active).
 template <class R, bool COUL, int MI, bool ENERGY, int G>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_lean(
     NearParams prm, R a24, R s6, R d2_max, const typename Traits<R>::V4* __restrict__ pos4,
@@ -434,7 +436,10 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_lean(
 // which no predicate accepts.  The pair terms are those of k_near_force (same predicates and
 // arithmetic); each lane sums the four forces of a chunk and folds them into a two-float
 // accumulator, and the group combines its G partial sums in FP64 with a fixed butterfly, so the
-// result does not depend on scheduling.
+// result does not depend on scheduling.  Bound by issue and the latency of the gathers: 30,000 water
+// atoms at 16 lanes 134 -> 113 us against one list entry per lane and step (65 % of the issue
+// slots); 22,824 chain atoms with special bonds 103 us, of which the search of the special lists,
+// needed only for pairs inside a molecule, took 16 us while it was unrolled with the entries.
 template <class R, bool COUL, int MI, int G>
 __global__ void __launch_bounds__(256) k_near_force_group(
     NearParams prm, const LJTable* __restrict__ ljt, const typename Traits<R>::V4* __restrict__ pos4,
@@ -608,7 +613,8 @@ __global__ void __launch_bounds__(256) k_near_force_group(
 // memory (two 16-byte broadcast loads per sample) when they fit.  Runs on the k-space stream
 // concurrently with the near pass and writes far_force[c]; k_add_far folds it into the force.
 // Bound by MUFU (two per term) when the chip is full; the lanes of an atom take every G-th sample and
-// are summed in FP64 by a fixed butterfly, so that few charged atoms still fill it (launch_rbe_force).
+// are summed in FP64 by a fixed butterfly, so that few charged atoms still fill it (launch_rbe_force):
+// 25,000 charged atoms in FP64 37 -> 27 us.
 constexpr int kRbeThreads = 128;
 
 template <class R, int G>
@@ -720,7 +726,10 @@ constexpr int kRhoStage = 256;
 
 // The fixed-point coordinates are formed while staging (k tile 0 also writes them for k_rbe_force).
 // rep_done: with few chunks per replica the block that finishes a replica's last item sums its
-// partials in chunk order and fills the records (kFusedChunks); otherwise k_rho_finish does.
+// partials in chunk order and fills the records (kFusedChunks); otherwise k_rho_finish does.  Bound by
+// MUFU (two per term) when the chip is full: 25,000 charged atoms in FP64 in chunks of 64 to 256
+// atoms 67 -> 28 us against chunks of 1024; 1,600 charged atoms 25 us with k_frac and k_rho_finish as
+// launches of their own, 16 us in one.
 constexpr int kFusedChunks = 32;
 
 template <class R, int KL>
@@ -809,8 +818,8 @@ __global__ void __launch_bounds__(256) k_rho_lanes(
 // Sum of the chunk partials of 32 consecutive k samples of one tile per block: lane = sample, so a
 // warp reads 32 consecutive partials, warp w takes the chunks w, w + warps, .. (FP64) and the warps
 // are added in order through shared memory (deterministic).
-// (One warp per sample read one 8-byte partial per 32-byte sector: 12.4 us at 390 chunks, 35 us for
-// 512 replicas of 100 samples.)
+// (One warp per sample read one 8-byte partial per 32-byte sector: 12.4 us at 390 chunks, now 7, 35 us
+// for 512 replicas of 100 samples.)
 constexpr int kFinishWarps = 16;   // at most; the launch uses as many as the longest chunk list needs
 
 template <class R>
@@ -1214,7 +1223,9 @@ __global__ void __launch_bounds__(128) k_eam_force(int n, int stride, int cap, d
 // chunks s, s + G, .. of four entries (the last chunk is filled with the slot itself, which the
 // predicate 0.01 < r^2 < rc^2 refuses); each term goes into a two-float accumulator, the lanes'
 // sums are combined in FP64 by a fixed butterfly.  Pass 1 also writes (x, y, z, F'(rho)) per slot, so
-// that pass 2 needs one gather per neighbour.  Pair physics as k_eam_fp and k_eam_force.
+// that pass 2 needs one gather per neighbour.  Bound by issue and the gathers: 256,000 atoms at 4 lanes
+// 80 + 165 -> 66 + 85 us (1 and 2 lanes: the step 1.5 and 1 % longer).  Pair physics as k_eam_fp and
+// k_eam_force.
 constexpr int kEamThreads = 1024;
 
 template <bool MI>

@@ -167,7 +167,9 @@ __device__ __forceinline__ void block_colsum(MlpSmem& S, float* v, float* out) {
   __syncthreads();
 }
 
-// One CTA = one group of 256 rows, 256 threads (thread t = row t).
+// One CTA = one group of 256 rows, 256 threads (thread t = row t).  Bound by the latency of one CTA's
+// chain of layers (16 groups fill 16 SMs): 16 groups 136 -> 55 us with 16-byte shared-memory rows, the
+// halving column sums and 4 x 4 register tiles of dW2.
 __global__ void __launch_bounds__(256, 1) k_mlp(MlpArgs args) {
   extern __shared__ unsigned char smem_raw[];
   MlpSmem& S = *reinterpret_cast<MlpSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);

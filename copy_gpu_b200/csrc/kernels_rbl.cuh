@@ -274,7 +274,8 @@ __global__ void __launch_bounds__(32 * kRblWarps) k_rbl_list_warp(
 // d^2 <= shell_hi (shell) are the reference's predicates as single comparisons (pair_d2_max,
 // pair_d2_min).  Stencil cells farther than rc from the box of the warp's atoms hold no pair and
 // are left out (rbl_gap2).  Lists identical entry for entry to k_rbl_list's, which also serves the
-// atoms whose own cell index differs from the cell they were binned into.
+// atoms whose own cell index differs from the cell they were binned into.  Bound by issue (66 % of
+// the slots): 101,440 chain atoms at rc 12 283 us against 355 with a warp per atom.
 constexpr int kRblBatch32 = 12;              // words of 32 candidates per batch
 constexpr int kRblBatchN = 32 * kRblBatch32;
 

