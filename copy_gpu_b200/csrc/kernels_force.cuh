@@ -95,6 +95,27 @@ __device__ __forceinline__ float erfc_shared(float x, float e) {
 }
 __device__ __forceinline__ double erfc_shared(double x, double) { return erfc(x); }
 
+// the same for two arguments side by side: e^(-a d2), and erfc with its Gaussian factors
+__device__ __forceinline__ Pair<float> exp_neg2(float a, Pair<float> d2) {
+  const Pair<float> m = mul2(mul2(both<float>(-a), d2), both<float>(1.44269504088896340736f));
+  Pair<float> r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(m.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(m.y));
+  return r;
+}
+__device__ __forceinline__ Pair<double> exp_neg2(double a, Pair<double> d2) { return {exp(-a * d2.x), exp(-a * d2.y)}; }
+__device__ __forceinline__ Pair<float> erfc_shared2(Pair<float> x, Pair<float> e) {
+  const Pair<float> one = both<float>(1.0f), u = fma2(both<float>(0.3275911f), x, one);
+  const Pair<float> w{rcp_r(u.x), rcp_r(u.y)};
+  const Pair<float> t = fma2(w, fma2(mul2(both<float>(-1.0f), u), w, one), w);
+  Pair<float> poly = fma2(both<float>(1.061405429f), t, both<float>(-1.453152027f));
+  poly = fma2(poly, t, both<float>(1.421413741f));
+  poly = fma2(poly, t, both<float>(-0.284496736f));
+  poly = fma2(poly, t, both<float>(0.254829592f));
+  return mul2(mul2(poly, t), e);
+}
+__device__ __forceinline__ Pair<double> erfc_shared2(Pair<double> x, Pair<double>) { return {erfc(x.x), erfc(x.y)}; }
+
 template <class R> __host__ __device__ __forceinline__ R lj24(const LJTable& t, int k);
 template <> __host__ __device__ __forceinline__ float lj24<float>(const LJTable& t, int k) { return t.lj24_f[k]; }
 template <> __host__ __device__ __forceinline__ double lj24<double>(const LJTable& t, int k) { return t.lj24_d[k]; }
@@ -434,14 +455,16 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_lean(
 // molecules, records) of the current one in flight together, the image offsets decoded in one
 // branch per chunk.  The filler entries of the last chunk hold the slot itself, at distance 0,
 // which no predicate accepts.  The pair terms are those of k_near_force (same predicates and
-// arithmetic); each lane sums the four forces of a chunk and folds them into a two-float
+// operations), two entries side by side in packed FP32x2 instructions, branch-free and selected
+// by the predicates; each lane sums the four forces of a chunk and folds them into a two-float
 // accumulator, and the group combines its G partial sums in FP64 with a fixed butterfly, so the
-// result does not depend on scheduling.  Bound by issue and the latency of the gathers: 30,000 water
-// atoms at 16 lanes 134 -> 113 us against one list entry per lane and step (65 % of the issue
-// slots); 22,824 chain atoms with special bonds 103 us, of which the search of the special lists,
-// needed only for pairs inside a molecule, took 16 us while it was unrolled with the entries.
+// result does not depend on scheduling.  Bound by issue and the latency of the gathers.  Five steps
+// of 30,000 water atoms at 16 lanes 1231 us with a branch per entry and predicate, 1120 packed;
+// 22,824 chain atoms with special bonds 777 -> 686 us (80 registers: 1120 and 709; the next chunk's
+// positions a step ahead: 1131 and 716).  The special lists, needed only for pairs inside a
+// molecule, are searched in one copy outside the unrolled entries, where they took 16 us a pass.
 template <class R, bool COUL, int MI, int G>
-__global__ void __launch_bounds__(256) k_near_force_group(
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 4 : 1) k_near_force_group(
     NearParams prm, const LJTable* __restrict__ ljt, const typename Traits<R>::V4* __restrict__ pos4,
     const int2* __restrict__ meta, const int* __restrict__ nbr, const int* __restrict__ count,
     const RepDev* __restrict__ reps, const int* __restrict__ rep_of_slot,
@@ -472,6 +495,8 @@ __global__ void __launch_bounds__(256) k_near_force_group(
   const R cs = (R)prm.coul_scale;
   const R qi = pi.w;
   const int trow = prm.ntypes > 1 ? mi.x * prm.ntypes : 0;
+  const int tmask = prm.ntypes > 1 ? ~0 : 0;
+  const R margin = prm.orig ? (R)0 : (R)1.0e-4;
   const int4* nbr4 = reinterpret_cast<const int4*>(nbr) + i;
   const int nch = active ? (min(count[i], prm.cap) + 3) >> 2 : 0;
   const int last = __reduce_max_sync(0xffffffffu, nch);
@@ -500,57 +525,83 @@ __global__ void __launch_bounds__(256) k_near_force_group(
         pj[k].z -= k2 == 1 ? w2 : (k2 == 2 ? -w2 : (R)0);
       }
     }
-    R gx = 0, gy = 0, gz = 0;
+    Pair<R> gx2 = both<R>(0), gy2 = both<R>(0), gz2 = both<R>(0);
     unsigned bonded = 0;   // entries of the atom's own bond-graph component (SPW)
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const R r0 = pj[k].x - pi.x, r1 = pj[k].y - pi.y, r2 = pj[k].z - pi.z;
-      const R d2 = r0 * r0 + r1 * r1 + r2 * r2;
-      if ((MI & 3) == kMiAll && !((prm.orig ? cut2 - d2 > (R)0 : cut2 - d2 > (R)1.0e-4) && d2 > (R)1.0e-4)) continue;
-      R f = 0;
+    for (int h = 0; h < 2; ++h) {
+      const V4 &pa = pj[2 * h], &pb = pj[2 * h + 1];
+      const Pair<R> rx{pa.x - pi.x, pb.x - pi.x}, ry{pa.y - pi.y, pb.y - pi.y}, rz{pa.z - pi.z, pb.z - pi.z};
+      const Pair<R> d2 = fma2(rz, rz, fma2(ry, ry, mul2(rx, rx)));
+      // the list predicate at rc (list reuse); every listed pair passes it otherwise
+      bool in[2] = {d2.x > (R)1.0e-4, d2.y > (R)1.0e-4};
+      if ((MI & 3) == kMiAll) {
+        in[0] = in[0] && cut2 - d2.x > margin;
+        in[1] = in[1] && cut2 - d2.y > margin;
+      }
+      Pair<R> t = both<R>(0);
       if (COUL) {
-        const R qq = qi * pj[k].w;
-        if (qq != (R)0) {
-          const R inv = rsqrt_r(d2);
-          const R dis = d2 * inv;
-          if (dis < rc && dis > (R)0.01) {
-            const R ex = exp_r(-aa * d2);
-            const R erfcv = erfc_shared(sa * dis, ex);
-            const R g = (erfcv * inv + c2 * ex) * inv;
-            f = -qq * g * inv * cs;
-            if (ENERGY) e_coul += qq * erfcv * inv * cs;
-          }
+        const Pair<R> qq{qi * pa.w, qi * pb.w};
+        if (qq.x != (R)0 || qq.y != (R)0) {   // the term of a pair with q_i q_j = 0 is 0
+          const Pair<R> inv{rsqrt_r(d2.x), rsqrt_r(d2.y)};
+          const Pair<R> dis = mul2(d2, inv);
+          const Pair<R> ex = exp_neg2(aa, d2);
+          const Pair<R> erfcv = erfc_shared2(mul2(both<R>(sa), dis), ex);
+          const Pair<R> qi2 = mul2(mul2(qq, inv), both<R>(cs));
+          const Pair<R> g = mul2(fma2(erfcv, inv, mul2(both<R>(c2), ex)), inv);
+          const Pair<R> f = mul2(qi2, g);
+          const bool cx = ((MI & 3) != kMiAll || in[0]) && dis.x < rc && dis.x > (R)0.01;
+          const bool cy = ((MI & 3) != kMiAll || in[1]) && dis.y < rc && dis.y > (R)0.01;
+          t.x = cx ? -f.x : (R)0;
+          t.y = cy ? -f.y : (R)0;
+          if (ENERGY) e_coul += (cx ? qi2.x * erfcv.x : (R)0) + (cy ? qi2.y * erfcv.y : (R)0);
         }
       }
-      R fl0 = 0, fl1 = 0, fl2 = 0;
-      bool same = false;
-      int tj = 0;
+      Pair<R> qx = rx, qy = ry, qz = rz, l2 = d2;
+      bool lj[2] = {in[0], in[1]};
+      if ((MI & 3) == kMiLJ) {   // MinDistanceVec
+        const R box[3] = {Traits<R>::box(rp, 0), Traits<R>::box(rp, 1), Traits<R>::box(rp, 2)};
+        min_image(qx.x, qy.x, qz.x, box);
+        min_image(qx.y, qy.y, qz.y, box);
+        l2 = fma2(qz, qz, fma2(qy, qy, mul2(qx, qx)));
+        lj[0] = l2.x > (R)1.0e-4;
+        lj[1] = l2.y > (R)1.0e-4;
+      }
+      if ((MI & 3) != kMiAll) {
+        lj[0] = lj[0] && l2.x < cut2;
+        lj[1] = lj[1] && l2.y < cut2;
+      }
+      int tj[2] = {0, 0};
       if (typed) {
-        same = MOLEC && (mj[k].y == mi.y);
-        tj = prm.ntypes > 1 ? mj[k].x : 0;
-        if (SPW && same) bonded |= 1u << k;
-      }
-      if (!same) {
-        R q0 = r0, q1 = r1, q2 = r2;
-        R dl2 = d2;
-        if ((MI & 3) == kMiLJ) {
-          const R box[3] = {Traits<R>::box(rp, 0), Traits<R>::box(rp, 1), Traits<R>::box(rp, 2)};
-          min_image(q0, q1, q2, box);
-          dl2 = q0 * q0 + q1 * q1 + q2 * q2;
-        }
-        if (dl2 < cut2 && dl2 > (R)0.0001) {
-          const R inv2 = rcp_r(dl2);
-          const R sd6 = lj_s6[trow + tj] * inv2 * inv2 * inv2;
-          const R a24 = lj_a[trow + tj];
-          const R scal = a24 * (((R)2 * sd6 - (R)1) * sd6) * inv2;
-          fl0 = scal * q0; fl1 = scal * q1; fl2 = scal * q2;
-          if (ENERGY) e_lj += -a24 / (R)6 * (sd6 - (R)1) * sd6;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          const bool same = MOLEC && mj[2 * h + k].y == mi.y;
+          tj[k] = mj[2 * h + k].x & tmask;
+          if (SPW && same && ((MI & 3) != kMiAll || in[k])) bonded |= 1u << (2 * h + k);
+          lj[k] = lj[k] && !same;
         }
       }
-      gx += f * r0 + fl0;
-      gy += f * r1 + fl1;
-      gz += f * r2 + fl2;
+      const Pair<R> i2{rcp_r(l2.x), rcp_r(l2.y)};
+      const Pair<R> sd6 = mul2(mul2(mul2(Pair<R>{lj_s6[trow + tj[0]], lj_s6[trow + tj[1]]}, i2), i2), i2);
+      const Pair<R> a24{lj_a[trow + tj[0]], lj_a[trow + tj[1]]};
+      Pair<R> sc = mul2(mul2(a24, mul2(fma2(both<R>(2), sd6, both<R>(-1)), sd6)), i2);
+      sc.x = lj[0] ? sc.x : (R)0;
+      sc.y = lj[1] ? sc.y : (R)0;
+      if (ENERGY) {
+        if (lj[0]) e_lj += -a24.x / (R)6 * (sd6.x - (R)1) * sd6.x;
+        if (lj[1]) e_lj += -a24.y / (R)6 * (sd6.y - (R)1) * sd6.y;
+      }
+      if ((MI & 3) == kMiLJ) {
+        gx2 = fma2(sc, qx, fma2(t, rx, gx2));
+        gy2 = fma2(sc, qy, fma2(t, ry, gy2));
+        gz2 = fma2(sc, qz, fma2(t, rz, gz2));
+      } else {
+        t = add2(t, sc);
+        gx2 = fma2(t, rx, gx2);
+        gy2 = fma2(t, ry, gy2);
+        gz2 = fma2(t, rz, gz2);
+      }
     }
+    R gx = gx2.x + gx2.y, gy = gy2.x + gy2.y, gz = gz2.x + gz2.y;
     if (SPW) {
       // LJ of pairs inside the component, a dozen per atom, with the special-bond weight of the
       // pair: one copy of the partner search, outside the unrolled entries
