@@ -172,13 +172,14 @@ PAIR_PROFILE = {
     # profiles/pair_kernels_all_workloads.md
     "electrolyte": {"kernel": "k_near_lean", "atoms": 1_000_000, "dram_bytes": 390.7e6, "warp_inst": 111.9e6},
     "batched": {"kernel": "k_near_lean", "atoms": 2_266_365, "dram_bytes": 813.0e6, "warp_inst": 339.2e6},
-    "eam": {"kernel": "k_eam_fp_smem + k_eam_force_smem", "atoms": 256_000, "dram_bytes": 126.3e6, "warp_inst": 77.44e6},
-    "water": {"kernel": "k_near_force_group (16 lanes)", "atoms": 30_000, "dram_bytes": 69.85e6,
-              "warp_inst": 75.92e6},
+    "eam": {"kernel": "k_eam_fp_smem + k_eam_force_smem", "atoms": 256_000, "dram_bytes": 126.3e6,
+            "warp_inst": 77.44e6},
+    "water": {"kernel": "k_near_force_group (16 lanes)", "atoms": 30_000, "dram_bytes": 69.8e6,
+              "warp_inst": 56.2e6},
     "lj": {"kernel": "k_near_lean (16 lanes, FP64)", "atoms": 4_000, "dram_bytes": 1.45e6, "warp_inst": 1.55e6},
     "molecular": {"kernel": "k_rbl_force (8 lanes)", "atoms": 101_440, "dram_bytes": 47.9e6, "warp_inst": 89.4e6},
-    "molecular_verlet": {"kernel": "k_near_force_group (16 lanes)", "atoms": 97_600, "dram_bytes": 175.68e6,
-                         "warp_inst": 233.34e6},
+    "molecular_verlet": {"kernel": "k_near_force_group (16 lanes)", "atoms": 22_824, "dram_bytes": 43.7e6,
+                         "warp_inst": 53.3e6},
 }
 
 
