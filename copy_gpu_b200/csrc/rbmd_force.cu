@@ -2892,6 +2892,13 @@ rbmd_status rbmd_force_step(rbmd_force* f, int32_t n_steps, void* stream) {
     CK(cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s));   // longest overflowed row of this call
     k_set_step<<<1, 1, 0, s>>>(f->d_step, f->step_count);
     CK(cudaGetLastError());
+    // the sampler of a step launched directly reads d_step on the k-space stream before that stream
+    // joins the step's fork, so the stream waits for the write here (a replay after a list overflow
+    // finds the index of the abandoned attempt there)
+    if (f->is_rbe()) {
+      CK(cudaEventRecord(f->ev_fork, s));
+      CK(cudaStreamWaitEvent(f->side, f->ev_fork, 0));
+    }
     f->in_step = true;
     rbmd_status gs = f->fp64 ? run_steps<double>(f, n_steps, s) : run_steps<float>(f, n_steps, s);
     f->in_step = false;

@@ -9,6 +9,8 @@
   charged atoms against the FP64 oracle, no worse than 1e-5 of the largest force (FP32 bar).
 * A step call that starts with the graph of an earlier call: many short calls, with force calls, an
   injected k-set and velocities read back between them, bit for bit as without graphs.
+* A step call replayed because its list overflowed draws the k-sets of the call's own steps: bit for bit
+  the trajectory of a run whose first capacity is large enough.
 """
 import numpy as np
 import pytest
@@ -137,3 +139,29 @@ def test_step_calls_from_the_graph(cuda, kind, skin):
     for a, b in zip(*[o[0] for o in out]):
         assert np.array_equal(a, b)
     assert out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("proposal", ["gauss", "gauss_iid"])
+@pytest.mark.parametrize("n_steps,skin", [(1, 0.0), (1, 0.3), (5, 0.3), (12, 0.0)])
+def test_step_replay_draws_its_own_k_sets(cuda, proposal, n_steps, skin):
+    import torch
+    out = []
+    for capacity in (0, 8):   # 0: by density; 8: every call's first attempt overflows on a fresh handle
+        s = systems.electrolyte(1500, seed=23)
+        cfg = systems.electrolyte_config(P=40, precision="fp32", seed=7)
+        cfg["hyper_parameters"]["neighbor"]["skin"] = skin
+        cfg["hyper_parameters"]["coulomb"]["proposal"] = proposal
+        if capacity:
+            cfg["hyper_parameters"]["neighbor"]["capacity"] = capacity
+        dev = to_dev(s, cuda)
+        ff = make_ff(cfg, s, dev)
+        ff.step(n_steps)
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        got = [dev[k].cpu().numpy() for k in ("pos", "vel", "force")] + [ff.get_ksamples(40)]
+        ff.step(2)
+        torch.cuda.synchronize()
+        out.append(got + [dev["pos"].cpu().numpy()])
+        ff.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
