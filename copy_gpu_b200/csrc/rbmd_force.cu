@@ -124,7 +124,7 @@ struct rbmd_force {
   int tpa_list = 0, tpa_near = 128;     // list build: 0 = one warp per cell, 1 = one warp per atom, else
                                         // threads per block of k_nlist; threads per block of the force pass
   double mean_listed = 0;               // listed neighbours per atom expected from the density
-  int rbl_list_warp = -1;               // RBL list build: -1 one warp per cell, 1 one warp per atom, 0 one thread per atom
+  int rbl_list_warp = -1;               // RBL list build: -1 by size (rbl_list_build), 1 one warp per atom, 0 one thread per atom
   int rbl_lanes = 0;                    // RBL force pass lanes per atom (0: by size)
   int num_sms = 148;                    // SMs of the bound device (cudaDevAttrMultiProcessorCount)
   int near_variant = 1;                 // 1: k_near_lean where it applies (lean_ok), 0: k_near_force
@@ -869,12 +869,36 @@ void launch_nlist(rbmd_force* f, cudaStream_t s) {
   f->launches++;
 }
 
+// RBL list build when the configuration leaves it open: 2 one warp per cell, 1 one warp per atom, 0 one
+// thread per atom.  The cell build takes the same time whatever fills its lanes: it loses with few atoms
+// per cell, and, while all its warps fit the chip at once, its time does not shrink with the system.
+// Measured on B200 (list, microseconds; LJ at density 0.8 unless noted; c = atoms per cell):
+//   * 2,000 atoms c 12.5: cell 82, warp 52; 6,000 atoms 91 / 95; 10,000 101 / 123; 46,000 234 / 465.
+//     FP64 10,000 atoms c 12.5: 152 / 139; 20,000 195 / 252.  Hence 64 atoms per SM, 100 in FP64.
+//   * up to 320 atoms per SM, against one warp per atom: c 1.6 40,000 atoms 123 / 107; c 2.7 46,000
+//     115 / 160.  Stencils of 7 cells per axis: c 0.8 40,000 atoms 424 / 207, c 7.3 46,000 417 / 809.
+//   * above, against one thread per atom: 60,000 atoms c 2.7 148 / 181 (FP64 208 / 212), copper (c 1.3)
+//     62,500 atoms 189 / 117; 150,000 atoms c 3 338 / 263, c 6.4 361 / 349, c 9 402 / 462, chains
+//     (c 21.6) 583 / 813; 600,000 atoms c 0.8 6300 / 1078; 7 cells per axis, c 7.3, 150,000 1209 / 775.
+int rbl_list_build(const rbmd_force* f) {
+  if (f->num_cycles > 3) return 0;   // stencil tables hold kRblStencilMax cells
+  if (f->rbl_list_warp >= 0) return f->rbl_list_warp;
+  const int per_sm = f->n / f->num_sms;
+  const bool few = per_sm < 10 * 32;
+  const double per_cell = (double)f->n / std::max(1, f->ncell_total);
+  bool cell = per_sm >= (f->fp64 ? 100 : 64);
+  if (few) cell = cell && per_cell >= (f->num_cycles < 3 ? 2.5 : 6.0);
+  else cell = f->num_cycles < 3 && per_cell >= (per_sm < 420 ? 2.5 : 8.0);
+  return cell ? 2 : (few ? 1 : 0);
+}
+
 template <class R>
 void launch_rbl_list(rbmd_force* f, cudaStream_t s) {
   PhaseScope ps(f, kPhList, s);
   const int* rp = f->nrep > 1 ? f->d_rep_of : nullptr;
   const int side = 2 * f->num_cycles + 1, ncs = side * side * side;
-  if (f->rbl_list_warp < 0 && ncs <= kRblStencilMax) {   // warp per cell
+  const int build = rbl_list_build(f);
+  if (build == 2) {   // warp per cell
     const long long items = (long long)f->ncell_total * f->list_parts;
     const size_t smem = (size_t)kRblWarps * rbl_cell_bytes<R>(ncs);
     k_rbl_list_cell<R, sizeof(R) == 4 ? 4 : 2>
@@ -883,7 +907,7 @@ void launch_rbl_list(rbmd_force* f, cudaStream_t s) {
             f->nrep > 1 ? f->d_cell_rep : nullptr, f->num_cycles, (R)f->rc, (R)f->rs,
             pair_d2_max<R>((R)f->rs, true, false), pair_d2_min<R>((R)f->rs), pair_d2_max<R>((R)f->rc, true, false),
             (R)1, f->core_cap, f->shell_cap, f->stride, f->d_nbr, f->d_count, f->d_count2, f->d_maxcount, f->d_status);
-  } else if (f->rbl_list_warp > 0 && ncs <= kRblStencilMax) {
+  } else if (build == 1) {
     k_rbl_list_warp<R><<<(f->n + kRblWarps - 1) / kRblWarps, 32 * kRblWarps, 0, s>>>(
         f->n, (const typename Traits<R>::V4*)f->d_pos4, f->d_cell_start, f->d_reps, rp, f->num_cycles, (R)f->rc,
         (R)f->rs, f->core_cap, f->shell_cap, f->stride, f->d_nbr, f->d_count, f->d_count2, f->d_maxcount,

@@ -1,0 +1,73 @@
+"""Kernels chosen by size against the ones that a configuration can force: the same answers on both
+sides of each line, and the choice no slower than what it replaced (event times of the phase, best of
+several windows, with a margin of 30 % for the spread of single launches)."""
+import numpy as np
+import pytest
+
+from copy_gpu_b200 import systems
+from tests.helpers import jitter, make_ff, to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _phase_us(s, cfg, phase, windows=5, calls=3):
+    """Shortest mean time of one phase of a force call, in microseconds."""
+    dev = {k: v for k, v in to_dev(s, "cuda", with_vel=False).items()}
+    ff = make_ff(cfg, s, dev)
+    ff.Execute()
+    ff.profile(True)
+    best, last = 1e30, ff.phase_ms()[phase]
+    for _ in range(windows):
+        for _ in range(calls):
+            ff.Execute()
+        now = ff.phase_ms()[phase]
+        best, last = min(best, (now[0] - last[0]) / (now[1] - last[1])), now
+    assert ff.status() == 0
+    ff.close()
+    return 1e3 * best
+
+
+def _rbl_config(prec, rc, rcore, mode):
+    cfg = systems.lj_config(cutoff=rc, precision=prec)
+    cfg["hyper_parameters"]["neighbor"].update(type="RBL", r_core=rcore, neighbor_sample_num=50)
+    cfg["tuning"] = {"rbl_list": mode}
+    return cfg
+
+
+# (atoms, density, cutoff, core radius): sparse cells (one thread per atom), few atoms (one warp per
+# atom), and two sizes at which one warp per cell is the fastest
+@pytest.mark.parametrize("n,rho,rc,rcore", [(150000, 0.1, 6.0, 2.0), (150000, 0.8, 2.5, 1.25), (2000, 0.8, 5.0, 2.5),
+                                            (40000, 0.8, 5.0, 2.5), (150000, 0.8, 5.0, 2.5)])
+def test_rbl_list_choice_is_not_slower(cuda, n, rho, rc, rcore):
+    s = systems.electrolyte(n, rho=rho, ion_frac=0.0)
+    us = {m: _phase_us(s, _rbl_config("fp32", rc, rcore, m), "neighbor_list") for m in ("auto", "warp", "thread")}
+    assert us["auto"] <= 1.3 * min(us["warp"], us["thread"]), us
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("case", ["below", "above", "dense", "wide", "outside"])
+def test_rbl_list_choice_same_lists(cuda, prec, case):
+    import torch
+    # below / above: the first size at which a warp takes a cell, and one atom less; dense: about 54 atoms
+    # a cell and many batches of candidates; wide: 7 stencil cells per axis; outside: atoms beyond the faces
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if case in ("below", "above"):
+        s = systems.electrolyte((100 if prec == "fp64" else 64) * sms - (case == "below"), ion_frac=0.0)
+        rc, rcore = 5.0, 2.5
+    else:
+        s = systems.lj_fcc(ncell=16, seed=4)
+        s["pos"] = jitter(s["pos"], s["lo"], s["hi"], 0.08, seed=5)
+        rc, rcore = {"dense": (8.0, 4.2), "wide": (5.9, 2.0), "outside": (5.0, 2.6)}[case]
+        if case == "outside":
+            s["pos"][:500] += np.random.default_rng(8).uniform(-1.2, 1.2, size=(500, 3))
+    out = []
+    for mode in ("auto", "thread"):
+        dev = to_dev(s, cuda)
+        ff = make_ff(_rbl_config(prec, rc, rcore, mode), s, dev)
+        ff.Execute()
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        out.append(ff.neighbors(1024) + ff.rbl_lists()[:2] + (dev["force"].cpu().numpy(),))
+        ff.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
