@@ -372,21 +372,45 @@ bool lean_ok(const rbmd_force* f) {
          (f->skin > 0 || !f->minimg);
 }
 
-// Lanes per atom of the near pass when neither the configuration nor the autotuner gave them
-// (B200, microseconds a pass).  Lean pass, electrolyte lists of 78 entries, FP32: 4,000 atoms 1 lane
-// 29 / 16 lanes 10.1; 8,000 8 lanes 14.2 / 16 lanes 15.5; 16,000 1 lane 28 / 8 lanes 15.6; 32,000
-// 4 lanes 21.6 / 8 lanes 22.5; 128,000 1 lane 49 / 4 lanes 44; 256,000 82 / 80, beyond which the
-// FP64 sums of the lanes cost more than they spread (FP64 crosses at 128,000: 109 / 110).  General
-// pass with long lists: water (556 listed) 30,000 atoms 1 lane 409 / 4 lanes 165 / 16 lanes 120 / 32
-// lanes 132, 4,800 359 / 78 / 32 / 37; chains (505 listed) 22,824 427 / 179 / 125 / 142.
+// Lanes per atom of the near pass when neither the configuration nor the autotuner gave them.  Lanes
+// spread a small system over the chip; once it is full they cost the FP64 sums of the lanes, idle lanes in
+// rows shorter than their chunks and, in the branch-free general pass in FP64, an erfc for every listed
+// pair beside a charged one.  Measured on B200 (near pass, microseconds, 1 / 4 / 8 / 16 lanes):
+//   * lean pass, 52 listed, FP32: 4,000 atoms 19 / 11 / 8.5 / 8.5, 20,000 19 / 11 / 13, 70,000 21 / 21,
+//     150,000 27 / 31; with charges 100,000 28 / 27, 200,000 42 / 41.  FP64: 40,000 27 / 24, 70,000 31 / 33;
+//     with charges 70,000 67 / 56, 150,000 106 / 103, 200,000 123 / 135.
+//     20 listed, FP32: 20,000 13 / 11, 40,000 13 / 13, 100,000 15 / 17; FP64 20,000 15 / 13, 40,000 15 / 17.
+//     6 listed, FP32: 20,000 8.5 / 8.5, 200,000 14 / 19; FP64 20,000 11 / 11, 200,000 19 / 33.
+//     419 listed, FP32: 100,000 136 / 110, 200,000 229 / 194; FP64 200,000 435 / 427.
+//   * general pass (two LJ types), 52 listed, FP32: 8,000 47 / 13 / 11 / 11, 30,000 52 / 17 / 19 / 21,
+//     1,000,000 291 / 240 / 316 / 441 (with charges 283 / 270).  FP64: 8,000 43 / 15 / 13 / 15, 80,000 56 / 52,
+//     300,000 136 / 160; with charges 4,000 58 / 21 / 15 / 19, 36,000 68 / 64, 60,000 70 / 100, 300,000
+//     223 / 448.
+//     20 listed, FP32: 60,000 25 / 18, 300,000 47 / 54 with charges; FP64 10,000 23 / 13, 60,000 25 / 27.
+//     6 listed, FP32: 10,000 13 / 8.5, 60,000 13 / 15 with charges, 1,000,000 64 / 99; FP64 10,000 13 / 11,
+//     with charges 14 / 17.
+//   * general pass, long lists: water (556 listed) 4,800 atoms 429 / 84 / 50 / 35, 30,000 476 / 136 / 116 /
+//     112, 300,000 1366 / 944 / 949 / 982, chains (505 listed) 228,240 1104 / 732 / 703 / 725 in FP32; water
+//     in FP64 30,000 861 / 603 / 549 / 539, 48,000 944 / 958 / 898 / 902, 60,000 1040 / 1115 / 1072 / 1114.
 int near_lanes(const rbmd_force* f) {
   if (f->lanes_set) return f->near_lanes;
   const int per_sm = f->n / f->num_sms;
-  const bool lean = lean_ok(f);
-  if (!lean && f->mean_listed >= 128.0) return 16;
-  if (per_sm < 40) return 16;
-  if (per_sm < 160) return 8;
-  return !lean || per_sm < (f->fp64 ? 700 : 1400) ? 4 : 1;
+  const bool lean = lean_ok(f), coul = f->with_coul_near();
+  const double listed = f->mean_listed;
+  if (!lean && listed >= 128.0) {
+    if (f->fp64) return per_sm < 330 ? 16 : 1;
+    return per_sm < 1000 ? 16 : 8;
+  }
+  // atoms per SM below which four lanes beat one thread: [lean][FP64][charges][rows of 128, 40, 12, fewer]
+  constexpr int any = 1 << 30;
+  static const int four[2][2][2][4] = {
+      {{{any, any, 500, 200}, {any, any, 500, 200}}, {{any, 700, 200, 100}, {any, 270, 100, 0}}},
+      {{{1400, 470, 270, 135}, {1400, 1000, 270, 135}}, {{1400, 400, 200, 100}, {1400, 1000, 200, 100}}}};
+  const int row = listed >= 128.0 ? 0 : (listed >= 40.0 ? 1 : (listed >= 12.0 ? 2 : 3));
+  if (per_sm >= four[lean][f->fp64][coul][row]) return 1;
+  const bool heavy = !lean && f->fp64 && coul;   // every lane pays for an FP64 erfc
+  if (per_sm < 40) return heavy ? 8 : 16;
+  return per_sm < 100 && row <= 1 && !heavy ? 8 : 4;
 }
 
 // The lean near pass and the per-atom list build run beside the k-space stream and use no shared

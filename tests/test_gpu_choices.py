@@ -71,3 +71,26 @@ def test_rbl_list_choice_same_lists(cuda, prec, case):
         ff.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def _two_types(n, rho, prec, charged):
+    """Atoms of two LJ types (the general near pass), one in ten charged."""
+    s = systems.electrolyte(n, rho=rho, ion_frac=0.1)
+    s["type"] = (np.arange(n) % 2).astype(np.int32)
+    s["eps"], s["sigma"] = np.array([1.0, 0.8]), np.array([1.0, 0.95])
+    if not charged:
+        s["charge"][:] = 0
+        return s, systems.lj_config(cutoff=2.5, precision=prec)
+    return s, systems.electrolyte_config(P=32, precision=prec)
+
+
+@pytest.mark.parametrize("n,rho,prec,charged", [(300000, 0.8, "fp64", True), (300000, 0.8, "fp64", False),
+                                                (1000000, 0.1, "fp32", False), (60000, 0.1, "fp64", True),
+                                                (30000, 0.8, "fp32", True), (4000, 0.8, "fp64", True)])
+def test_near_lanes_choice_is_not_slower(cuda, n, rho, prec, charged):
+    s, cfg = _two_types(n, rho, prec, charged)
+    us = {}
+    for lanes in (0, 1, 4, 8, 16):
+        cfg["tuning"] = {"force_lanes": lanes} if lanes else {}
+        us[lanes] = _phase_us(s, cfg, "force")
+    assert us[0] <= 1.3 * min(us[k] for k in (1, 4, 8, 16)), us
