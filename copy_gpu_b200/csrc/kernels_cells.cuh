@@ -172,12 +172,14 @@ __device__ __forceinline__ unsigned long long ord_key(double x) {
 // row of consecutive x cells is ordered by x, which lets the list build skip the candidates
 // beyond the cutoff in x by binary search.  Cells above kMaxCellAtoms keep the scatter order
 // (flagged by the scan).
-// nparts > 1 (cells of many atoms): a cell is shared by nparts warps, each ranking its share of the
+// SPLIT (cells of many atoms): a cell is shared by nparts warps, each ranking its share of the
 // atoms against all of them (30,000 water atoms fill 216 cells, 54 blocks of one warp per cell:
-// 37 -> 16 us with parts).
+// 37 -> 16 us with parts).  Without it no index is divided: the warps of empty cells, most of a dilute
+// or droplet system, do little else (300,000 atoms at 0.05 atoms a cell, whole sort: 1887 us with 64-bit
+// divisions, 1239 without any).
 constexpr int kSortWarps = 4;   // warps per block of k_cell_sort_gather
 
-template <class R>
+template <class R, bool SPLIT>
 __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
     int ncell, int nparts, const int* __restrict__ start, const int* __restrict__ tmp_slot_atom,
     const double* __restrict__ pos, const double* __restrict__ charge,
@@ -189,12 +191,20 @@ __global__ void __launch_bounds__(32 * kSortWarps) k_cell_sort_gather(
   __shared__ int ids[kSortWarps][kMaxCellAtoms];
   __shared__ Key keys[kSortWarps][kMaxCellAtoms];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long item = (long long)blockIdx.x * kSortWarps + w;
-  const int cell = (int)(item / nparts), part = (int)(item % nparts);
+  const unsigned item = blockIdx.x * kSortWarps + w;   // below 2^32: ncell + atoms / 32 warps
+  int cell = (int)item, part = 0;
+  if (SPLIT) {
+    cell = (int)(item / (unsigned)nparts);
+    part = (int)(item % (unsigned)nparts);
+  }
   if (cell >= ncell) return;
   if (rebuild && !rebuild[cell_rep ? cell_rep[cell] : 0]) return;
   const int s0 = start[cell], n = start[cell + 1] - s0;
-  const int k0 = (int)((long long)n * part / nparts), k1 = (int)((long long)n * (part + 1) / nparts);
+  int k0 = 0, k1 = n;
+  if (SPLIT) {
+    k0 = (int)((long long)n * part / nparts);
+    k1 = (int)((long long)n * (part + 1) / nparts);
+  }
   if (k0 == k1) return;
   const bool sortable = n <= kMaxCellAtoms;
   if (sortable)

@@ -988,7 +988,8 @@ void launch_sort(rbmd_force* f, cudaStream_t s, bool bin, bool regather) {
   // one warp per 32 atoms of a cell on average
   const int parts = std::max(1, (int)((f->n + 32LL * f->ncell_total - 1) / (32LL * f->ncell_total)));
   const long long sort_items = (long long)f->ncell_total * parts;
-  k_cell_sort_gather<R><<<(unsigned)((sort_items + kSortWarps - 1) / kSortWarps), 32 * kSortWarps, 0, s>>>(
+  auto kern = parts > 1 ? k_cell_sort_gather<R, true> : k_cell_sort_gather<R, false>;
+  kern<<<(unsigned)((sort_items + kSortWarps - 1) / kSortWarps), 32 * kSortWarps, 0, s>>>(
       f->ncell_total, parts, f->d_cell_start, f->d_tmp, f->at.pos, f->at.charge, f->at.type,
       molecular_mode(f) == 2 ? f->d_comp : f->at.molecule,
       rep_of, f->d_reps, f->d_slot_atom, f->d_atom_slot, (typename Traits<R>::V4*)f->d_pos4, nullptr,
