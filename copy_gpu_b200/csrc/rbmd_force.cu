@@ -1348,6 +1348,12 @@ __global__ void k_snapshot(long long m, const double* __restrict__ pos, const do
   }
 }
 
+// charged atom of each atom (the others keep what was there): the inverse of qidx
+__global__ void k_charge_index(int nq, const int* __restrict__ qidx, int* __restrict__ cidx) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < nq) cidx[qidx[c]] = c;
+}
+
 // The samplers' step index (by value: the host counter moves on while the call's work is queued).
 __global__ void k_set_step(long long* step, long long value) { *step = value; }
 
@@ -2538,10 +2544,14 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     CK(dalloc(&f->d_qidx, (size_t)std::max(1, f->nq)));
     if (f->nq > 0)
       CK(cudaMemcpy(f->d_qidx, qidx.data(), sizeof(int) * f->nq, cudaMemcpyHostToDevice));
-    std::vector<int> cidx(n, -1);
-    for (int c = 0; c < f->nq; ++c) cidx[qidx[c]] = c;
     CK(dalloc(&f->d_cidx, n));
-    CK(cudaMemcpy(f->d_cidx, cidx.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    CK(cudaMemset(f->d_cidx, 0xff, sizeof(int) * n));   // -1
+    if (f->nq > 0) {
+      // on the device: filled on the host and copied it took 0.6 of 6.5 ms of a bind of 200,000 atoms
+      k_charge_index<<<(f->nq + 255) / 256, 256>>>(f->nq, f->d_qidx, f->d_cidx);
+      CK(cudaGetLastError());
+      CK(cudaStreamSynchronize(nullptr));
+    }
     const int recb = fp64 ? sizeof(KRec64) : sizeof(KRec32);
     if (f->coul_type == "EWALD") {
       // EWALD: the cube m in [-kmax, kmax]^3 \ {0} (ExecPointLocator::ExecuteOnKNeighbor,
