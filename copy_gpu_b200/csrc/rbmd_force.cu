@@ -1145,7 +1145,8 @@ void launch_near_t(rbmd_force* f, cudaStream_t s) {
   if constexpr ((MI & 3) != kMiLJ && (MI & kMiSpecial) == 0) {
     // one LJ coefficient pair for all types, no molecules: the lean pass
     if (lean_ok(f)) {
-      if (g >= 16) launch_near_lean<R, COUL, MI, 16>(f, s, p);
+      if (g >= 32) launch_near_lean<R, COUL, MI, 32>(f, s, p);
+      else if (g == 16) launch_near_lean<R, COUL, MI, 16>(f, s, p);
       else if (g == 8) launch_near_lean<R, COUL, MI, 8>(f, s, p);
       else if (g == 4) launch_near_lean<R, COUL, MI, 4>(f, s, p);
       else launch_near_lean<R, COUL, MI, 1>(f, s, p);

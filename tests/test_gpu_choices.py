@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 from copy_gpu_b200 import systems
-from tests.helpers import jitter, make_ff, to_dev
+from tests.helpers import jitter, make_ff, rel_err, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +94,35 @@ def test_near_lanes_choice_is_not_slower(cuda, n, rho, prec, charged):
         cfg["tuning"] = {"force_lanes": lanes} if lanes else {}
         us[lanes] = _phase_us(s, cfg, "force")
     assert us[0] <= 1.3 * min(us[k] for k in (1, 4, 8, 16)), us
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("charged", [False, True])
+def test_every_forced_lane_count_runs(cuda, prec, charged):
+    """Lanes 1 .. 32 of the pass for one LJ coefficient pair: the parity bars against one thread per atom,
+    and in FP64 sums in another order for every count (rows of about 210 entries, 54 chunks; the butterfly
+    adds rows of up to 32 chunks alike with 16 and 32 lanes), so that no count runs as another one (FP32
+    adds the chunks in two-float sums, exact enough to agree)."""
+    import torch
+    s = systems.electrolyte(3000, ion_frac=0.2, seed=9)
+    if not charged:
+        s["charge"][:] = 0
+    out = {}
+    for lanes in (1, 4, 8, 16, 32):
+        cfg = (systems.electrolyte_config(P=16, cutoff=4.0, precision=prec) if charged
+               else systems.lj_config(cutoff=4.0, precision=prec))
+        cfg["tuning"] = {"force_lanes": lanes}
+        dev = to_dev(s, cuda)
+        ff = make_ff(cfg, s, dev)
+        if charged:
+            ff.set_ksamples(np.array([[1, 0, 0], [0, 1, 0], [0, 0, 1], [1, 1, 0]] * 4, np.int32))
+        ff.Execute()
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        out[lanes] = dev["force"].cpu().numpy()
+        ff.close()
+    bar = 1e-5 if prec == "fp32" else 1e-11
+    for a in out:
+        assert rel_err(out[a], out[1]) <= bar
+        for b in out:
+            assert prec == "fp32" or a == b or not np.array_equal(out[a], out[b]), (a, b)
