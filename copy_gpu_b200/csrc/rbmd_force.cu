@@ -365,11 +365,25 @@ int molecular_mode(const rbmd_force* f) {
   return f->at.molecule != nullptr ? 1 : 0;
 }
 
-// k_near_lean applies: one LJ coefficient pair for all types, no molecules, no per-pair minimum
-// image (a Verlet skin, or boxes of >= 3 cells per axis).
+// k_near_lean forms the LJ term as (ka u - kb) d^-8 with u = d^-6, ka = 2 c s6^2, kb = c s6 (c = -24 eps):
+// ka, kb and the smallest d^-8 have to be normal numbers of the run precision, or 0 for atoms without LJ.
+// In FP32 that ends at sigma of about 1180 for eps = 1 and at a cutoff of about 55,000; beyond,
+// k_near_force's (2 s6 u - 1) s6 u keeps the range.
+template <class R>
+bool lean_range(const rbmd_force* f) {
+  const volatile R c = lj24<R>(f->ljt_h, 0), s6 = sig6<R>(f->ljt_h, 0);
+  const volatile R kb = c * s6, c2 = (R)2 * c, c2s = c2 * s6, ka = c2s * s6;   // in the kernel's order
+  const volatile R rc2 = (R)f->rc * (R)f->rc, i2 = (R)1 / rc2, i4 = i2 * i2, i8 = i4 * i4;
+  if (!std::isfinite(c2) || !std::isnormal(i8)) return false;
+  if (c == (R)0 || s6 == (R)0) return true;
+  return std::isnormal(ka) && std::isnormal(kb) && std::isfinite(c2s);
+}
+
+// k_near_lean applies: one LJ coefficient pair for all types within its range, no molecules, no
+// per-pair minimum image (a Verlet skin, or boxes of >= 3 cells per axis).
 bool lean_ok(const rbmd_force* f) {
   return f->near_variant >= 1 && !f->is_rbl() && !f->is_eam() && f->nt_eff == 1 && molecular_mode(f) == 0 &&
-         (f->skin > 0 || !f->minimg);
+         (f->skin > 0 || !f->minimg) && (f->fp64 ? lean_range<double>(f) : lean_range<float>(f));
 }
 
 // Lanes per atom of the near pass when neither the configuration nor the autotuner gave them.  Lanes

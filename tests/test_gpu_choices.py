@@ -126,3 +126,31 @@ def test_every_forced_lane_count_runs(cuda, prec, charged):
         assert rel_err(out[a], out[1]) <= bar
         for b in out:
             assert prec == "fp32" or a == b or not np.array_equal(out[a], out[b]), (a, b)
+
+
+@pytest.mark.parametrize("skin", [0.0, 0.3])
+@pytest.mark.parametrize("scale,sigma", [(2000.0, 2000.0), (1100.0, 1100.0), (2e5, 100.0), (1.0, 0.0)])
+def test_lj_range_in_float(cuda, scale, sigma, skin):
+    """LJ in units whose 48 eps sigma^12 (or d^-8) leaves the range of floats, and just inside it: the FP32
+    pass against the FP64 pass at the same float positions, parity bar of FP32."""
+    import torch
+    s = systems.lj_fcc(ncell=7, seed=3)
+    s["pos"] = (jitter(s["pos"], s["lo"], s["hi"], 0.05, seed=4) * scale).astype(np.float32).astype(np.float64)
+    s["hi"] = s["hi"] * scale
+    s["sigma"] = np.array([sigma])
+    s["pos"] = np.minimum(s["pos"], np.nextafter(s["hi"].astype(np.float32), np.float32(0)).astype(np.float64))
+    out = []
+    for prec in ("fp32", "fp64"):
+        cfg = systems.lj_config(cutoff=2.5 * scale, precision=prec)
+        cfg["hyper_parameters"]["neighbor"]["skin"] = skin * scale
+        dev = to_dev(s, cuda)
+        ff = make_ff(cfg, s, dev)
+        ff.Execute()
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        out.append(dev["force"].cpu().numpy())
+        ff.close()
+    if sigma == 0.0:
+        assert not out[0].any() and not out[1].any()
+    else:
+        assert rel_err(out[0], out[1]) <= 1e-5
