@@ -7,6 +7,8 @@
   entry, from a few atoms to cells of more than 32 atoms and several batches of candidates.
 * Lanes per charged atom of the RBE force and short structure-factor chunks: one to a few thousand
   charged atoms against the FP64 oracle, no worse than 1e-5 of the largest force (FP32 bar).
+* Lanes per atom with types, molecules, special bonds and boxes of two cells per axis (per-pair minimum
+  image) against one thread per atom, forces and energies: the parity bars of each precision.
 * A step call that starts with the graph of an earlier call: many short calls, with force calls, an
   injected k-set and velocities read back between them, bit for bit as without graphs.
 * A step call replayed because its list overflowed draws the k-sets of the call's own steps: bit for bit
@@ -165,3 +167,49 @@ def test_step_replay_draws_its_own_k_sets(cuda, proposal, n_steps, skin):
         ff.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("case,skin", [("water", 0.0), ("water", 0.5), ("water_small", 0.0), ("chains", 0.0),
+                                       ("chains", 0.5), ("chains_small", 0.0), ("chains_nospecial", 0.0),
+                                       ("chains_nospecial", 0.5), ("types", 0.0), ("types", 0.3),
+                                       ("types_small", 0.0), ("one_type", 0.0), ("one_type", 0.3)])
+def test_lanes_match_one_thread(cuda, prec, case, skin):
+    import torch
+    if case.startswith("water"):
+        s = systems.water(n_mol=300 if case == "water" else 90, seed=6)
+        cfg = systems.water_config(P=16, precision=prec, cutoff=6.0)   # edges 20.8 and 13.9: 3 and 2 cells
+    elif case.startswith("chains"):
+        s = systems.molecular(n_chain=27 if case != "chains_small" else 8, chain_len=12, n_ion_pairs=4, step=1.5,
+                              cell=8.0, seed=5)
+        cfg = systems.molecular_config(P=16, cutoff=9.0, precision=prec,
+                                       special=None if case == "chains_nospecial" else (0.0, 0.2, 0.5))
+    else:   # two LJ coefficient pairs; one_type: the general pass forced by near_variant 0
+        s = systems.electrolyte(200 if case == "types_small" else 1500, ion_frac=0.4, seed=8)   # 2 and 4 cells
+        cfg = systems.electrolyte_config(P=16, precision=prec)
+        if case != "one_type":
+            s["eps"], s["sigma"] = np.array([1.0, 0.7, 0.7]), np.array([1.0, 0.9, 0.9])
+    cfg["hyper_parameters"]["neighbor"]["skin"] = skin
+    out = []
+    for lanes in (1, 4, 8, 16, 32):
+        cfg["tuning"] = {"force_lanes": lanes, "force_block": 128, "near_variant": 0 if case == "one_type" else 1}
+        dev = to_dev(s, cuda)
+        ff = make_ff(cfg, s, dev)
+        if "bonds" in s:
+            keys = ("molecule", "bonds", "bond_type", "bond_coeffs", "angles", "angle_type", "angle_coeffs",
+                    "dihedrals", "dihedral_type", "dihedral_coeffs")
+            ff.set_topology(*[s[k] for k in keys[:7 if case == "chains_nospecial" else 10]])
+        ff.Execute()
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        e = ff.energy()
+        out.append((dev["force"].cpu().numpy(), e["lj"], e["coul_real"]))
+        ff.close()
+    # energies: the parity bar of FP64; in FP32 each lane adds up to 4 x 140 terms in a float, so that a row's
+    # sum carries at most 560 x 2^-25 = 1.7e-5 of the terms it adds, of either sign from row to row
+    bar, ebar = (1e-5, 1.7e-5) if prec == "fp32" else (1e-11, 1e-10)
+    for f, lj, coul in out[1:]:
+        assert rel_err(f, out[0][0]) <= bar
+        scale = max(1.0, abs(out[0][1]), abs(out[0][2]))
+        assert abs(lj - out[0][1]) <= ebar * scale
+        assert abs(coul - out[0][2]) <= ebar * scale
