@@ -1,8 +1,9 @@
 """Kernel variants chosen by size, at the edges of their rules.
 
-* EAM in FP32 with the spline rows in shared memory (tables up to the shared-memory limit, one row
-  longer falls back to the global tables) against the FP64 passes on the same file: 1e-5 of the force
-  rms, the FP32 parity bar; boxes of 2 cells per axis (per-pair minimum image) and of 3.
+* EAM in FP32 with the spline rows in shared memory (the longest table that fits; one row more falls
+  back to the global tables) against the FP64 passes on the same file and the same float positions, to
+  what the float image positions allow (see the test); boxes of 2 cells per axis (per-pair minimum
+  image) and of 3.
 * RBL lists built by one warp per cell (the default) equal those of one thread per atom entry for
   entry, from a few atoms to cells of more than 32 atoms and several batches of candidates.
 * Lanes per charged atom of the RBE force and short structure-factor chunks: one to a few thousand
@@ -36,16 +37,24 @@ def _eam_force(s, path, prec, cuda):
     return dev["force"].cpu().numpy(), e["eam_embed"] + e["eam_pair"]
 
 
-@pytest.mark.parametrize("ncell,npts", [(4, 5000), (5, 5000), (5, 64), (9, 5000), (6, 7262), (6, 9000)])
+@pytest.mark.parametrize("ncell,npts", [(4, 5000), (5, 5000), (5, 64), (9, 5000), (6, "longest"), (6, "one more"),
+                                        (6, 9000)])
 def test_eam_rows_in_shared_memory(cuda, tmp_path, ncell, npts):
+    import torch
+    if isinstance(npts, str):   # two tables of npts + 1 rows of 16 bytes in a block's shared memory
+        limit = torch.cuda.get_device_properties(0).shared_memory_per_block_optin
+        npts = limit // 32 - 1 + (npts == "one more")
     p = dict(systems.JOHNSON_CU, npts=npts)
     path = systems.write_johnson_setfl(str(tmp_path / "j.setfl"), p)
     s = systems.eam_fcc(ncell=ncell, seed=3)
+    s["pos"] = s["pos"].astype(np.float32).astype(np.float64)
+    s["pos"][s["pos"] >= s["hi"]] = 0.0
     f32, e32 = _eam_force(s, path, "fp32", cuda)
     f64, e64 = _eam_force(s, path, "fp64", cuda)
-    # the FP32 pass differentiates the value rows, the FP64 pass reads the rounded derivative rows:
-    # with npts rows over 5 A the float row values carry 6e-8 npts / 12 of a row's slope
-    bar = 1e-5 + 6e-8 * npts / 12
+    # a neighbour's image lies within 2 L, where floats round to 2^-24 x 2 L; displacements of 0.131 A per axis
+    # make the force, so that a shift of all neighbours by that much is 2^-23 L / 0.131 of its rms (8e-6 at 18 A
+    # and 5e-6 at 33 A measured, the same with tables in global memory)
+    bar = max(1e-5, 2.0 ** -23 * s["hi"][0] / 0.131)
     assert rel_err(f32, f64) <= bar, rel_err(f32, f64)
     assert abs(e32 - e64) <= 1e-6 * abs(e64)
 
