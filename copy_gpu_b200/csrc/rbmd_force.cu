@@ -257,6 +257,10 @@ struct rbmd_force {
   cudaEvent_t ev_tail = nullptr;   // end of the k-space stream's work of a step (after the join)
   long long step_count = 0;
   long long* d_step = nullptr;   // step index of the k-samplers on the device (graph replay)
+  double* d_snap_thermo = nullptr;   // with d_snap: lambda and xi, noise counter, conditioning spectrum and its flag
+  long long* d_snap_lstep = nullptr;
+  float* d_snap_spec = nullptr;
+  int* d_snap_spec_init = nullptr;
   long long* d_lstep = nullptr;  // Langevin noise counter (advanced after every application)
   double langevin_gamma = 100.0; // execution.langevin_gamma (the reference hard-codes 100)
   bool langevin_shared = false;  // compat.langevin_reference: m = 1, kBT = 1, one xi for all
@@ -483,6 +487,7 @@ void free_all(rbmd_force* f) {
   free_topology(f);
   dfree(f->d_host32);
   dfree(f->d_snap); dfree(f->d_snap_img); dfree(f->d_step); dfree(f->d_lstep);
+  dfree(f->d_snap_thermo); dfree(f->d_snap_lstep); dfree(f->d_snap_spec); dfree(f->d_snap_spec_init);
   if (f->graph_exec) cudaGraphExecDestroy(f->graph_exec);
   f->graph_exec = nullptr;
   if (f->graph_multi) cudaGraphExecDestroy(f->graph_multi);
@@ -1348,12 +1353,37 @@ __global__ void k_f64_to_f32(long long m, const double* __restrict__ a, float* _
     b[k] = (float)a[k];
 }
 
+// What steps carry on besides the atoms: thermostat, Langevin noise counter, conditioning spectrum of the
+// proposal (nullable).
+struct CarriedState {
+  double *lambda, *xi;
+  long long* lstep;
+  float* spec;
+  int* spec_init;
+};
+__device__ __forceinline__ void copy_carried(const CarriedState& from, const CarriedState& to, int nrep, long long k,
+                                             long long stride) {
+  for (long long r = k; r < nrep; r += stride) {
+    to.lambda[r] = from.lambda[r];
+    to.xi[r] = from.xi[r];
+    if (from.spec) to.spec_init[r] = from.spec_init[r];
+  }
+  if (from.spec)
+    for (long long j = k; j < (long long)nrep * kPropBands; j += stride) to.spec[j] = from.spec[j];
+  if (k == 0) *to.lstep = *from.lstep;
+}
+__global__ void k_restore_carried(CarriedState from, CarriedState to, int nrep) {
+  copy_carried(from, to, nrep, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+}
+
 // State at the start of a step call, for its replay when a list overflows: one launch for the four
-// arrays.
+// arrays and the carried state.
 __global__ void k_snapshot(long long m, const double* __restrict__ pos, const double* __restrict__ vel,
                            const double* __restrict__ force, const int* __restrict__ image,
-                           double* __restrict__ snap, int* __restrict__ snap_img) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < m; k += (long long)gridDim.x * blockDim.x) {
+                           double* __restrict__ snap, int* __restrict__ snap_img, CarriedState from, CarriedState to,
+                           int nrep) {
+  const long long k0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  for (long long k = k0; k < m; k += stride) {
     const double x = pos[k], v = vel[k], f = force[k];
     const int g = image ? image[k] : 0;
     snap[k] = x;
@@ -1361,6 +1391,7 @@ __global__ void k_snapshot(long long m, const double* __restrict__ pos, const do
     snap[2 * m + k] = f;
     if (image) snap_img[k] = g;
   }
+  copy_carried(from, to, nrep, k0, stride);
 }
 
 // charged atom of each atom (the others keep what was there): the inverse of qidx
@@ -2954,13 +2985,24 @@ rbmd_status rbmd_force_step(rbmd_force* f, int32_t n_steps, void* stream) {
   if (!f->at.vel || !f->at.mass) return RBMD_ERR_STATE;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t n = f->n;
-  if (!f->d_snap) CK(dalloc(&f->d_snap, 9 * n));
+  if (!f->d_snap) {
+    CK(dalloc(&f->d_snap, 9 * n));
+    CK(dalloc(&f->d_snap_thermo, 2 * (size_t)f->nrep));
+    CK(dalloc(&f->d_snap_lstep, 1));
+    if (f->d_spec) {
+      CK(dalloc(&f->d_snap_spec, (size_t)f->nrep * kPropBands));
+      CK(dalloc(&f->d_snap_spec_init, (size_t)f->nrep));
+    }
+  }
   if (f->at.image && !f->d_snap_img) CK(dalloc(&f->d_snap_img, 3 * n));
+  const CarriedState now{f->d_lambda, f->d_xi, f->d_lstep, f->d_spec, f->d_spec_init};
+  const CarriedState kept{f->d_snap_thermo, f->d_snap_thermo + f->nrep, f->d_snap_lstep, f->d_snap_spec,
+                          f->d_snap_spec_init};
   const long long step0 = f->step_count;
   const bool pend0 = f->pending_scale;
   for (int attempt = 0; attempt < 4; ++attempt) {
     k_snapshot<<<(unsigned)std::min<size_t>((3 * n + 255) / 256, 32ull * f->num_sms), 256, 0, s>>>(
-        3 * (long long)n, f->at.pos, f->at.vel, f->at.force, f->at.image, f->d_snap, f->d_snap_img);
+        3 * (long long)n, f->at.pos, f->at.vel, f->at.force, f->at.image, f->d_snap, f->d_snap_img, now, kept, f->nrep);
     CK(cudaGetLastError());
     f->launches = 0;
     CK(cudaMemsetAsync(f->d_maxcount, 0, 2 * sizeof(int), s));   // longest overflowed row of this call
@@ -2991,6 +3033,8 @@ rbmd_status rbmd_force_step(rbmd_force* f, int32_t n_steps, void* stream) {
     CK(cudaMemcpyAsync(f->at.force, f->d_snap + 6 * n, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s));
     if (f->at.image)
       CK(cudaMemcpyAsync(f->at.image, f->d_snap_img, sizeof(int) * 3 * n, cudaMemcpyDeviceToDevice, s));
+    k_restore_carried<<<(f->nrep + 255) / 256, 256, 0, s>>>(kept, now, f->nrep);
+    CK(cudaGetLastError());
     f->step_count = step0;
     f->pending_scale = pend0;
   }

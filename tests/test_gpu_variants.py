@@ -12,8 +12,9 @@
   image) against one thread per atom, forces and energies: the parity bars of each precision.
 * A step call that starts with the graph of an earlier call: many short calls, with force calls, an
   injected k-set and velocities read back between them, bit for bit as without graphs.
-* A step call replayed because its list overflowed draws the k-sets of the call's own steps: bit for bit
-  the trajectory of a run whose first capacity is large enough.
+* A step call replayed because its list overflowed draws the k-sets of the call's own steps and starts from
+  its thermostat, noise counter and conditioning spectrum: bit for bit the trajectory of a run whose
+  first capacity is large enough.
 """
 import numpy as np
 import pytest
@@ -152,20 +153,26 @@ def test_step_calls_from_the_graph(cuda, kind, skin):
     assert out[0][1] == out[1][1]
 
 
-@pytest.mark.parametrize("proposal", ["gauss", "gauss_iid"])
+@pytest.mark.parametrize("kind", ["gauss", "gauss_iid", "learned", "nose_hoover", "langevin"])
 @pytest.mark.parametrize("n_steps,skin", [(1, 0.0), (1, 0.3), (5, 0.3), (12, 0.0)])
-def test_step_replay_draws_its_own_k_sets(cuda, proposal, n_steps, skin):
+def test_step_replay_draws_its_own_k_sets(cuda, kind, n_steps, skin):
     import torch
+    from oracle import mlp
     out = []
     for capacity in (0, 8):   # 0: by density; 8: every call's first attempt overflows on a fresh handle
         s = systems.electrolyte(1500, seed=23)
         cfg = systems.electrolyte_config(P=40, precision="fp32", seed=7)
         cfg["hyper_parameters"]["neighbor"]["skin"] = skin
-        cfg["hyper_parameters"]["coulomb"]["proposal"] = proposal
+        if kind in ("gauss", "gauss_iid", "learned"):
+            cfg["hyper_parameters"]["coulomb"]["proposal"] = kind
+        else:   # a thermostat with a state of its own
+            cfg["execution"].update({"ensemble": "NVT", "temp_ctrl_type": kind.upper(), "temperature": [1.0, 1.0, 0.1]})
         if capacity:
             cfg["hyper_parameters"]["neighbor"]["capacity"] = capacity
         dev = to_dev(s, cuda)
         ff = make_ff(cfg, s, dev)
+        if kind == "learned":
+            ff.proposal_params(mlp.init_params(2, scale=0.5))
         ff.step(n_steps)
         torch.cuda.synchronize()
         assert ff.status() == 0
