@@ -2848,6 +2848,7 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
   f->bound = true;
   f->list_valid = false;
   f->rebuild_clear = false;
+  f->presampled = false;
   f->step_count = 0;
   f->pending_scale = false;
   return RBMD_OK;

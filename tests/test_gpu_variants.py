@@ -229,3 +229,28 @@ def test_lanes_match_one_thread(cuda, prec, case, skin):
         scale = max(1.0, abs(out[0][1]), abs(out[0][2]))
         assert abs(lj - out[0][1]) <= ebar * scale
         assert abs(coul - out[0][2]) <= ebar * scale
+
+
+@pytest.mark.parametrize("proposal", ["gauss", "gauss_iid"])
+def test_steps_after_a_second_bind(cuda, proposal):
+    """A handle bound to new arrays after steps draws their k-sets anew: bit for bit a fresh handle."""
+    import torch
+    cfg = systems.electrolyte_config(P=40, precision="fp32", seed=7)
+    cfg["hyper_parameters"]["coulomb"]["proposal"] = proposal
+    s = systems.electrolyte(1500, seed=23)
+    out = []
+    for first in (False, True):
+        dev = to_dev(s, cuda)
+        ff = make_ff(cfg, s, dev)
+        if first:
+            ff.step(3)
+            dev = to_dev(s, cuda)
+            ff.Init(dev["pos"], dev["force"], vel=dev["vel"], mass=dev["mass"], charge=dev["charge"],
+                    type=dev["type"], image=dev["image"])
+        ff.step(3)
+        torch.cuda.synchronize()
+        assert ff.status() == 0
+        out.append([dev[k].cpu().numpy() for k in ("pos", "vel", "force")])
+        ff.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
