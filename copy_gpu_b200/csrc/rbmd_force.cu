@@ -257,10 +257,6 @@ struct rbmd_force {
   cudaEvent_t ev_tail = nullptr;   // end of the k-space stream's work of a step (after the join)
   long long step_count = 0;
   long long* d_step = nullptr;   // step index of the k-samplers on the device (graph replay)
-  double* d_snap_thermo = nullptr;   // with d_snap: lambda and xi, noise counter, conditioning spectrum and its flag
-  long long* d_snap_lstep = nullptr;
-  float* d_snap_spec = nullptr;
-  int* d_snap_spec_init = nullptr;
   long long* d_lstep = nullptr;  // Langevin noise counter (advanced after every application)
   double langevin_gamma = 100.0; // execution.langevin_gamma (the reference hard-codes 100)
   bool langevin_shared = false;  // compat.langevin_reference: m = 1, kBT = 1, one xi for all
@@ -487,7 +483,6 @@ void free_all(rbmd_force* f) {
   free_topology(f);
   dfree(f->d_host32);
   dfree(f->d_snap); dfree(f->d_snap_img); dfree(f->d_step); dfree(f->d_lstep);
-  dfree(f->d_snap_thermo); dfree(f->d_snap_lstep); dfree(f->d_snap_spec); dfree(f->d_snap_spec_init);
   if (f->graph_exec) cudaGraphExecDestroy(f->graph_exec);
   f->graph_exec = nullptr;
   if (f->graph_multi) cudaGraphExecDestroy(f->graph_multi);
@@ -1366,9 +1361,9 @@ __device__ __forceinline__ void copy_carried(const CarriedState& from, const Car
   for (long long r = k; r < nrep; r += stride) {
     to.lambda[r] = from.lambda[r];
     to.xi[r] = from.xi[r];
-    if (from.spec) to.spec_init[r] = from.spec_init[r];
+    if (from.spec && to.spec) to.spec_init[r] = from.spec_init[r];
   }
-  if (from.spec)
+  if (from.spec && to.spec)
     for (long long j = k; j < (long long)nrep * kPropBands; j += stride) to.spec[j] = from.spec[j];
   if (k == 0) *to.lstep = *from.lstep;
 }
@@ -2986,19 +2981,15 @@ rbmd_status rbmd_force_step(rbmd_force* f, int32_t n_steps, void* stream) {
   if (!f->at.vel || !f->at.mass) return RBMD_ERR_STATE;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t n = f->n;
-  if (!f->d_snap) {
-    CK(dalloc(&f->d_snap, 9 * n));
-    CK(dalloc(&f->d_snap_thermo, 2 * (size_t)f->nrep));
-    CK(dalloc(&f->d_snap_lstep, 1));
-    if (f->d_spec) {
-      CK(dalloc(&f->d_snap_spec, (size_t)f->nrep * kPropBands));
-      CK(dalloc(&f->d_snap_spec_init, (size_t)f->nrep));
-    }
-  }
+  // positions, velocities and forces, then the carried state, in one allocation
+  const size_t nr = (size_t)f->nrep;
+  if (!f->d_snap) CK(dalloc(&f->d_snap, 9 * n + 2 * nr + 1 + (nr * kPropBands + 1) / 2 + (nr + 1) / 2));
   if (f->at.image && !f->d_snap_img) CK(dalloc(&f->d_snap_img, 3 * n));
+  double* small = f->d_snap + 9 * n;
   const CarriedState now{f->d_lambda, f->d_xi, f->d_lstep, f->d_spec, f->d_spec_init};
-  const CarriedState kept{f->d_snap_thermo, f->d_snap_thermo + f->nrep, f->d_snap_lstep, f->d_snap_spec,
-                          f->d_snap_spec_init};
+  const CarriedState kept{small, small + nr, (long long*)(small + 2 * nr),
+                          f->d_spec ? (float*)(small + 2 * nr + 1) : nullptr,
+                          f->d_spec ? (int*)(small + 2 * nr + 1 + (nr * kPropBands + 1) / 2) : nullptr};
   const long long step0 = f->step_count;
   const bool pend0 = f->pending_scale;
   for (int attempt = 0; attempt < 4; ++attempt) {
