@@ -11,6 +11,16 @@
 namespace rbmd {
 
 // cell index of a position, BinPointsWorklet semantics (truncate, clamp to [0, dims-1])
+// Cell index of coordinate x along axis d, unclamped to the box but bounded, so that sums with stencil
+// offsets and cell counts stay in 32 bits for an atom far outside (an overflowed sum read cell_start out
+// of range).  No pair is accepted so far out, whatever cells are searched.
+constexpr int kCellIndexMax = 1 << 30;
+template <class R>
+__device__ __forceinline__ int cell_index(const RepDev& rp, int d, R x) {
+  const int c = (int)div_rn(sub_rn(x, Traits<R>::lo(rp, d)), Traits<R>::dx(rp, d));
+  return max(-kCellIndexMax, min(kCellIndexMax, c));
+}
+
 template <class R>
 __device__ __forceinline__ int cell_of_pos(const RepDev& rp, R x, R y, R z) {
   R p[3] = {x, y, z};
@@ -388,7 +398,7 @@ __device__ int nlist_thread(int i, const typename Traits<R>::V4 pi, const RepDev
   int ci[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d)
-    ci[d] = (int)div_rn(sub_rn(pix[d], Traits<R>::lo(rp, d)), Traits<R>::dx(rp, d));
+    ci[d] = cell_index<R>(rp, d, pix[d]);
   const R cut2 = mul_rn(rc, rc);
   const int nc = num_cycles;
   const int dx0 = rp.dims[0], dx1 = rp.dims[1], dx2 = rp.dims[2];
@@ -487,7 +497,7 @@ __global__ void __launch_bounds__(256) k_nlist_warp(
   int ci[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d)
-    ci[d] = (int)div_rn(sub_rn(pix[d], Traits<R>::lo(rp, d)), Traits<R>::dx(rp, d));
+    ci[d] = cell_index<R>(rp, d, pix[d]);
   const R cut2 = mul_rn(rc, rc);
   const int dx0 = rp.dims[0], dx1 = rp.dims[1], dx2 = rp.dims[2];
   const bool x_contig = ci[0] - 1 >= 0 && ci[0] + 1 < dx0;

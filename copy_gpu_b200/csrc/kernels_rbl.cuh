@@ -53,7 +53,7 @@ __device__ __forceinline__ void rbl_list_slot(
   int ci[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d)
-    ci[d] = (int)div_rn(sub_rn(pix[d], Traits<R>::lo(rp, d)), Traits<R>::dx(rp, d));
+    ci[d] = cell_index<R>(rp, d, pix[d]);
   const R rc2 = mul_rn(rc, rc), rs2 = mul_rn(rs, rs);
   const int nc = num_cycles;
   const int dx0 = rp.dims[0], dx1 = rp.dims[1], dx2 = rp.dims[2];
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(32 * kRblWarps) k_rbl_list_warp(
   int ci[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d)
-    ci[d] = (int)div_rn(sub_rn(pix[d], Traits<R>::lo(rp, d)), Traits<R>::dx(rp, d));
+    ci[d] = cell_index<R>(rp, d, pix[d]);
   const R rc2 = mul_rn(rc, rc), rs2 = mul_rn(rs, rs);
   const int nc = num_cycles, side = 2 * num_cycles + 1, ncs = side * side * side;
   const int dims[3] = {rp.dims[0], rp.dims[1], rp.dims[2]};

@@ -64,3 +64,30 @@ def test_cell_list_edges(cuda, oracle_lib, prec, case):
         assert rel_err(ref[2], want) <= TOL[prec]
     else:
         assert ref[0][0] == 0 and not ref[2].any()
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("block", [0, 1, 128])
+@pytest.mark.parametrize("far", [1e30, -1e30, np.inf, -np.inf])
+def test_atom_far_outside(cuda, prec, block, far):
+    """An atom whose cell index saturates has no neighbours and leaves the others' rows alone."""
+    import torch
+    s = systems.lj_fcc(ncell=6, seed=2)
+    s["pos"] = jitter(s["pos"], s["lo"], s["hi"], 0.05, seed=5)
+    out = []
+    for k in (None, 0, 1, 2):   # nowhere, then along each axis
+        p = dict(s, pos=s["pos"].copy())
+        if k is not None:
+            p["pos"][11, k] = far
+        cfg = systems.lj_config(cutoff=2.5, precision=prec)
+        cfg["tuning"] = {"list_block": block, "force_block": 64}
+        dev = to_dev(p, cuda)
+        ff = make_ff(cfg, p, dev)
+        ff.Execute()
+        torch.cuda.synchronize()
+        c, ids = ff.neighbors(128)
+        assert (ff.status() != 0) == (k is not None and not np.isfinite(far))
+        out.append([set(ids[i, :c[i]].tolist()) for i in range(len(c))])
+        ff.close()
+    for rows in out[1:]:
+        assert not rows[11] and all(r == ref - {11} for i, (r, ref) in enumerate(zip(rows, out[0])) if i != 11)
