@@ -268,9 +268,11 @@ def kspace_noise(ff, steps, warm=3):
     return acc / cnt
 
 
-STEP_LAUNCH_GRAPH = ("cuda graph replay: the first step launched directly, then graphs of 8 captured steps "
-                     "and single-step graphs for the rest; phase_ms_per_step from a second pass of the "
-                     "same length with phase events, kernels launched one by one")
+STEP_LAUNCH_GRAPH = ("cuda graph replay: graphs of 8 captured steps and single-step graphs for the rest; the first "
+                     "step of a call is launched directly unless an earlier call left the state that the graph "
+                     "starts from; the first call of 8 steps or more also captures the 8-step graph, about 3 ms; "
+                     "phase_ms_per_step from a second pass of the same length with phase events, kernels "
+                     "launched one by one")
 STEP_LAUNCH_NOGRAPH = "kernels launched one by one (--no-graph); phase_ms_per_step from a second pass"
 
 
