@@ -493,8 +493,7 @@ void free_all(rbmd_force* f) {
   f->ev_begin = nullptr;
   if (f->h_status) cudaFreeHost(f->h_status);
   f->h_status = nullptr;
-  if (f->h_maxcount) cudaFreeHost(f->h_maxcount);
-  f->h_maxcount = nullptr;
+  f->h_maxcount = nullptr;   // part of h_status
   if (f->side) cudaStreamDestroy(f->side);
   f->side = nullptr;
   if (f->cstream) cudaStreamDestroy(f->cstream);
@@ -2535,8 +2534,9 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
   CK(dalloc(&f->d_eslot, 2 * n));
   CK(cudaMemset(f->d_eslot, 0, sizeof(double) * 2 * n));
   CK(dalloc(&f->d_esum, 32));
-  CK(cudaMallocHost(&f->h_status, sizeof(uint32_t)));
-  CK(cudaMallocHost(&f->h_maxcount, 2 * sizeof(int)));
+  // status word and row counts in one pinned allocation (1.2 ms each, a quarter of a small system's bind)
+  CK(cudaMallocHost(&f->h_status, sizeof(uint32_t) + 2 * sizeof(int)));
+  f->h_maxcount = reinterpret_cast<int*>(f->h_status + 1);
   {
     // the k-space chain is short next to the near pass it overlaps: at the highest priority its
     // blocks take SMs as soon as near-pass blocks retire, so the join rarely waits
