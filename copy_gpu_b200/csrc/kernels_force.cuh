@@ -870,8 +870,9 @@ __global__ void __launch_bounds__(256) k_rho_lanes(
 // Sum of the chunk partials of 32 consecutive k samples of one tile per block: lane = sample, so a
 // warp reads 32 consecutive partials, warp w takes the chunks w, w + warps, .. (FP64) and the warps
 // are added in order through shared memory (deterministic).
-// (One warp per sample read one 8-byte partial per 32-byte sector: 12.4 us at 390 chunks, now 7, 35 us
-// for 512 replicas of 100 samples.)
+// (One warp per sample read one 8-byte partial per 32-byte sector: 12.5 us at 390 chunks of 305 samples,
+// now 10.8.  Systems of up to kFusedChunks chunks per replica, such as batches of small replicas, have no
+// launch of it.)
 constexpr int kFinishWarps = 16;   // at most; the launch uses as many as the longest chunk list needs
 
 template <class R>

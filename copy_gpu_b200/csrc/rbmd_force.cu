@@ -2619,7 +2619,7 @@ rbmd_status rbmd_force_bind(rbmd_force* f, const rbmd_atoms_dev* a) {
     CK(dalloc(&f->d_rho, (size_t)f->Ptot));
     CK(dalloc(&f->d_ek, (size_t)f->Ptot));
     // structure-factor work items (replica, chunk, tile): a block has 32*kKL samples per warp and
-    // at most 8 warps; chunks are sized for about four resident waves of blocks
+    // at most 8 warps
     const int warps = std::min(8, (std::min(f->P, 8 * 32 * kKL) + 32 * kKL - 1) / (32 * kKL));
     f->rho_threads = 32 * warps;
     f->ktile = f->rho_threads * kKL;
