@@ -1,6 +1,6 @@
 """Kernels chosen by size against the ones that a configuration can force: the same answers on both
 sides of each line, and the choice no slower than what it replaced (event times of the phase, best of
-several windows, with a margin of 30 % for the spread of single launches)."""
+15 calls, with a margin of 30 % for their spread)."""
 import numpy as np
 import pytest
 
@@ -10,16 +10,15 @@ from tests.helpers import jitter, make_ff, rel_err, to_dev
 pytestmark = pytest.mark.gpu
 
 
-def _phase_us(s, cfg, phase, windows=5, calls=3):
-    """Shortest mean time of one phase of a force call, in microseconds."""
-    dev = {k: v for k, v in to_dev(s, "cuda", with_vel=False).items()}
+def _phase_us(s, cfg, phase, calls=15):
+    """Shortest time of one phase of a force call, in microseconds."""
+    dev = to_dev(s, "cuda", with_vel=False)
     ff = make_ff(cfg, s, dev)
     ff.Execute()
     ff.profile(True)
     best, last = 1e30, ff.phase_ms()[phase]
-    for _ in range(windows):
-        for _ in range(calls):
-            ff.Execute()
+    for _ in range(calls):
+        ff.Execute()
         now = ff.phase_ms()[phase]
         best, last = min(best, (now[0] - last[0]) / (now[1] - last[1])), now
     assert ff.status() == 0
